@@ -113,6 +113,7 @@ typedef struct instance {
     cudaStream_t wb_stream; /* carries the copy of the normalised input back to the caller, beside the forward (made on first use) */
     cudaEvent_t ev_wb;
     int wb_pending;
+    size_t device_bytes; /* allocated by the plan: activations, staging, result (weights belong to the engine) */
     void **allocs;
     int nallocs, capallocs;
     void **hostmem; /* host arrays the launches' descriptors point to */
@@ -139,28 +140,55 @@ typedef struct instance {
     int runs, graph_state; /* graph_state: 0 not tried, 1 usable, -1 capture failed or switched off */
     int graph_from;        /* first launch inside the graph (the ones before it are issued directly every forward) */
     int graph_launches;    /* kernel launches one replay stands for */
-} instance;
-
-struct thb_engine {
-    thb_model *model;
-    int mode, dtype, ngpus;
-    float range;
-    int strict_math;
-    /* shape the instances were planned for */
-    int N, C, H, W, rank, cp;
-    int built;
     int input_s2d; /* the network input is staged space-to-depth for a stride-2 first convolution */
     int input_neigh; /* uint8 engine, 3x3 / stride 1 / pad 1 first convolution on a three-plane float batch: the boundary kernel
                       * stages every pixel's 27 quantised neighbours as the channels of that pixel (taps outside the image: the
                       * byte of 0.0), and the layer runs as a 1x1 convolution over them -- no gather, no border classes */
     int input_pad16; /* the network input is staged with 16 channels per pixel (zeros behind the real ones) for a stride-1
                       * first convolution, which then runs as a 16-channel convolution through the patch kernel */
+} instance;
+
+/* What an engine keeps per input shape: the planned launches and activation memory of every GPU (`inst`) and, once a
+ * host-input forward was pipelined, of its sub-batches.  Weights are not in here: they belong to the engine (wblob). */
+typedef struct shape_plan {
+    int N, C, H, W, rank, cp;
+    int built; /* GPUs used, 0: not built */
     instance inst[8];
     /* Host-input forwards are pipelined: the batch slice of each GPU is cut into `chunks` sub-batches, each with its own
      * plan instance and stream on that GPU, so that the host-to-device copy of one sub-batch runs under the kernels of
      * the one before it.  Built on the first such forward; chunk c of GPU g is pipe[g * chunks + c]. */
     instance pipe[32];
     int chunks, pipe_built, pipe_chunks;
+    int peer_gather;
+    unsigned long long used; /* forward counter of the last use */
+} shape_plan;
+
+/* Packed weights and per-channel constants in device memory, kept by the engine and found again by what they were made
+ * from: every plan of the same network on a device (a sub-batch, another batch size, another image size) shares them. */
+typedef struct {
+    int device, key[20];
+    void *ptr;
+    float meta[2]; /* uint8 weights: their quantisation */
+} wblob;
+
+/* Plans kept per engine.  A program whose last batch is short, or that alternates between a few image sizes, comes back
+ * to a shape it used before: planning again costs milliseconds (a hundred allocations and the graph capture) against
+ * hundreds of microseconds for the forward.  Bounded in number and, so that rarely used shapes do not pin device memory,
+ * in bytes: plans beyond MAX_PLAN_BYTES are dropped least recently used first, whatever their number. */
+enum { MAX_PLANS = 4 };
+static const size_t MAX_PLAN_BYTES = (size_t)12 << 30;
+
+struct thb_engine {
+    thb_model *model;
+    int mode, dtype, ngpus;
+    float range;
+    int strict_math;
+    shape_plan *plans[MAX_PLANS];
+    shape_plan *cur; /* the plan of the last forward (or the one being built) */
+    unsigned long long clock;
+    wblob *blobs;
+    int nblobs, capblobs;
+    int out_of_memory; /* the last plan failed for want of device memory */
     float *h_out;
     size_t h_out_bytes;
     float *h_stage; /* pinned staging buffer for float batches that arrive in pageable host memory */
@@ -179,13 +207,17 @@ static int esize_of(int dtype) { return dtype == THB_F32 ? 4 : dtype == THB_U8 ?
 static int ru(int v, int m) { return (v + m - 1) / m * m; }
 
 /* ---- device allocations owned by an instance ---- */
-static void *dalloc(instance *I, size_t bytes)
+static void *dalloc(thb_engine *E, instance *I, size_t bytes)
 {
     void *p = 0;
-    if (cudaMalloc(&p, bytes ? bytes : 16) != cudaSuccess) {
+    const cudaError_t e = cudaMalloc(&p, bytes ? bytes : 16);
+    if (e != cudaSuccess) {
+        E->out_of_memory = e == cudaErrorMemoryAllocation;
+        cudaGetLastError();
         thb_set_error("cudaMalloc of %zu bytes failed on device %d", bytes, I->device);
         return 0;
     }
+    I->device_bytes += bytes;
     if (I->nallocs == I->capallocs) {
         I->capallocs = I->capallocs ? I->capallocs * 2 : 64;
         I->allocs = realloc(I->allocs, I->capallocs * sizeof(void *));
@@ -202,14 +234,39 @@ static void host_keep(instance *I, void *p)
     }
     I->hostmem[I->nhost++] = p;
 }
-static void *dupload(instance *I, const void *host, size_t bytes)
+
+/* ---- weights and constants, owned by the engine ---- */
+enum blob_tag { BL_SCALE = 1, BL_SHIFT, BL_SLOPE, BL_BIAS, BL_FACTOR, BL_ADDEND, BL_GEMV, BL_CONV, BL_KINFO, BL_WSAT };
+enum { BLOB_KEY = sizeof(((wblob *)0)->key) / sizeof(int) };
+
+static wblob *blob_find(thb_engine *E, int device, const int *key)
 {
-    void *p = dalloc(I, bytes);
-    if (p && cudaMemcpy(p, host, bytes, cudaMemcpyHostToDevice) != cudaSuccess) {
-        thb_set_error("upload of %zu bytes failed", bytes);
+    for (int i = 0; i < E->nblobs; i++)
+        if (E->blobs[i].device == device && !memcmp(E->blobs[i].key, key, sizeof(E->blobs[i].key))) return &E->blobs[i];
+    return 0;
+}
+/* upload `bytes` and keep them under `key` (on the instance's device, which is current) */
+static wblob *blob_add(thb_engine *E, int device, const int *key, const void *host, size_t bytes)
+{
+    void *p = 0;
+    const cudaError_t e = cudaMalloc(&p, bytes ? bytes : 16);
+    if (e != cudaSuccess || cudaMemcpy(p, host, bytes, cudaMemcpyHostToDevice) != cudaSuccess) {
+        E->out_of_memory = e == cudaErrorMemoryAllocation;
+        cudaGetLastError();
+        if (p) cudaFree(p);
+        thb_set_error("upload of %zu bytes failed on device %d", bytes, device);
         return 0;
     }
-    return p;
+    if (E->nblobs == E->capblobs) {
+        E->capblobs = E->capblobs ? E->capblobs * 2 : 256;
+        E->blobs = realloc(E->blobs, E->capblobs * sizeof(wblob));
+    }
+    wblob *b = &E->blobs[E->nblobs++];
+    memset(b, 0, sizeof(*b));
+    b->device = device;
+    memcpy(b->key, key, sizeof(b->key));
+    b->ptr = p;
+    return b;
 }
 
 /* ---- shape rules ---- */
@@ -379,17 +436,23 @@ static int sole_consumer(planner *P, int node)
     return -1;
 }
 
-static float *upload_floats(planner *P, const float *src, int n, int padded)
+/* A small per-channel array on the device: `n` words padded with zeros to `padded`, shared by node, purpose and contents. */
+static void *upload_words(planner *P, int node, int tag, const void *src, int n, int padded)
 {
-    float *tmp = calloc(padded, sizeof(float));
-    memcpy(tmp, src, sizeof(float) * n);
-    float *d = dupload(P->I, tmp, sizeof(float) * padded);
+    unsigned *tmp = calloc(padded > 0 ? padded : 1, sizeof(unsigned));
+    memcpy(tmp, src, sizeof(unsigned) * n);
+    unsigned long long h = 1469598103934665603ull;
+    for (int i = 0; i < padded; i++) h = (h ^ tmp[i]) * 1099511628211ull;
+    const int key[BLOB_KEY] = {node, tag, n, padded, (int)h, (int)(h >> 32)};
+    wblob *b = blob_find(P->E, P->I->device, key);
+    if (!b) b = blob_add(P->E, P->I->device, key, tmp, sizeof(unsigned) * padded);
     free(tmp);
-    return d;
+    return b ? b->ptr : 0;
 }
 
 static int fill_act(planner *P, thb_act *a, const thb_node *n, int C)
 {
+    const int node = (int)(n - P->M->nodes);
     a->kind = n->act_kind;
     a->threshold = n->act_threshold;
     a->value = n->act_value;
@@ -405,10 +468,157 @@ static int fill_act(planner *P, thb_act *a, const thb_node *n, int C)
             return -1;
         }
         for (int i = 0; i < C; i++) tmp[i] = n->nslope ? n->slope[i] : n->slope[0];
-        a->slope = dupload(P->I, tmp, sizeof(float) * padded);
+        a->slope = upload_words(P, node, BL_SLOPE, tmp, padded, padded);
         free(tmp);
         if (!a->slope) return -1;
     }
+    return 0;
+}
+
+/* Where a planned convolution's weights come from and how they are laid out over the descriptor's Cout x Cin x kH x kW. */
+enum { WS_PLAIN, WS_DECONV, WS_FLAT, WS_S2D, WS_NEIGH, WS_PAD16, WS_DILATED, WS_DUAL };
+typedef struct {
+    const thb_node *n;
+    int bn, dual_conv, dual_bn, kind;
+    float self_coef, res_coef; /* WS_DUAL */
+    int permute_hw, ld;        /* WS_FLAT: positions per channel and stored channels of the flattened input */
+    int s2d_padH, s2d_padW;
+} wsource;
+
+/* The weights in the descriptor's [Cout][Cin][kH][kW] order; a new array, or the node's own (then *owned = 0). */
+static float *weights_oihw(const thb_model *M, const thb_conv_desc *d, const wsource *ws, int u8, int *owned)
+{
+    const thb_node *n = ws->n;
+    const int kH = d->kH, kW = d->kW, Cin = d->Cin;
+    float *fold = 0, *w = 0;
+    const float *src = n->weight;
+    if (u8 && ws->bn >= 0) {
+        const size_t per = (size_t)n->Cin * n->kH * n->kW;
+        src = fold = malloc(sizeof(float) * per * n->Cout);
+#pragma omp parallel for schedule(static)
+        for (int co = 0; co < n->Cout; co++)
+            for (size_t k = 0; k < per; k++) fold[co * per + k] = n->weight[co * per + k] * M->nodes[ws->bn].scale[co];
+    }
+    *owned = 1;
+    if (ws->kind == WS_PLAIN) {
+        if (fold) return fold;
+        *owned = 0;
+        return n->weight;
+    }
+    const size_t count = (size_t)d->Cout * Cin * kH * kW;
+    w = calloc(count ? count : 1, sizeof(float));
+    switch (ws->kind) {
+    case WS_DECONV: {
+        /* column (kh*kW + kw)*Cp + co  <-  W[ci][co][kh][kw] */
+        const int taps = n->kH * n->kW, Cp = d->Cout / taps;
+        for (int ci = 0; ci < Cin; ci++)
+            for (int co = 0; co < n->Cout; co++)
+                for (int t = 0; t < taps; t++)
+                    w[((size_t)t * Cp + co) * Cin + ci] = src[((size_t)ci * n->Cout + co) * taps + t];
+        break;
+    }
+    case WS_FLAT:
+#pragma omp parallel for schedule(static)
+        for (int o = 0; o < n->Cout; o++)
+            for (int k = 0; k < n->Cin; k++)
+                w[(size_t)o * Cin + (size_t)(k % ws->permute_hw) * ws->ld + k / ws->permute_hw] = src[(size_t)o * n->Cin + k];
+        break;
+    case WS_S2D:
+        /* W'[co][(ph*2 + pw)*Cin + c][dh][dw] = W[co][c][2*(dh - pad') + ph + pad][...] where that row exists */
+        for (int co = 0; co < n->Cout; co++)
+            for (int c = 0; c < n->Cin; c++)
+                for (int r = 0; r < n->kH; r++)
+                    for (int q = 0; q < n->kW; q++) {
+                        const int tr = r - n->padH + 2 * ws->s2d_padH, tq = q - n->padW + 2 * ws->s2d_padW; /* >= 0 */
+                        const int dh = tr / 2, ph = tr % 2, dw = tq / 2, pw = tq % 2;
+                        w[(((size_t)co * Cin + (ph * 2 + pw) * n->Cin + c) * kH + dh) * kW + dw] =
+                            src[(((size_t)co * n->Cin + c) * n->kH + r) * n->kW + q];
+                    }
+        break;
+    case WS_NEIGH:
+        /* W'[co][(r*3 + s)*3 + c] = W[co][c][r][s]: the order the boundary kernel stores a pixel's neighbours in */
+        for (int co = 0; co < n->Cout; co++)
+            for (int c = 0; c < 3; c++)
+                for (int t = 0; t < 9; t++) w[(size_t)co * 27 + t * 3 + c] = src[((size_t)co * 3 + c) * 9 + t];
+        break;
+    case WS_PAD16:
+        for (int co = 0; co < n->Cout; co++)
+            memcpy(w + (size_t)co * 16 * kH * kW, src + (size_t)co * n->Cin * kH * kW, sizeof(float) * n->Cin * kH * kW);
+        break;
+    case WS_DILATED: {
+        const int dlH = n->dlH > 0 ? n->dlH : 1, dlW = n->dlW > 0 ? n->dlW : 1;
+        for (long oc = 0; oc < (long)n->Cout * Cin; oc++)
+            for (int r = 0; r < n->kH; r++)
+                for (int q = 0; q < n->kW; q++) w[(oc * kH + r * dlH) * kW + q * dlW] = src[(oc * n->kH + r) * n->kW + q];
+        break;
+    }
+    case WS_DUAL: {
+        const thb_node *c2 = &M->nodes[ws->dual_conv];
+        const int c1n = n->Cin, c2n = c2->Cin;
+        for (int co = 0; co < n->Cout; co++) {
+            const float s1 = ws->self_coef * (ws->bn >= 0 ? M->nodes[ws->bn].scale[co] : 1.f);
+            const float s2 = ws->res_coef * (ws->dual_bn >= 0 ? M->nodes[ws->dual_bn].scale[co] : 1.f);
+            float *row = w + (size_t)co * (c1n + c2n);
+            for (int ci = 0; ci < c1n; ci++) row[ci] = s1 * n->weight[(size_t)co * c1n + ci];
+            for (int ci = 0; ci < c2n; ci++) row[c1n + ci] = s2 * c2->weight[(size_t)co * c2n + ci];
+        }
+        break;
+    }
+    }
+    free(fold);
+    return w;
+}
+
+/* Packed weights and gather table of a planned convolution: the engine's, when a plan with the same layout made them
+ * before (another batch or image size nearly always has it), else packed here and uploaded. */
+static int conv_weights(planner *P, step *s, thb_conv_desc *d, const wsource *ws)
+{
+    thb_engine *E = P->E;
+    const int dev = P->I->device, node = (int)(ws->n - P->M->nodes), u8 = E->dtype == THB_U8;
+    int key[BLOB_KEY] = {node, BL_CONV, ws->kind, ws->bn, ws->dual_conv, ws->dual_bn, ws->permute_hw, ws->ld, ws->s2d_padH * 16 + ws->s2d_padW,
+                         d->Cout, d->Cin, d->kH, d->kW, d->Cin_pad, d->Ktot_pad, d->Cout_pad, d->cin1, d->in_row_pitch ? d->in_ld : 0};
+    wblob *w = blob_find(E, dev, key);
+    if (!w) {
+        const size_t wbytes = thb_conv_weight_bytes(d), kwords = thb_conv_kinfo_words(d);
+        const size_t sat = (size_t)d->Cout * (d->kH + 1) * (d->kW + 1);
+        void *packed = malloc(wbytes);
+        int *kinfo = malloc(kwords * sizeof(int)), *wsat = 0, owned = 0;
+        unsigned char *wq = 0;
+        float *src = weights_oihw(P->M, d, ws, u8, &owned), sub = 0, mult = 0;
+        if (u8) {
+            /* lowp/lowp_basic.c:156-157: weights and bias quantised over their own ranges */
+            const long wn = (long)d->Cout * d->Cin * d->kH * d->kW;
+            wq = malloc(wn);
+            thb_lowp_quantize(src, wn, wq, &sub, &mult);
+            wsat = malloc(sizeof(int) * sat);
+        }
+        const int rc = thb_conv_pack_weights_host(d, u8 ? 0 : src, wq, packed, kinfo, wsat);
+        int ok = !rc;
+        if (ok) {
+            key[1] = BL_KINFO;
+            ok = blob_add(E, dev, key, kinfo, kwords * sizeof(int)) != 0;
+        }
+        if (ok && wsat) {
+            key[1] = BL_WSAT;
+            ok = blob_add(E, dev, key, wsat, sizeof(int) * sat) != 0;
+        }
+        if (ok) {
+            /* last: its presence says that all of them are there */
+            key[1] = BL_CONV;
+            w = blob_add(E, dev, key, packed, wbytes);
+            if (w) { w->meta[0] = sub; w->meta[1] = mult; }
+        }
+        if (owned) free(src);
+        free(packed); free(kinfo); free(wsat); free(wq);
+        if (rc) thb_set_error("weight packing failed (%d)", rc);
+        if (!w) return -1;
+    }
+    d->w = w->ptr;
+    s->w_sub = w->meta[0]; s->w_mult = w->meta[1];
+    key[1] = BL_KINFO;
+    d->kinfo = blob_find(E, dev, key)->ptr;
+    key[1] = BL_WSAT;
+    d->wsat = u8 ? blob_find(E, dev, key)->ptr : 0;
     return 0;
 }
 
@@ -417,6 +627,7 @@ static int fill_act(planner *P, thb_act *a, const thb_node *n, int C)
 static int plan_gemm_group(planner *P, int i)
 {
     thb_engine *E = P->E;
+    instance *I = P->I;
     thb_model *M = P->M;
     thb_node *n = &M->nodes[i];
     const value *in = &P->val[n->in[0]];
@@ -425,9 +636,9 @@ static int plan_gemm_group(planner *P, int i)
     int is_linear = n->op == OP_LINEAR, is_deconv = n->op == OP_DECONV;
     /* stride-2 first convolution on a space-to-depth input (see instance_build): rewritten as a stride-1 convolution
      * over 4*Cin channels.  Input row 2*oh - pad + r is block row oh + floor((r - pad)/2), phase (r - pad) mod 2. */
-    const int s2d = E->input_s2d && n->in[0] == 0 && n->op == OP_CONV;
-    const int pad16 = E->input_pad16 && n->in[0] == 0 && n->op == OP_CONV;  /* 16 stored channels, zeros behind the real ones */
-    const int neigh = E->input_neigh && n->in[0] == 0 && n->op == OP_CONV;  /* 27 neighbours per pixel: a 1x1 convolution */
+    const int s2d = I->input_s2d && n->in[0] == 0 && n->op == OP_CONV;
+    const int pad16 = I->input_pad16 && n->in[0] == 0 && n->op == OP_CONV;  /* 16 stored channels, zeros behind the real ones */
+    const int neigh = I->input_neigh && n->in[0] == 0 && n->op == OP_CONV;  /* 27 neighbours per pixel: a 1x1 convolution */
     const int s2d_padH = (n->padH + 1) / 2, s2d_padW = (n->padW + 1) / 2;
     const int s2d_kH = (n->kH - 1 - n->padH) / 2 + s2d_padH + 1, s2d_kW = (n->kW - 1 - n->padW) / 2 + s2d_padW + 1;
 
@@ -462,8 +673,8 @@ static int plan_gemm_group(planner *P, int i)
     } else if (s2d) {
         /* the logical input is still [N, Cin, 2H', 2W']: output size from the original geometry */
         os.C = n->Cout;
-        os.H = conv_out(E->H, n->kH, 2, n->padH);
-        os.W = conv_out(E->W, n->kW, 2, n->padW);
+        os.H = conv_out(E->cur->H, n->kH, 2, n->padH);
+        os.W = conv_out(E->cur->W, n->kW, 2, n->padW);
         Cin = 4 * n->Cin;
         kH = s2d_kH; kW = s2d_kW;
     } else {
@@ -612,8 +823,8 @@ static int plan_gemm_group(planner *P, int i)
                 hs[c] = 1.f;
             }
         }
-        if (bn >= 0 && dual_conv < 0) { scale = dupload(P->I, hs, sizeof(float) * Cp); scale_h = hs; }
-        if ((dual_conv >= 0 || bn >= 0 || n->bias) && !is_deconv) { shift = dupload(P->I, hh, sizeof(float) * Cp); shift_h = hh; }
+        if (bn >= 0 && dual_conv < 0) { scale = upload_words(P, i, BL_SCALE, hs, Cp, Cp); scale_h = hs; }
+        if ((dual_conv >= 0 || bn >= 0 || n->bias) && !is_deconv) { shift = upload_words(P, i, BL_SHIFT, hh, Cp, Cp); shift_h = hh; }
         if (scale_h) host_keep(P->I, hs); else free(hs);
         if (shift_h) host_keep(P->I, hh); else free(hh);
     }
@@ -631,19 +842,25 @@ static int plan_gemm_group(planner *P, int i)
         s->N = is.N; s->K = Kp; s->M = n->Cout; s->in_ld[0] = permute_hw ? in_ld : in->ld;
         s->scale = scale; s->shift = shift;
         if (act >= 0 && fill_act(P, &s->act, &M->nodes[act], n->Cout)) return -1;
-        size_t es = esize_of(dtype);
-        unsigned char *hw = calloc((size_t)n->Cout * Kp, es);
-        for (int o = 0; o < n->Cout; o++)
-            for (int k = 0; k < n->Cin; k++) {
-                long dst = k;
-                if (permute_hw) { int c = k / permute_hw, hw_ = k % permute_hw; dst = (long)hw_ * in->ld + c; }
-                float v = n->weight[(size_t)o * n->Cin + k];
-                if (dtype == THB_F32) ((float *)hw)[(size_t)o * Kp + dst] = v;
-                else ((unsigned short *)hw)[(size_t)o * Kp + dst] = thb_float_to_half_bits(v, dtype == THB_BF16);
-            }
-        s->w = dupload(P->I, hw, (size_t)n->Cout * Kp * es);
-        free(hw);
-        if (!s->w) return -1;
+        const int key[BLOB_KEY] = {i, BL_GEMV, Kp, permute_hw, in->ld};
+        wblob *wb = blob_find(E, P->I->device, key);
+        if (!wb) {
+            const size_t es = esize_of(dtype);
+            unsigned char *hw = calloc((size_t)n->Cout * Kp, es);
+#pragma omp parallel for schedule(static)
+            for (int o = 0; o < n->Cout; o++)
+                for (int k = 0; k < n->Cin; k++) {
+                    long dst = k;
+                    if (permute_hw) { int c = k / permute_hw, hw_ = k % permute_hw; dst = (long)hw_ * in->ld + c; }
+                    float v = n->weight[(size_t)o * n->Cin + k];
+                    if (dtype == THB_F32) ((float *)hw)[(size_t)o * Kp + dst] = v;
+                    else ((unsigned short *)hw)[(size_t)o * Kp + dst] = thb_float_to_half_bits(v, dtype == THB_BF16);
+                }
+            wb = blob_add(E, P->I->device, key, hw, (size_t)n->Cout * Kp * es);
+            free(hw);
+        }
+        if (!wb) return -1;
+        s->w = wb->ptr;
         s->flops_node = i;
         return cur;
     }
@@ -681,122 +898,62 @@ static int plan_gemm_group(planner *P, int i)
     if (neigh) d->padH = d->padW = 0;
     d->self_coef = 1.f; d->res_coef = 0.f; d->relu_thr = -1;
     int Cp_out = ru(n->Cout, al);
-    float *w_oihw = n->weight, *w_tmp = 0;
-    float *w_fold = 0, *b_fold = 0; /* uint8: weights and bias with the batch normalisation folded in */
+    wsource ws = {n, bn, dual_conv, dual_bn, WS_PLAIN, self_coef, res_coef, permute_hw, in->ld, s2d_padH, s2d_padW};
+    float *b_fold = 0; /* uint8: bias with the batch normalisation folded in (the weights: conv_weights) */
     const float *bias_eff = n->bias;
     if (dtype == THB_U8 && bn >= 0) {
-        const size_t per = (size_t)n->Cin * n->kH * n->kW;
-        w_fold = malloc(sizeof(float) * per * n->Cout);
         b_fold = malloc(sizeof(float) * n->Cout);
-        for (int co = 0; co < n->Cout; co++) {
-            const float sc = M->nodes[bn].scale[co];
-            for (size_t k = 0; k < per; k++) w_fold[co * per + k] = n->weight[co * per + k] * sc;
-            b_fold[co] = (n->bias ? n->bias[co] * sc : 0.f) + M->nodes[bn].shift[co];
-        }
-        w_oihw = w_fold;
+        for (int co = 0; co < n->Cout; co++)
+            b_fold[co] = (n->bias ? n->bias[co] * M->nodes[bn].scale[co] : 0.f) + M->nodes[bn].shift[co];
         bias_eff = b_fold;
     }
     if (is_deconv) {
-        /* column matrix [N*H*W][kH*kW*Cp]: column (kh*kW + kw)*Cp + co  <-  W[ci][co][kh][kw] */
+        /* column matrix [N*H*W][kH*kW*Cp] */
+        ws.kind = WS_DECONV;
         d->Cout = kH * kW * Cp_out; d->kH = d->kW = 1; d->dH = d->dW = 1; d->padH = d->padW = 0;
         d->oH = H; d->oW = W;
-        w_tmp = calloc((size_t)d->Cout * Cin, sizeof(float));
-        for (int ci = 0; ci < Cin; ci++)
-            for (int co = 0; co < n->Cout; co++)
-                for (int t = 0; t < kH * kW; t++)
-                    w_tmp[((size_t)t * Cp_out + co) * Cin + ci] = n->weight[((size_t)ci * n->Cout + co) * kH * kW + t];
-        w_oihw = w_tmp;
     } else if (is_linear) {
         d->Cout = n->Cout; d->oH = d->oW = 1;
-        if (permute_hw && w_fold) { free(w_fold); free(b_fold); thb_set_error("batch-norm after a flattened Linear is not supported in Lowp"); return -1; }
-        if (permute_hw) {
-            w_tmp = calloc((size_t)n->Cout * Cin, sizeof(float));
-            for (int o = 0; o < n->Cout; o++)
-                for (int k = 0; k < n->Cin; k++) {
-                    int c = k / permute_hw, hw_ = k % permute_hw;
-                    w_tmp[(size_t)o * Cin + (size_t)hw_ * in->ld + c] = n->weight[(size_t)o * n->Cin + k];
-                }
-            w_oihw = w_tmp;
-        }
+        if (permute_hw && b_fold) { free(b_fold); thb_set_error("batch-norm after a flattened Linear is not supported in Lowp"); return -1; }
+        if (permute_hw) ws.kind = WS_FLAT;
     } else if (s2d) {
+        ws.kind = WS_S2D;
         d->Cout = n->Cout; d->oH = os.H; d->oW = os.W;
         d->dH = d->dW = 1; d->padH = s2d_padH; d->padW = s2d_padW;
-        /* W'[co][(ph*2 + pw)*Cin + c][dh][dw] = W[co][c][2*(dh - pad') + ph + pad][...] where that row exists */
-        w_tmp = calloc((size_t)n->Cout * Cin * kH * kW, sizeof(float));
-        for (int co = 0; co < n->Cout; co++)
-            for (int c = 0; c < n->Cin; c++)
-                for (int r = 0; r < n->kH; r++)
-                    for (int q = 0; q < n->kW; q++) {
-                        int tr = r - n->padH + 2 * s2d_padH, tq = q - n->padW + 2 * s2d_padW; /* >= 0 */
-                        int dh = tr / 2, ph = tr % 2, dw = tq / 2, pw = tq % 2;
-                        w_tmp[(((size_t)co * Cin + (ph * 2 + pw) * n->Cin + c) * kH + dh) * kW + dw] =
-                            (w_fold ? w_fold : n->weight)[(((size_t)co * n->Cin + c) * n->kH + r) * n->kW + q];
-                    }
-        w_oihw = w_tmp;
     } else if (neigh) {
-        /* W'[co][(r*3 + s)*3 + c] = W[co][c][r][s]: the order the boundary kernel stores a pixel's neighbours in */
+        ws.kind = WS_NEIGH;
         d->Cout = n->Cout; d->oH = os.H; d->oW = os.W;
-        const float *src = w_fold ? w_fold : n->weight;
-        w_tmp = calloc((size_t)n->Cout * 27, sizeof(float));
-        for (int co = 0; co < n->Cout; co++)
-            for (int c = 0; c < 3; c++)
-                for (int r = 0; r < 3; r++)
-                    for (int q = 0; q < 3; q++)
-                        w_tmp[(size_t)co * 27 + (r * 3 + q) * 3 + c] = src[(((size_t)co * 3 + c) * 3 + r) * 3 + q];
-        w_oihw = w_tmp;
     } else if (pad16) {
         /* the same convolution over 16 input channels, the added ones with zero weights */
+        ws.kind = WS_PAD16;
         d->Cout = n->Cout; d->oH = os.H; d->oW = os.W;
         d->Cin = 16;
         d->BN = 64; /* (the patch kernel's tile, also below 33 output channels) */
-        const float *src = w_fold ? w_fold : n->weight;
-        w_tmp = calloc((size_t)n->Cout * 16 * kH * kW, sizeof(float));
-        for (int co = 0; co < n->Cout; co++)
-            memcpy(w_tmp + (size_t)co * 16 * kH * kW, src + (size_t)co * n->Cin * kH * kW, sizeof(float) * n->Cin * kH * kW);
-        w_oihw = w_tmp;
     } else {
         d->Cout = n->Cout; d->oH = os.H; d->oW = os.W;
         if (honour) {
             d->padH = padT; d->padW = padL;
-            if (ekH != n->kH || ekW != n->kW) {
-                /* dilation: the kernel written out at its full extent, zeros between the taps */
-                const float *src = w_fold ? w_fold : n->weight;
-                const int dlH = n->dlH > 0 ? n->dlH : 1, dlW = n->dlW > 0 ? n->dlW : 1;
-                w_tmp = calloc((size_t)n->Cout * Cin * ekH * ekW, sizeof(float));
-                for (long oc = 0; oc < (long)n->Cout * Cin; oc++)
-                    for (int r = 0; r < n->kH; r++)
-                        for (int q = 0; q < n->kW; q++)
-                            w_tmp[(oc * ekH + r * dlH) * ekW + q * dlW] = src[(oc * n->kH + r) * n->kW + q];
-                w_oihw = w_tmp;
-            }
+            /* dilation: the kernel written out at its full extent, zeros between the taps */
+            if (ekH != n->kH || ekW != n->kW) ws.kind = WS_DILATED;
         }
     }
     if (dual_conv >= 0) {
         /* [Cout][cin1 + cin2] weights: each convolution's rows scaled by its batch-norm and its coefficient of the sum */
         const thb_node *c2 = &M->nodes[dual_conv];
         const value *v2 = &P->val[c2->in[0]];
-        const int c1n = n->Cin, c2n = c2->Cin;
-        w_tmp = malloc(sizeof(float) * (size_t)n->Cout * (c1n + c2n));
-        for (int co = 0; co < n->Cout; co++) {
-            const float s1 = self_coef * (bn >= 0 ? M->nodes[bn].scale[co] : 1.f);
-            const float s2 = res_coef * (dual_bn >= 0 ? M->nodes[dual_bn].scale[co] : 1.f);
-            float *row = w_tmp + (size_t)co * (c1n + c2n);
-            for (int ci = 0; ci < c1n; ci++) row[ci] = s1 * n->weight[(size_t)co * c1n + ci];
-            for (int ci = 0; ci < c2n; ci++) row[c1n + ci] = s2 * c2->weight[(size_t)co * c2n + ci];
-        }
-        w_oihw = w_tmp;
-        d->Cin = c1n + c2n;
-        d->cin1 = c1n;
+        ws.kind = WS_DUAL;
+        d->Cin = n->Cin + c2->Cin;
+        d->cin1 = n->Cin;
         d->x2_ld = v2->ld; d->x2_H = v2->s.H; d->x2_W = v2->s.W; d->x2_d = c2->dH;
     }
     if (pool >= 0) d->BN = 64;
-    if (thb_conv_geometry(d)) { free(w_tmp); thb_set_error("unsupported convolution geometry %dx%d", kH, kW); return -1; }
+    if (thb_conv_geometry(d)) { free(b_fold); thb_set_error("unsupported convolution geometry %dx%d", kH, kW); return -1; }
     if (pool >= 0 && !thb_conv_maxpool_supported(d, M->nodes[pool].kH, 2, M->nodes[pool].padH)) {
         pool = -1;
         d->BN = 0;
         thb_conv_geometry(d);
     }
-    if (dual_conv < 0 && in_ld < d->Cin_pad) { free(w_tmp); thb_set_error("internal: input stride %d below padded channels %d", in_ld, d->Cin_pad); return -1; }
+    if (dual_conv < 0 && in_ld < d->Cin_pad) { free(b_fold); thb_set_error("internal: input stride %d below padded channels %d", in_ld, d->Cin_pad); return -1; }
     /* Splitting a reduction over CTAs changes the order in which its fp32 partial sums are added, and whether a layer is
      * split depends on how many tiles the (sub-)batch gives it: with it, a batch sharded over GPUs or cut into sub-batches
      * no longer reproduces the whole batch bit for bit.  That identity is worth more than the few-tile layers' time, so
@@ -825,26 +982,7 @@ static int plan_gemm_group(planner *P, int i)
         }
     }
 
-    size_t wbytes = thb_conv_weight_bytes(d), kwords = thb_conv_kinfo_words(d);
-    void *packed = malloc(wbytes);
-    int *kinfo = malloc(kwords * sizeof(int)), *wsat = 0;
-    unsigned char *wq = 0;
-    if (dtype == THB_U8) {
-        /* lowp/lowp_basic.c:156-157: weights and bias quantised over their own ranges */
-        long wn = (long)d->Cout * d->Cin * d->kH * d->kW;
-        wq = malloc(wn);
-        thb_lowp_quantize(w_oihw, wn, wq, &s->w_sub, &s->w_mult);
-        wsat = malloc(sizeof(int) * d->Cout * (d->kH + 1) * (d->kW + 1));
-    }
-    int rc = thb_conv_pack_weights_host(d, dtype == THB_U8 ? 0 : w_oihw, wq, packed, kinfo, wsat);
-    free(w_tmp); free(w_fold);
-    if (!rc) {
-        d->w = dupload(P->I, packed, wbytes);
-        d->kinfo = dupload(P->I, kinfo, kwords * sizeof(int));
-        if (wsat) d->wsat = dupload(P->I, wsat, sizeof(int) * d->Cout * (d->kH + 1) * (d->kW + 1));
-    }
-    free(packed); free(kinfo); free(wsat); free(wq);
-    if (rc || !d->w || !d->kinfo) { if (rc) thb_set_error("weight packing failed (%d)", rc); return -1; }
+    if (conv_weights(P, s, d, &ws)) { free(b_fold); return -1; }
     if (dtype != THB_F32) {
         s->tmap = aligned_alloc(64, sizeof(thb_tmap));
         if (thb_conv_make_tmap(d, s->tmap)) { thb_set_error("TMA descriptor creation failed"); return -1; }
@@ -870,7 +1008,7 @@ static int plan_gemm_group(planner *P, int i)
         float out_sub = -E->range / 2, out_mult = 255 / E->range; /* lowp_basic.c:137-138 */
         int *addend = malloc(sizeof(int) * n->Cout);
         thb_lowp_bias_addends(bq, n->Cout, b_sub, b_mult, out_mult, addend);
-        d->bias_add = dupload(P->I, addend, sizeof(int) * n->Cout);
+        d->bias_add = upload_words(P, i, BL_ADDEND, addend, n->Cout, n->Cout);
         free(addend); free(bq);
         s->out_sub = out_sub; s->out_mult = out_mult;
         int ohw = d->oH * d->oW;
@@ -931,7 +1069,7 @@ static int plan_gemm_group(planner *P, int i)
         g->padH = n->padH; g->padW = n->padW; g->oH = os.H; g->oW = os.W;
         /* SpatialFullConvolution.c:229-238: the bias GEMM runs with beta = 11 whenever a bias exists */
         g->beta = E->strict_math ? 1.f : 11.f;
-        if (n->bias) g->bias = upload_floats(P, n->bias, n->Cout, ru(n->Cout, 64));
+        if (n->bias) g->bias = upload_words(P, i, BL_BIAS, n->bias, n->Cout, ru(n->Cout, 64));
         if (act >= 0 && fill_act(P, &g->act, &M->nodes[act], n->Cout)) return -1;
         return cur;
     }
@@ -1004,13 +1142,13 @@ static int plan_node(planner *P, int i)
         s->pixels = (long)in->s.N * in->s.H * in->s.W; s->C = C;
         if (n->op == OP_BN) {
             if (n->C != C) { thb_set_error("batch-norm over %d channels applied to %d", n->C, C); return -1; }
-            s->scale = upload_floats(P, n->scale, C, ru(C, 64));
-            s->shift = upload_floats(P, n->shift, C, ru(C, 64));
+            s->scale = upload_words(P, i, BL_SCALE, n->scale, C, ru(C, 64));
+            s->shift = upload_words(P, i, BL_SHIFT, n->shift, C, ru(C, 64));
             if (act >= 0 && fill_act(P, &s->act, &M->nodes[act], C)) return -1;
         } else if (n->op == OP_SCALE) {
             float *f = malloc(sizeof(float) * C);
             for (int c = 0; c < C; c++) f[c] = n->factor;
-            s->scale = upload_floats(P, f, C, ru(C, 64));
+            s->scale = upload_words(P, i, BL_FACTOR, f, C, ru(C, 64));
             free(f);
         } else if (fill_act(P, &s->act, n, C))
             return -1;
@@ -1097,7 +1235,7 @@ static int plan_node(planner *P, int i)
         int chan_dim = (in->s.rank == 4 || in->s.rank == 2) ? 1 : 0;
         if (dim == 0 && chan_dim == 1) {
             /* JoinTable.c:46-57 / Concat.c:21-76 along the batch dimension: the inputs' images one after the other */
-            if (P->I->slice_n != E->N) { thb_set_error("concatenation along the batch dimension needs the whole batch on one GPU"); return -1; }
+            if (P->I->slice_n != E->cur->N) { thb_set_error("concatenation along the batch dimension needs the whole batch on one GPU"); return -1; }
             shape os = in->s;
             os.N = 0;
             for (int k = 0; k < n->nin; k++) {
@@ -1265,7 +1403,7 @@ static int plan_node(planner *P, int i)
             step_in(s, in); step_out(s, out);
             s->pixels = (long)os.N * os.H * os.W; s->C = len; s->flag = n->slice_from;
         } else if (which == 0) {
-            if (P->I->slice_n != E->N) { thb_set_error("a slice along the batch dimension needs the whole batch on one GPU"); return -1; }
+            if (P->I->slice_n != E->cur->N) { thb_set_error("a slice along the batch dimension needs the whole batch on one GPU"); return -1; }
             os.N = len;
             materialise(P, out, os);
             s = new_step(P, ST_COPY);
@@ -1303,7 +1441,7 @@ static int plan_node(planner *P, int i)
     }
     case OP_LOGSOFTMAX: {
         if (in->s.flat) { thb_set_error("LogSoftMax on a flattened spatial tensor is not supported"); return -1; }
-        if (P->I->slice_n != E->N && !E->strict_math) { thb_set_error("LogSoftMax as the reference computes it needs the whole batch on one GPU"); return -1; }
+        if (P->I->slice_n != E->cur->N && !E->strict_math) { thb_set_error("LogSoftMax as the reference computes it needs the whole batch on one GPU"); return -1; }
         materialise(P, out, in->s);
         s = new_step(P, ST_LOGSOFTMAX);
         step_in(s, in); step_out(s, out);
@@ -1316,7 +1454,7 @@ static int plan_node(planner *P, int i)
         /* Normalize.c:12-44: per row of a 2-D tensor, over the whole tensor (batch included) otherwise */
         if (in->s.flat || in->coff || in->ld != ru(in->s.C, al)) { thb_set_error("Normalize needs a dense tensor"); return -1; }
         const int per_row = in->s.rank == 2;
-        if (!per_row && P->I->slice_n != E->N) { thb_set_error("Normalize over a whole batch tensor needs the batch on one GPU"); return -1; }
+        if (!per_row && P->I->slice_n != E->cur->N) { thb_set_error("Normalize over a whole batch tensor needs the batch on one GPU"); return -1; }
         materialise(P, out, in->s);
         s = new_step(P, ST_NORMALIZE);
         step_in(s, in); step_out(s, out);
@@ -1425,8 +1563,8 @@ static int instance_build(thb_engine *E, instance *I, int device, int slice_off,
     CU(cudaStreamCreateWithFlags(&I->stream, cudaStreamNonBlocking));
     CU(cudaEventCreate(&I->ev0));
     CU(cudaEventCreate(&I->ev1));
-    I->d_status = dalloc(I, sizeof(int));
-    I->d_minmax = dalloc(I, 2 * sizeof(float));
+    I->d_status = dalloc(E, I, sizeof(int));
+    I->d_minmax = dalloc(E, I, 2 * sizeof(float));
     if (!I->d_status || !I->d_minmax) return -1;
     CU(cudaMemset(I->d_status, 0, sizeof(int)));
 
@@ -1444,21 +1582,21 @@ static int instance_build(thb_engine *E, instance *I, int device, int slice_off,
     }
     P.uses[M->output]++;
 
-    shape in = {slice_n, E->C, E->H, E->W, E->rank, 0, 0, 0, 0};
+    shape in = {slice_n, E->cur->C, E->cur->H, E->cur->W, E->cur->rank, 0, 0, 0, 0};
     {
         /* a stride-2 convolution on very few channels as the only consumer of the float input: stage the input
          * space-to-depth so that the gathered 16-byte chunks carry four times as many useful channels */
         thb_node *c1 = M->nnodes > 1 ? &M->nodes[1] : 0;
         const char *off = getenv("THB200_NO_S2D"), *u8off = getenv("THB200_NO_S2D_U8");
-        E->input_s2d = c1 && c1->op == OP_CONV && c1->in[0] == 0 && P.uses[0] == 1 && c1->dH == 2 && c1->dW == 2 &&
-                       4 * E->C <= 16 && c1->Cin == E->C && E->H % 2 == 0 && E->W % 2 == 0 && E->rank == 4 &&
+        I->input_s2d = c1 && c1->op == OP_CONV && c1->in[0] == 0 && P.uses[0] == 1 && c1->dH == 2 && c1->dW == 2 &&
+                       4 * E->cur->C <= 16 && c1->Cin == E->cur->C && E->cur->H % 2 == 0 && E->cur->W % 2 == 0 && E->cur->rank == 4 &&
                        /* a float batch, or three-plane byte images (converted and regrouped by one kernel) in the 16-bit modes */
-                       (E->cp == 0 || (E->cp == 3 && E->dtype != THB_U8)) &&
+                       (E->cur->cp == 0 || (E->cur->cp == 3 && E->dtype != THB_U8)) &&
                        (E->dtype == THB_F16 || E->dtype == THB_BF16 || (E->dtype == THB_U8 && !(u8off && atoi(u8off)))) &&
                        c1->padH <= c1->kH - 1 && c1->padW <= c1->kW - 1 &&
                        !(E->honour_pads && (c1->pad2H != c1->padH || c1->pad2W != c1->padW || c1->dlH > 1 || c1->dlW > 1 || c1->autopad || c1->refl_pad)) &&
                        !(off && atoi(off));
-        if (E->input_s2d) { in.C = 4 * E->C; in.H = E->H / 2; in.W = E->W / 2; }
+        if (I->input_s2d) { in.C = 4 * E->cur->C; in.H = E->cur->H / 2; in.W = E->cur->W / 2; }
     }
     {
         /* A stride-1 convolution with at most 64 output channels on very few input channels (VGG, the segmentation net):
@@ -1466,8 +1604,8 @@ static int instance_build(thb_engine *E, instance *I, int device, int slice_off,
          * 16-byte chunks that are mostly padding. */
         thb_node *c1 = M->nnodes > 1 ? &M->nodes[1] : 0;
         const char *off = getenv("THB200_NO_PAD16");
-        E->input_pad16 = !E->input_s2d && c1 && c1->op == OP_CONV && c1->in[0] == 0 && P.uses[0] == 1 && c1->dH == 1 && c1->dW == 1 &&
-                         E->C <= 8 && c1->Cin == E->C && c1->Cout <= 64 && c1->kH <= 8 && c1->kW <= 8 && c1->kH * c1->kW > 1 &&
+        I->input_pad16 = !I->input_s2d && c1 && c1->op == OP_CONV && c1->in[0] == 0 && P.uses[0] == 1 && c1->dH == 1 && c1->dW == 1 &&
+                         E->cur->C <= 8 && c1->Cin == E->cur->C && c1->Cout <= 64 && c1->kH <= 8 && c1->kW <= 8 && c1->kH * c1->kW > 1 &&
                          c1->padH < c1->kH && c1->padW < c1->kW && (E->dtype == THB_F16 || E->dtype == THB_BF16) &&
                          !(E->honour_pads && (c1->pad2H != c1->padH || c1->pad2W != c1->padW || c1->dlH > 1 || c1->dlW > 1 || c1->autopad || c1->refl_pad)) &&
                          !(off && atoi(off));
@@ -1476,21 +1614,21 @@ static int instance_build(thb_engine *E, instance *I, int device, int slice_off,
         /* uint8: a 3x3 / stride 1 / pad 1 first convolution on three planes of a float batch */
         thb_node *c1 = M->nnodes > 1 ? &M->nodes[1] : 0;
         const char *off = getenv("THB200_NO_NEIGH_U8");
-        E->input_neigh = E->dtype == THB_U8 && !E->input_s2d && E->cp == 0 && E->C == 3 && E->rank == 4 && c1 && c1->op == OP_CONV &&
+        I->input_neigh = E->dtype == THB_U8 && !I->input_s2d && E->cur->cp == 0 && E->cur->C == 3 && E->cur->rank == 4 && c1 && c1->op == OP_CONV &&
                          c1->in[0] == 0 && P.uses[0] == 1 && c1->Cin == 3 && c1->kH == 3 && c1->kW == 3 && c1->dH == 1 && c1->dW == 1 &&
                          c1->padH == 1 && c1->padW == 1 &&
                          !(E->honour_pads && (c1->pad2H != c1->padH || c1->pad2W != c1->padW || c1->dlH > 1 || c1->dlW > 1 || c1->autopad || c1->refl_pad)) &&
                          !(off && atoi(off));
-        if (E->input_neigh) in.C = 27;
+        if (I->input_neigh) in.C = 27;
     }
     materialise(&P, &P.val[0], in);
-    if (E->input_pad16) {
+    if (I->input_pad16) {
         value *v = &P.val[0];
         v->ld = 16;
         I->nbufs--; /* re-create the buffer with 16 channels per pixel */
         v->buf = new_buf(&P, (size_t)in.N * in.H * in.W * v->ld * esize_of(E->dtype));
     }
-    if (E->input_s2d) {
+    if (I->input_s2d) {
         /* When the rewritten convolution's kernel row fills one 128-byte K block, store the staged rows with their
          * zero padding: one copy then fetches a whole kernel row of an output pixel (thb_conv_desc.in_row_pitch). */
         thb_node *c1 = &M->nodes[1];
@@ -1519,11 +1657,11 @@ static int instance_build(thb_engine *E, instance *I, int device, int slice_off,
         I->out_shape = I->out_val.s;
         I->out_count = (long)I->out_shape.N * I->out_shape.C * I->out_shape.H * I->out_shape.W;
         I->arena_bytes = pack_arena(I);
-        I->arena = dalloc(I, I->arena_bytes);
-        size_t in_bytes = (size_t)slice_n * E->C * E->H * E->W * sizeof(float);
-        I->d_in = dalloc(I, in_bytes);
-        I->d_img = dalloc(I, (size_t)slice_n * E->H * E->W * 4);
-        I->d_out = dalloc(I, (size_t)(I->out_count ? I->out_count : 1) * sizeof(float));
+        I->arena = dalloc(E, I, I->arena_bytes);
+        size_t in_bytes = (size_t)slice_n * E->cur->C * E->cur->H * E->cur->W * sizeof(float);
+        I->d_in = dalloc(E, I, in_bytes);
+        I->d_img = dalloc(E, I, (size_t)slice_n * E->cur->H * E->cur->W * 4);
+        I->d_out = dalloc(E, I, (size_t)(I->out_count ? I->out_count : 1) * sizeof(float));
         if (!I->arena || !I->d_in || !I->d_out || !I->d_img) rc = -1;
         /* padded channels are never read as data, but stale NaN/Inf bit patterns would poison the
          * zero-weight products: start from a clean arena */
@@ -1731,8 +1869,8 @@ static int boundary_out(thb_engine *E, instance *I, float *dst);
  * flops: algorithmic FLOPs of the launch (2 * MACs of the convolution / Linear it computes), 0 otherwise. */
 int thb_engine_profile(thb_engine *E, int iters, int max_steps, int *kinds, float *ms, double *flops)
 {
-    if (!E || !E->built || iters < 1 || (!E->last_has_x && !E->last_cp)) return -1;
-    instance *I = &E->inst[0];
+    if (!E || !E->cur || iters < 1 || (!E->last_has_x && !E->last_cp)) return -1;
+    instance *I = &E->cur->inst[0];
     if (cudaSetDevice(I->device) != cudaSuccess) return -1;
     const int total = I->nsteps + 2;
     const int n = total < max_steps ? total : max_steps;
@@ -1742,9 +1880,9 @@ int thb_engine_profile(thb_engine *E, int iters, int max_steps, int *kinds, floa
     int rc = 0;
     for (int it = 0; it < iters && !rc; it++) {
         float q_sub = 0, q_mult = 0;
-        rc = lowp_input_range(E, E->inst, 1, E->last_has_x, E->last_cp, E->C, E->H, E->W, E->last_mean, E->last_std, &q_sub, &q_mult);
+        rc = lowp_input_range(E, E->cur->inst, 1, E->last_has_x, E->last_cp, E->cur->C, E->cur->H, E->cur->W, E->last_mean, E->last_std, &q_sub, &q_mult);
         cudaEventRecord(evs[0], I->stream);
-        if (!rc) rc = boundary_in(E, I, E->last_has_x, 0, E->last_cp, E->last_bgr, E->C, E->H, E->W, E->last_mean, E->last_std, q_sub, q_mult);
+        if (!rc) rc = boundary_in(E, I, E->last_has_x, 0, E->last_cp, E->last_bgr, E->cur->C, E->cur->H, E->cur->W, E->last_mean, E->last_std, q_sub, q_mult);
         cudaEventRecord(evs[1], I->stream);
         if (!rc) rc = run_steps_ev(E, I, evs + 1, 0, I->nsteps);
         if (!rc) rc = boundary_out(E, I, I->d_out);
@@ -1779,8 +1917,8 @@ int thb_engine_profile(thb_engine *E, int iters, int max_steps, int *kinds, floa
  * companion of thb_engine_profile's flops for a per-launch "slower of the two roofs" bound. */
 int thb_engine_profile_bytes(thb_engine *E, int max_steps, double *bytes)
 {
-    if (!E || !E->built) return -1;
-    instance *I = &E->inst[0];
+    if (!E || !E->cur) return -1;
+    instance *I = &E->cur->inst[0];
     const int total = I->nsteps + 2;
     const int n = total < max_steps ? total : max_steps;
     for (int t = 0; t < n; t++) {
@@ -1834,11 +1972,24 @@ thb_engine *thb_engine_create(thb_model *model, int mode, float lowp_range, int 
     return E;
 }
 
+static void plan_drop(thb_engine *E, int slot)
+{
+    shape_plan *p = E->plans[slot];
+    if (!p) return;
+    for (int g = 0; g < 8; g++) instance_free(&p->inst[g]);
+    for (int g = 0; g < 32; g++) instance_free(&p->pipe[g]);
+    if (E->cur == p) E->cur = 0;
+    free(p);
+    E->plans[slot] = 0;
+}
+
 void thb_engine_destroy(thb_engine *E)
 {
     if (!E) return;
-    for (int g = 0; g < 8; g++) instance_free(&E->inst[g]);
-    for (int g = 0; g < 32; g++) instance_free(&E->pipe[g]);
+    for (int i = 0; i < MAX_PLANS; i++) plan_drop(E, i);
+    for (int i = 0; i < E->nblobs; i++)
+        if (cudaSetDevice(E->blobs[i].device) == cudaSuccess) cudaFree(E->blobs[i].ptr);
+    free(E->blobs);
     thb_host_free_pinned(E->h_out);
     thb_host_free_pinned(E->h_stage);
     thb_model_release(E->model);
@@ -1868,13 +2019,68 @@ void thb_slice_sub_batches(int n, int S, int c, int *offset, int *count)
     *count = (n * cut[S][c + 1] + 8) / 16 - *offset;
 }
 
-static int engine_build(thb_engine *E, int N, int C, int H, int W, int rank, int cp)
+static size_t plan_bytes(const shape_plan *p)
 {
-    for (int g = 0; g < 8; g++) instance_free(&E->inst[g]);
-    for (int g = 0; g < 32; g++) instance_free(&E->pipe[g]);
-    E->built = 0;
-    E->pipe_built = 0;
-    E->N = N; E->C = C; E->H = H; E->W = W; E->rank = rank; E->cp = cp;
+    size_t b = 0;
+    for (int g = 0; g < 8; g++) b += p->inst[g].device_bytes;
+    for (int g = 0; g < 32; g++) b += p->pipe[g].device_bytes;
+    return b;
+}
+
+/* the least recently used plan other than `keep`, -1: none */
+static int plan_oldest(thb_engine *E, const shape_plan *keep)
+{
+    int v = -1;
+    for (int i = 0; i < MAX_PLANS; i++)
+        if (E->plans[i] && E->plans[i] != keep && (v < 0 || E->plans[i]->used < E->plans[v]->used)) v = i;
+    return v;
+}
+
+static int plan_build(thb_engine *E);
+
+/* Make the plan of this input shape the current one, building it when it is not kept. */
+static int select_plan(thb_engine *E, int N, int C, int H, int W, int rank, int cp)
+{
+    E->clock++;
+    for (int i = 0; i < MAX_PLANS; i++) {
+        shape_plan *p = E->plans[i];
+        if (p && p->N == N && p->C == C && p->H == H && p->W == W && p->rank == rank && p->cp == cp) {
+            p->used = E->clock;
+            E->cur = p;
+            return 0;
+        }
+    }
+    int slot = -1;
+    for (int i = 0; i < MAX_PLANS && slot < 0; i++)
+        if (!E->plans[i]) slot = i;
+    if (slot < 0) plan_drop(E, slot = plan_oldest(E, 0));
+    for (;;) {
+        shape_plan *p = E->plans[slot] = E->cur = calloc(1, sizeof(*p));
+        if (!p) { thb_set_error("out of memory"); return -1; }
+        p->N = N; p->C = C; p->H = H; p->W = W; p->rank = rank; p->cp = cp;
+        p->used = E->clock;
+        if (!plan_build(E)) break;
+        plan_drop(E, slot);
+        /* no room on the device: the other shapes' plans make way, one at a time */
+        const int v = E->out_of_memory ? plan_oldest(E, 0) : -1;
+        if (v < 0) return -1;
+        plan_drop(E, v);
+    }
+    size_t total = 0;
+    for (int i = 0; i < MAX_PLANS; i++)
+        if (E->plans[i]) total += plan_bytes(E->plans[i]);
+    for (int v; total > MAX_PLAN_BYTES && (v = plan_oldest(E, E->cur)) >= 0;) {
+        total -= plan_bytes(E->plans[v]);
+        plan_drop(E, v);
+    }
+    return 0;
+}
+
+static int plan_build(thb_engine *E)
+{
+    const int N = E->cur->N, C = E->cur->C, H = E->cur->H, W = E->cur->W, cp = E->cur->cp;
+    E->cur->peer_gather = E->peer_gather;
+    E->out_of_memory = 0;
     int G = E->ngpus < N ? E->ngpus : N;
     if (G < 1) G = 1;
     int dev0 = 0;
@@ -1883,45 +2089,45 @@ static int engine_build(thb_engine *E, int N, int C, int H, int W, int rank, int
     for (int g = 0; g < G; g++) {
         int off, n;
         thb_slice_batch(N, G, g, &off, &n);
-        if (instance_build(E, &E->inst[g], dev0 + g, off, n)) return -1;
+        if (instance_build(E, &E->cur->inst[g], dev0 + g, off, n)) return -1;
     }
     /* gather target: GPU 0 holds the whole result when peer copies are usable */
-    if (G > 1 && E->peer_gather) {
+    if (G > 1 && E->cur->peer_gather) {
         for (int g = 1; g < G; g++) {
             int can = 0;
-            cudaDeviceCanAccessPeer(&can, E->inst[0].device, E->inst[g].device);
-            if (!can) E->peer_gather = 0;
+            cudaDeviceCanAccessPeer(&can, E->cur->inst[0].device, E->cur->inst[g].device);
+            if (!can) E->cur->peer_gather = 0;
         }
-        if (E->peer_gather) {
+        if (E->cur->peer_gather) {
             /* direct copies over NVLink need the access switched on from the sending GPU's side (a second request is
              * answered with cudaErrorPeerAccessAlreadyEnabled, which is fine) */
             for (int g = 1; g < G; g++) {
-                cudaSetDevice(E->inst[g].device);
-                const cudaError_t pe = cudaDeviceEnablePeerAccess(E->inst[0].device, 0);
-                if (pe != cudaSuccess && pe != cudaErrorPeerAccessAlreadyEnabled) E->peer_gather = 0;
+                cudaSetDevice(E->cur->inst[g].device);
+                const cudaError_t pe = cudaDeviceEnablePeerAccess(E->cur->inst[0].device, 0);
+                if (pe != cudaSuccess && pe != cudaErrorPeerAccessAlreadyEnabled) E->cur->peer_gather = 0;
                 cudaGetLastError();
             }
         }
-        if (E->peer_gather) {
+        if (E->cur->peer_gather) {
             long total = 0;
-            for (int g = 0; g < G; g++) total += E->inst[g].out_count;
-            cudaSetDevice(E->inst[0].device);
-            E->inst[0].d_out = dalloc(&E->inst[0], (size_t)total * sizeof(float));
-            if (!E->inst[0].d_out) return -1;
+            for (int g = 0; g < G; g++) total += E->cur->inst[g].out_count;
+            cudaSetDevice(E->cur->inst[0].device);
+            E->cur->inst[0].d_out = dalloc(E, &E->cur->inst[0], (size_t)total * sizeof(float));
+            if (!E->cur->inst[0].d_out) return -1;
         }
     }
-    E->built = G;
+    E->cur->built = G;
     /* Sub-batches per GPU for pipelined host-input forwards.  Two sub-batches hide about 0.6 of the input copy (measured
      * at ~50 GB/s from pinned memory) and cost every launch's fill and drain a second time (~6 us each, with a margin):
      * worth it for a float batch of ResNet-50 (154 MB, 2.8 ms of copy), not for the same batch as byte images (38 MB).
      * The uint8 engine needs the input range of the whole batch before any kernel can start. */
     const int per_gpu = N / G;
     const double in_mb = (double)per_gpu * (cp ? (double)H * W * cp : (double)C * H * W * 4) / 1e6;
-    const double copy_ms = in_mb / 50.0, refill_ms = E->inst[0].nsteps * 0.006 * 1.5 + 0.1;
-    E->chunks = E->dtype == THB_U8 || per_gpu < 32 || copy_ms * 0.6 <= refill_ms ? 1 : 2;
+    const double copy_ms = in_mb / 50.0, refill_ms = E->cur->inst[0].nsteps * 0.006 * 1.5 + 0.1;
+    E->cur->chunks = E->dtype == THB_U8 || per_gpu < 32 || copy_ms * 0.6 <= refill_ms ? 1 : 2;
     const char *ce = getenv("THB200_CHUNKS");
-    if (ce) E->chunks = atoi(ce) < 1 || E->dtype == THB_U8 ? 1 : atoi(ce) > 4 ? 4 : atoi(ce);
-    if (E->chunks > per_gpu || E->whole_batch) E->chunks = 1;
+    if (ce) E->cur->chunks = atoi(ce) < 1 || E->dtype == THB_U8 ? 1 : atoi(ce) > 4 ? 4 : atoi(ce);
+    if (E->cur->chunks > per_gpu || E->whole_batch) E->cur->chunks = 1;
     return 0;
 }
 
@@ -1931,17 +2137,17 @@ void thb_set_pipeline_chunks(int n) { g_chunks_override = n < 0 ? 0 : n > 4 ? 4 
 /* plan instances of the sub-batches (first pipelined forward of this shape with S sub-batches per GPU) */
 static int pipe_build(thb_engine *E, int S)
 {
-    const int G = E->built;
-    for (int g = 0; g < 32; g++) instance_free(&E->pipe[g]);
-    E->pipe_built = 0;
+    const int G = E->cur->built;
+    for (int g = 0; g < 32; g++) instance_free(&E->cur->pipe[g]);
+    E->cur->pipe_built = 0;
     for (int g = 0; g < G; g++)
         for (int c = 0; c < S; c++) {
             int off, n;
-            thb_slice_sub_batches(E->inst[g].slice_n, S, c, &off, &n);
-            if (instance_build(E, &E->pipe[g * S + c], E->inst[g].device, E->inst[g].slice_off + off, n)) return -1;
+            thb_slice_sub_batches(E->cur->inst[g].slice_n, S, c, &off, &n);
+            if (instance_build(E, &E->cur->pipe[g * S + c], E->cur->inst[g].device, E->cur->inst[g].slice_off + off, n)) return -1;
         }
-    E->pipe_built = G * S;
-    E->pipe_chunks = S;
+    E->cur->pipe_built = G * S;
+    E->cur->pipe_chunks = S;
     return 0;
 }
 
@@ -1995,13 +2201,13 @@ static int boundary_in(thb_engine *E, instance *I, int has_x, int inplace, int c
 {
     int rc;
     void *in_ptr = bufptr(I, I->in_val.buf, 0, E->dtype);
-    if (has_x && E->input_neigh)
+    if (has_x && I->input_neigh)
         rc = thb_preprocess_neigh_u8(I->d_in, inplace ? I->d_in : 0, I->slice_n, H, W, mean, std, in_ptr, I->in_val.ld, q_sub, q_mult,
                                      I->stream);
-    else if (has_x && E->input_s2d && E->dtype == THB_U8)
+    else if (has_x && I->input_s2d && E->dtype == THB_U8)
         rc = thb_preprocess_s2d_u8(I->d_in, inplace ? I->d_in : 0, I->slice_n, C, H, W, mean, std, in_ptr, I->in_val.ld, q_sub,
                                    q_mult, I->stream);
-    else if (has_x && E->input_s2d)
+    else if (has_x && I->input_s2d)
         rc = thb_preprocess_s2d_padded(I->d_in, inplace ? I->d_in : 0, I->slice_n, C, H, W, mean, std, E->dtype, in_ptr,
                                        I->in_val.ld, I->in_val.row_pitch ? I->in_val.row_pitch : W / 2,
                                        I->in_val.pad_left, I->stream);
@@ -2015,7 +2221,7 @@ static int boundary_in(thb_engine *E, instance *I, int has_x, int inplace, int c
         rc = thb_preprocess_images_lowp(I->d_img, I->slice_n, H, W, W * cp, bgr, mean, std, in_ptr, I->in_val.ld, &q_sub,
                                         &q_mult, I->stream);
         set_dynamic_quant(I, q_sub, q_mult);
-    } else if (E->input_s2d)
+    } else if (I->input_s2d)
         rc = thb_preprocess_images_s2d(I->d_img, I->slice_n, H, W, W * cp, bgr, mean, std, E->dtype, in_ptr, I->in_val.ld,
                                        I->in_val.row_pitch ? I->in_val.row_pitch : W / 2, I->in_val.pad_left, I->stream);
     else
@@ -2109,25 +2315,23 @@ int thb_engine_forward(thb_engine *E, float *x, unsigned char **images, int stri
 {
     if (N < 1 || C < 1 || H < 1 || W < 1) { thb_set_error("empty input"); return -1; }
     if (E->dtype == THB_U8 && !x) rank = 4; /* the lowp image loader always builds a 4-D tensor (lowp_basic.c:87-92) */
-    if (!E->built || E->N != N || E->C != C || E->H != H || E->W != W || E->rank != rank || E->cp != cp) {
-        if (engine_build(E, N, C, H, W, rank, cp)) return -1;
-    }
+    if (select_plan(E, N, C, H, W, rank, cp)) return -1;
     /* host input (a float batch or byte images): run the sub-batch instances so that copies and kernels overlap */
-    instance *set = E->inst;
-    int G = E->built;
-    int peer_gather = E->peer_gather;
-    int S = g_chunks_override ? g_chunks_override : E->chunks;
-    if (E->dtype == THB_U8 || S > E->inst[0].slice_n || E->whole_batch) S = 1;
+    instance *set = E->cur->inst;
+    int G = E->cur->built;
+    const int peer_gather = E->cur->peer_gather;
+    int S = g_chunks_override ? g_chunks_override : E->cur->chunks;
+    if (E->dtype == THB_U8 || S > E->cur->inst[0].slice_n || E->whole_batch) S = 1;
     if (S > 1) {
-        if ((!E->pipe_built || E->pipe_chunks != S) && pipe_build(E, S)) return -1;
-        set = E->pipe;
-        G = E->pipe_built;
+        if ((!E->cur->pipe_built || E->cur->pipe_chunks != S) && pipe_build(E, S)) return -1;
+        set = E->cur->pipe;
+        G = E->cur->pipe_built;
     }
     /* Peer gather: every GPU's part of the result ends up in GPU 0's result buffer (the first instance's, sized for the
      * whole batch), which goes to the host in one copy.  Instances on GPU 0 write their part there directly; the others
      * send theirs with cudaMemcpyPeerAsync on their own stream -- also when a GPU's slice runs as pipelined sub-batches. */
-    float *gather = E->built > 1 && peer_gather ? E->inst[0].d_out : 0;
-    const int dev0 = E->inst[0].device;
+    float *gather = E->cur->built > 1 && peer_gather ? E->cur->inst[0].d_out : 0;
+    const int dev0 = E->cur->inst[0].device;
     const size_t img_elems = (size_t)C * H * W;
     float q_sub = 0, q_mult = 0;
 
@@ -2297,29 +2501,29 @@ float thb_engine_last_ms(thb_engine *E) { return E ? E->last_ms : -1.f; }
  * on the launching stream; max over GPUs.  No host<->device copy of the batch or the result is inside. */
 float thb_engine_time_forward(thb_engine *E, int iters)
 {
-    if (!E || !E->built || iters < 1 || (!E->last_has_x && !E->last_cp)) return -1.f;
-    const int G = E->built;
+    if (!E || !E->cur || iters < 1 || (!E->last_has_x && !E->last_cp)) return -1.f;
+    const int G = E->cur->built;
     cudaEvent_t t0[8], t1[8];
     for (int g = 0; g < G; g++) {
-        if (cudaSetDevice(E->inst[g].device) != cudaSuccess) return -1.f;
+        if (cudaSetDevice(E->cur->inst[g].device) != cudaSuccess) return -1.f;
         cudaEventCreate(&t0[g]);
         cudaEventCreate(&t1[g]);
-        cudaEventRecord(t0[g], E->inst[g].stream);
+        cudaEventRecord(t0[g], E->cur->inst[g].stream);
     }
     int rc = 0;
     for (int it = 0; it < iters && !rc; it++) {
         float q_sub = 0, q_mult = 0;
-        rc = lowp_input_range(E, E->inst, G, E->last_has_x, E->last_cp, E->C, E->H, E->W, E->last_mean, E->last_std, &q_sub, &q_mult);
+        rc = lowp_input_range(E, E->cur->inst, G, E->last_has_x, E->last_cp, E->cur->C, E->cur->H, E->cur->W, E->last_mean, E->last_std, &q_sub, &q_mult);
         for (int g = 0; g < G && !rc; g++) {
-            instance *I = &E->inst[g];
+            instance *I = &E->cur->inst[g];
             if (cudaSetDevice(I->device) != cudaSuccess) rc = -1;
-            else rc = device_forward(E, I, E->last_has_x, 0, E->last_cp, E->last_bgr, E->C, E->H, E->W, E->last_mean, E->last_std,
+            else rc = device_forward(E, I, E->last_has_x, 0, E->last_cp, E->last_bgr, E->cur->C, E->cur->H, E->cur->W, E->last_mean, E->last_std,
                                      q_sub, q_mult, 0, I->d_out);
         }
     }
     float worst = 0;
     for (int g = 0; g < G; g++) {
-        instance *I = &E->inst[g];
+        instance *I = &E->cur->inst[g];
         cudaSetDevice(I->device);
         cudaEventRecord(t1[g], I->stream);
         if (cudaStreamSynchronize(I->stream) != cudaSuccess) rc = -1;
