@@ -207,6 +207,9 @@ int thb_minmax_normalized(const float *x_nchw, int N, int C, int H, int W, const
 /* NHWC dtype -> NCHW fp32 (dequantising u8 with q*inv_mult + sub) */
 int thb_postprocess(const void *x, int dtype, int N, int H, int W, int C, int x_ld, float q_sub, float q_invmult,
                     float *y_nchw, thb_stream s);
+/* the same, leaving a copy of the launch status word in *status_out with the result (both may be pinned host memory) */
+int thb_postprocess_status(const void *x, int dtype, int N, int H, int W, int C, int x_ld, float q_sub, float q_invmult,
+                           float *y_nchw, const int *status, int *status_out, thb_stream s);
 
 /* ---- pooling: SpatialMaxPooling.c:74-247, SpatialAveragePooling.c:71-207, lowp_SpatialMaxPooling.c ---- */
 int thb_maxpool(int dtype, const void *x, int N, int H, int W, int C, int x_ld, int kH, int kW, int dH, int dW,

@@ -254,6 +254,9 @@ int THB200_SetDevices(int ngpus);
 /* THProcessFloat cuts each GPU's batch slice into sub-batches so that the host-to-device copy of one runs under the
  * kernels of the one before; 0 = chosen from the input size (default, also THB200_CHUNKS), 1 = off, up to 4 */
 int THB200_SetPipelineChunks(int chunks);
+/* THProcessFloat on a batch that stays as it is: the normalised values are not written back to the caller's buffer */
+int THB200_ProcessFloatConst(THNETWORK *network, const float *data, int batchsize, int width, int height, int nplanes,
+                             float **result, int *outwidth, int *outheight);
 /* pinned host memory for input batches, so that THProcessFloat's copies run at full PCIe speed */
 void *THB200_HostAlloc(size_t bytes);
 void THB200_HostFree(void *p);

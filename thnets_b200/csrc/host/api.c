@@ -317,22 +317,35 @@ static int publish(THNETWORK *network, const thb_result *r, float **result, int 
     return (int)r->count;
 }
 
-int THProcessFloat(THNETWORK *network, float *data, int batchsize, int width, int height, int nplanes, float **result,
-                   int *outwidth, int *outheight)
+static int process_float(THNETWORK *network, float *data, int batchsize, int width, int height, int nplanes, int inplace,
+                         float **result, int *outwidth, int *outheight)
 {
     thb_netx *x = netx(network);
     thb_result r;
     if (ensure_engine(x)) return fatal_or(0);
+    if (thb_engine_forward(x->engine, data, 0, 0, 0, 0, batchsize, nplanes, height, width, 4, network->mean, network->std,
+                           inplace, &r))
+        return fatal_or(0);
+    return publish(network, &r, result, outwidth, outheight);
+}
+
+int THProcessFloat(THNETWORK *network, float *data, int batchsize, int width, int height, int nplanes, float **result,
+                   int *outwidth, int *outheight)
+{
     /* the reference leaves the normalised values in the caller's buffer; identity statistics need no write-back */
     int trivial = 1;
     for (int c = 0; c < 3; c++)
         if (network->mean[c] != 0 || network->std[c] != 1) trivial = 0;
     const char *keep = getenv("THB200_KEEP_INPUT");
-    int inplace = !trivial && !(keep && atoi(keep));
-    if (thb_engine_forward(x->engine, data, 0, 0, 0, 0, batchsize, nplanes, height, width, 4, network->mean, network->std,
-                           inplace, &r))
-        return fatal_or(0);
-    return publish(network, &r, result, outwidth, outheight);
+    return process_float(network, data, batchsize, width, height, nplanes, !trivial && !(keep && atoi(keep)), result, outwidth,
+                         outheight);
+}
+
+/* THProcessFloat without its side effect: the caller's batch is read only, so a caller that wants to keep it needs no copy. */
+int THB200_ProcessFloatConst(THNETWORK *network, const float *data, int batchsize, int width, int height, int nplanes,
+                             float **result, int *outwidth, int *outheight)
+{
+    return process_float(network, (float *)data, batchsize, width, height, nplanes, 0, result, outwidth, outheight);
 }
 
 int THProcessImages(THNETWORK *network, unsigned char **images, int batchsize, int width, int height, int stride,

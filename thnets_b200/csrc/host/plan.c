@@ -126,6 +126,7 @@ typedef struct instance {
     float *d_minmax;
     float h_minmax[2];    /* host copy of the slice's input extremes (uint8 engine) */
     int *d_status;
+    int *h_status;        /* pinned: the boundary kernel out leaves a copy of *d_status here with every result */
     abuf *bufs;
     int nbufs;
     step *steps;
@@ -159,6 +160,7 @@ typedef struct shape_plan {
      * the one before it.  Built on the first such forward; chunk c of GPU g is pipe[g * chunks + c]. */
     instance pipe[32];
     int chunks, pipe_built, pipe_chunks;
+    const unsigned char *cut; /* boundaries of the sub-batches in sixteenths (sub_batch_cuts), NULL: thb_slice_sub_batches */
     int peer_gather;
     unsigned long long used; /* forward counter of the last use */
 } shape_plan;
@@ -1550,6 +1552,7 @@ static void instance_free(instance *I)
     if (I->ev_wb) cudaEventDestroy(I->ev_wb);
     if (I->wb_stream) cudaStreamDestroy(I->wb_stream);
     if (I->stream) cudaStreamDestroy(I->stream);
+    thb_host_free_pinned(I->h_status);
     free(I->allocs); free(I->steps); free(I->bufs);
     memset(I, 0, sizeof(*I));
 }
@@ -1567,6 +1570,9 @@ static int instance_build(thb_engine *E, instance *I, int device, int slice_off,
     I->d_minmax = dalloc(E, I, 2 * sizeof(float));
     if (!I->d_status || !I->d_minmax) return -1;
     CU(cudaMemset(I->d_status, 0, sizeof(int)));
+    I->h_status = thb_host_alloc_pinned(sizeof(int));
+    if (!I->h_status) { thb_set_error("pinned allocation failed"); return -1; }
+    *I->h_status = 0;
 
     planner P;
     memset(&P, 0, sizeof(P));
@@ -2076,9 +2082,66 @@ static int select_plan(thb_engine *E, int N, int C, int H, int W, int rank, int 
     return 0;
 }
 
+/* Ways to cut a batch into sub-batches, boundaries in sixteenths: growing ones where the results' way back is the longest
+ * part (the first result leaves early and each later one is computed under the copy before it), shrinking ones where the
+ * inputs' way in is (little is left to compute when the last input arrives), even ones between. */
+static const unsigned char sub_batch_cuts[][5] = {
+    {0, 16}, {0, 6, 16}, {0, 8, 16}, {0, 11, 16}, {0, 3, 8, 16}, {0, 5, 11, 16}, {0, 7, 13, 16},
+    {0, 1, 3, 7, 16}, {0, 2, 6, 11, 16}, {0, 4, 8, 12, 16}, {0, 5, 10, 14, 16},
+};
+
+/* Sub-batches per GPU of a host-input forward: the cut with the earliest last result in a model of the three stages a
+ * sub-batch goes through -- its copy to the device, its kernels, its result's copy back -- each one at a time.  Copies run
+ * at 50 GB/s (measured on PCIe from and to pinned memory: 55-57); a launch takes its share of the arithmetic (at 0.8
+ * PFLOP/s in the tensor-core modes, 1.4 in uint8, 20 TFLOP/s in fp32, what large layers reach) or of the bytes (4.5 TB/s),
+ * and 5 us for its fill and drain however small its sub-batch is.  The uint8 engine needs the range of a whole float batch
+ * before any kernel can start; its byte images have a static one. */
+static void choose_sub_batches(thb_engine *E)
+{
+    shape_plan *p = E->cur;
+    instance *I = &p->inst[0];
+    p->chunks = 1;
+    p->cut = 0;
+    if ((E->dtype == THB_U8 && !p->cp) || I->slice_n < 2) return;
+    const double rate = E->dtype == THB_F32 ? 20e6 : E->dtype == THB_U8 ? 1.4e9 : 0.8e9; /* per microsecond */
+    const double t_in = (double)I->slice_n * p->H * p->W * (p->cp ? p->cp : 4.0 * p->C) / 50e3;
+    const double t_out = 4.0 * I->out_count / 50e3;
+    double t_k = 0;
+    for (int t = 0; t < I->nsteps; t++) {
+        const step *s = &I->steps[t];
+        double us = (double)s->out_pixels * s->out_C * esize_of(s->dtype) * 2 / 4.5e6;
+        if (s->kind == ST_CONV) {
+            const thb_conv_desc *d = &s->conv;
+            const double f = 2.0 * d->N * d->oH * d->oW * (double)d->Cout * d->Cin * d->kH * d->kW / rate;
+            if (f > us) us = f;
+        }
+        t_k += us;
+    }
+    const double fixed = I->nsteps * 5.0;
+    double best = 0;
+    for (unsigned c = 0; c < sizeof(sub_batch_cuts) / sizeof(sub_batch_cuts[0]); c++) {
+        const unsigned char *cut = sub_batch_cuts[c];
+        double in = 0, k = 0, out = 0;
+        int S = 0, ok = 1;
+        do {
+            const double f = (cut[S + 1] - cut[S]) / 16.0;
+            if (cut[S + 1] < 16 && I->slice_n * (cut[S + 1] - cut[S]) < 16) ok = 0; /* (every sub-batch at least an image) */
+            in += f * t_in;
+            k = (in > k ? in : k) + f * t_k + fixed;
+            out = (k > out ? k : out) + f * t_out;
+        } while (cut[++S] < 16);
+        if (!ok || S > I->slice_n) continue;
+        if (c == 0 || out < 0.97 * best) {
+            best = out;
+            p->chunks = S;
+            p->cut = S > 1 ? cut : 0;
+        }
+    }
+}
+
 static int plan_build(thb_engine *E)
 {
-    const int N = E->cur->N, C = E->cur->C, H = E->cur->H, W = E->cur->W, cp = E->cur->cp;
+    const int N = E->cur->N, cp = E->cur->cp;
     E->cur->peer_gather = E->peer_gather;
     E->out_of_memory = 0;
     int G = E->ngpus < N ? E->ngpus : N;
@@ -2117,17 +2180,13 @@ static int plan_build(thb_engine *E)
         }
     }
     E->cur->built = G;
-    /* Sub-batches per GPU for pipelined host-input forwards.  Two sub-batches hide about 0.6 of the input copy (measured
-     * at ~50 GB/s from pinned memory) and cost every launch's fill and drain a second time (~6 us each, with a margin):
-     * worth it for a float batch of ResNet-50 (154 MB, 2.8 ms of copy), not for the same batch as byte images (38 MB).
-     * The uint8 engine needs the input range of the whole batch before any kernel can start. */
-    const int per_gpu = N / G;
-    const double in_mb = (double)per_gpu * (cp ? (double)H * W * cp : (double)C * H * W * 4) / 1e6;
-    const double copy_ms = in_mb / 50.0, refill_ms = E->cur->inst[0].nsteps * 0.006 * 1.5 + 0.1;
-    E->cur->chunks = E->dtype == THB_U8 || per_gpu < 32 || copy_ms * 0.6 <= refill_ms ? 1 : 2;
+    choose_sub_batches(E);
     const char *ce = getenv("THB200_CHUNKS");
-    if (ce) E->cur->chunks = atoi(ce) < 1 || E->dtype == THB_U8 ? 1 : atoi(ce) > 4 ? 4 : atoi(ce);
-    if (E->cur->chunks > per_gpu || E->whole_batch) E->cur->chunks = 1;
+    if (ce) {
+        E->cur->chunks = atoi(ce) < 1 || (E->dtype == THB_U8 && !cp) ? 1 : atoi(ce) > 4 ? 4 : atoi(ce);
+        E->cur->cut = 0;
+    }
+    if (E->cur->chunks > N / G || E->whole_batch) E->cur->chunks = 1;
     return 0;
 }
 
@@ -2143,7 +2202,13 @@ static int pipe_build(thb_engine *E, int S)
     for (int g = 0; g < G; g++)
         for (int c = 0; c < S; c++) {
             int off, n;
-            thb_slice_sub_batches(E->cur->inst[g].slice_n, S, c, &off, &n);
+            if (E->cur->cut && S == E->cur->chunks) {
+                const unsigned char *cut = E->cur->cut;
+                const int sn = E->cur->inst[g].slice_n;
+                off = (sn * cut[c] + 8) / 16;
+                n = (sn * cut[c + 1] + 8) / 16 - off;
+            } else
+                thb_slice_sub_batches(E->cur->inst[g].slice_n, S, c, &off, &n);
             if (instance_build(E, &E->cur->pipe[g * S + c], E->cur->inst[g].device, E->cur->inst[g].slice_off + off, n)) return -1;
         }
     E->cur->pipe_built = G * S;
@@ -2236,8 +2301,8 @@ static int boundary_out(thb_engine *E, instance *I, float *dst)
 {
     const value *ov = &I->out_val;
     float inv = ov->q_mult ? (float)(1.0 / ov->q_mult) : 0;
-    if (thb_postprocess(bufptr(I, ov->buf, ov->coff, E->dtype), E->dtype, ov->s.N, ov->s.H, ov->s.W, ov->s.C, ov->ld,
-                        ov->q_sub, inv, dst, I->stream)) { thb_set_error("postprocess launch failed"); return -1; }
+    if (thb_postprocess_status(bufptr(I, ov->buf, ov->coff, E->dtype), E->dtype, ov->s.N, ov->s.H, ov->s.W, ov->s.C, ov->ld,
+                               ov->q_sub, inv, dst, I->d_status, I->h_status, I->stream)) { thb_set_error("postprocess launch failed"); return -1; }
     return 0;
 }
 
@@ -2275,15 +2340,33 @@ static int host_is_pageable(const void *p)
     return a.type == cudaMemoryTypeUnregistered;
 }
 
-/* host-to-host copy by all the host threads OpenMP gives this process (1 MB blocks) */
+/* host-to-host copy; from a quarter of a megabyte on by all the host threads OpenMP gives this process */
 static void parallel_copy(void *dst, const void *src, size_t bytes)
 {
-    const size_t blk = (size_t)1 << 20;
+    const size_t blk = (size_t)128 << 10;
     const long nb = (long)((bytes + blk - 1) / blk);
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (nb > 2)
     for (long b = 0; b < nb; b++) {
         const size_t o = (size_t)b * blk;
         memcpy((char *)dst + o, (const char *)src + o, bytes - o < blk ? bytes - o : blk);
+    }
+}
+
+/* Byte images, each wherever the caller has it, to one tightly packed array.  The threads share blocks of rows, so that
+ * one large image is spread over them as well as a batch of small ones. */
+static void stage_images(unsigned char *dst, unsigned char *const *images, int n, int H, size_t row, size_t stride)
+{
+    const int rows = row >= ((size_t)64 << 10) ? 1 : (int)(((size_t)64 << 10) / row);
+    const int per = (H + rows - 1) / rows;
+    const long items = (long)n * per;
+#pragma omp parallel for schedule(static) if (items > 4)
+    for (long t = 0; t < items; t++) {
+        const int i = (int)(t / per), r0 = (int)(t % per) * rows, r1 = r0 + rows < H ? r0 + rows : H;
+        unsigned char *d = dst + ((size_t)i * H + r0) * row;
+        const unsigned char *s = images[i] + (size_t)r0 * stride;
+        if (stride == row) memcpy(d, s, (size_t)(r1 - r0) * row);
+        else
+            for (int r = r0; r < r1; r++, d += row, s += stride) memcpy(d, s, row);
     }
 }
 
@@ -2294,7 +2377,7 @@ static void parallel_copy(void *dst, const void *src, size_t bytes)
  * device. */
 static void stage_planes_normalised(float *dst, float *src, long p0, long p1, int C, long HW, const float *mean, const float *std)
 {
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if ((p1 - p0) * HW > 65536)
     for (long p = p0; p < p1; p++) {
         const int c = (int)(p % C);
         float *s = src + p * HW, *d = dst + p * HW;
@@ -2310,6 +2393,9 @@ static void stage_planes_normalised(float *dst, float *src, long p0, long p1, in
     }
 }
 
+/* bytes staged per copy to the device, and up to which size a result is written to the host by the kernel that makes it */
+static const size_t STAGE_PIECE = (size_t)4 << 20, DIRECT_RESULT_BYTES = (size_t)2 << 20;
+
 int thb_engine_forward(thb_engine *E, float *x, unsigned char **images, int stride, int bgr, int cp, int N, int C, int H,
                        int W, int rank, const float *mean, const float *std, int inplace, thb_result *res)
 {
@@ -2321,7 +2407,7 @@ int thb_engine_forward(thb_engine *E, float *x, unsigned char **images, int stri
     int G = E->cur->built;
     const int peer_gather = E->cur->peer_gather;
     int S = g_chunks_override ? g_chunks_override : E->cur->chunks;
-    if (E->dtype == THB_U8 || S > E->cur->inst[0].slice_n || E->whole_batch) S = 1;
+    if ((E->dtype == THB_U8 && x) || S > E->cur->inst[0].slice_n || E->whole_batch) S = 1;
     if (S > 1) {
         if ((!E->cur->pipe_built || E->cur->pipe_chunks != S) && pipe_build(E, S)) return -1;
         set = E->cur->pipe;
@@ -2332,23 +2418,28 @@ int thb_engine_forward(thb_engine *E, float *x, unsigned char **images, int stri
      * send theirs with cudaMemcpyPeerAsync on their own stream -- also when a GPU's slice runs as pipelined sub-batches. */
     float *gather = E->cur->built > 1 && peer_gather ? E->cur->inst[0].d_out : 0;
     const int dev0 = E->cur->inst[0].device;
+    /* A small result is written by the boundary kernel into the pinned result buffer itself, which saves the copy that would
+     * otherwise start when the kernels have ended (about 6 us for a few kilobytes). */
+    long total = 0;
+    for (int g = 0; g < G; g++) total += set[g].out_count;
+    const int direct = !gather && (size_t)total * sizeof(float) <= DIRECT_RESULT_BYTES;
     const size_t img_elems = (size_t)C * H * W;
     float q_sub = 0, q_mult = 0;
 
-    long total = 0;
-    for (int g = 0; g < G; g++) total += set[g].out_count;
     if ((size_t)total * sizeof(float) > E->h_out_bytes) {
         thb_host_free_pinned(E->h_out);
         E->h_out_bytes = (size_t)total * sizeof(float);
         E->h_out = thb_host_alloc_pinned(E->h_out_bytes);
         if (!E->h_out) { thb_set_error("pinned result allocation failed"); return -1; }
     }
-    /* A float batch in pageable memory (what a caller of the reference passes) goes through a pinned buffer of the
-     * library, filled slice by slice by the host's threads, so that the copy to the device runs at link speed and under
-     * the previous slice's kernels (THB200_NO_STAGING=1: hand the caller's pointer to the driver as it is). */
+    /* A batch in pageable memory (what a caller of the reference passes) goes through a pinned buffer of the library, piece
+     * by piece, filled by the host's threads: the copy of a piece to the device runs at link speed under the filling of the
+     * next one, and images that lie apart in memory leave as one copy per piece.  The driver's own staging of 256 separate
+     * pictures took 4.5 ms of an 8.1 ms call; small batches gain too, since the driver stages and waits for those inside the
+     * call.  (THB200_NO_STAGING=1: hand the caller's pointers to the driver as they are.) */
     int staged = 0;
     const size_t in_bytes = x ? (size_t)N * img_elems * sizeof(float) : (size_t)N * H * W * cp;
-    if (in_bytes >= ((size_t)8 << 20) && (x || (size_t)stride == (size_t)W * cp) && host_is_pageable(x ? (const void *)x : images[0])) {
+    if (host_is_pageable(x ? (const void *)x : images[0])) {
         const char *ns = getenv("THB200_NO_STAGING");
         staged = !(ns && atoi(ns));
         if (staged && in_bytes > E->h_stage_bytes) {
@@ -2368,9 +2459,9 @@ int thb_engine_forward(thb_engine *E, float *x, unsigned char **images, int stri
     E->last_has_x = x != 0; E->last_cp = cp; E->last_bgr = bgr;
     for (int k = 0; k < 3; k++) { E->last_mean[k] = mean[k]; E->last_std[k] = std[k]; }
 
-    /* The uint8 engine needs the input range of the whole batch before any kernel can start: it stages every slice, then
-     * measures, then launches.  The other modes launch a slice's kernels as soon as its copy is queued. */
-    const int two_phase = E->dtype == THB_U8;
+    /* The uint8 engine needs the input range of the whole float batch before any kernel can start: it stages every slice, then
+     * measures, then launches (byte images come with a static range).  The other modes launch a slice's kernels as soon as its copy is queued. */
+    const int two_phase = E->dtype == THB_U8 && x;
     cudaEvent_t ev_call = 0;
     if (th_debug > 1 && cudaSetDevice(set[0].device) == cudaSuccess && cudaEventCreate(&ev_call) == cudaSuccess)
         cudaEventRecord(ev_call, set[0].stream);
@@ -2388,12 +2479,11 @@ int thb_engine_forward(thb_engine *E, float *x, unsigned char **images, int stri
                     const size_t bytes = (size_t)I->slice_n * img_elems * sizeof(float);
                     const float *src = x + (size_t)I->slice_off * img_elems;
                     if (staged) {
-                        /* in pieces of about 16 MB (whole planes): the copy to the device of one piece runs while the host
-                         * threads fill the next */
+                        /* in pieces of whole planes: the copy to the device of one piece runs while the host threads fill the next */
                         float *st = E->h_stage + (size_t)I->slice_off * img_elems;
                         float *xs = x + (size_t)I->slice_off * img_elems;
                         const long HW = (long)H * W, planes = (long)I->slice_n * C;
-                        long per_piece = (((long)16 << 20) / (long)sizeof(float)) / HW;
+                        long per_piece = (long)(STAGE_PIECE / sizeof(float)) / HW;
                         if (per_piece < 1) per_piece = 1;
                         for (long p0 = 0; p0 < planes; p0 += per_piece) {
                             const long p1 = p0 + per_piece < planes ? p0 + per_piece : planes;
@@ -2404,19 +2494,25 @@ int thb_engine_forward(thb_engine *E, float *x, unsigned char **images, int stri
                         }
                     } else
                         CU(cudaMemcpyAsync(I->d_in, src, bytes, cudaMemcpyHostToDevice, I->stream));
+                } else if (staged) {
+                    const size_t row = (size_t)W * cp, img_bytes = (size_t)H * row;
+                    unsigned char *st = (unsigned char *)E->h_stage + (size_t)I->slice_off * img_bytes;
+                    int per_piece = (int)(STAGE_PIECE / img_bytes);
+                    if (per_piece < 1) per_piece = 1;
+                    for (int n = 0; n < I->slice_n; n += per_piece) {
+                        const int cnt = I->slice_n - n < per_piece ? I->slice_n - n : per_piece;
+                        stage_images(st + (size_t)n * img_bytes, images + I->slice_off + n, cnt, H, row, stride);
+                        CU(cudaMemcpyAsync(I->d_img + (size_t)n * img_bytes, st + (size_t)n * img_bytes, (size_t)cnt * img_bytes,
+                                           cudaMemcpyHostToDevice, I->stream));
+                    }
                 } else if ((size_t)stride == (size_t)W * cp) {
-                    /* tightly packed rows: one copy per run of images that also follow one another in host memory */
+                    /* pinned, tightly packed rows: one copy per run of images that also follow one another in host memory */
                     const size_t img_bytes = (size_t)H * W * cp;
                     for (int n = 0; n < I->slice_n;) {
                         int run = 1;
                         while (n + run < I->slice_n && images[I->slice_off + n + run] == images[I->slice_off + n + run - 1] + img_bytes) run++;
-                        const unsigned char *src = images[I->slice_off + n];
-                        if (staged) {
-                            unsigned char *st = (unsigned char *)E->h_stage + (size_t)(I->slice_off + n) * img_bytes;
-                            parallel_copy(st, src, (size_t)run * img_bytes);
-                            src = st;
-                        }
-                        CU(cudaMemcpyAsync(I->d_img + (size_t)n * img_bytes, src, (size_t)run * img_bytes, cudaMemcpyHostToDevice, I->stream));
+                        CU(cudaMemcpyAsync(I->d_img + (size_t)n * img_bytes, images[I->slice_off + n], (size_t)run * img_bytes,
+                                           cudaMemcpyHostToDevice, I->stream));
                         n += run;
                     }
                 } else {
@@ -2428,14 +2524,14 @@ int thb_engine_forward(thb_engine *E, float *x, unsigned char **images, int stri
             }
             long off = 0;
             for (int k = 0; k < g; k++) off += set[k].out_count;
-            float *dst = gather && I->device == dev0 ? gather + off : I->d_out;
+            float *dst = gather && I->device == dev0 ? gather + off : direct ? E->h_out + off : I->d_out;
             if (device_forward(E, I, x != 0, inplace, cp, bgr, C, H, W, mean, std, q_sub, q_mult,
                                x && inplace ? x + (size_t)I->slice_off * img_elems : 0, dst)) return -1;
             CU(cudaEventRecord(I->ev1, I->stream));
             if (gather) {
                 if (I->device != dev0)
                     CU(cudaMemcpyPeerAsync(gather + off, dev0, I->d_out, I->device, (size_t)I->out_count * sizeof(float), I->stream));
-            } else
+            } else if (!direct)
                 CU(cudaMemcpyAsync(E->h_out + off, I->d_out, (size_t)I->out_count * sizeof(float), cudaMemcpyDeviceToHost, I->stream));
         }
     }
@@ -2462,9 +2558,9 @@ int thb_engine_forward(thb_engine *E, float *x, unsigned char **images, int stri
         }
         I->last_ms = ms;
         if (ms > ms_max) ms_max = ms;
-        int status = 0;
-        CU(cudaMemcpy(&status, I->d_status, sizeof(int), cudaMemcpyDeviceToHost));
+        const int status = *(volatile int *)I->h_status;
         if (status) {
+            *I->h_status = 0;
             cudaMemset(I->d_status, 0, sizeof(int));
             thb_set_error("a device-side wait timed out (code %d) on device %d", status, I->device);
             return -1;

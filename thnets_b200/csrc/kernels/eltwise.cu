@@ -413,9 +413,11 @@ __global__ void __launch_bounds__(256) minmax_kernel(const float *x, int C, long
 
 // ---- NHWC Tin -> NCHW Tout through a 32x32 shared-memory transpose ---------------------------------
 template <typename Tin, typename Tout>
-__global__ void nhwc_to_nchw_kernel(const Tin *x, int HW, int C, int x_ld, float q_sub, float q_invmult, Tout *y)
+__global__ void nhwc_to_nchw_kernel(const Tin *x, int HW, int C, int x_ld, float q_sub, float q_invmult, Tout *y,
+                                    const int *status, int *status_out)
 {
     __shared__ float tile[32][33];
+    if (status && (blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x | threadIdx.y) == 0) *status_out = *status;
     const int n = blockIdx.z, hw0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
     for (int r = threadIdx.y; r < 32; r += blockDim.y) {
         const int hw = hw0 + r, c = c0 + threadIdx.x;
@@ -433,6 +435,21 @@ __global__ void nhwc_to_nchw_kernel(const Tin *x, int HW, int C, int x_ld, float
             dt<Tout>::st(y + ((size_t)n * C + c) * HW + hw, tile[threadIdx.x][r]);
         }
     }
+}
+
+// The same for one position per image (a classifier's scores): neither side needs transposing, so consecutive threads
+// write consecutive values -- `y` may be pinned host memory, where scattered 4-byte stores would cost a transaction each.
+template <typename Tin>
+__global__ void rows_to_float_kernel(const Tin *x, long total, int C, int x_ld, float q_sub, float q_invmult, float *y,
+                                     const int *status, int *status_out)
+{
+    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (status && i == 0) *status_out = *status;
+    if (i >= total) return;
+    const long n = i / C;
+    float v = dt<Tin>::ld(x + n * x_ld + (i - n * C));
+    if (sizeof(Tin) == 1) v = __fadd_rn(__fmul_rn(v, q_invmult), q_sub);
+    y[i] = v;
 }
 
 // ---- pooling ------------------------------------------------------------------------------------------
@@ -956,15 +973,27 @@ int thb_minmax_normalized(const float *x, int N, int C, int H, int W, const floa
     return THB_LAUNCH_CHECK("minmax_kernel");
 }
 
-int thb_postprocess(const void *x, int dtype, int N, int H, int W, int C, int x_ld, float q_sub, float q_invmult,
-                    float *y, thb_stream s)
+int thb_postprocess_status(const void *x, int dtype, int N, int H, int W, int C, int x_ld, float q_sub, float q_invmult,
+                           float *y, const int *status, int *status_out, thb_stream s)
 {
     const int HW = H * W;
     if ((long)N * HW * C == 0) return THB_OK;
+    if (HW == 1) {
+        const long total = (long)N * C;
+        DISPATCH_ANY_DTYPE(dtype, (rows_to_float_kernel<T><<<nblocks(total), 256, 0, (cudaStream_t)s>>>(
+                                      (const T *)x, total, C, x_ld, q_sub, q_invmult, y, status, status_out)));
+        return THB_LAUNCH_CHECK("rows_to_float_kernel");
+    }
     dim3 grid((HW + 31) / 32, (C + 31) / 32, N), block(32, 8);
     DISPATCH_ANY_DTYPE(dtype, (nhwc_to_nchw_kernel<T, float><<<grid, block, 0, (cudaStream_t)s>>>(
-                                  (const T *)x, HW, C, x_ld, q_sub, q_invmult, y)));
+                                  (const T *)x, HW, C, x_ld, q_sub, q_invmult, y, status, status_out)));
     return THB_LAUNCH_CHECK("nhwc_to_nchw_kernel");
+}
+
+int thb_postprocess(const void *x, int dtype, int N, int H, int W, int C, int x_ld, float q_sub, float q_invmult,
+                    float *y, thb_stream s)
+{
+    return thb_postprocess_status(x, dtype, N, H, W, C, x_ld, q_sub, q_invmult, y, 0, 0, s);
 }
 
 int thb_to_nchw(int dtype, const void *x, int N, int H, int W, int C, int x_ld, void *y, thb_stream s)
@@ -973,7 +1002,7 @@ int thb_to_nchw(int dtype, const void *x, int N, int H, int W, int C, int x_ld, 
     if ((long)N * HW * C == 0) return THB_OK;
     dim3 grid((HW + 31) / 32, (C + 31) / 32, N), block(32, 8);
     DISPATCH_ANY_DTYPE(dtype, (nhwc_to_nchw_kernel<T, T><<<grid, block, 0, (cudaStream_t)s>>>(
-                                  (const T *)x, HW, C, x_ld, 0.f, 1.f, (T *)y)));
+                                  (const T *)x, HW, C, x_ld, 0.f, 1.f, (T *)y, 0, 0)));
     return THB_LAUNCH_CHECK("nhwc_to_nchw_kernel");
 }
 
