@@ -14,6 +14,10 @@
  * two ends by the pre/postprocess kernels.
  */
 #include <cuda_runtime_api.h>
+#ifdef __SSE2__
+#include <emmintrin.h>
+#endif
+#include <omp.h>
 #include <math.h>
 #include <stdarg.h>
 #include <stdio.h>
@@ -141,6 +145,12 @@ typedef struct instance {
     int runs, graph_state; /* graph_state: 0 not tried, 1 usable, -1 capture failed or switched off */
     int graph_from;        /* first launch inside the graph (the ones before it are issued directly every forward) */
     int graph_launches;    /* kernel launches one replay stands for */
+    /* Sliced start: a large batch is copied in `slices` parts on a stream of its own, and the first `prefix` launches run on
+     * each part as it arrives (set up by choose_slices; 0: the launches wait for the whole batch) */
+    int prefix, slices;
+    double hidden_us; /* modelled gain */
+    cudaStream_t copy_stream;
+    cudaEvent_t ev_slice;
     int input_s2d; /* the network input is staged space-to-depth for a stride-2 first convolution */
     int input_neigh; /* uint8 engine, 3x3 / stride 1 / pad 1 first convolution on a three-plane float batch: the boundary kernel
                       * stages every pixel's 27 quantised neighbours as the channels of that pixel (taps outside the image: the
@@ -1492,6 +1502,82 @@ static int plan_node(planner *P, int i)
     return -1;
 }
 
+/* Can launch `s` run on some of its images?  (The planned convolutions and poolings whose images are independent; what
+ * they add is the image offset of every operand, exec_step.) */
+static int sliceable(const instance *I, const step *s)
+{
+    switch (s->kind) {
+    case ST_CONV: return s->conv.N == I->slice_n && s->scratch_buf < 0 && !s->in_off0 && !s->out_off0;
+    case ST_MAXPOOL: return s->N == I->slice_n;
+    case ST_CSUM: case ST_ZERO: return s->pixels % I->slice_n == 0;
+    default: return 0;
+    }
+}
+
+/* Microseconds of a launch on the whole slice, roughly: its share of the arithmetic (at 0.5 PFLOP/s in the 16-bit modes,
+ * 0.9 in uint8, 20 TFLOP/s in fp32, what the layers of a large batch reach on average) or of the bytes (4.5 TB/s), whichever
+ * is more. */
+static double model_us(const step *s)
+{
+    double elems = (double)s->out_pixels * s->out_C * 2, us = 0;
+    if (s->kind == ST_CONV) {
+        const thb_conv_desc *d = &s->conv;
+        const double rate = s->dtype == THB_F32 ? 20e6 : s->dtype == THB_U8 ? 0.9e9 : 0.5e9; /* per microsecond */
+        us = 2.0 * d->N * d->oH * d->oW * (double)d->Cout * d->Cin * d->kH * d->kW / rate;
+        elems = (double)d->N * d->H * d->W * d->Cin + elems * (s->nin > 1 ? 1 : 0.5);
+    }
+    const double b = elems * esize_of(s->dtype) / 4.5e6;
+    return us > b ? us : b;
+}
+
+/* microseconds of a slice's input on its way to the device (measured: 55 GB/s from pinned memory) */
+static double copy_in_us(const thb_engine *E, const instance *I)
+{
+    const shape_plan *p = E->cur;
+    return (double)I->slice_n * p->H * p->W * (p->cp ? p->cp : 4.0 * p->C) / 50e3;
+}
+
+/* A batch of 256 pictures takes 0.7 ms to arrive, a fifth of a ResNet-50 forward.  The first launches of a network are the
+ * ones with the most pixels, which lose nothing on a part of the batch: they follow the copy part by part, and the rest of the
+ * network runs on the whole batch.  (Cutting the whole network into sub-batches instead repeats the fill and drain of all its
+ * small layers: ResNet-50 on 96 + 160 pictures, 4.35 ms of kernels instead of 3.65.)  Of 2 to 8 parts, the count that hides
+ * most of the copy: launches join as long as a part of theirs keeps the chip busy for 6 us, until they take as long as the
+ * copy; a launch costs 5 us more on every part (measured: 3 to 7 launches in 4 parts are within 2 % of one another, 9 in 7 parts
+ * lose 6 %). */
+static void choose_slices(thb_engine *E, instance *I)
+{
+    I->prefix = I->slices = 0;
+    if ((E->dtype == THB_U8 && !E->cur->cp) || E->cur->cp == 2 || E->whole_batch || I->in_val.buf < 0) return;
+    const char *off = getenv("THB200_NO_SLICES");
+    if (off && atoi(off)) return;
+    const double t_in = copy_in_us(E, I);
+    double best = 20;
+    for (int m = 2; m <= 8 && m <= I->slice_n / 2; m++) {
+        double us = 0;
+        int p = 0;
+        while (p < I->nsteps && us < t_in && sliceable(I, &I->steps[p])) {
+            const double k = model_us(&I->steps[p]);
+            if (k > 0 && k < 6 * m) break;
+            us += k;
+            p++;
+        }
+        const double gain = (us < t_in ? us : t_in) * (m - 1) / m - 5.0 * p * m;
+        if (gain <= best) continue;
+        best = gain;
+        I->prefix = p;
+        I->slices = m;
+        I->hidden_us = gain;
+    }
+}
+
+/* part c of a sliced start: the first one is half as large as the others, so that the kernels start early */
+static void slice_part(const instance *I, int c, int *i0, int *cnt)
+{
+    const int w = 2 * I->slices - 1, n = I->slice_n;
+    *i0 = c ? (int)((long)n * (2 * c - 1) / w) : 0;
+    *cnt = (int)((long)n * (2 * c + 1) / w) - *i0;
+}
+
 /* liveness-based packing of the activation buffers into one arena */
 static size_t pack_arena(instance *I)
 {
@@ -1510,6 +1596,12 @@ static size_t pack_arena(instance *I)
                 b->last = t;
             }
     }
+    /* a sliced start runs its launches part by part: whatever they touch is alive until the last part has run them all */
+    for (int b = 0; b < I->nbufs; b++)
+        if (I->prefix && I->bufs[b].last >= 0 && I->bufs[b].first < I->prefix) {
+            I->bufs[b].first = 0;
+            if (I->bufs[b].last < I->prefix - 1) I->bufs[b].last = I->prefix - 1;
+        }
     /* the network input lives from the preprocess launch (before step 0); the output until the postprocess */
     if (I->in_val.buf >= 0) I->bufs[I->in_val.buf].first = -1;
     if (I->out_val.buf >= 0) I->bufs[I->out_val.buf].last = I->nsteps;
@@ -1551,13 +1643,16 @@ static void instance_free(instance *I)
     if (I->ev1) cudaEventDestroy(I->ev1);
     if (I->ev_wb) cudaEventDestroy(I->ev_wb);
     if (I->wb_stream) cudaStreamDestroy(I->wb_stream);
+    if (I->copy_stream) { cudaStreamSynchronize(I->copy_stream); cudaStreamDestroy(I->copy_stream); }
+    if (I->ev_slice) cudaEventDestroy(I->ev_slice);
     if (I->stream) cudaStreamDestroy(I->stream);
     thb_host_free_pinned(I->h_status);
     free(I->allocs); free(I->steps); free(I->bufs);
     memset(I, 0, sizeof(*I));
 }
 
-static int instance_build(thb_engine *E, instance *I, int device, int slice_off, int slice_n)
+/* `whole`: the instance computes all of its GPU's images (not one of the pipelined sub-batches of them) */
+static int instance_build(thb_engine *E, instance *I, int device, int slice_off, int slice_n, int whole)
 {
     thb_model *M = E->model;
     memset(I, 0, sizeof(*I));
@@ -1662,6 +1757,7 @@ static int instance_build(thb_engine *E, instance *I, int device, int slice_off,
         I->out_val = P.val[M->output];
         I->out_shape = I->out_val.s;
         I->out_count = (long)I->out_shape.N * I->out_shape.C * I->out_shape.H * I->out_shape.W;
+        if (whole) choose_slices(E, I);
         I->arena_bytes = pack_arena(I);
         I->arena = dalloc(E, I, I->arena_bytes);
         size_t in_bytes = (size_t)slice_n * E->cur->C * E->cur->H * E->cur->W * sizeof(float);
@@ -1669,6 +1765,11 @@ static int instance_build(thb_engine *E, instance *I, int device, int slice_off,
         I->d_img = dalloc(E, I, (size_t)slice_n * E->cur->H * E->cur->W * 4);
         I->d_out = dalloc(E, I, (size_t)(I->out_count ? I->out_count : 1) * sizeof(float));
         if (!I->arena || !I->d_in || !I->d_out || !I->d_img) rc = -1;
+        if (!rc && I->prefix && (cudaStreamCreateWithFlags(&I->copy_stream, cudaStreamNonBlocking) != cudaSuccess ||
+                                 cudaEventCreateWithFlags(&I->ev_slice, cudaEventDisableTiming) != cudaSuccess)) {
+            thb_set_error("stream creation failed");
+            rc = -1;
+        }
         /* padded channels are never read as data, but stale NaN/Inf bit patterns would poison the
          * zero-weight products: start from a clean arena */
         if (!rc && cudaMemset(I->arena, 0, I->arena_bytes) != cudaSuccess) { thb_set_error("arena memset failed"); rc = -1; }
@@ -1685,110 +1786,152 @@ static void *bufptr(instance *I, int buf, int coff, int dtype)
     return buf < 0 ? 0 : I->arena + I->bufs[buf].offset + (size_t)coff * esize_of(dtype);
 }
 
-static int run_steps_ev(thb_engine *E, instance *I, cudaEvent_t *evs, int from, int to)
+/* One planned launch on the instance's stream; on images [img0, img0 + cnt) only when cnt > 0 (sliceable launches). */
+static int exec_step(instance *I, int t, int img0, int cnt)
 {
     thb_stream st = I->stream;
+    step part, *s = &I->steps[t];
+    const int dt = s->dtype;
+    const size_t es = esize_of(dt);
+    char *x0 = bufptr(I, s->in_buf[0], s->in_coff[0], dt);
+    if (x0 && s->in_off0) x0 += s->in_off0 * es;
+    char *y = bufptr(I, s->out_buf, s->out_coff, dt);
+    if (y && s->out_off0) y += s->out_off0 * es;
+    int rc = 0;
+    size_t res_off = 0, aux_off = 0, aux2_off = 0; /* bytes */
+    if (cnt > 0) {
+        part = *s;
+        s = &part;
+        thb_conv_desc *d = &s->conv;
+        switch (s->kind) {
+        case ST_CONV: {
+            const size_t opix = (size_t)d->oH * d->oW;
+            d->N = cnt;
+            x0 += (size_t)img0 * d->H * (d->in_row_pitch ? d->in_row_pitch : d->W) * d->in_ld * es;
+            y += (size_t)img0 * (s->pool_k ? (size_t)s->pool_oH * s->pool_oW : opix) * s->out_ld * es;
+            res_off = s->dual ? (size_t)img0 * d->x2_H * d->x2_W * d->x2_ld * es : img0 * opix * d->res_ld * es;
+            aux_off = sizeof(int) * (size_t)img0 * d->H * d->W;
+            aux2_off = sizeof(int) * img0 * opix;
+            break;
+        }
+        case ST_MAXPOOL:
+            s->N = cnt;
+            x0 += (size_t)img0 * s->H * s->W * s->in_ld[0] * es;
+            y += (size_t)img0 * s->oH * s->oW * s->out_ld * es;
+            break;
+        case ST_CSUM: case ST_ZERO: {
+            const long per = s->pixels / I->slice_n;
+            if (s->kind == ST_CSUM) x0 += (size_t)img0 * per * s->in_ld[0] * es;
+            aux_off = sizeof(int) * (size_t)img0 * per;
+            s->pixels = cnt * per;
+            break;
+        }
+        }
+    }
+    switch (s->kind) {
+    case ST_CONV: {
+        thb_conv_desc *d = &s->conv;
+        if (s->dual) d->x2 = (char *)bufptr(I, s->in_buf[1], s->in_coff[1], dt) + res_off;
+        else if (s->nin > 1) d->res = (char *)bufptr(I, s->in_buf[1], s->in_coff[1], dt) + res_off;
+        if (s->aux_buf >= 0) d->csum = (const int *)((char *)bufptr(I, s->aux_buf, 0, THB_U8) + aux_off);
+        if (s->aux2_buf >= 0) d->csum_out = (int *)((char *)bufptr(I, s->aux2_buf, 0, THB_U8) + aux2_off);
+        if (s->scratch_buf >= 0) d->splitk_scratch = (float *)bufptr(I, s->scratch_buf, 0, THB_U8);
+        rc = s->pool_k ? thb_conv_maxpool_fwd(d, s->pool_k, 2, s->pool_pad, s->pool_oH, s->pool_oW, x0, y, s->out_ld, st)
+                       : thb_conv_fwd(d, x0, y, st);
+        break;
+    }
+    case ST_GEMV:
+        rc = thb_gemv_fwd(dt, x0, s->N, s->K, s->in_ld[0], s->w, s->M, s->scale, s->shift, &s->act, y, s->out_ld, st);
+        break;
+    case ST_MAXPOOL:
+        rc = thb_maxpool(dt, x0, s->N, s->H, s->W, s->C, s->in_ld[0], s->kH, s->kW, s->dH, s->dW, s->padH, s->padW, s->oH,
+                         s->oW, y, s->out_ld, st);
+        break;
+    case ST_AVGPOOL:
+        rc = thb_avgpool(dt, x0, s->N, s->H, s->W, s->C, s->in_ld[0], s->kH, s->kW, s->dH, s->dW, s->padH, s->padW, s->oH,
+                         s->oW, s->flag, y, s->out_ld, st);
+        break;
+    case ST_AFFINE:
+        rc = thb_affine_act(dt, x0, s->pixels, s->C, s->in_ld[0], s->scale, s->shift, &s->act, y, s->out_ld, st);
+        break;
+    case ST_U8COMBINE:
+        rc = thb_u8_combine(x0, s->in_ld[0], bufptr(I, s->in_buf[1], s->in_coff[1], THB_U8), s->in_ld[1], (int)s->coef[0],
+                            (int)s->coef[1], s->thr, s->val, s->pixels, s->C, y, s->out_ld, st);
+        break;
+    case ST_U8THR:
+        rc = thb_u8_threshold(x0, s->pixels, s->C, s->in_ld[0], s->thr, s->val, y, s->out_ld, st);
+        break;
+    case ST_COMBINE: {
+        const void *xs[8];
+        for (int k = 0; k < s->nin; k++) xs[k] = bufptr(I, s->in_buf[k], s->in_coff[k], dt);
+        rc = thb_combine(dt, s->nin, xs, s->in_ld, s->coef, s->pixels, s->C, y, s->out_ld, st);
+        break;
+    }
+    case ST_COPY:
+        rc = thb_copy_channels(dt, x0, s->pixels, s->C, s->in_ld[0], y, s->out_ld, st);
+        break;
+    case ST_SOFTMAX:
+        rc = thb_softmax(dt, x0, s->pixels, s->C, s->in_ld[0], y, s->out_ld, st);
+        break;
+    case ST_COL2IM:
+        rc = thb_col2im(dt, x0, s->N, s->H, s->W, s->C, s->kH, s->kW, s->dH, s->dW, s->padH, s->padW, s->oH, s->oW,
+                        s->in_ld[0], s->beta, s->bias, &s->act, y, s->out_ld, st);
+        break;
+    case ST_ZERO:
+        if (s->pixels > 0 && cudaMemsetAsync((char *)bufptr(I, s->out_buf, 0, THB_U8) + aux_off, 0, sizeof(int) * (size_t)s->pixels, (cudaStream_t)st) != cudaSuccess) rc = -1;
+        break;
+    case ST_CSUM:
+        rc = thb_u8_channel_sum(x0, s->pixels, s->C, s->in_ld[0], (int *)((char *)bufptr(I, s->out_buf, 0, THB_U8) + aux_off), st);
+        break;
+    case ST_TO_NCHW:
+        rc = thb_to_nchw(dt, x0, s->N, s->H, s->W, s->C, s->in_ld[0], y, st);
+        break;
+    case ST_FROM_NCHW:
+        rc = thb_from_nchw(dt, x0, s->N, s->H, s->W, s->C, s->in_ld[0], y, s->out_ld, st);
+        break;
+    case ST_UPSAMPLE:
+        rc = thb_upsample2x(dt, x0, s->N, s->H, s->W, s->C, s->in_ld[0], y, s->out_ld, st);
+        break;
+    case ST_ZEROPAD:
+        rc = thb_zero_pad(dt, x0, s->N, s->H, s->W, s->C, s->in_ld[0], s->padW, s->kW, s->padH, s->kH, y, s->out_ld, st);
+        break;
+    case ST_REFLECTPAD:
+        rc = thb_reflect_pad(dt, x0, s->N, s->H, s->W, s->C, s->in_ld[0], s->padW, s->kW, s->padH, s->kH, y, s->out_ld, st);
+        break;
+    case ST_SLICEC:
+        rc = thb_slice_channels(dt, x0, s->pixels, s->flag, s->C, s->in_ld[0], y, s->out_ld, st);
+        break;
+    case ST_CMAX: {
+        const void *xs[8];
+        for (int k = 0; k < s->nin; k++) xs[k] = bufptr(I, s->in_buf[k], s->in_coff[k], dt);
+        rc = thb_cmax(dt, s->nin, xs, s->in_ld, s->pixels, s->C, y, s->out_ld, st);
+        break;
+    }
+    case ST_LOGSOFTMAX:
+        rc = thb_logsoftmax(dt, x0, s->pixels, s->C, s->in_ld[0], y, s->out_ld, s->flag, st);
+        break;
+    case ST_NORMALIZE:
+        rc = thb_l2_normalize(dt, x0, s->N, s->pixels, s->flag, (float *)bufptr(I, s->aux_buf, 0, THB_U8), y, st);
+        break;
+    case ST_UNPOOL:
+        rc = thb_max_unpool(dt, x0, s->in_ld[0], bufptr(I, s->in_buf[1], s->in_coff[1], dt), s->in_ld[1], s->N, s->H, s->W, s->C,
+                            s->kH, s->kW, s->dH, s->dW, s->padH, s->padW, s->oH, s->oW, y, s->out_ld, st);
+        break;
+    }
+    if (rc) thb_set_error("kernel launch %d (kind %d) failed: %d %s", t, s->kind, rc, thb_last_cuda_error());
+    return rc ? -1 : 0;
+}
+
+static int run_steps_ev(thb_engine *E, instance *I, cudaEvent_t *evs, int from, int to)
+{
     for (int t = from; t < to; t++) {
         step *s = &I->steps[t];
         const int dt = s->dtype;
-        void *x0 = bufptr(I, s->in_buf[0], s->in_coff[0], dt);
-        if (x0 && s->in_off0) x0 = (char *)x0 + s->in_off0 * esize_of(dt);
         void *y = bufptr(I, s->out_buf, s->out_coff, dt);
         if (y && s->out_off0) y = (char *)y + s->out_off0 * esize_of(dt);
-        int rc = 0;
         double t0 = 0;
         if (th_profile) { cudaStreamSynchronize(I->stream); t0 = th_seconds(); }
-        switch (s->kind) {
-        case ST_CONV: {
-            thb_conv_desc *d = &s->conv;
-            if (s->dual) d->x2 = bufptr(I, s->in_buf[1], s->in_coff[1], dt);
-            else if (s->nin > 1) d->res = bufptr(I, s->in_buf[1], s->in_coff[1], dt);
-            if (s->aux_buf >= 0) d->csum = (const int *)bufptr(I, s->aux_buf, 0, THB_U8);
-            if (s->aux2_buf >= 0) d->csum_out = (int *)bufptr(I, s->aux2_buf, 0, THB_U8);
-            if (s->scratch_buf >= 0) d->splitk_scratch = (float *)bufptr(I, s->scratch_buf, 0, THB_U8);
-            rc = s->pool_k ? thb_conv_maxpool_fwd(d, s->pool_k, 2, s->pool_pad, s->pool_oH, s->pool_oW, x0, y, s->out_ld, st)
-                           : thb_conv_fwd(d, x0, y, st);
-            break;
-        }
-        case ST_GEMV:
-            rc = thb_gemv_fwd(dt, x0, s->N, s->K, s->in_ld[0], s->w, s->M, s->scale, s->shift, &s->act, y, s->out_ld, st);
-            break;
-        case ST_MAXPOOL:
-            rc = thb_maxpool(dt, x0, s->N, s->H, s->W, s->C, s->in_ld[0], s->kH, s->kW, s->dH, s->dW, s->padH, s->padW, s->oH,
-                             s->oW, y, s->out_ld, st);
-            break;
-        case ST_AVGPOOL:
-            rc = thb_avgpool(dt, x0, s->N, s->H, s->W, s->C, s->in_ld[0], s->kH, s->kW, s->dH, s->dW, s->padH, s->padW, s->oH,
-                             s->oW, s->flag, y, s->out_ld, st);
-            break;
-        case ST_AFFINE:
-            rc = thb_affine_act(dt, x0, s->pixels, s->C, s->in_ld[0], s->scale, s->shift, &s->act, y, s->out_ld, st);
-            break;
-        case ST_U8COMBINE:
-            rc = thb_u8_combine(x0, s->in_ld[0], bufptr(I, s->in_buf[1], s->in_coff[1], THB_U8), s->in_ld[1], (int)s->coef[0],
-                                (int)s->coef[1], s->thr, s->val, s->pixels, s->C, y, s->out_ld, st);
-            break;
-        case ST_U8THR:
-            rc = thb_u8_threshold(x0, s->pixels, s->C, s->in_ld[0], s->thr, s->val, y, s->out_ld, st);
-            break;
-        case ST_COMBINE: {
-            const void *xs[8];
-            for (int k = 0; k < s->nin; k++) xs[k] = bufptr(I, s->in_buf[k], s->in_coff[k], dt);
-            rc = thb_combine(dt, s->nin, xs, s->in_ld, s->coef, s->pixels, s->C, y, s->out_ld, st);
-            break;
-        }
-        case ST_COPY:
-            rc = thb_copy_channels(dt, x0, s->pixels, s->C, s->in_ld[0], y, s->out_ld, st);
-            break;
-        case ST_SOFTMAX:
-            rc = thb_softmax(dt, x0, s->pixels, s->C, s->in_ld[0], y, s->out_ld, st);
-            break;
-        case ST_COL2IM:
-            rc = thb_col2im(dt, x0, s->N, s->H, s->W, s->C, s->kH, s->kW, s->dH, s->dW, s->padH, s->padW, s->oH, s->oW,
-                            s->in_ld[0], s->beta, s->bias, &s->act, y, s->out_ld, st);
-            break;
-        case ST_ZERO:
-            if (s->pixels > 0 && cudaMemsetAsync(bufptr(I, s->out_buf, 0, THB_U8), 0, sizeof(int) * (size_t)s->pixels, (cudaStream_t)st) != cudaSuccess) rc = -1;
-            break;
-        case ST_CSUM:
-            rc = thb_u8_channel_sum(x0, s->pixels, s->C, s->in_ld[0], (int *)bufptr(I, s->out_buf, 0, THB_U8), st);
-            break;
-        case ST_TO_NCHW:
-            rc = thb_to_nchw(dt, x0, s->N, s->H, s->W, s->C, s->in_ld[0], y, st);
-            break;
-        case ST_FROM_NCHW:
-            rc = thb_from_nchw(dt, x0, s->N, s->H, s->W, s->C, s->in_ld[0], y, s->out_ld, st);
-            break;
-        case ST_UPSAMPLE:
-            rc = thb_upsample2x(dt, x0, s->N, s->H, s->W, s->C, s->in_ld[0], y, s->out_ld, st);
-            break;
-        case ST_ZEROPAD:
-            rc = thb_zero_pad(dt, x0, s->N, s->H, s->W, s->C, s->in_ld[0], s->padW, s->kW, s->padH, s->kH, y, s->out_ld, st);
-            break;
-        case ST_REFLECTPAD:
-            rc = thb_reflect_pad(dt, x0, s->N, s->H, s->W, s->C, s->in_ld[0], s->padW, s->kW, s->padH, s->kH, y, s->out_ld, st);
-            break;
-        case ST_SLICEC:
-            rc = thb_slice_channels(dt, x0, s->pixels, s->flag, s->C, s->in_ld[0], y, s->out_ld, st);
-            break;
-        case ST_CMAX: {
-            const void *xs[8];
-            for (int k = 0; k < s->nin; k++) xs[k] = bufptr(I, s->in_buf[k], s->in_coff[k], dt);
-            rc = thb_cmax(dt, s->nin, xs, s->in_ld, s->pixels, s->C, y, s->out_ld, st);
-            break;
-        }
-        case ST_LOGSOFTMAX:
-            rc = thb_logsoftmax(dt, x0, s->pixels, s->C, s->in_ld[0], y, s->out_ld, s->flag, st);
-            break;
-        case ST_NORMALIZE:
-            rc = thb_l2_normalize(dt, x0, s->N, s->pixels, s->flag, (float *)bufptr(I, s->aux_buf, 0, THB_U8), y, st);
-            break;
-        case ST_UNPOOL:
-            rc = thb_max_unpool(dt, x0, s->in_ld[0], bufptr(I, s->in_buf[1], s->in_coff[1], dt), s->in_ld[1], s->N, s->H, s->W, s->C,
-                                s->kH, s->kW, s->dH, s->dW, s->padH, s->padW, s->oH, s->oW, y, s->out_ld, st);
-            break;
-        }
-        if (rc) { thb_set_error("kernel launch %d (kind %d) failed: %d %s", t, s->kind, rc, thb_last_cuda_error()); return -1; }
+        if (exec_step(I, t, 0, 0)) return -1;
         if (evs) cudaEventRecord(evs[t + 1], I->stream);
         if (th_minmax && y && s->out_pixels > 0 && s->out_C > 0 && s->kind != ST_ZERO && s->kind != ST_CSUM) {
             /* thapi.c:141-154, :197-202: smallest and largest value of every layer's output -- how a caller picks the
@@ -1825,9 +1968,10 @@ static int run_steps_ev(thb_engine *E, instance *I, cudaEvent_t *evs, int from, 
 /* The launches of one forward on the instance's stream: directly the first time, from then on as a replay of the
  * graph captured from them.  In the uint8 engine the convolutions that read the network input take kernel arguments
  * that change every forward (the input's quantisation is measured per batch, lowp_basic.c:299-321): the launches up to
- * and including the last of them are always issued directly and the graph holds the rest.  THB200_NO_GRAPH=1 and the
+ * and including the last of them are always issued directly and the graph holds the rest.  The same goes for the
+ * launches of a sliced start; `from`: the first launch that has not run on the slices already.  THB200_NO_GRAPH=1 and the
  * per-module profile mode launch everything directly. */
-static int run_steps(thb_engine *E, instance *I)
+static int run_steps(thb_engine *E, instance *I, int from)
 {
     if (I->graph_state == 0 && I->runs >= 1) {
         const char *ng = getenv("THB200_NO_GRAPH");
@@ -1835,6 +1979,7 @@ static int run_steps(thb_engine *E, instance *I)
         I->graph_from = 0;
         for (int t = 0; t < I->nsteps; t++)
             if (I->steps[t].kind == ST_CONV && I->steps[t].dyn_quant) I->graph_from = t + 1;
+        if (I->graph_from < I->prefix) I->graph_from = I->prefix;
         if (I->graph_from < I->nsteps && !(ng && atoi(ng)) && !th_profile && !th_minmax) {
             cudaGraph_t g = 0;
             if (cudaStreamBeginCapture(I->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
@@ -1851,7 +1996,7 @@ static int run_steps(thb_engine *E, instance *I)
     }
     I->runs++;
     if (I->graph_state == 1 && !th_profile && !th_minmax) {
-        if (I->graph_from && run_steps_ev(E, I, 0, 0, I->graph_from)) return -1;
+        if (from < I->graph_from && run_steps_ev(E, I, 0, from, I->graph_from)) return -1;
         if (cudaGraphLaunch(I->graph, I->stream) == cudaSuccess) {
             thb_count_launches(I->graph_launches);
             return 0;
@@ -1859,12 +2004,12 @@ static int run_steps(thb_engine *E, instance *I)
         thb_set_error("graph launch failed: %s", cudaGetErrorString(cudaGetLastError()));
         return -1;
     }
-    return run_steps_ev(E, I, 0, 0, I->nsteps);
+    return run_steps_ev(E, I, 0, from, I->nsteps);
 }
 
 static int lowp_input_range(thb_engine *E, instance *set, int G, int has_x, int cp, int C, int H, int W, const float *mean,
                             const float *std, float *q_sub, float *q_mult);
-static int boundary_in(thb_engine *E, instance *I, int has_x, int inplace, int cp, int bgr, int C, int H, int W,
+static int boundary_in(thb_engine *E, instance *I, int img0, int n, int has_x, int inplace, int cp, int bgr, int C, int H, int W,
                        const float *mean, const float *std, float q_sub, float q_mult);
 static int boundary_out(thb_engine *E, instance *I, float *dst);
 
@@ -1888,7 +2033,7 @@ int thb_engine_profile(thb_engine *E, int iters, int max_steps, int *kinds, floa
         float q_sub = 0, q_mult = 0;
         rc = lowp_input_range(E, E->cur->inst, 1, E->last_has_x, E->last_cp, E->cur->C, E->cur->H, E->cur->W, E->last_mean, E->last_std, &q_sub, &q_mult);
         cudaEventRecord(evs[0], I->stream);
-        if (!rc) rc = boundary_in(E, I, E->last_has_x, 0, E->last_cp, E->last_bgr, E->cur->C, E->cur->H, E->cur->W, E->last_mean, E->last_std, q_sub, q_mult);
+        if (!rc) rc = boundary_in(E, I, 0, I->slice_n, E->last_has_x, 0, E->last_cp, E->last_bgr, E->cur->C, E->cur->H, E->cur->W, E->last_mean, E->last_std, q_sub, q_mult);
         cudaEventRecord(evs[1], I->stream);
         if (!rc) rc = run_steps_ev(E, I, evs + 1, 0, I->nsteps);
         if (!rc) rc = boundary_out(E, I, I->d_out);
@@ -2091,11 +2236,9 @@ static const unsigned char sub_batch_cuts[][5] = {
 };
 
 /* Sub-batches per GPU of a host-input forward: the cut with the earliest last result in a model of the three stages a
- * sub-batch goes through -- its copy to the device, its kernels, its result's copy back -- each one at a time.  Copies run
- * at 50 GB/s (measured on PCIe from and to pinned memory: 55-57); a launch takes its share of the arithmetic (at 0.8
- * PFLOP/s in the tensor-core modes, 1.4 in uint8, 20 TFLOP/s in fp32, what large layers reach) or of the bytes (4.5 TB/s),
- * and 5 us for its fill and drain however small its sub-batch is.  The uint8 engine needs the range of a whole float batch
- * before any kernel can start; its byte images have a static one. */
+ * sub-batch goes through -- its copy to the device, its kernels (model_us, and 12 us for each launch's fill and drain however
+ * small the sub-batch is), its result's copy back -- each one at a time.  The uint8 engine needs the range of a whole float
+ * batch before any kernel can start; its byte images have a static one. */
 static void choose_sub_batches(thb_engine *E)
 {
     shape_plan *p = E->cur;
@@ -2103,21 +2246,10 @@ static void choose_sub_batches(thb_engine *E)
     p->chunks = 1;
     p->cut = 0;
     if ((E->dtype == THB_U8 && !p->cp) || I->slice_n < 2) return;
-    const double rate = E->dtype == THB_F32 ? 20e6 : E->dtype == THB_U8 ? 1.4e9 : 0.8e9; /* per microsecond */
-    const double t_in = (double)I->slice_n * p->H * p->W * (p->cp ? p->cp : 4.0 * p->C) / 50e3;
-    const double t_out = 4.0 * I->out_count / 50e3;
+    const double t_in = copy_in_us(E, I), t_out = 4.0 * I->out_count / 50e3;
     double t_k = 0;
-    for (int t = 0; t < I->nsteps; t++) {
-        const step *s = &I->steps[t];
-        double us = (double)s->out_pixels * s->out_C * esize_of(s->dtype) * 2 / 4.5e6;
-        if (s->kind == ST_CONV) {
-            const thb_conv_desc *d = &s->conv;
-            const double f = 2.0 * d->N * d->oH * d->oW * (double)d->Cout * d->Cin * d->kH * d->kW / rate;
-            if (f > us) us = f;
-        }
-        t_k += us;
-    }
-    const double fixed = I->nsteps * 5.0;
+    for (int t = 0; t < I->nsteps; t++) t_k += model_us(&I->steps[t]);
+    const double fixed = I->nsteps * 12.0;
     double best = 0;
     for (unsigned c = 0; c < sizeof(sub_batch_cuts) / sizeof(sub_batch_cuts[0]); c++) {
         const unsigned char *cut = sub_batch_cuts[c];
@@ -2131,6 +2263,7 @@ static void choose_sub_batches(thb_engine *E)
             out = (k > out ? k : out) + f * t_out;
         } while (cut[++S] < 16);
         if (!ok || S > I->slice_n) continue;
+        if (c == 0 && I->slices) out -= I->hidden_us;
         if (c == 0 || out < 0.97 * best) {
             best = out;
             p->chunks = S;
@@ -2152,7 +2285,7 @@ static int plan_build(thb_engine *E)
     for (int g = 0; g < G; g++) {
         int off, n;
         thb_slice_batch(N, G, g, &off, &n);
-        if (instance_build(E, &E->cur->inst[g], dev0 + g, off, n)) return -1;
+        if (instance_build(E, &E->cur->inst[g], dev0 + g, off, n, 1)) return -1;
     }
     /* gather target: GPU 0 holds the whole result when peer copies are usable */
     if (G > 1 && E->cur->peer_gather) {
@@ -2209,7 +2342,7 @@ static int pipe_build(thb_engine *E, int S)
                 n = (sn * cut[c + 1] + 8) / 16 - off;
             } else
                 thb_slice_sub_batches(E->cur->inst[g].slice_n, S, c, &off, &n);
-            if (instance_build(E, &E->cur->pipe[g * S + c], E->cur->inst[g].device, E->cur->inst[g].slice_off + off, n)) return -1;
+            if (instance_build(E, &E->cur->pipe[g * S + c], E->cur->inst[g].device, E->cur->inst[g].slice_off + off, n, 0)) return -1;
         }
     E->cur->pipe_built = G * S;
     E->cur->pipe_chunks = S;
@@ -2260,37 +2393,42 @@ static int lowp_input_range(thb_engine *E, instance *set, int G, int has_x, int 
     return 0;
 }
 
-/* The boundary kernel in: the staged input (I->d_in: NCHW fp32, or I->d_img: HWC bytes) -> the engine's layout and type. */
-static int boundary_in(thb_engine *E, instance *I, int has_x, int inplace, int cp, int bgr, int C, int H, int W,
+/* The boundary kernel in: images [img0, img0 + n) of the staged input (I->d_in: NCHW fp32, or I->d_img: HWC bytes) -> the
+ * engine's layout and type. */
+static int boundary_in(thb_engine *E, instance *I, int img0, int n, int has_x, int inplace, int cp, int bgr, int C, int H, int W,
                        const float *mean, const float *std, float q_sub, float q_mult)
 {
     int rc;
-    void *in_ptr = bufptr(I, I->in_val.buf, 0, E->dtype);
+    const value *iv = &I->in_val;
+    const size_t stored = (size_t)iv->s.H * (iv->row_pitch ? iv->row_pitch : iv->s.W) * iv->ld; /* elements of an image */
+    void *in_ptr = (char *)bufptr(I, iv->buf, 0, E->dtype) + img0 * stored * esize_of(E->dtype);
+    float *d_in = I->d_in + (size_t)img0 * C * H * W;
+    const unsigned char *d_img = I->d_img + (size_t)img0 * H * W * cp;
     if (has_x && I->input_neigh)
-        rc = thb_preprocess_neigh_u8(I->d_in, inplace ? I->d_in : 0, I->slice_n, H, W, mean, std, in_ptr, I->in_val.ld, q_sub, q_mult,
+        rc = thb_preprocess_neigh_u8(d_in, inplace ? d_in : 0, n, H, W, mean, std, in_ptr, I->in_val.ld, q_sub, q_mult,
                                      I->stream);
     else if (has_x && I->input_s2d && E->dtype == THB_U8)
-        rc = thb_preprocess_s2d_u8(I->d_in, inplace ? I->d_in : 0, I->slice_n, C, H, W, mean, std, in_ptr, I->in_val.ld, q_sub,
+        rc = thb_preprocess_s2d_u8(d_in, inplace ? d_in : 0, n, C, H, W, mean, std, in_ptr, I->in_val.ld, q_sub,
                                    q_mult, I->stream);
     else if (has_x && I->input_s2d)
-        rc = thb_preprocess_s2d_padded(I->d_in, inplace ? I->d_in : 0, I->slice_n, C, H, W, mean, std, E->dtype, in_ptr,
+        rc = thb_preprocess_s2d_padded(d_in, inplace ? d_in : 0, n, C, H, W, mean, std, E->dtype, in_ptr,
                                        I->in_val.ld, I->in_val.row_pitch ? I->in_val.row_pitch : W / 2,
                                        I->in_val.pad_left, I->stream);
     else if (has_x)
-        rc = thb_preprocess(I->d_in, inplace ? I->d_in : 0, I->slice_n, C, H, W, mean, std, E->dtype, in_ptr, I->in_val.ld,
+        rc = thb_preprocess(d_in, inplace ? d_in : 0, n, C, H, W, mean, std, E->dtype, in_ptr, I->in_val.ld,
                             q_sub, q_mult, I->stream);
     else if (cp == 2) /* one YUYV frame (THProcessYUYV) */
         rc = E->dtype == THB_U8 ? THB_ERR_UNSUPPORTED
-                                : thb_preprocess_yuyv(I->d_img, H, W, mean, std, E->dtype, in_ptr, I->in_val.ld, I->stream);
+                                : thb_preprocess_yuyv(d_img, H, W, mean, std, E->dtype, in_ptr, I->in_val.ld, I->stream);
     else if (E->dtype == THB_U8) {
-        rc = thb_preprocess_images_lowp(I->d_img, I->slice_n, H, W, W * cp, bgr, mean, std, in_ptr, I->in_val.ld, &q_sub,
+        rc = thb_preprocess_images_lowp(d_img, n, H, W, W * cp, bgr, mean, std, in_ptr, I->in_val.ld, &q_sub,
                                         &q_mult, I->stream);
         set_dynamic_quant(I, q_sub, q_mult);
     } else if (I->input_s2d)
-        rc = thb_preprocess_images_s2d(I->d_img, I->slice_n, H, W, W * cp, bgr, mean, std, E->dtype, in_ptr, I->in_val.ld,
+        rc = thb_preprocess_images_s2d(d_img, n, H, W, W * cp, bgr, mean, std, E->dtype, in_ptr, I->in_val.ld,
                                        I->in_val.row_pitch ? I->in_val.row_pitch : W / 2, I->in_val.pad_left, I->stream);
     else
-        rc = thb_preprocess_images(I->d_img, I->slice_n, H, W, W * cp, cp, bgr, mean, std, E->dtype, in_ptr,
+        rc = thb_preprocess_images(d_img, n, H, W, W * cp, cp, bgr, mean, std, E->dtype, in_ptr,
                                    I->in_val.ld, I->stream);
     if (rc) { thb_set_error("preprocess launch failed: %s", thb_last_cuda_error()); return -1; }
     return 0;
@@ -2313,7 +2451,7 @@ static int boundary_out(thb_engine *E, instance *I, float *dst)
 static int device_forward(thb_engine *E, instance *I, int has_x, int inplace, int cp, int bgr, int C, int H, int W,
                           const float *mean, const float *std, float q_sub, float q_mult, float *writeback, float *dst)
 {
-    if (boundary_in(E, I, has_x, inplace, cp, bgr, C, H, W, mean, std, q_sub, q_mult)) return -1;
+    if (boundary_in(E, I, 0, I->slice_n, has_x, inplace, cp, bgr, C, H, W, mean, std, q_sub, q_mult)) return -1;
     if (writeback) {
         /* the normalised values go back to the caller on a stream of their own: the link is full duplex and the forward does
          * not wait for them (the caller does, before THProcessFloat returns) */
@@ -2327,7 +2465,7 @@ static int device_forward(thb_engine *E, instance *I, int has_x, int inplace, in
         I->wb_pending = 1;
     }
     CU(cudaEventRecord(I->ev0, I->stream));
-    if (run_steps(E, I)) return -1;
+    if (run_steps(E, I, 0)) return -1;
     return boundary_out(E, I, dst);
 }
 
@@ -2340,15 +2478,51 @@ static int host_is_pageable(const void *p)
     return a.type == cudaMemoryTypeUnregistered;
 }
 
-/* host-to-host copy; from a quarter of a megabyte on by all the host threads OpenMP gives this process */
+/* Copy into the pinned staging buffer past the caches.  The device reads the buffer next and the host never does: lines left
+ * dirty in sixteen cores' caches have to be snooped out of them, at half the link's rate (38.5 MB staged and copied to the
+ * device, eight pieces: 1.00 ms with memcpy, 0.83-0.88 ms with these stores; 0.71 ms is the copy alone). */
+static void copy_past_caches(void *dst, const void *src, size_t n)
+{
+#ifdef __SSE2__
+    char *d = dst;
+    const char *s = src;
+    const size_t head = (64 - ((size_t)d & 63)) & 63;
+    if (n >= 256) {
+        memcpy(d, s, head);
+        d += head; s += head; n -= head;
+        for (; n >= 64; n -= 64, d += 64, s += 64) {
+            const __m128i a = _mm_loadu_si128((const __m128i *)s), b = _mm_loadu_si128((const __m128i *)(s + 16));
+            const __m128i c = _mm_loadu_si128((const __m128i *)(s + 32)), e = _mm_loadu_si128((const __m128i *)(s + 48));
+            _mm_stream_si128((__m128i *)d, a);
+            _mm_stream_si128((__m128i *)(d + 16), b);
+            _mm_stream_si128((__m128i *)(d + 32), c);
+            _mm_stream_si128((__m128i *)(d + 48), e);
+        }
+        _mm_sfence();
+    }
+    memcpy(d, s, n);
+#else
+    memcpy(dst, src, n);
+#endif
+}
+
+/* Threads that fill the staging buffer: eight already keep ahead of the link, and more of them disturb the thread that
+ * issues the copies and launches (OMP_NUM_THREADS bounds them too). */
+static int stage_threads(void)
+{
+    const int n = omp_get_max_threads();
+    return n > 8 ? 8 : n;
+}
+
+/* host-to-host copy; from a quarter of a megabyte on by several threads */
 static void parallel_copy(void *dst, const void *src, size_t bytes)
 {
     const size_t blk = (size_t)128 << 10;
     const long nb = (long)((bytes + blk - 1) / blk);
-#pragma omp parallel for schedule(static) if (nb > 2)
+#pragma omp parallel for schedule(static) if (nb > 2) num_threads(stage_threads())
     for (long b = 0; b < nb; b++) {
         const size_t o = (size_t)b * blk;
-        memcpy((char *)dst + o, (const char *)src + o, bytes - o < blk ? bytes - o : blk);
+        copy_past_caches((char *)dst + o, (const char *)src + o, bytes - o < blk ? bytes - o : blk);
     }
 }
 
@@ -2359,14 +2533,14 @@ static void stage_images(unsigned char *dst, unsigned char *const *images, int n
     const int rows = row >= ((size_t)64 << 10) ? 1 : (int)(((size_t)64 << 10) / row);
     const int per = (H + rows - 1) / rows;
     const long items = (long)n * per;
-#pragma omp parallel for schedule(static) if (items > 4)
+#pragma omp parallel for schedule(static) if (items > 4) num_threads(stage_threads())
     for (long t = 0; t < items; t++) {
         const int i = (int)(t / per), r0 = (int)(t % per) * rows, r1 = r0 + rows < H ? r0 + rows : H;
         unsigned char *d = dst + ((size_t)i * H + r0) * row;
         const unsigned char *s = images[i] + (size_t)r0 * stride;
-        if (stride == row) memcpy(d, s, (size_t)(r1 - r0) * row);
+        if (stride == row) copy_past_caches(d, s, (size_t)(r1 - r0) * row);
         else
-            for (int r = r0; r < r1; r++, d += row, s += stride) memcpy(d, s, row);
+            for (int r = r0; r < r1; r++, d += row, s += stride) copy_past_caches(d, s, row);
     }
 }
 
@@ -2377,24 +2551,94 @@ static void stage_images(unsigned char *dst, unsigned char *const *images, int n
  * device. */
 static void stage_planes_normalised(float *dst, float *src, long p0, long p1, int C, long HW, const float *mean, const float *std)
 {
-#pragma omp parallel for schedule(static) if ((p1 - p0) * HW > 65536)
+#pragma omp parallel for schedule(static) if ((p1 - p0) * HW > 65536) num_threads(stage_threads())
     for (long p = p0; p < p1; p++) {
         const int c = (int)(p % C);
         float *s = src + p * HW, *d = dst + p * HW;
         if (c < 3) {
             const float m = mean[c], sd = std[c];
-            for (long i = 0; i < HW; i++) {
+            long i = 0;
+#ifdef __SSE2__
+            const __m128 vm = _mm_set1_ps(m), vs = _mm_set1_ps(sd);
+            if (((size_t)d & 15) == 0)
+                for (; i + 4 <= HW; i += 4) {
+                    const __m128 v = _mm_div_ps(_mm_sub_ps(_mm_loadu_ps(s + i), vm), vs);
+                    _mm_storeu_ps(s + i, v);
+                    _mm_stream_ps(d + i, v);
+                }
+            _mm_sfence();
+#endif
+            for (; i < HW; i++) {
                 const float v = (s[i] - m) / sd;
                 s[i] = v;
                 d[i] = v;
             }
         } else
-            memcpy(d, s, (size_t)HW * sizeof(float));
+            copy_past_caches(d, s, (size_t)HW * sizeof(float));
     }
 }
 
 /* bytes staged per copy to the device, and up to which size a result is written to the host by the kernel that makes it */
 static const size_t STAGE_PIECE = (size_t)4 << 20, DIRECT_RESULT_BYTES = (size_t)2 << 20;
+
+typedef struct {
+    float *x;               /* NCHW floats, or */
+    unsigned char **images; /* HWC bytes */
+    size_t stride;
+    int cp, C, H, W;
+    int staged;    /* by way of the engine's pinned buffer */
+    int host_norm; /* normalised in place on the way, with these statistics */
+    const float *mean, *std;
+} input_batch;
+
+/* Images [i0, i0 + cnt) of an instance's slice to its input buffer, by copies on stream `st`. */
+static int send_images(thb_engine *E, instance *I, const input_batch *in, int i0, int cnt, cudaStream_t st)
+{
+    const long HW = (long)in->H * in->W;
+    const size_t first = (size_t)(I->slice_off + i0);
+    if (in->x) {
+        const long C = in->C, planes = cnt * C;
+        float *dst = I->d_in + (size_t)i0 * C * HW, *xs = in->x + first * C * HW, *stage = E->h_stage + first * C * HW;
+        if (!in->staged) {
+            CU(cudaMemcpyAsync(dst, xs, (size_t)planes * HW * sizeof(float), cudaMemcpyHostToDevice, st));
+            return 0;
+        }
+        /* in pieces of whole planes: the copy to the device of one piece runs while the host threads fill the next */
+        long per_piece = (long)(STAGE_PIECE / sizeof(float)) / HW;
+        if (per_piece < 1) per_piece = 1;
+        for (long p0 = 0; p0 < planes; p0 += per_piece) {
+            const long p1 = p0 + per_piece < planes ? p0 + per_piece : planes;
+            const size_t o = (size_t)p0 * HW, n = (size_t)(p1 - p0) * HW;
+            if (in->host_norm) stage_planes_normalised(stage, xs, p0, p1, in->C, HW, in->mean, in->std);
+            else parallel_copy(stage + o, xs + o, n * sizeof(float));
+            CU(cudaMemcpyAsync(dst + o, stage + o, n * sizeof(float), cudaMemcpyHostToDevice, st));
+        }
+        return 0;
+    }
+    const size_t row = (size_t)in->W * in->cp, img_bytes = in->H * row;
+    unsigned char *dst = I->d_img + i0 * img_bytes, **images = in->images + first;
+    if (in->staged) {
+        unsigned char *stage = (unsigned char *)E->h_stage + first * img_bytes;
+        int per_piece = (int)(STAGE_PIECE / img_bytes);
+        if (per_piece < 1) per_piece = 1;
+        for (int n = 0; n < cnt; n += per_piece) {
+            const int k = cnt - n < per_piece ? cnt - n : per_piece;
+            stage_images(stage + n * img_bytes, images + n, k, in->H, row, in->stride);
+            CU(cudaMemcpyAsync(dst + n * img_bytes, stage + n * img_bytes, k * img_bytes, cudaMemcpyHostToDevice, st));
+        }
+    } else if (in->stride == row) {
+        /* pinned, tightly packed rows: one copy per run of images that also follow one another in host memory */
+        for (int n = 0; n < cnt;) {
+            int run = 1;
+            while (n + run < cnt && images[n + run] == images[n + run - 1] + img_bytes) run++;
+            CU(cudaMemcpyAsync(dst + n * img_bytes, images[n], run * img_bytes, cudaMemcpyHostToDevice, st));
+            n += run;
+        }
+    } else
+        for (int n = 0; n < cnt; n++)
+            CU(cudaMemcpy2DAsync(dst + n * img_bytes, row, images[n], in->stride, row, in->H, cudaMemcpyHostToDevice, st));
+    return 0;
+}
 
 int thb_engine_forward(thb_engine *E, float *x, unsigned char **images, int stride, int bgr, int cp, int N, int C, int H,
                        int W, int rank, const float *mean, const float *std, int inplace, thb_result *res)
@@ -2455,6 +2699,7 @@ int thb_engine_forward(thb_engine *E, float *x, unsigned char **images, int stri
     const float *host_mean = mean, *host_std = std;
     const int host_norm = staged && x && inplace;
     if (host_norm) { mean = zero3; std = one3; inplace = 0; }
+    const input_batch src = {x, images, (size_t)stride, cp, C, H, W, staged, host_norm, host_mean, host_std};
     /* what the device-resident timing loop needs to repeat this forward from the staged input */
     E->last_has_x = x != 0; E->last_cp = cp; E->last_bgr = bgr;
     for (int k = 0; k < 3; k++) { E->last_mean[k] = mean[k]; E->last_std[k] = std[k]; }
@@ -2473,60 +2718,30 @@ int thb_engine_forward(thb_engine *E, float *x, unsigned char **images, int stri
         for (int g = 0; g < G; g++) {
             instance *I = &set[g];
             CU(cudaSetDevice(I->device));
+            const int sliced = S == 1 && I->slices && !two_phase && !inplace && !th_profile && !th_minmax;
             if (phase == 0) {
-                /* stage the input slice */
-                if (x) {
-                    const size_t bytes = (size_t)I->slice_n * img_elems * sizeof(float);
-                    const float *src = x + (size_t)I->slice_off * img_elems;
-                    if (staged) {
-                        /* in pieces of whole planes: the copy to the device of one piece runs while the host threads fill the next */
-                        float *st = E->h_stage + (size_t)I->slice_off * img_elems;
-                        float *xs = x + (size_t)I->slice_off * img_elems;
-                        const long HW = (long)H * W, planes = (long)I->slice_n * C;
-                        long per_piece = (long)(STAGE_PIECE / sizeof(float)) / HW;
-                        if (per_piece < 1) per_piece = 1;
-                        for (long p0 = 0; p0 < planes; p0 += per_piece) {
-                            const long p1 = p0 + per_piece < planes ? p0 + per_piece : planes;
-                            const size_t o = (size_t)p0 * HW, cnt = (size_t)(p1 - p0) * HW;
-                            if (host_norm) stage_planes_normalised(st, xs, p0, p1, C, HW, host_mean, host_std);
-                            else parallel_copy(st + o, xs + o, cnt * sizeof(float));
-                            CU(cudaMemcpyAsync(I->d_in + o, st + o, cnt * sizeof(float), cudaMemcpyHostToDevice, I->stream));
-                        }
-                    } else
-                        CU(cudaMemcpyAsync(I->d_in, src, bytes, cudaMemcpyHostToDevice, I->stream));
-                } else if (staged) {
-                    const size_t row = (size_t)W * cp, img_bytes = (size_t)H * row;
-                    unsigned char *st = (unsigned char *)E->h_stage + (size_t)I->slice_off * img_bytes;
-                    int per_piece = (int)(STAGE_PIECE / img_bytes);
-                    if (per_piece < 1) per_piece = 1;
-                    for (int n = 0; n < I->slice_n; n += per_piece) {
-                        const int cnt = I->slice_n - n < per_piece ? I->slice_n - n : per_piece;
-                        stage_images(st + (size_t)n * img_bytes, images + I->slice_off + n, cnt, H, row, stride);
-                        CU(cudaMemcpyAsync(I->d_img + (size_t)n * img_bytes, st + (size_t)n * img_bytes, (size_t)cnt * img_bytes,
-                                           cudaMemcpyHostToDevice, I->stream));
+                if (sliced) {
+                    for (int c = 0; c < I->slices; c++) {
+                        int i0, cnt;
+                        slice_part(I, c, &i0, &cnt);
+                        if (send_images(E, I, &src, i0, cnt, I->copy_stream)) return -1;
+                        CU(cudaEventRecord(I->ev_slice, I->copy_stream));
+                        CU(cudaStreamWaitEvent(I->stream, I->ev_slice, 0));
+                        if (boundary_in(E, I, i0, cnt, x != 0, 0, cp, bgr, C, H, W, mean, std, q_sub, q_mult)) return -1;
+                        if (c == 0) CU(cudaEventRecord(I->ev0, I->stream));
+                        for (int t = 0; t < I->prefix; t++)
+                            if (exec_step(I, t, i0, cnt)) return -1;
                     }
-                } else if ((size_t)stride == (size_t)W * cp) {
-                    /* pinned, tightly packed rows: one copy per run of images that also follow one another in host memory */
-                    const size_t img_bytes = (size_t)H * W * cp;
-                    for (int n = 0; n < I->slice_n;) {
-                        int run = 1;
-                        while (n + run < I->slice_n && images[I->slice_off + n + run] == images[I->slice_off + n + run - 1] + img_bytes) run++;
-                        CU(cudaMemcpyAsync(I->d_img + (size_t)n * img_bytes, images[I->slice_off + n], (size_t)run * img_bytes,
-                                           cudaMemcpyHostToDevice, I->stream));
-                        n += run;
-                    }
-                } else {
-                    for (int n = 0; n < I->slice_n; n++)
-                        CU(cudaMemcpy2DAsync(I->d_img + (size_t)n * H * W * cp, (size_t)W * cp, images[I->slice_off + n], stride,
-                                             (size_t)W * cp, H, cudaMemcpyHostToDevice, I->stream));
-                }
+                } else if (send_images(E, I, &src, 0, I->slice_n, I->stream)) return -1;
                 if (two_phase) continue;
             }
             long off = 0;
             for (int k = 0; k < g; k++) off += set[k].out_count;
             float *dst = gather && I->device == dev0 ? gather + off : direct ? E->h_out + off : I->d_out;
-            if (device_forward(E, I, x != 0, inplace, cp, bgr, C, H, W, mean, std, q_sub, q_mult,
-                               x && inplace ? x + (size_t)I->slice_off * img_elems : 0, dst)) return -1;
+            if (sliced) {
+                if (run_steps(E, I, I->prefix) || boundary_out(E, I, dst)) return -1;
+            } else if (device_forward(E, I, x != 0, inplace, cp, bgr, C, H, W, mean, std, q_sub, q_mult,
+                                      x && inplace ? x + (size_t)I->slice_off * img_elems : 0, dst)) return -1;
             CU(cudaEventRecord(I->ev1, I->stream));
             if (gather) {
                 if (I->device != dev0)
