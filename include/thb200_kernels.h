@@ -136,6 +136,11 @@ int thb_conv_make_tmap(const thb_conv_desc *d, thb_tmap *out);
 int thb_conv_fwd(const thb_conv_desc *d, const void *x, void *y, thb_stream s);
 /* the split count that suits a convolution's tile count (1: none) and the scratch bytes it needs; THB200_NO_SPLITK=1: always 1 */
 int thb_conv_splitk_plan(const thb_conv_desc *d, size_t *scratch_bytes);
+/* The other way to share a reduction (F16 / BF16): with splits = 2, 4 or 8 and no splitk_scratch the S CTAs of a cluster work on
+ * one tile and add their parts through distributed shared memory, in rank order, in the same launch.  thb_conv_few_splits: the
+ * split that suits this tile count (1: none); thb_conv_few_supported: the kernel of few tiles takes this convolution. */
+int thb_conv_few_splits(const thb_conv_desc *d);
+int thb_conv_few_supported(const thb_conv_desc *d);
 
 /* Convolution + epilogue as above (no residual) + max pooling with a pk x pk window (2 or 3), stride 2 and padding ppad
  * in ONE launch: the convolution's own output is never written, only the [N][pH][pW][y_ld] pooled tensor.  Replaces

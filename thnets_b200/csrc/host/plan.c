@@ -984,6 +984,15 @@ static int plan_gemm_group(planner *P, int i)
             thb_conv_geometry(d);
         }
     }
+    if (!want_split && pool < 0 && P->I->slice_n > 0 && is.N == P->I->slice_n && (dtype == THB_F16 || dtype == THB_BF16)) {
+        /* Few tiles: the CTAs of a cluster share each tile's reduction.  The split follows from the batch of the whole call, so
+         * that a GPU's slice of it, or a sub-batch, adds its partial sums in the same order as the whole batch on one GPU. */
+        thb_conv_desc whole = *d;
+        whole.N = E->cur->N;
+        whole.out_ld = ru(d->Cout, al);
+        d->splits = thb_conv_few_splits(&whole);
+        if (d->splits < 2) d->splits = 0;
+    }
     if (want_split && pool < 0 && dual_conv < 0 && (dtype == THB_F16 || dtype == THB_BF16) && !thb_conv_patch_supported(d)) {
         /* a launch of few tiles: several CTAs share each tile's reduction, through an fp32 scratch that lives for this launch */
         size_t sk_bytes = 0;

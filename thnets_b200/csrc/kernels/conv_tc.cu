@@ -25,6 +25,7 @@
 // No im2col buffer exists anywhere.  Every wait is bounded: a wait that runs out records a code in
 // *status and the CTA drains and exits.
 #include "common.cuh"
+#include "conv_maps.cuh"
 #include <cuda.h>
 #include <string.h>
 #include <stdio.h>
@@ -1264,7 +1265,7 @@ __global__ void __launch_bounds__(256) splitk_finish_kernel(const ConvTcParams p
 // Diagnostic launcher switches (THB200_* environment variables), read ONCE: a launch costs no getenv call.
 // thb_conv_reload_knobs() re-reads them (the tests change them between cases).  -1 = not set.
 struct ConvKnobs {
-    int pair_min_kb, u8_fast, reverse, epi_groups, epi_bufs, pdl, conv_l1, half_taps, a_tma, test_withhold;
+    int pair_min_kb, u8_fast, reverse, epi_groups, epi_bufs, pdl, conv_l1, half_taps, a_tma, test_withhold, few_tiles, few_stages;
     long pair_min_units;
     long long wait_limit;
 };
@@ -1289,6 +1290,8 @@ void read_knobs()
     g_knobs.half_taps = env_int("THB200_HALF_TAPS", -1);
     g_knobs.a_tma = env_int("THB200_A_TMA", -1);
     g_knobs.test_withhold = env_int("THB200_TEST_WITHHOLD", 0);
+    g_knobs.few_tiles = env_int("THB200_FEW_TILES", -1);
+    g_knobs.few_stages = env_int("THB200_FEW_STAGES", -1);
     const char *wl = getenv("THB200_WAIT_LIMIT_CYCLES");
     g_knobs.wait_limit = wl && atoll(wl) > 0 ? atoll(wl) : 4000000000ll;
     g_knobs_read = true;
@@ -1569,39 +1572,63 @@ const CUtensorMap *activation_tmap(const thb_conv_desc *d, const void *x, int mo
     return &e.map;
 }
 
-// Descriptor of the packed weights read in boxes 64 bytes wide (SWIZZLE_64B), for convolutions whose taps are 64 bytes.
-struct WHalfEntry {
+// Descriptor of the packed weights read in boxes of box_rows channels x 128 or 64 bytes (SWIZZLE_64B: convolutions whose taps
+// are 64 bytes).
+struct WBoxEntry {
     const void *w;
-    int ktot, cout_pad, bn, dtype;
+    int ktot, cout_pad, rows, bytes, dtype;
     alignas(64) CUtensorMap map;
 };
-const CUtensorMap *weights_half_tmap(const thb_conv_desc *d)
+const CUtensorMap *weights_box_tmap(const thb_conv_desc *d, int box_rows, int box_bytes)
 {
-    static WHalfEntry cache[256];
+    static WBoxEntry cache[512];
     static int used = 0, next = 0;
     for (int i = 0; i < used; i++) {
-        WHalfEntry &e = cache[i];
-        if (e.w == d->w && e.ktot == d->Ktot_pad && e.cout_pad == d->Cout_pad && e.bn == d->BN && e.dtype == d->dtype) return &e.map;
+        WBoxEntry &e = cache[i];
+        if (e.w == d->w && e.ktot == d->Ktot_pad && e.cout_pad == d->Cout_pad && e.rows == box_rows && e.bytes == box_bytes && e.dtype == d->dtype)
+            return &e.map;
     }
     encode_tiled_fn enc = get_encode_fn();
     if (!enc) return nullptr;
-    WHalfEntry &e = cache[used < 256 ? used++ : (next++ % 256)];
+    WBoxEntry &e = cache[used < 512 ? used++ : (next++ % 512)];
     e.w = nullptr;
     const int es = d->dtype == THB_U8 ? 1 : 2;
     CUtensorMapDataType t = d->dtype == THB_U8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8
                             : d->dtype == THB_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
     cuuint64_t dims[2] = {(cuuint64_t)d->Ktot_pad, (cuuint64_t)d->Cout_pad};
     cuuint64_t strides[1] = {(cuuint64_t)d->Ktot_pad * es};
-    cuuint32_t box[2] = {(cuuint32_t)(64 / es), (cuuint32_t)d->BN};
+    cuuint32_t box[2] = {(cuuint32_t)(box_bytes / es), (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
     if (enc(&e.map, t, 2, const_cast<void *>(d->w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            box_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return nullptr;
-    e.w = d->w; e.ktot = d->Ktot_pad; e.cout_pad = d->Cout_pad; e.bn = d->BN; e.dtype = d->dtype;
+    e.w = d->w; e.ktot = d->Ktot_pad; e.cout_pad = d->Cout_pad; e.rows = box_rows; e.bytes = box_bytes; e.dtype = d->dtype;
     return &e.map;
 }
 
 }  // namespace
+
+// upper corner of the im2col bounding box: representable, and leaving a box of at least one position
+static bool box_corner_ok(int upper, int dim_plus_pad) { return upper >= -128 && upper <= 127 && dim_plus_pad + upper >= 1; }
+// limits of a rank-4 im2col descriptor: box corners in [-128, 127], traversal strides up to 8, tap offsets below 256
+bool thb_im2col_ok(const thb_conv_desc *d)
+{
+    return d->dH <= 8 && d->dW <= 8 && d->padH <= 127 && d->padW <= 127 && d->kH <= 256 && d->kW <= 256 && d->oH >= 1 && d->oW >= 1 &&
+           box_corner_ok((d->oH - 1) * d->dH + 1 - d->H - d->padH, d->H + d->padH) &&
+           box_corner_ok((d->oW - 1) * d->dW + 1 - d->W - d->padW, d->W + d->padW);
+}
+const CUtensorMap *thb_matrix_tmap(const void *x, long rows, int cols, int ld, int dtype, int box_cols)
+{
+    return matrix_tmap(x, rows, cols, ld, dtype, box_cols);
+}
+const CUtensorMap *thb_activation_tmap(const thb_conv_desc *d, const void *x, int mode) { return activation_tmap(d, x, mode); }
+const CUtensorMap *thb_weights_tmap(const thb_conv_desc *d, int box_rows) { return weights_box_tmap(d, box_rows, 128); }
+ThbConvLaunch thb_conv_launch_knobs()
+{
+    const ConvKnobs &kn = knobs();
+    return {kn.pdl, kn.test_withhold, num_sms(), kn.a_tma, kn.few_tiles, kn.few_stages, kn.wait_limit};
+}
 
 extern "C" void thb_simt_reload_knobs(void);
 extern "C" void thb_conv_reload_knobs(void)
@@ -1632,9 +1659,6 @@ extern "C" int thb_conv_make_tmap(const thb_conv_desc *d, thb_tmap *out)
     }
     return THB_OK;
 }
-
-// upper corner of the im2col bounding box: representable, and leaving a box of at least one position
-static bool box_corner_ok(int upper, int dim_plus_pad) { return upper >= -128 && upper <= 127 && dim_plus_pad + upper >= 1; }
 
 extern "C" int thb_conv_padded_rows_supported(int dtype)
 {
@@ -1708,13 +1732,9 @@ extern "C" int thb_conv_fwd_tc(const thb_conv_desc *d, const void *x, void *y, t
     // a 1x1 stride-1 unpadded convolution (and every Linear) reads a plain [pixels][Cin] matrix: TMA loads it
     p.a_tma = d->kH == 1 && d->kW == 1 && d->dH == 1 && d->dW == 1 && d->padH == 0 && d->padW == 0 &&
               d->oH == d->H && d->oW == d->W;
-    // anything else whose taps are whole 128-byte channel slabs goes through im2col-mode TMA, within the limits of
-    // a rank-4 descriptor: box corners in [-128, 127], traversal strides up to 8, tap offsets below 256
+    // anything else whose taps are whole 128-byte channel slabs goes through im2col-mode TMA
     const int bke = 128 / es;
-    const bool im2col_ok = d->dH <= 8 && d->dW <= 8 && d->padH <= 127 && d->padW <= 127 &&
-                           d->kH <= 256 && d->kW <= 256 && d->oH >= 1 && d->oW >= 1 &&
-                           box_corner_ok((d->oH - 1) * d->dH + 1 - d->H - d->padH, d->H + d->padH) &&
-                           box_corner_ok((d->oW - 1) * d->dW + 1 - d->W - d->padW, d->W + d->padW);
+    const bool im2col_ok = thb_im2col_ok(d);
     if (!p.a_tma && im2col_ok && d->Cin_pad % bke == 0 && d->Ktot_pad == d->kH * d->kW * d->Cin_pad) p.a_tma = 2;
     // taps of 64 bytes (uint8 with 64 channels, 16-bit types with 32): half a K block; two taps per block, each as its own
     // 64-byte-wide copy
@@ -1756,7 +1776,7 @@ extern "C" int thb_conv_fwd_tc(const thb_conv_desc *d, const void *x, void *y, t
     }
     ConvTmaps maps = {&tm, ta, nullptr, nullptr};
     if (p.half) {
-        maps.w = weights_half_tmap(d);
+        maps.w = weights_box_tmap(d, d->BN, 64);
         if (!maps.w) return thb_note_launch(cudaErrorUnknown, "conv_tc: weight tensor map");
     }
     if (d->dtype != THB_U8 && d->BN >= 64) {
