@@ -202,6 +202,13 @@ int thb_preprocess_yuyv(const unsigned char *frame, int H, int W, const float *m
  * (F16 / BF16): THProcessImages feeding a stride-2 first convolution (thapi.c:20-46 arithmetic) */
 int thb_preprocess_images_s2d(const unsigned char *img, int N, int H, int W, int stride, int bgr, const float *mean3,
                               const float *std3, int dtype, void *y, int y_ld, int row_pitch, int pad_left, thb_stream s);
+/* Space-to-depth by f (2, 4, ...) of NCHW floats (bytes = 0) or HWC RGB bytes (bytes = 1), for a first convolution of stride f:
+ * channel (ph*f + pw)*C + c of stored pixel (bh, bw) is plane c of pixel (f*bh + ph, f*bw + pw); pixels beyond the image are
+ * zeros.  Rows row_pitch stored pixels apart behind pad_left zero ones; any side lengths, y_ld >= C*f*f (zeros behind).
+ * U8: q_sub, q_mult (host) are the quantisation of a float batch, or are set to the image loader's static one. */
+int thb_preprocess_s2d_any(const void *src, int bytes, float *x_inplace, int N, int C, int H, int W, int f, int stride, int bgr,
+                           const float *mean3, const float *std3, int dtype, void *y, int y_ld, int row_pitch, int pad_left,
+                           float *q_sub, float *q_mult, thb_stream s);
 /* u8 HWC RGB images -> quantised NHWC u8 with the static input range the lowp image loader derives from mean/std
  * (lowp/lowp_basic.c:82-131); returns that range as *q_sub, *q_mult (host) */
 int thb_preprocess_images_lowp(const unsigned char *img, int N, int H, int W, int stride, int bgr, const float *mean3,
@@ -276,6 +283,8 @@ int thb_max_unpool(int dtype, const void *v, int v_ld, const void *pool_in, int 
 
 /* per-pixel sum of the first C bytes (zero-point correction term of the u8 convolution) */
 int thb_u8_channel_sum(const void *x, long pixels, int C, int x_ld, int *csum, thb_stream s);
+/* the same for rows of W pixels stored row_pitch pixels apart behind pad_left padding pixels (0, 0: dense); csum stays dense */
+int thb_u8_channel_sum_rows(const void *x, long pixels, int C, int x_ld, int W, int row_pitch, int pad_left, int *csum, thb_stream s);
 /* channels-innermost -> plain NCHW flatten order of the same dtype (View feeding anything but a Linear) */
 int thb_to_nchw(int dtype, const void *x, int N, int H, int W, int C, int x_ld, void *y, thb_stream s);
 

@@ -151,7 +151,7 @@ typedef struct instance {
     double hidden_us; /* modelled gain */
     cudaStream_t copy_stream;
     cudaEvent_t ev_slice;
-    int input_s2d; /* the network input is staged space-to-depth for a stride-2 first convolution */
+    int input_s2d; /* the network input is staged space-to-depth by this factor, the stride of the first convolution (0: as it is) */
     int input_neigh; /* uint8 engine, 3x3 / stride 1 / pad 1 first convolution on a three-plane float batch: the boundary kernel
                       * stages every pixel's 27 quantised neighbours as the channels of that pixel (taps outside the image: the
                       * byte of 0.0), and the layer runs as a 1x1 convolution over them -- no gather, no border classes */
@@ -494,7 +494,7 @@ typedef struct {
     int bn, dual_conv, dual_bn, kind;
     float self_coef, res_coef; /* WS_DUAL */
     int permute_hw, ld;        /* WS_FLAT: positions per channel and stored channels of the flattened input */
-    int s2d_padH, s2d_padW;
+    int s2d, s2d_padH, s2d_padW;
 } wsource;
 
 /* The weights in the descriptor's [Cout][Cin][kH][kW] order; a new array, or the node's own (then *owned = 0). */
@@ -536,14 +536,14 @@ static float *weights_oihw(const thb_model *M, const thb_conv_desc *d, const wso
                 w[(size_t)o * Cin + (size_t)(k % ws->permute_hw) * ws->ld + k / ws->permute_hw] = src[(size_t)o * n->Cin + k];
         break;
     case WS_S2D:
-        /* W'[co][(ph*2 + pw)*Cin + c][dh][dw] = W[co][c][2*(dh - pad') + ph + pad][...] where that row exists */
+        /* W'[co][(ph*f + pw)*Cin + c][dh][dw] = W[co][c][f*(dh - pad') + ph + pad][...] where that row exists */
         for (int co = 0; co < n->Cout; co++)
             for (int c = 0; c < n->Cin; c++)
                 for (int r = 0; r < n->kH; r++)
                     for (int q = 0; q < n->kW; q++) {
-                        const int tr = r - n->padH + 2 * ws->s2d_padH, tq = q - n->padW + 2 * ws->s2d_padW; /* >= 0 */
-                        const int dh = tr / 2, ph = tr % 2, dw = tq / 2, pw = tq % 2;
-                        w[(((size_t)co * Cin + (ph * 2 + pw) * n->Cin + c) * kH + dh) * kW + dw] =
+                        const int f = ws->s2d, tr = r - n->padH + f * ws->s2d_padH, tq = q - n->padW + f * ws->s2d_padW; /* >= 0 */
+                        const int dh = tr / f, ph = tr % f, dw = tq / f, pw = tq % f;
+                        w[(((size_t)co * Cin + (ph * f + pw) * n->Cin + c) * kH + dh) * kW + dw] =
                             src[(((size_t)co * n->Cin + c) * n->kH + r) * n->kW + q];
                     }
         break;
@@ -587,7 +587,7 @@ static int conv_weights(planner *P, step *s, thb_conv_desc *d, const wsource *ws
 {
     thb_engine *E = P->E;
     const int dev = P->I->device, node = (int)(ws->n - P->M->nodes), u8 = E->dtype == THB_U8;
-    int key[BLOB_KEY] = {node, BL_CONV, ws->kind, ws->bn, ws->dual_conv, ws->dual_bn, ws->permute_hw, ws->ld, ws->s2d_padH * 16 + ws->s2d_padW,
+    int key[BLOB_KEY] = {node, BL_CONV, ws->kind, ws->bn, ws->dual_conv, ws->dual_bn, ws->permute_hw, ws->ld, (ws->s2d * 16 + ws->s2d_padH) * 16 + ws->s2d_padW,
                          d->Cout, d->Cin, d->kH, d->kW, d->Cin_pad, d->Ktot_pad, d->Cout_pad, d->cin1, d->in_row_pitch ? d->in_ld : 0};
     wblob *w = blob_find(E, dev, key);
     if (!w) {
@@ -646,13 +646,13 @@ static int plan_gemm_group(planner *P, int i)
     const int dtype = E->dtype, al = align_of(dtype);
     shape is = in->s, os = is;
     int is_linear = n->op == OP_LINEAR, is_deconv = n->op == OP_DECONV;
-    /* stride-2 first convolution on a space-to-depth input (see instance_build): rewritten as a stride-1 convolution
-     * over 4*Cin channels.  Input row 2*oh - pad + r is block row oh + floor((r - pad)/2), phase (r - pad) mod 2. */
-    const int s2d = I->input_s2d && n->in[0] == 0 && n->op == OP_CONV;
+    /* first convolution of stride f on a space-to-depth input (see instance_build): rewritten as a stride-1 convolution
+     * over f*f*Cin channels.  Input row f*oh - pad + r is block row oh + floor((r - pad)/f), phase (r - pad) mod f. */
+    const int s2d = n->in[0] == 0 && n->op == OP_CONV ? I->input_s2d : 0, s2d_f = s2d ? s2d : 1;
     const int pad16 = I->input_pad16 && n->in[0] == 0 && n->op == OP_CONV;  /* 16 stored channels, zeros behind the real ones */
     const int neigh = I->input_neigh && n->in[0] == 0 && n->op == OP_CONV;  /* 27 neighbours per pixel: a 1x1 convolution */
-    const int s2d_padH = (n->padH + 1) / 2, s2d_padW = (n->padW + 1) / 2;
-    const int s2d_kH = (n->kH - 1 - n->padH) / 2 + s2d_padH + 1, s2d_kW = (n->kW - 1 - n->padW) / 2 + s2d_padW + 1;
+    const int s2d_padH = (n->padH + s2d_f - 1) / s2d_f, s2d_padW = (n->padW + s2d_f - 1) / s2d_f;
+    const int s2d_kH = (n->kH - 1 - n->padH) / s2d_f + s2d_padH + 1, s2d_kW = (n->kW - 1 - n->padW) / s2d_f + s2d_padW + 1;
 
     /* ---- geometry ---- */
     int kH = n->kH, kW = n->kW, Cin = n->Cin, H = is.H, W = is.W, in_ld = in->ld, permute_hw = 0;
@@ -683,11 +683,12 @@ static int plan_gemm_group(planner *P, int i)
         Cin = 27;
         kH = kW = 1;
     } else if (s2d) {
-        /* the logical input is still [N, Cin, 2H', 2W']: output size from the original geometry */
+        /* the logical input is still [N, Cin, H, W]: output size from the original geometry */
         os.C = n->Cout;
-        os.H = conv_out(E->cur->H, n->kH, 2, n->padH);
-        os.W = conv_out(E->cur->W, n->kW, 2, n->padW);
-        Cin = 4 * n->Cin;
+        os.H = conv_out(E->cur->H, n->kH, s2d, n->padH);
+        os.W = conv_out(E->cur->W, n->kW, s2d, n->padW);
+        if (os.H < 1 || os.W < 1) { thb_set_error("Given input size: (%dx%dx%d). Output size is too small", n->Cin, E->cur->H, E->cur->W); return -1; }
+        Cin = s2d == 2 ? 4 * n->Cin : in->ld; /* (stride 4: every stored channel, the unused ones with zero weights) */
         kH = s2d_kH; kW = s2d_kW;
     } else {
         if (is.rank < 3) { thb_set_error("convolution needs a 3D or 4D input"); return -1; }
@@ -890,6 +891,7 @@ static int plan_gemm_group(planner *P, int i)
             step_in(cs, in);
             cs->in_ld[0] = in_ld;
             cs->pixels = (long)is.N * H * W; cs->C = Cin; cs->out_buf = csum_buf;
+            cs->W = W; cs->oW = in->row_pitch; cs->padW = in->pad_left;
             if (!is_linear) inw->csum_buf = csum_buf + 1;
         }
     }
@@ -910,7 +912,7 @@ static int plan_gemm_group(planner *P, int i)
     if (neigh) d->padH = d->padW = 0;
     d->self_coef = 1.f; d->res_coef = 0.f; d->relu_thr = -1;
     int Cp_out = ru(n->Cout, al);
-    wsource ws = {n, bn, dual_conv, dual_bn, WS_PLAIN, self_coef, res_coef, permute_hw, in->ld, s2d_padH, s2d_padW};
+    wsource ws = {n, bn, dual_conv, dual_bn, WS_PLAIN, self_coef, res_coef, permute_hw, in->ld, s2d, s2d_padH, s2d_padW};
     float *b_fold = 0; /* uint8: bias with the batch normalisation folded in (the weights: conv_weights) */
     const float *bias_eff = n->bias;
     if (dtype == THB_U8 && bn >= 0) {
@@ -1694,19 +1696,19 @@ static int instance_build(thb_engine *E, instance *I, int device, int slice_off,
 
     shape in = {slice_n, E->cur->C, E->cur->H, E->cur->W, E->cur->rank, 0, 0, 0, 0};
     {
-        /* a stride-2 convolution on very few channels as the only consumer of the float input: stage the input
-         * space-to-depth so that the gathered 16-byte chunks carry four times as many useful channels */
+        /* a convolution of stride 2 or 4 on very few channels as the only consumer of the input: stage the input space-to-depth,
+         * so that the copy engine can load it (16 channels a pixel in padded rows, or 64) instead of a gather of 16-byte chunks
+         * that are mostly padding */
         thb_node *c1 = M->nnodes > 1 ? &M->nodes[1] : 0;
         const char *off = getenv("THB200_NO_S2D"), *u8off = getenv("THB200_NO_S2D_U8");
-        I->input_s2d = c1 && c1->op == OP_CONV && c1->in[0] == 0 && P.uses[0] == 1 && c1->dH == 2 && c1->dW == 2 &&
-                       4 * E->cur->C <= 16 && c1->Cin == E->cur->C && E->cur->H % 2 == 0 && E->cur->W % 2 == 0 && E->cur->rank == 4 &&
-                       /* a float batch, or three-plane byte images (converted and regrouped by one kernel) in the 16-bit modes */
-                       (E->cur->cp == 0 || (E->cur->cp == 3 && E->dtype != THB_U8)) &&
+        const int f = c1 && c1->op == OP_CONV && c1->dH == c1->dW ? c1->dH : 0;
+        I->input_s2d = (f == 2 || (f == 4 && E->dtype != THB_U8)) && c1->in[0] == 0 && P.uses[0] == 1 && 4 * E->cur->C <= 16 &&
+                       c1->Cin == E->cur->C && (E->cur->cp == 0 || E->cur->cp == 3) &&
                        (E->dtype == THB_F16 || E->dtype == THB_BF16 || (E->dtype == THB_U8 && !(u8off && atoi(u8off)))) &&
                        c1->padH <= c1->kH - 1 && c1->padW <= c1->kW - 1 &&
                        !(E->honour_pads && (c1->pad2H != c1->padH || c1->pad2W != c1->padW || c1->dlH > 1 || c1->dlW > 1 || c1->autopad || c1->refl_pad)) &&
-                       !(off && atoi(off));
-        if (I->input_s2d) { in.C = 4 * E->cur->C; in.H = E->cur->H / 2; in.W = E->cur->W / 2; }
+                       !(off && atoi(off)) ? f : 0;
+        if (I->input_s2d) { in.C = f * f * E->cur->C; in.H = (E->cur->H + f - 1) / f; in.W = (E->cur->W + f - 1) / f; }
     }
     {
         /* A stride-1 convolution with at most 64 output channels on very few input channels (VGG, the segmentation net):
@@ -1738,15 +1740,20 @@ static int instance_build(thb_engine *E, instance *I, int device, int slice_off,
         I->nbufs--; /* re-create the buffer with 16 channels per pixel */
         v->buf = new_buf(&P, (size_t)in.N * in.H * in.W * v->ld * esize_of(E->dtype));
     }
-    if (I->input_s2d) {
-        /* When the rewritten convolution's kernel row fills one 128-byte K block, store the staged rows with their
-         * zero padding: one copy then fetches a whole kernel row of an output pixel (thb_conv_desc.in_row_pitch). */
+    if (I->input_s2d == 4) {
+        value *v = &P.val[0];
+        v->ld = 64; /* one 128-byte slab a pixel */
+        I->nbufs--;
+        v->buf = new_buf(&P, (size_t)in.N * in.H * in.W * v->ld * esize_of(E->dtype));
+    }
+    if (I->input_s2d == 2) {
+        /* When the rewritten convolution's kernel row fills one 128-byte K block (uint8: half of one), store the staged rows with
+         * their zero padding: one copy then fetches a whole kernel row of an output pixel (thb_conv_desc.in_row_pitch). */
         thb_node *c1 = &M->nodes[1];
         const int padW = (c1->padW + 1) / 2, kW = (c1->kW - 1 - c1->padW) / 2 + padW + 1;
         const char *off = getenv("THB200_NO_PADDED_ROWS");
         value *v = &P.val[0];
-        /* (16-bit types only: the uint8 loader and the channel-sum pass write and read dense rows) */
-        if (E->dtype != THB_U8 && kW * v->ld * esize_of(E->dtype) == 128 && thb_conv_padded_rows_supported(E->dtype) &&
+        if (kW * v->ld * esize_of(E->dtype) == (E->dtype == THB_U8 ? 64 : 128) && thb_conv_padded_rows_supported(E->dtype) &&
             !(off && atoi(off))) {
             v->pad_left = padW;
             v->row_pitch = (padW + in.W + kW - 1 + 3) & ~3;
@@ -1830,7 +1837,7 @@ static int exec_step(instance *I, int t, int img0, int cnt)
             break;
         case ST_CSUM: case ST_ZERO: {
             const long per = s->pixels / I->slice_n;
-            if (s->kind == ST_CSUM) x0 += (size_t)img0 * per * s->in_ld[0] * es;
+            if (s->kind == ST_CSUM) x0 += (size_t)img0 * (s->oW ? per / s->W * s->oW : per) * s->in_ld[0] * es;
             aux_off = sizeof(int) * (size_t)img0 * per;
             s->pixels = cnt * per;
             break;
@@ -1890,7 +1897,7 @@ static int exec_step(instance *I, int t, int img0, int cnt)
         if (s->pixels > 0 && cudaMemsetAsync((char *)bufptr(I, s->out_buf, 0, THB_U8) + aux_off, 0, sizeof(int) * (size_t)s->pixels, (cudaStream_t)st) != cudaSuccess) rc = -1;
         break;
     case ST_CSUM:
-        rc = thb_u8_channel_sum(x0, s->pixels, s->C, s->in_ld[0], (int *)((char *)bufptr(I, s->out_buf, 0, THB_U8) + aux_off), st);
+        rc = thb_u8_channel_sum_rows(x0, s->pixels, s->C, s->in_ld[0], s->W > 0 ? s->W : 1, s->oW, s->padW, (int *)((char *)bufptr(I, s->out_buf, 0, THB_U8) + aux_off), st);
         break;
     case ST_TO_NCHW:
         rc = thb_to_nchw(dt, x0, s->N, s->H, s->W, s->C, s->in_ld[0], y, st);
@@ -2413,16 +2420,18 @@ static int boundary_in(thb_engine *E, instance *I, int img0, int n, int has_x, i
     void *in_ptr = (char *)bufptr(I, iv->buf, 0, E->dtype) + img0 * stored * esize_of(E->dtype);
     float *d_in = I->d_in + (size_t)img0 * C * H * W;
     const unsigned char *d_img = I->d_img + (size_t)img0 * H * W * cp;
-    if (has_x && I->input_neigh)
+    const int f = I->input_s2d, W2 = f ? (W + f - 1) / f : 0, pitch = iv->row_pitch ? iv->row_pitch : W2;
+    /* (even sides and stride 2 in the 16-bit modes have kernels of their own) */
+    if (f && (E->dtype == THB_U8 || f != 2 || ((H | W) & 1))) {
+        rc = thb_preprocess_s2d_any(has_x ? (const void *)d_in : d_img, !has_x, inplace ? d_in : 0, n, C, H, W, f, W * cp, bgr, mean, std,
+                                    E->dtype, in_ptr, iv->ld, pitch, iv->pad_left, &q_sub, &q_mult, I->stream);
+        if (!has_x && E->dtype == THB_U8) set_dynamic_quant(I, q_sub, q_mult);
+    } else if (has_x && I->input_neigh)
         rc = thb_preprocess_neigh_u8(d_in, inplace ? d_in : 0, n, H, W, mean, std, in_ptr, I->in_val.ld, q_sub, q_mult,
                                      I->stream);
-    else if (has_x && I->input_s2d && E->dtype == THB_U8)
-        rc = thb_preprocess_s2d_u8(d_in, inplace ? d_in : 0, n, C, H, W, mean, std, in_ptr, I->in_val.ld, q_sub,
-                                   q_mult, I->stream);
-    else if (has_x && I->input_s2d)
-        rc = thb_preprocess_s2d_padded(d_in, inplace ? d_in : 0, n, C, H, W, mean, std, E->dtype, in_ptr,
-                                       I->in_val.ld, I->in_val.row_pitch ? I->in_val.row_pitch : W / 2,
-                                       I->in_val.pad_left, I->stream);
+    else if (has_x && f)
+        rc = thb_preprocess_s2d_padded(d_in, inplace ? d_in : 0, n, C, H, W, mean, std, E->dtype, in_ptr, iv->ld, pitch, iv->pad_left,
+                                       I->stream);
     else if (has_x)
         rc = thb_preprocess(d_in, inplace ? d_in : 0, n, C, H, W, mean, std, E->dtype, in_ptr, I->in_val.ld,
                             q_sub, q_mult, I->stream);
@@ -2433,9 +2442,8 @@ static int boundary_in(thb_engine *E, instance *I, int img0, int n, int has_x, i
         rc = thb_preprocess_images_lowp(d_img, n, H, W, W * cp, bgr, mean, std, in_ptr, I->in_val.ld, &q_sub,
                                         &q_mult, I->stream);
         set_dynamic_quant(I, q_sub, q_mult);
-    } else if (I->input_s2d)
-        rc = thb_preprocess_images_s2d(d_img, n, H, W, W * cp, bgr, mean, std, E->dtype, in_ptr, I->in_val.ld,
-                                       I->in_val.row_pitch ? I->in_val.row_pitch : W / 2, I->in_val.pad_left, I->stream);
+    } else if (f)
+        rc = thb_preprocess_images_s2d(d_img, n, H, W, W * cp, bgr, mean, std, E->dtype, in_ptr, iv->ld, pitch, iv->pad_left, I->stream);
     else
         rc = thb_preprocess_images(d_img, n, H, W, W * cp, cp, bgr, mean, std, E->dtype, in_ptr,
                                    I->in_val.ld, I->stream);

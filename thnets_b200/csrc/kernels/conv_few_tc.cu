@@ -447,8 +447,8 @@ int launch(const CUtensorMap *w, const CUtensorMap *a, const CUtensorMap *a2, co
 //   3x3 256->256 @14x14, 8 images, 52 tiles of 36          17.3 / 15.6 / 11.2 / 9.0 / 15.0
 //   3x3 128->128 @28x28, 8 images, 98 tiles of 18          12.9 / 10.0 /  8.7 / 14.1
 //   1x1 512->128 @28x28, 8 images, 98 tiles of 8            8.9 /  6.5 /  7.0
-// So: eight K blocks or more, at least two of them to a CTA, up to one CTA per SM -- two per SM where four K blocks stay,
-// but not in clusters of eight (ResNet-18 on 4 images: 193 us with those, 173 without).
+// So: eight K blocks or more, at least two of them to a CTA, up to one CTA per SM -- two per SM where four K blocks stay, but
+// not in clusters of eight.
 extern "C" int thb_conv_few_splits(const thb_conv_desc *d)
 {
     const ThbConvLaunch kn = thb_conv_launch_knobs();
@@ -521,8 +521,9 @@ extern "C" int thb_conv_few_fwd(const thb_conv_desc *d, const void *x, void *y, 
     if (!w || !a || !a2) return thb_note_launch(cudaErrorUnknown, "conv_few: tensor map");
     const int per = (p.nkb + p.splits - 1) / p.splits;
     const int ctas = ((p.P + BM - 1) / BM) * p.n_tiles * p.splits;
-    // stages: as many as let two CTAs onto an SM; one more where an SM gets one CTA at most (0.3 to 1 us of 6 to 10)
-    p.stages = kn.few_stages > 0 ? kn.few_stages : (p.splits > 1 ? 3 : 4) + (ctas <= kn.sms);
+    // stages: as many as fit the CTAs an SM gets.  Clusters always leave room for two CTAs to an SM, or a GPC holds too few of
+    // them at once (ResNet-18 on 4 images: 193 us with a fourth stage, 168 with three)
+    p.stages = kn.few_stages > 0 ? kn.few_stages : p.splits > 1 || ctas > 2 * kn.sms ? 3 : ctas > kn.sms ? 4 : 5;
     if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
     if (p.stages > per) p.stages = per;
     const int smem = 1024 + BAR_BYTES + (p.splits > 1 ? RECV_BYTES : 0) + p.stages * STAGE_BYTES;

@@ -1518,7 +1518,7 @@ const CUtensorMap *activation_tmap(const thb_conv_desc *d, const void *x, int mo
         return matrix_tmap(x, (long)d->N * d->H * d->W, d->Cin_pad, d->in_ld, d->dtype, d->dtype == THB_U8 ? 128 : 64);
     static ATmapEntry cache[512];
     static int used = 0, next = 0;
-    const int geom[8] = {d->kH, d->kW, d->dH, d->dW, d->padH, mode == 3 ? d->in_row_pitch : d->padW, d->oH, d->oW};
+    const int geom[8] = {d->kH, d->kW, d->dH, d->dW, d->padH, mode == 3 || mode == 5 ? d->in_row_pitch : d->padW, d->oH, d->oW};
     for (int i = 0; i < used; i++) {
         ATmapEntry &e = cache[i];
         if (e.x == x && e.mode == mode && e.N == d->N && e.H == d->H && e.W == d->W && e.cin_pad == d->Cin_pad &&
@@ -1541,12 +1541,12 @@ const CUtensorMap *activation_tmap(const thb_conv_desc *d, const void *x, int mo
                                  (cuuint64_t)d->H * d->W * d->in_ld * es};
         int lower[2] = {-d->padW, -d->padH};
         int upper[2] = {(d->oW - 1) * d->dW + 1 - d->W - d->padW, (d->oH - 1) * d->dH + 1 - d->H - d->padH};
-        if (mode == 3) {
-            // Rows stored with their zero padding, kW taps = 128 bytes, stride 1: "pixel" w of this tensor is the
-            // 128-byte window that starts at stored pixel w, i.e. the kW taps of output column w.  Windows overlap
+        if (mode == 3 || mode == 5) {
+            // Rows stored with their zero padding, kW taps = 128 bytes (mode 5: 64), stride 1: "pixel" w of this tensor is the
+            // window of that size that starts at stored pixel w, i.e. the kW taps of output column w.  Windows overlap
             // (the pixel stride is smaller than the window), there are oW of them per row, and no horizontal
             // padding is left for the copy engine to supply.
-            dims[0] = (cuuint64_t)(128 / es);
+            dims[0] = (cuuint64_t)((mode == 5 ? 64 : 128) / es);
             dims[1] = (cuuint64_t)d->oW;
             strides[1] = (cuuint64_t)d->in_row_pitch * d->in_ld * es;
             strides[2] = (cuuint64_t)d->H * d->in_row_pitch * d->in_ld * es;
@@ -1554,17 +1554,17 @@ const CUtensorMap *activation_tmap(const thb_conv_desc *d, const void *x, int mo
             upper[0] = 0;
         }
         cuuint32_t estr[4] = {1, (cuuint32_t)d->dW, (cuuint32_t)d->dH, 1};
-        // mode 4: a tap is 64 bytes of channels; the box is 64 bytes wide and lands as rows of 64 bytes with the 64-byte swizzle
-        if (enc(&e.map, t, 4, const_cast<void *>(x), dims, strides, lower, upper, (cuuint32_t)((mode == 4 ? 64 : 128) / es),
+        // modes 4 and 5: a tap (a row of taps) is 64 bytes of channels; the box is 64 bytes wide and lands as rows of 64 bytes with the 64-byte swizzle
+        if (enc(&e.map, t, 4, const_cast<void *>(x), dims, strides, lower, upper, (cuuint32_t)((mode >= 4 ? 64 : 128) / es),
                 (cuuint32_t)BM, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                mode == 4 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                mode >= 4 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return nullptr;
         // Drivers up to CUDA 13.1 encode im2col descriptors of tensors smaller than 128 KiB with a flag (bit 21 of
         // the second 64-bit word) that makes the load misbehave; CUTLASS clears it for those drivers, and so do we.
         int drv = 0;
         if (cudaDriverGetVersion(&drv) == cudaSuccess && drv <= 13010 &&
-            (size_t)d->N * d->H * (mode == 3 ? d->in_row_pitch : d->W) * d->in_ld * es < 131072)
+            (size_t)d->N * d->H * (mode == 3 || mode == 5 ? d->in_row_pitch : d->W) * d->in_ld * es < 131072)
             reinterpret_cast<uint64_t *>(&e.map)[1] &= ~(1ull << 21);
     }
     e.x = x; e.mode = mode; e.N = d->N; e.H = d->H; e.W = d->W; e.cin_pad = d->Cin_pad; e.in_ld = d->in_ld; e.dtype = d->dtype;
@@ -1758,10 +1758,17 @@ extern "C" int thb_conv_fwd_tc(const thb_conv_desc *d, const void *x, void *y, t
             p.slabs = 1;
             p.tma_kw = 1;
             p.tma_padw = 0;
+        } else if (im2col_ok && d->dW == 1 && d->kW * d->Cin_pad * 2 == bke && d->Ktot_pad == (d->kH * (bke / 2) + bke - 1) / bke * bke) {
+            // a kernel row of taps is 64 bytes: two rows to a K block, each its own copy (the uint8 space-to-depth first layer)
+            p.a_tma = 2;
+            p.half = 1;
+            p.ntaps = d->kH;
+            p.tma_kw = 1;
+            p.tma_padw = 0;
         }
     }
     if (p.half) {
-        tmap_mode = 4;
+        tmap_mode = d->in_row_pitch ? 5 : 4;
         p.slabs = 1;
         if (kn.half_taps == 0) p.half = 0, p.a_tma = 0;
     }

@@ -210,6 +210,67 @@ __global__ void preprocess_s2d_kernel(const float *x, float *x_inplace, int N, i
     }
 }
 
+// The same for any block size f (a first convolution of stride f), any plane count with C*f*f stored channels or fewer, and
+// image sides that f does not divide (the missing pixels are zeros, in uint8 the byte 0.0 quantises to, which the zero point
+// cancels).  One thread per stored 16-byte group; SRC: NCHW floats or HWC bytes.
+struct S2dArgs {
+    const void *src;
+    float *x_inplace;  // floats: where the normalised values go back to, or null
+    int N, C, H, W, f, stride, bgr;
+    float3 mean, std_;  // bytes: 1 / std
+    int y_ld, row_pitch, pad_left;
+    float q_mult, zr;   // uint8 floats
+    int3 q_sub;         // uint8 bytes (lowp_images.c)
+    float3 q_mul;
+    int q_zero;         // uint8: the byte of 0.0
+};
+template <typename T, bool BYTES>
+__global__ void preprocess_s2d_any_kernel(const S2dArgs a, T *y)
+{
+    constexpr int VN = Vec<T>::N;
+    const int H2 = (a.H + a.f - 1) / a.f, W2 = (a.W + a.f - 1) / a.f, groups = a.y_ld / VN;
+    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long pix = t / groups;
+    if (pix >= (long)a.N * H2 * a.row_pitch) return;
+    const int c0 = (int)(t - pix * groups) * VN;
+    const long n = pix / ((long)H2 * a.row_pitch);
+    const int rem = (int)(pix - n * (long)H2 * a.row_pitch), bh = rem / a.row_pitch, bw = rem - bh * a.row_pitch - a.pad_left;
+    const bool real = bw >= 0 && bw < W2;
+    const float m[3] = {a.mean.x, a.mean.y, a.mean.z}, sd[3] = {a.std_.x, a.std_.y, a.std_.z};
+    const int qs[3] = {a.q_sub.x, a.q_sub.y, a.q_sub.z};
+    const float qm[3] = {a.q_mul.x, a.q_mul.y, a.q_mul.z};
+    int blk = c0 / a.C, c = c0 - blk * a.C, ph = blk / a.f, pw = blk - ph * a.f;  // stepped, not divided, from here on
+    float v[VN];
+#pragma unroll
+    for (int i = 0; i < VN; i++) {
+        float val = 0.f;
+        if (real && ph < a.f) {
+            const int h = bh * a.f + ph, w = bw * a.f + pw;
+            if (h < a.H && w < a.W) {
+                if (BYTES) {
+                    const uint8_t *px = reinterpret_cast<const uint8_t *>(a.src) + ((size_t)n * a.H + h) * a.stride + (size_t)w * a.C;
+                    const float b = (float)px[a.bgr ? a.C - 1 - c : c];
+                    if (sizeof(T) == 1) val = (float)((int)roundf(__fmul_rn(b - (float)qs[c], qm[c])) & 255);
+                    else val = __fmul_rn(__fsub_rn(__fmul_rn(b, 0.003921568f), m[c]), sd[c]);
+                } else {
+                    const long idx = ((n * a.C + c) * a.H + h) * a.W + w;
+                    val = reinterpret_cast<const float *>(a.src)[idx];
+                    if (c < 3) val = __fdiv_rn(__fsub_rn(val, m[c]), sd[c]);
+                    if (a.x_inplace) a.x_inplace[idx] = val;
+                    if (sizeof(T) == 1) val = (float)(((int)(roundf(val * a.q_mult) - a.zr)) & 255);
+                }
+            } else if (sizeof(T) == 1)
+                val = (float)a.q_zero;
+        }
+        v[i] = val;
+        if (++c == a.C) {
+            c = 0;
+            if (++pw == a.f) { pw = 0; ph++; }
+        }
+    }
+    Vec<T>::store(y + pix * a.y_ld + c0, v);
+}
+
 // uint8 engine, 3x3 / stride 1 / pad 1 first convolution on a three-plane float batch: every pixel's 27 neighbours,
 // normalised and quantised as preprocess_kernel does, become the channels of that pixel of an [N][H][W][32] byte tensor
 // (channel (r*3 + s)*3 + c = plane c of pixel (h - 1 + r, w - 1 + s)); neighbours outside the image hold the byte that 0.0
@@ -779,14 +840,19 @@ __global__ void col2im_kernel(const T *cols, int N, int H, int W, int Cout, int 
 // G lanes per pixel (a power of two up to 32): neighbouring lanes read neighbouring 16-byte chunks, so a warp's load covers
 // whole pixels' contiguous bytes; bytes are summed four at a time (dp4a against ones) and the G partial sums by shuffles.
 template <int G>
-__global__ void u8_channel_sum_kernel(const uint8_t *x, long pixels, int C, int x_ld, int *csum)
+__global__ void u8_channel_sum_kernel(const uint8_t *x, long pixels, int C, int x_ld, int W, int row_pitch, int pad_left, int *csum)
 {
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const long pix = t / G;
     const int g = (int)(t % G);
     int s = 0;
     if (pix < pixels) {
-        const uint8_t *p = x + pix * x_ld;
+        long at = pix;
+        if (row_pitch) {  // rows stored with their padding
+            const long row = pix / W;
+            at = row * row_pitch + pad_left + (pix - row * W);
+        }
+        const uint8_t *p = x + at * x_ld;
         for (int c0 = g * 16; c0 < C; c0 += G * 16) {
             const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p + c0));
             uint32_t w[4] = {v.x, v.y, v.z, v.w};
@@ -834,6 +900,23 @@ __global__ void u8_channel_sum_wide_kernel(const uint8_t *x, int C, int x_ld, in
 }  // namespace
 
 // =================================================================================================
+// The static input range of the lowp image loader: its float expressions, in its order (lowp_basic.c:102-119).
+static void lowp_image_range(const float *mean3, const float *std3, float *q_sub, float *q_mult, int *sub, float *mul)
+{
+    float mn = 1e30f, mx = -1e30f, m;
+    for (int i = 0; i < 3; i++) {
+        if (-mean3[i] / std3[i] < mn) mn = -mean3[i] / std3[i];
+        if ((1 - mean3[i]) / std3[i] > mx) mx = (1 - mean3[i]) / std3[i];
+    }
+    m = (mx - mn) ? 255 / (mx - mn) : 0;
+    for (int i = 0; i < 3; i++) {
+        sub[i] = (int)roundf(255 * (mean3[i] + std3[i] * mn));
+        mul[i] = m / (255 * std3[i]);
+    }
+    *q_sub = mn;
+    *q_mult = m;
+}
+
 extern "C" {
 
 int thb_channel_align(int dtype) { return dtype == THB_F32 ? 4 : dtype == THB_U8 ? 16 : 8; }
@@ -933,26 +1016,50 @@ int thb_preprocess_images_lowp(const unsigned char *img, int N, int H, int W, in
                                const float *std3, void *y, int y_ld, float *q_sub, float *q_mult, thb_stream s)
 {
     if (y_ld % 16) return THB_ERR_ARG;
-    // the loader's float expressions, in its order (lowp_basic.c:102-119)
-    float mn = 1e30f, mx = -1e30f, m;
-    for (int i = 0; i < 3; i++) {
-        if (-mean3[i] / std3[i] < mn) mn = -mean3[i] / std3[i];
-        if ((1 - mean3[i]) / std3[i] > mx) mx = (1 - mean3[i]) / std3[i];
-    }
-    m = (mx - mn) ? 255 / (mx - mn) : 0;
     int sub[3];
     float mul[3];
-    for (int i = 0; i < 3; i++) {
-        sub[i] = (int)roundf(255 * (mean3[i] + std3[i] * mn));
-        mul[i] = m / (255 * std3[i]);
-    }
-    *q_sub = mn;
-    *q_mult = m;
+    lowp_image_range(mean3, std3, q_sub, q_mult, sub, mul);
     const long pix = (long)N * H * W;
     if (pix == 0) return THB_OK;
     preprocess_images_u8_kernel<<<nblocks(pix), 256, 0, (cudaStream_t)s>>>(img, N, H, W, stride, bgr, make_int3(sub[0], sub[1], sub[2]),
                                                                             make_float3(mul[0], mul[1], mul[2]), (uint8_t *)y, y_ld);
     return THB_LAUNCH_CHECK("preprocess_images_u8_kernel");
+}
+
+int thb_preprocess_s2d_any(const void *src, int bytes, float *x_inplace, int N, int C, int H, int W, int f, int stride, int bgr,
+                           const float *mean3, const float *std3, int dtype, void *y, int y_ld, int row_pitch, int pad_left,
+                           float *q_sub, float *q_mult, thb_stream s)
+{
+    if (f < 2 || C < 1 || (bytes && C != 3) || y_ld % thb_channel_align(dtype) || y_ld < C * f * f) return THB_ERR_ARG;
+    const int W2 = (W + f - 1) / f, H2 = (H + f - 1) / f;
+    if (pad_left < 0 || row_pitch < pad_left + W2) return THB_ERR_ARG;
+    S2dArgs a;
+    a.src = src; a.x_inplace = bytes ? nullptr : x_inplace;
+    a.N = N; a.C = C; a.H = H; a.W = W; a.f = f; a.stride = stride; a.bgr = bgr;
+    a.mean = make_float3(mean3[0], mean3[1], mean3[2]);
+    a.std_ = bytes ? make_float3(1 / std3[0], 1 / std3[1], 1 / std3[2]) : make_float3(std3[0], std3[1], std3[2]);
+    a.y_ld = y_ld; a.row_pitch = row_pitch; a.pad_left = pad_left;
+    a.q_mult = a.zr = 0; a.q_sub = make_int3(0, 0, 0); a.q_mul = make_float3(0, 0, 0); a.q_zero = 0;
+    if (dtype == THB_U8) {
+        if (bytes) {
+            int sub[3];
+            float mul[3];
+            lowp_image_range(mean3, std3, q_sub, q_mult, sub, mul);
+            a.q_sub = make_int3(sub[0], sub[1], sub[2]);
+            a.q_mul = make_float3(mul[0], mul[1], mul[2]);
+        }
+        a.q_mult = *q_mult;
+        a.zr = roundf(*q_sub * *q_mult);
+        a.q_zero = (int)-a.zr & 255;
+    }
+    const long total = (long)N * H2 * row_pitch * (y_ld / thb_channel_align(dtype));
+    if (total == 0) return THB_OK;
+    if (bytes) {
+        DISPATCH_ANY_DTYPE(dtype, (preprocess_s2d_any_kernel<T, true><<<nblocks(total), 256, 0, (cudaStream_t)s>>>(a, (T *)y)));
+    } else {
+        DISPATCH_ANY_DTYPE(dtype, (preprocess_s2d_any_kernel<T, false><<<nblocks(total), 256, 0, (cudaStream_t)s>>>(a, (T *)y)));
+    }
+    return THB_LAUNCH_CHECK("preprocess_s2d_any_kernel");
 }
 
 int thb_minmax_normalized(const float *x, int N, int C, int H, int W, const float *mean3, const float *std3,
@@ -1152,14 +1259,20 @@ int thb_col2im(int dtype, const void *cols, int N, int H, int W, int Cout, int k
 
 int thb_u8_channel_sum(const void *x, long pixels, int C, int x_ld, int *csum, thb_stream s)
 {
+    return thb_u8_channel_sum_rows(x, pixels, C, x_ld, 1, 0, 0, csum, s);
+}
+
+int thb_u8_channel_sum_rows(const void *x, long pixels, int C, int x_ld, int W, int row_pitch, int pad_left, int *csum, thb_stream s)
+{
     if (pixels == 0) return THB_OK;
-    if (C >= 2048 && pixels <= 65535) {
+    if (W < 1 || (row_pitch && row_pitch < pad_left + W)) return THB_ERR_ARG;
+    if (!row_pitch && C >= 2048 && pixels <= 65535) {
         u8_channel_sum_wide_kernel<<<(unsigned)pixels, 256, 0, (cudaStream_t)s>>>((const uint8_t *)x, C, x_ld, csum);
         return THB_LAUNCH_CHECK("u8_channel_sum_wide_kernel");
     }
     const int chunks = (C + 15) / 16;
 #define CSUM_CASE(G)                                                                                                      \
-    u8_channel_sum_kernel<G><<<nblocks(pixels * G), 256, 0, (cudaStream_t)s>>>((const uint8_t *)x, pixels, C, x_ld, csum)
+    u8_channel_sum_kernel<G><<<nblocks(pixels * G), 256, 0, (cudaStream_t)s>>>((const uint8_t *)x, pixels, C, x_ld, W, row_pitch, pad_left, csum)
     if (chunks <= 1) CSUM_CASE(1);
     else if (chunks <= 2) CSUM_CASE(2);
     else if (chunks <= 4) CSUM_CASE(4);
