@@ -1,176 +1,291 @@
 // fp32 implicit-GEMM convolution with exact FFMA accumulation (the fp32 mode's 1e-4 parity path).
 //
 // D[pixel][cout] = sum_k A[pixel][k] * Wk[k][cout], k = tap*Cin_pad + c over NHWC fp32 activations.
-// Block tile (16*TM) pixels x 64 output channels, K step 16, 256 threads, TM x 4 outputs per thread.
-// The A tile is gathered as float4 channel chunks (zero outside the image) and stored transposed in
-// shared memory; global loads of the next K step are issued before the current one is consumed.
 //
-// Few pixels (batch 1): the tile grid alone leaves most SMs idle and each CTA walks the whole reduction alone.  Then the
-// K steps are split over the CTAs of a thread-block cluster (grid z, up to 8): every CTA accumulates its share, the
-// others leave their partial tiles in their own shared memory, and the cluster's first CTA adds them up through
-// distributed shared memory in rank order (so the result does not depend on timing) and runs the epilogue.
+// What bounds it is the FP32 pipe (74 TFLOP/s) once operands reach the registers cheaply, so:
+//   * a thread owns 8 pixels x 8 channels and multiplies with fma.rn.f32x2, two channels an instruction, which leaves half
+//     of the issue slots to the loads and to the duplication of the pixel operand;
+//   * a CTA's tile is 128 pixels x 64 or 128 channels, the K block 32; both operands arrive by 16-byte cp.async (channel
+//     chunks of pixels through the gather table, zeros outside the image) in a ring of three stages, pixel rows of 128 bytes
+//     swizzled by XOR so that neither the copies nor the 16-byte reads of four k at a time meet in a bank;
+//   * launches of few tiles: the K blocks of a tile are shared by the S CTAs of a thread-block cluster.  Each leaves its partial tile in its shared memory, and every CTA adds the S parts of its share of
+//     the rows, in rank order, through distributed shared memory (no atomics, the result does not depend on timing).
+// Measured: the table at thb_conv_fwd_simt.
 #include "common.cuh"
+#include "conv_maps.cuh"
 #include <cooperative_groups.h>
+#include <stdlib.h>
 #include <string.h>
 namespace cg = cooperative_groups;
 
 namespace {
 
+constexpr int BM = 128, BK = 32, STAGES = 3;
+
 struct ConvSimtParams {
     const float *x, *w;
     float *y;
     const int *kinfo;
-    int P, H, W, in_ld, oW, oHW, dH, dW, padH, padW, Cout, Cout_pad, out_ld, nkb, n_kchunks;
+    int P, H, W, in_ld, oW, oHW, dH, dW, padH, padW, Cout, Cout_pad, out_ld, Ktot, n_kchunks;
     const float *scale, *shift, *slope, *res;
     int res_ld;
     float self_coef, res_coef;
     int act_kind;
     float act_th, act_val, act_alpha;
+    int splits, pdl;
 };
 
 int g_no_split = -1;  // THB200_NO_SPLITK, read once
 
-template <int TM, bool SPLIT>
-__global__ void __launch_bounds__(256) conv_simt_kernel(const ConvSimtParams p)
+__device__ __forceinline__ uint64_t dup2(float a)
 {
-    constexpr int BMT = 16 * TM, BNT = 64, BK = 16;
-    constexpr int A_LOADS = (BMT * 4 + 255) / 256;
-    __shared__ __align__(16) float As[BK][BMT + 4];
-    __shared__ __align__(16) float Bs[BK][BNT];
-    __shared__ float red[SPLIT ? TM * 4 : 1][SPLIT ? 256 : 1];  // this CTA's partial tile, read by the cluster's first CTA
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
+    return r;
+}
+__device__ __forceinline__ uint64_t pair2(float a, float b)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpair2(uint64_t v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ void fma2(uint64_t &c, uint64_t a, uint64_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b)); }
 
-    const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
-    const int m0 = blockIdx.x * BMT, n0 = blockIdx.y * BNT;
-
-    // gather bookkeeping for this thread's A chunks
-    int a_row[A_LOADS], a_ih0[A_LOADS], a_iw0[A_LOADS], a_pix[A_LOADS];
-    const int a_chunk = t & 3;
-#pragma unroll
-    for (int i = 0; i < A_LOADS; i++) {
-        int idx = t + i * 256;
-        int r = idx >> 2;
-        a_row[i] = r;
-        int pm = m0 + r;
-        if (idx < BMT * 4 && pm < p.P) {
-            int n = pm / p.oHW, rem = pm - n * p.oHW;
-            int oh = rem / p.oW, ow = rem - oh * p.oW;
-            a_ih0[i] = oh * p.dH - p.padH;
-            a_iw0[i] = ow * p.dW - p.padW;
-            a_pix[i] = n * p.H * p.W;
-        } else {
-            a_ih0[i] = a_iw0[i] = 0;
-            a_pix[i] = -1;
-        }
-    }
-    const int b_k = t >> 4, b_c = (t & 15) * 4;
-
-    float acc[TM][4];
-#pragma unroll
-    for (int i = 0; i < TM; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
-
-    float4 a_reg[A_LOADS], b_reg;
-    auto load_global = [&](int kb) {
-        const int g = kb * 4 + a_chunk;
-        const int ki = g < p.n_kchunks ? p.kinfo[g] : -1;
-        const int dh = (ki >> 24) & 0x7f, dw = (ki >> 16) & 0xff, coff = (ki & 0xffff) * 4;
-#pragma unroll
-        for (int i = 0; i < A_LOADS; i++) {
-            const int ih = a_ih0[i] + dh, iw = a_iw0[i] + dw;
-            const bool ok = ki >= 0 && a_pix[i] >= 0 && (unsigned)ih < (unsigned)p.H && (unsigned)iw < (unsigned)p.W;
-            a_reg[i] = ok ? *reinterpret_cast<const float4 *>(p.x + (size_t)(a_pix[i] + ih * p.W + iw) * p.in_ld + coff)
-                          : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        b_reg = *reinterpret_cast<const float4 *>(p.w + (size_t)(kb * BK + b_k) * p.Cout_pad + n0 + b_c);
-    };
-    auto store_smem = [&]() {
-#pragma unroll
-        for (int i = 0; i < A_LOADS; i++) {
-            if (t + i * 256 < BMT * 4) {
-                const int r = a_row[i], k = a_chunk * 4;
-                As[k + 0][r] = a_reg[i].x;
-                As[k + 1][r] = a_reg[i].y;
-                As[k + 2][r] = a_reg[i].z;
-                As[k + 3][r] = a_reg[i].w;
-            }
-        }
-        *reinterpret_cast<float4 *>(&Bs[b_k][b_c]) = b_reg;
-    };
-
-    // this CTA's share of the K steps
-    const int kb0 = SPLIT ? (int)((long)p.nkb * blockIdx.z / gridDim.z) : 0;
-    const int kb1 = SPLIT ? (int)((long)p.nkb * (blockIdx.z + 1) / gridDim.z) : p.nkb;
-    if (kb0 < kb1) load_global(kb0);
-    for (int kb = kb0; kb < kb1; kb++) {
-        store_smem();
-        __syncthreads();
-        if (kb + 1 < kb1) load_global(kb + 1);
-#pragma unroll
-        for (int k = 0; k < BK; k++) {
-            float a[TM];
-            const float4 b = *reinterpret_cast<const float4 *>(&Bs[k][tx * 4]);
-#pragma unroll
-            for (int i = 0; i < TM; i++) a[i] = As[k][ty * TM + i];
-#pragma unroll
-            for (int i = 0; i < TM; i++) {
-                acc[i][0] = fmaf(a[i], b.x, acc[i][0]);
-                acc[i][1] = fmaf(a[i], b.y, acc[i][1]);
-                acc[i][2] = fmaf(a[i], b.z, acc[i][2]);
-                acc[i][3] = fmaf(a[i], b.w, acc[i][3]);
-            }
-        }
-        __syncthreads();
-    }
-
-    if (SPLIT) {
-        cg::cluster_group cluster = cg::this_cluster();
-        if (blockIdx.z != 0) {
-#pragma unroll
-            for (int i = 0; i < TM; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) red[i * 4 + j][t] = acc[i][j];
-        }
-        cluster.sync();
-        if (blockIdx.z == 0) {
-            for (unsigned r = 1; r < gridDim.z; r++) {
-                const float *remote = cluster.map_shared_rank(&red[0][0], r);
-#pragma unroll
-                for (int i = 0; i < TM; i++)
-#pragma unroll
-                    for (int j = 0; j < 4; j++) acc[i][j] += remote[(i * 4 + j) * 256 + t];
-            }
-        }
-        cluster.sync();  // the others' shared memory must outlive the reads above
-        if (blockIdx.z != 0) return;
-    }
-    const int c0 = n0 + tx * 4;
-    if (c0 >= p.Cout) return;
+// Four channels of one pixel: y = act(self * (acc * scale + shift) + res_coef * residual), channels >= Cout zero.
+struct Affine4 {
     float sc[4], sh[4], sl[4];
+    __device__ Affine4(const ConvSimtParams &p, int c0)
+    {
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        const int c = c0 + j;
-        sc[j] = c < p.Cout ? (p.scale ? p.scale[c] : 1.f) : 0.f;
-        sh[j] = c < p.Cout ? (p.shift ? p.shift[c] : 0.f) : 0.f;
-        sl[j] = (c < p.Cout && p.slope) ? p.slope[c] : 0.f;
+        for (int j = 0; j < 4; j++) {
+            const int c = c0 + j;
+            sc[j] = c < p.Cout ? (p.scale ? p.scale[c] : 1.f) : 0.f;
+            sh[j] = c < p.Cout ? (p.shift ? p.shift[c] : 0.f) : 0.f;
+            sl[j] = (c < p.Cout && p.slope) ? p.slope[c] : 0.f;
+        }
     }
-#pragma unroll
-    for (int i = 0; i < TM; i++) {
-        const int pm = m0 + ty * TM + i;
-        if (pm >= p.P) continue;
-        float v[4];
+    __device__ void store(const ConvSimtParams &p, int pm, int c0, const float (&acc)[4]) const
+    {
         float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
         if (p.res) r = *reinterpret_cast<const float4 *>(p.res + (size_t)pm * p.res_ld + c0);
         const float rr[4] = {r.x, r.y, r.z, r.w};
+        float v[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            float val = acc[i][j] * sc[j] + sh[j];
+            float val = acc[j] * sc[j] + sh[j];
             if (p.res) val = p.self_coef * val + p.res_coef * rr[j];
-            val = thb_apply_act(val, p.act_kind, p.act_th, p.act_val, p.act_alpha, sl[j]);
+            if (p.act_kind == THB_ACT_THRESHOLD) val = val > p.act_th ? val : p.act_val;
+            else if (p.act_kind != THB_ACT_NONE) val = thb_apply_act(val, p.act_kind, p.act_th, p.act_val, p.act_alpha, sl[j]);
             v[j] = (c0 + j < p.Cout) ? val : 0.f;
         }
         *reinterpret_cast<float4 *>(p.y + (size_t)pm * p.out_ld + c0) = make_float4(v[0], v[1], v[2], v[3]);
     }
+};
+
+template <int BN, bool SPLIT>
+__global__ void __launch_bounds__(2 * BN, BN == 64 ? 3 : 2) conv_simt_kernel(const ConvSimtParams p)
+{
+    constexpr int NT = 2 * BN, A_BYTES = BM * 128, B_BYTES = BK * BN * 4, STAGE = A_BYTES + B_BYTES;
+    constexpr int A_ROWS = BM * 8 / NT, B_ROWS = BK * (BN / 4) / NT;
+    extern __shared__ __align__(1024) uint8_t smem[];
+
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int tx = lane & 7, ty = lane >> 3;
+    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+    const int wm = (warp & 3) * 32, wn = (warp >> 2) * 64;  // this warp's 32 pixels x 64 channels
+
+    // this thread's share of the copies: one 16-byte chunk of K of A_ROWS pixel rows, B_ROWS chunks of weight rows
+    const int chunk = t & 7;
+    int a_ih[A_ROWS], a_iw[A_ROWS], a_pix[A_ROWS];  // position of tap (0, 0); first pixel of the image, -1: no pixel
+#pragma unroll
+    for (int j = 0; j < A_ROWS; j++) {
+        const int pm = m0 + (t >> 3) + j * (NT / 8);
+        a_pix[j] = -1;
+        a_ih[j] = a_iw[j] = 0;
+        if (pm < p.P) {
+            const int n = pm / p.oHW, rem = pm - n * p.oHW;
+            const int oh = rem / p.oW, ow = rem - oh * p.oW;
+            a_ih[j] = oh * p.dH - p.padH;
+            a_iw[j] = ow * p.dW - p.padW;
+            a_pix[j] = n * p.H * p.W;
+        }
+    }
+    const int b_row = t / (BN / 4), b_c = (t % (BN / 4)) * 4;
+
+    const int nkb = (p.Ktot + BK - 1) / BK;
+    const int kb0 = SPLIT ? (int)((long)nkb * blockIdx.z / gridDim.z) : 0;
+    const int kb1 = SPLIT ? (int)((long)nkb * (blockIdx.z + 1) / gridDim.z) : nkb;
+
+    auto load_b = [&](int kb, int s) {
+        const uint32_t dst = smem_u32(smem + s * STAGE + A_BYTES);
+#pragma unroll
+        for (int j = 0; j < B_ROWS; j++) {
+            const int r = b_row + j * (NT / (BN / 4)), k = kb * BK + r;
+            cp_async16(dst + (r * BN + b_c) * 4, p.w + (size_t)(k < p.Ktot ? k : 0) * p.Cout_pad + n0 + b_c, k < p.Ktot ? 16u : 0u);
+        }
+    };
+    auto load_a = [&](int kb, int s) {
+        const int g = kb * 8 + chunk;
+        const int ki = g < p.n_kchunks ? __ldg(p.kinfo + g) : -1;
+        const int dh = (ki >> 24) & 0x7f, dw = (ki >> 16) & 0xff, coff = (ki & 0xffff) * 4;
+        const uint32_t dst = smem_u32(smem + s * STAGE);
+#pragma unroll
+        for (int j = 0; j < A_ROWS; j++) {
+            const int r = (t >> 3) + j * (NT / 8);
+            const int ih = a_ih[j] + dh, iw = a_iw[j] + dw;
+            const bool ok = ki >= 0 && a_pix[j] >= 0 && (unsigned)ih < (unsigned)p.H && (unsigned)iw < (unsigned)p.W;
+            const float *src = ok ? p.x + (size_t)(a_pix[j] + ih * p.W + iw) * p.in_ld + coff : p.x;
+            cp_async16(dst + r * 128 + ((chunk ^ (r & 7)) << 4), src, ok ? 16u : 0u);
+        }
+    };
+
+    // (weights do not depend on the launch before: their first copies go out ahead of the wait)
+    int next = kb0;
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; s++)
+        if (kb0 + s < kb1) load_b(kb0 + s, s);
+    if (p.pdl) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; s++) {
+        if (next < kb1) load_a(next++, s);
+        cp_async_commit();
+    }
+
+    uint64_t acc[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = 0;
+
+    int s = 0;
+    for (int kb = kb0; kb < kb1; kb++) {
+        cp_async_wait<STAGES - 2>();
+        __syncthreads();
+        {
+            const int ns = s == 0 ? STAGES - 1 : s - 1;  // the stage everyone has just left
+            if (next < kb1) {
+                load_b(next, ns);
+                load_a(next, ns);
+                next++;
+            }
+            cp_async_commit();
+        }
+        const uint8_t *sA = smem + s * STAGE + (wm + ty) * 128;
+        const float *sB = reinterpret_cast<const float *>(smem + s * STAGE + A_BYTES) + wn + tx * 4;
+#pragma unroll
+        for (int kc = 0; kc < 8; kc++) {
+            const int off0 = (kc ^ ty) << 4, off1 = off0 ^ 64;  // rows ty + 4i: (row & 7) is ty for even i, ty + 4 for odd
+            float4 a[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) a[i] = *reinterpret_cast<const float4 *>(sA + i * 512 + (i & 1 ? off1 : off0));
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const float4 b0 = *reinterpret_cast<const float4 *>(sB + (kc * 4 + k) * BN);
+                const float4 b1 = *reinterpret_cast<const float4 *>(sB + (kc * 4 + k) * BN + 32);
+                const uint64_t b[4] = {pair2(b0.x, b0.y), pair2(b0.z, b0.w), pair2(b1.x, b1.y), pair2(b1.z, b1.w)};
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const uint64_t av = dup2(k == 0 ? a[i].x : k == 1 ? a[i].y : k == 2 ? a[i].z : a[i].w);
+#pragma unroll
+                    for (int j = 0; j < 4; j++) fma2(acc[i][j], av, b[j]);
+                }
+            }
+        }
+        if (++s == STAGES) s = 0;
+    }
+    cp_async_wait<0>();
+
+    if (!SPLIT) {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int c0 = n0 + wn + tx * 4 + 32 * h;
+            if (c0 >= p.Cout) continue;
+            const Affine4 f(p, c0);
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int pm = m0 + wm + ty + 4 * i;
+                if (pm >= p.P) continue;
+                const float2 u = unpair2(acc[i][2 * h]), v = unpair2(acc[i][2 * h + 1]);
+                const float o[4] = {u.x, u.y, v.x, v.y};
+                f.store(p, pm, c0, o);
+            }
+        }
+        return;
+    }
+    float *red = reinterpret_cast<float *>(smem);  // this CTA's part of the tile, [BM][BN], over the stages
+    __syncthreads();                               // (everyone has left them)
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const float2 u = unpair2(acc[i][2 * h]), v = unpair2(acc[i][2 * h + 1]);
+            *reinterpret_cast<float4 *>(red + (wm + ty + 4 * i) * BN + wn + tx * 4 + 32 * h) = make_float4(u.x, u.y, v.x, v.y);
+        }
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    const int S = (int)gridDim.z, rows = BM / S, r0 = (int)blockIdx.z * rows;
+    for (int it = t; it < rows * (BN / 4); it += NT) {
+        const int r = r0 + it / (BN / 4), c = (it % (BN / 4)) * 4, pm = m0 + r, c0 = n0 + c;
+        if (pm >= p.P || c0 >= p.Cout) continue;
+        float acc4[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int q = 0; q < S; q++) {
+            const float4 v = *reinterpret_cast<const float4 *>(cluster.map_shared_rank(red, q) + r * BN + c);
+            acc4[0] += v.x; acc4[1] += v.y; acc4[2] += v.z; acc4[3] += v.w;
+        }
+        const Affine4 f(p, c0);
+        f.store(p, pm, c0, acc4);
+    }
+    cluster.sync();  // the parts must outlive the reads above
+}
+
+template <int BN, bool SPLIT> int launch_simt(const ConvSimtParams &p, int sms, cudaStream_t st)
+{
+    auto kern = conv_simt_kernel<BN, SPLIT>;
+    constexpr int need = STAGES * (BM * 128 + BK * BN * 4);
+    static bool set[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64 || !set[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 115712);
+        if (e == cudaSuccess && SPLIT) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e != cudaSuccess) return thb_note_launch(e, "conv_simt_kernel attributes");
+        if (dev >= 0 && dev < 64) set[dev] = true;
+    }
+    // A launch of one to two CTAs per SM: three would fit, and the scheduler packs clusters before it spreads them (240 CTAs in
+    // clusters of two ran on 80 SMs: 90 us instead of 65), so they ask for the shared memory that leaves room for two.
+    const long ctas = (long)((p.P + BM - 1) / BM) * (p.Cout_pad / BN) * p.splits;
+    const int smem = ctas > sms && ctas <= 2L * sms && need < 115712 ? 115712 : need;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((p.P + BM - 1) / BM, p.Cout_pad / BN, p.splits);
+    cfg.blockDim = dim3(2 * BN);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (SPLIT) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = attr[n].val.clusterDim.y = 1;
+        attr[n].val.clusterDim.z = p.splits;
+        n++;
+    }
+    if (p.pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n].val.programmaticStreamSerializationAllowed = 1;
+        n++;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    const cudaError_t le = cudaLaunchKernelEx(&cfg, kern, p);
+    return thb_note_launch(le != cudaSuccess ? le : cudaGetLastError(), "conv_simt_kernel");
 }
 
 }  // namespace
@@ -189,49 +304,35 @@ extern "C" int thb_conv_fwd_simt(const thb_conv_desc *d, const void *x, void *y,
     p.H = d->H; p.W = d->W; p.in_ld = d->in_ld; p.oW = d->oW; p.oHW = d->oH * d->oW;
     p.dH = d->dH; p.dW = d->dW; p.padH = d->padH; p.padW = d->padW;
     p.Cout = d->Cout; p.Cout_pad = d->Cout_pad; p.out_ld = d->out_ld;
-    p.nkb = d->Ktot_pad / 16; p.n_kchunks = d->Ktot_pad / 4;
+    p.Ktot = d->Ktot_pad; p.n_kchunks = d->Ktot_pad / 4;
     p.scale = d->scale; p.shift = d->shift; p.slope = d->act.kind == THB_ACT_PRELU ? d->act.slope : nullptr;
     p.res = (const float *)d->res; p.res_ld = d->res_ld; p.self_coef = d->self_coef; p.res_coef = d->res_coef;
     p.act_kind = d->act.kind; p.act_th = d->act.threshold; p.act_val = d->act.value; p.act_alpha = d->act.alpha;
     if (p.P <= 0) return THB_OK;
-    const int gy = d->Cout_pad / 64;
-    cudaStream_t st = (cudaStream_t)s;
-    if ((long)((p.P + 127) / 128) * gy >= 120) {
-        conv_simt_kernel<8, false><<<dim3((p.P + 127) / 128, gy), 256, 0, st>>>(p);
-    } else {
-        // how many CTAs share one tile's reduction: enough to give every SM about two CTAs, at least four K steps each
-        const long ctas = (long)((p.P + 31) / 32) * gy;
-        static int sms = 0;
-        int &no_split = g_no_split;
-        if (!sms) {
-            int dev = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            if (sms <= 0) sms = 148;
-        }
-        if (no_split < 0) {
-            const char *e = getenv("THB200_NO_SPLITK");
-            no_split = e && atoi(e) ? 1 : 0;
-        }
-        int split = 1;
-        while (split < 8 && ctas * split * 2 <= 2L * sms && p.nkb / (split * 2) >= 4) split *= 2;
-        if (split == 1 || no_split) {
-            conv_simt_kernel<2, false><<<dim3((p.P + 31) / 32, gy), 256, 0, st>>>(p);
-        } else {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3((p.P + 31) / 32, gy, split);
-            cfg.blockDim = dim3(256);
-            cfg.stream = st;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = 1;
-            attr[0].val.clusterDim.y = 1;
-            attr[0].val.clusterDim.z = split;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            const cudaError_t le = cudaLaunchKernelEx(&cfg, conv_simt_kernel<2, true>, p);
-            if (le != cudaSuccess) return thb_note_launch(le, "conv_simt_kernel (split K)");
-        }
+    if (g_no_split < 0) {
+        const char *e = getenv("THB200_NO_SPLITK");
+        g_no_split = e && atoi(e) ? 1 : 0;
     }
-    return THB_LAUNCH_CHECK("conv_simt_kernel");
+    const ThbConvLaunch kn = thb_conv_launch_knobs();
+    p.pdl = kn.pdl;
+    const cudaStream_t st = (cudaStream_t)s;
+    // Tiles of 64 channels, the reduction split while that leaves at most three CTAs to an SM (what its registers hold); measured,
+    // us before / unsplit / split in 2 / 4 / 8 (16 in clusters beyond the portable size):
+    //   64->64 3x3 @57x57, 9 images, 229 tiles of 18 K blocks      72 / 65 / 66
+    //   128->128 3x3 @29x29, 9 images, 120 of 36                   82 / 70 / 65 / 64
+    //   256->256 3x3 @15x15, 9 images, 64 of 72                   144 / 133 / 71 / 63 / 77
+    //   512->512 3x3 @8x8, 9 images, 40 of 144                    160 / - / 137 / 120 / 89
+    //   64->192 5x5 @27x27, 1 image, 18 of 50                      31 / - / 51 / 28 / 27
+    //   384->256 3x3 @13x13, 1 image, 8 of 108                     34 / - / 102 / 53 / 29
+    // Large layers: tiles of 128 channels (128->128 3x3 @28x28, 64 images: 401 / 332 with 64, 320 with 128).
+    const long tiles = (long)((p.P + BM - 1) / BM) * (d->Cout_pad / 64);
+    const int nkb = (p.Ktot + BK - 1) / BK;
+    p.splits = 1;
+    if (!g_no_split) {
+        while (p.splits < 8 && tiles * 2 * p.splits <= 3L * kn.sms && nkb >= 2 * p.splits) p.splits *= 2;
+        if (p.splits == 8 && tiles * 16 <= 2L * kn.sms && nkb >= 32) p.splits = 16;
+    }
+    if (p.splits > 1) return launch_simt<64, true>(p, kn.sms, st);
+    if (d->Cout_pad % 128 == 0 && tiles >= 200) return launch_simt<128, false>(p, kn.sms, st);
+    return launch_simt<64, false>(p, kn.sms, st);
 }
