@@ -10,6 +10,29 @@
 extern "C" int thb_note_launch(cudaError_t e, const char *what);
 #define THB_LAUNCH_CHECK(what) thb_note_launch(cudaGetLastError(), what)
 
+// Programmatic dependent launch.  A kernel launched by thb_launch may be set up while its predecessor in the stream still runs:
+// it calls pdl_enter() before its first access to global memory.  (THB200_PDL=0 launches plainly; pdl_enter is then free.)
+__device__ __forceinline__ void pdl_enter()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+int thb_pdl_enabled();  // conv_tc.cu
+template <typename... Params, typename... Args>
+inline void thb_launch(void (*kernel)(Params...), dim3 grid, dim3 block, thb_stream s, Args... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = (cudaStream_t)s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = thb_pdl_enabled() ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);  // (an error stays for THB_LAUNCH_CHECK)
+}
+
 template <typename T> struct dt;
 template <> struct dt<float> {
     static __device__ __forceinline__ float ld(const float *p) { return *p; }

@@ -106,6 +106,7 @@ template <typename T>
 __global__ void preprocess_kernel(const float *x, float *x_inplace, int N, int C, long HW, float3 mean, float3 std_,
                                   T *y, int y_ld, float q_min, float q_mult)
 {
+    pdl_enter();
     constexpr int VN = Vec<T>::N;
     const long pix = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (pix >= (long)N * HW) return;
@@ -141,6 +142,7 @@ template <typename T>
 __global__ void preprocess_s2d_kernel(const float *x, float *x_inplace, int N, int C, int H, int W, float3 mean,
                                       float3 std_, T *y, int y_ld, int row_pitch, int pad_left, float q_min, float q_mult)
 {
+    pdl_enter();
     const float zr = roundf(q_min * q_mult);  // uint8 only: the quantisation of preprocess_kernel
     constexpr int VN = Vec<T>::N;
     const int H2 = H / 2, W2 = W / 2;
@@ -227,6 +229,7 @@ struct S2dArgs {
 template <typename T, bool BYTES>
 __global__ void preprocess_s2d_any_kernel(const S2dArgs a, T *y)
 {
+    pdl_enter();
     constexpr int VN = Vec<T>::N;
     const int H2 = (a.H + a.f - 1) / a.f, W2 = (a.W + a.f - 1) / a.f, groups = a.y_ld / VN;
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -280,6 +283,7 @@ __global__ void preprocess_s2d_any_kernel(const S2dArgs a, T *y)
 __global__ void preprocess_neigh_u8_kernel(const float *x, float *x_inplace, int N, int H, int W, float3 mean, float3 std_,
                                            uint8_t *y, int y_ld, float q_min, float q_mult)
 {
+    pdl_enter();
     const long pix = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const long HW = (long)H * W;
     if (pix >= (long)N * HW) return;
@@ -319,6 +323,7 @@ template <typename T>
 __global__ void preprocess_images_kernel(const uint8_t *img, int N, int H, int W, int stride, int cp, int bgr, float3 mean,
                                          float3 istd, T *y, int y_ld)
 {
+    pdl_enter();
     constexpr int VN = Vec<T>::N;
     const long pix = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (pix >= (long)N * H * W) return;
@@ -350,6 +355,7 @@ template <typename T>
 __global__ void preprocess_images_s2d_kernel(const uint8_t *img, int N, int H, int W, int stride, int bgr, float3 mean, float3 istd,
                                              T *y, int y_ld, int row_pitch, int pad_left)
 {
+    pdl_enter();
     constexpr int VN = Vec<T>::N;
     const int H2 = H / 2, W2 = W / 2;
     const long pix = (long)blockIdx.x * blockDim.x + threadIdx.x;  // over the stored (padded) pixels
@@ -383,6 +389,7 @@ __global__ void preprocess_images_s2d_kernel(const uint8_t *img, int N, int H, i
 template <typename T>
 __global__ void preprocess_yuyv_kernel(const uint8_t *frame, int H, int W, float3 mean, float3 istd, T *y, int y_ld)
 {
+    pdl_enter();
     constexpr int VN = Vec<T>::N;
     const long pair = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const int W2 = W / 2;
@@ -415,6 +422,7 @@ __global__ void preprocess_yuyv_kernel(const uint8_t *frame, int H, int W, float
 __global__ void preprocess_images_u8_kernel(const uint8_t *img, int N, int H, int W, int stride, int bgr, int3 sub, float3 mult,
                                             uint8_t *y, int y_ld)
 {
+    pdl_enter();
     const long pix = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (pix >= (long)N * H * W) return;
     const long n = pix / ((long)H * W);
@@ -437,6 +445,7 @@ __global__ void preprocess_images_u8_kernel(const uint8_t *img, int N, int H, in
 // deviation are monotone, so the extremes of the normalised values are the normalised extremes, bit for bit.
 __global__ void __launch_bounds__(256) minmax_kernel(const float *x, int C, long HW, int pieces, float3 mean, float3 std_, float *minmax)
 {
+    pdl_enter();
     const long plane = blockIdx.x / pieces;
     const int piece = blockIdx.x % pieces, c = (int)(plane % C);
     const long per = (HW + pieces - 1) / pieces, i0 = piece * per, i1 = min(HW, i0 + per);
@@ -477,6 +486,7 @@ template <typename Tin, typename Tout>
 __global__ void nhwc_to_nchw_kernel(const Tin *x, int HW, int C, int x_ld, float q_sub, float q_invmult, Tout *y,
                                     const int *status, int *status_out)
 {
+    pdl_enter();
     __shared__ float tile[32][33];
     if (status && (blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x | threadIdx.y) == 0) *status_out = *status;
     const int n = blockIdx.z, hw0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
@@ -504,6 +514,7 @@ template <typename Tin>
 __global__ void rows_to_float_kernel(const Tin *x, long total, int C, int x_ld, float q_sub, float q_invmult, float *y,
                                      const int *status, int *status_out)
 {
+    pdl_enter();
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (status && i == 0) *status_out = *status;
     if (i >= total) return;
@@ -518,6 +529,7 @@ template <typename T, bool IS_MAX>
 __global__ void pool_kernel(const T *x, int N, int H, int W, int C, int x_ld, int kH, int kW, int dH, int dW, int padH,
                             int padW, int oH, int oW, int count_include_pad, T *y, int y_ld)
 {
+    pdl_enter();
     constexpr int VN = Vec<T>::N;
     const int cvecs = (C + VN - 1) / VN;
     const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -567,6 +579,7 @@ __global__ void pool_kernel(const T *x, int N, int H, int W, int C, int x_ld, in
 template <typename T>
 __global__ void __launch_bounds__(256) global_avgpool_kernel(const T *x, int HW, int C, int x_ld, T *y, int y_ld)
 {
+    pdl_enter();
     constexpr int VN = Vec<T>::N;
     __shared__ float part[8][32][VN + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -621,6 +634,7 @@ template <typename T2>
 __global__ void maxpool3s2_kernel(const uint4 *__restrict__ x, int N, int H, int W, int cvecs, int x_ld8, int padH, int padW,
                                   int oH, int oW, int strip, int nstrips, uint32_t neg_inf2, uint4 *__restrict__ y, int y_ld8)
 {
+    pdl_enter();
     const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (long)N * nstrips * oW * cvecs) return;
     const int cv = (int)(idx % cvecs);
@@ -657,6 +671,7 @@ template <typename T>
 __global__ void affine_act_kernel(const T *x, long pixels, int C, int x_ld, const float *scale, const float *shift,
                                   thb_act act, T *y, int y_ld)
 {
+    pdl_enter();
     constexpr int VN = Vec<T>::N;
     const int cvecs = (C + VN - 1) / VN;
     const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -681,6 +696,7 @@ __global__ void affine_act_kernel(const T *x, long pixels, int C, int x_ld, cons
 
 __global__ void u8_threshold_kernel(const uint8_t *x, long pixels, int C, int x_ld, int thr, int val, uint8_t *y, int y_ld)
 {
+    pdl_enter();
     const int cvecs = (C + 15) / 16;
     const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= pixels * cvecs) return;
@@ -701,6 +717,7 @@ __global__ void u8_threshold_kernel(const uint8_t *x, long pixels, int C, int x_
 __global__ void u8_combine_kernel(const uint8_t *a, int a_ld, const uint8_t *b, int b_ld, int ca, int cb, int addend,
                                   int thr, int val, long pixels, int C, uint8_t *y, int y_ld)
 {
+    pdl_enter();
     const int cvecs = (C + 15) / 16;
     const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= pixels * cvecs) return;
@@ -730,6 +747,7 @@ struct CombineArgs {
 template <typename T>
 __global__ void combine_kernel(CombineArgs a, long pixels, int C, T *y, int y_ld)
 {
+    pdl_enter();
     constexpr int VN = Vec<T>::N;
     const int cvecs = (C + VN - 1) / VN;
     const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -754,6 +772,7 @@ __global__ void combine_kernel(CombineArgs a, long pixels, int C, T *y, int y_ld
 template <typename T>
 __global__ void copy_channels_kernel(const T *x, long pixels, int cvecs, int x_ld, T *y, int y_ld)
 {
+    pdl_enter();
     constexpr int VN = Vec<T>::N;
     const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= pixels * cvecs) return;
@@ -776,6 +795,7 @@ __device__ __forceinline__ float exp_minus_approx(float d)
 template <typename T>
 __global__ void softmax_kernel(const T *x, long pixels, int C, int x_ld, T *y, int y_ld)
 {
+    pdl_enter();
     const long pix = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (pix >= pixels) return;
@@ -797,6 +817,7 @@ __global__ void col2im_kernel(const T *cols, int N, int H, int W, int Cout, int 
                               int padW, int oH, int oW, int cols_ld, int Cp, float beta, const float *bias, thb_act act,
                               T *y, int y_ld)
 {
+    pdl_enter();
     constexpr int VN = Vec<T>::N;
     const int cvecs = Cp / VN;
     const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -842,6 +863,7 @@ __global__ void col2im_kernel(const T *cols, int N, int H, int W, int Cout, int 
 template <int G>
 __global__ void u8_channel_sum_kernel(const uint8_t *x, long pixels, int C, int x_ld, int W, int row_pitch, int pad_left, int *csum)
 {
+    pdl_enter();
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const long pix = t / G;
     const int g = (int)(t % G);
@@ -876,6 +898,7 @@ __global__ void u8_channel_sum_kernel(const uint8_t *x, long pixels, int C, int 
 // the same with a whole block per pixel, for the few-pixel, many-channel inputs of Linear layers
 __global__ void u8_channel_sum_wide_kernel(const uint8_t *x, int C, int x_ld, int *csum)
 {
+    pdl_enter();
     const uint8_t *p = x + (size_t)blockIdx.x * x_ld;
     int s = 0;
     for (int c0 = threadIdx.x * 16; c0 < C; c0 += blockDim.x * 16) {
@@ -927,8 +950,7 @@ int thb_preprocess(const float *x, float *x_inplace, int N, int C, int H, int W,
     const long HW = (long)H * W, pix = (long)N * HW;
     if (pix == 0) return THB_OK;
     float3 m = make_float3(mean3[0], mean3[1], mean3[2]), sd = make_float3(std3[0], std3[1], std3[2]);
-    DISPATCH_ANY_DTYPE(dtype, (preprocess_kernel<T><<<nblocks(pix), 256, 0, (cudaStream_t)s>>>(
-                                  x, x_inplace, N, C, HW, m, sd, (T *)y, y_ld, q_sub, q_mult)));
+    DISPATCH_ANY_DTYPE(dtype, (thb_launch(preprocess_kernel<T>, nblocks(pix), 256, s, x, x_inplace, N, C, HW, m, sd, (T *)y, y_ld, q_sub, q_mult)));
     return THB_LAUNCH_CHECK("preprocess_kernel");
 }
 
@@ -939,8 +961,7 @@ int thb_preprocess_s2d_padded(const float *x, float *x_inplace, int N, int C, in
     const long pix = (long)N * (H / 2) * row_pitch;
     if (pix == 0) return THB_OK;
     float3 m = make_float3(mean3[0], mean3[1], mean3[2]), sd = make_float3(std3[0], std3[1], std3[2]);
-    DISPATCH_FLOAT_DTYPE(dtype, (preprocess_s2d_kernel<T><<<nblocks(pix), 256, 0, (cudaStream_t)s>>>(
-                                    x, x_inplace, N, C, H, W, m, sd, (T *)y, y_ld, row_pitch, pad_left, 0.f, 0.f)));
+    DISPATCH_FLOAT_DTYPE(dtype, (thb_launch(preprocess_s2d_kernel<T>, nblocks(pix), 256, s, x, x_inplace, N, C, H, W, m, sd, (T *)y, y_ld, row_pitch, pad_left, 0.f, 0.f)));
     return THB_LAUNCH_CHECK("preprocess_s2d_kernel");
 }
 
@@ -951,7 +972,7 @@ int thb_preprocess_s2d_u8(const float *x, float *x_inplace, int N, int C, int H,
     const long pix = (long)N * (H / 2) * (W / 2);
     if (pix == 0) return THB_OK;
     float3 m = make_float3(mean3[0], mean3[1], mean3[2]), sd = make_float3(std3[0], std3[1], std3[2]);
-    preprocess_s2d_kernel<uint8_t><<<nblocks(pix), 256, 0, (cudaStream_t)s>>>(x, x_inplace, N, C, H, W, m, sd, (uint8_t *)y, y_ld,
+    thb_launch(preprocess_s2d_kernel<uint8_t>, nblocks(pix), 256, s, x, x_inplace, N, C, H, W, m, sd, (uint8_t *)y, y_ld,
                                                                               W / 2, 0, q_sub, q_mult);
     return THB_LAUNCH_CHECK("preprocess_s2d_kernel<u8>");
 }
@@ -963,7 +984,7 @@ int thb_preprocess_neigh_u8(const float *x, float *x_inplace, int N, int H, int 
     const long pix = (long)N * H * W;
     if (pix == 0) return THB_OK;
     float3 m = make_float3(mean3[0], mean3[1], mean3[2]), sd = make_float3(std3[0], std3[1], std3[2]);
-    preprocess_neigh_u8_kernel<<<nblocks(pix), 256, 0, (cudaStream_t)s>>>(x, x_inplace, N, H, W, m, sd, (uint8_t *)y, y_ld, q_sub, q_mult);
+    thb_launch(preprocess_neigh_u8_kernel, nblocks(pix), 256, s, x, x_inplace, N, H, W, m, sd, (uint8_t *)y, y_ld, q_sub, q_mult);
     return THB_LAUNCH_CHECK("preprocess_neigh_u8_kernel");
 }
 
@@ -981,8 +1002,7 @@ int thb_preprocess_images(const unsigned char *img, int N, int H, int W, int str
     if (cp != 1 && cp != 3) return THB_ERR_ARG;
     float3 m = make_float3(mean3[0], mean3[1], mean3[2]);
     float3 is = make_float3(1 / std3[0], 1 / std3[1], 1 / std3[2]);
-    DISPATCH_FLOAT_DTYPE(dtype, (preprocess_images_kernel<T><<<nblocks(pix), 256, 0, (cudaStream_t)s>>>(
-                                    img, N, H, W, stride, cp, bgr, m, is, (T *)y, y_ld)));
+    DISPATCH_FLOAT_DTYPE(dtype, (thb_launch(preprocess_images_kernel<T>, nblocks(pix), 256, s, img, N, H, W, stride, cp, bgr, m, is, (T *)y, y_ld)));
     return THB_LAUNCH_CHECK("preprocess_images_kernel");
 }
 
@@ -994,7 +1014,7 @@ int thb_preprocess_yuyv(const unsigned char *frame, int H, int W, const float *m
     const long pairs = (long)H * (W / 2);
     float3 m = make_float3(mean3[0], mean3[1], mean3[2]);
     float3 is = make_float3(1 / std3[0], 1 / std3[1], 1 / std3[2]);
-    DISPATCH_FLOAT_DTYPE(dtype, (preprocess_yuyv_kernel<T><<<nblocks(pairs), 256, 0, (cudaStream_t)s>>>(frame, H, W, m, is, (T *)y, y_ld)));
+    DISPATCH_FLOAT_DTYPE(dtype, (thb_launch(preprocess_yuyv_kernel<T>, nblocks(pairs), 256, s, frame, H, W, m, is, (T *)y, y_ld)));
     return THB_LAUNCH_CHECK("preprocess_yuyv_kernel");
 }
 
@@ -1007,8 +1027,7 @@ int thb_preprocess_images_s2d(const unsigned char *img, int N, int H, int W, int
     if (pix == 0) return THB_OK;
     float3 m = make_float3(mean3[0], mean3[1], mean3[2]);
     float3 is = make_float3(1 / std3[0], 1 / std3[1], 1 / std3[2]);
-    DISPATCH_FLOAT_DTYPE(dtype, (preprocess_images_s2d_kernel<T><<<nblocks(pix), 256, 0, (cudaStream_t)s>>>(
-                                    img, N, H, W, stride, bgr, m, is, (T *)y, y_ld, row_pitch, pad_left)));
+    DISPATCH_FLOAT_DTYPE(dtype, (thb_launch(preprocess_images_s2d_kernel<T>, nblocks(pix), 256, s, img, N, H, W, stride, bgr, m, is, (T *)y, y_ld, row_pitch, pad_left)));
     return THB_LAUNCH_CHECK("preprocess_images_s2d_kernel");
 }
 
@@ -1021,7 +1040,7 @@ int thb_preprocess_images_lowp(const unsigned char *img, int N, int H, int W, in
     lowp_image_range(mean3, std3, q_sub, q_mult, sub, mul);
     const long pix = (long)N * H * W;
     if (pix == 0) return THB_OK;
-    preprocess_images_u8_kernel<<<nblocks(pix), 256, 0, (cudaStream_t)s>>>(img, N, H, W, stride, bgr, make_int3(sub[0], sub[1], sub[2]),
+    thb_launch(preprocess_images_u8_kernel, nblocks(pix), 256, s, img, N, H, W, stride, bgr, make_int3(sub[0], sub[1], sub[2]),
                                                                             make_float3(mul[0], mul[1], mul[2]), (uint8_t *)y, y_ld);
     return THB_LAUNCH_CHECK("preprocess_images_u8_kernel");
 }
@@ -1055,9 +1074,9 @@ int thb_preprocess_s2d_any(const void *src, int bytes, float *x_inplace, int N, 
     const long total = (long)N * H2 * row_pitch * (y_ld / thb_channel_align(dtype));
     if (total == 0) return THB_OK;
     if (bytes) {
-        DISPATCH_ANY_DTYPE(dtype, (preprocess_s2d_any_kernel<T, true><<<nblocks(total), 256, 0, (cudaStream_t)s>>>(a, (T *)y)));
+        DISPATCH_ANY_DTYPE(dtype, (thb_launch(preprocess_s2d_any_kernel<T, true>, nblocks(total), 256, s, a, (T *)y)));
     } else {
-        DISPATCH_ANY_DTYPE(dtype, (preprocess_s2d_any_kernel<T, false><<<nblocks(total), 256, 0, (cudaStream_t)s>>>(a, (T *)y)));
+        DISPATCH_ANY_DTYPE(dtype, (thb_launch(preprocess_s2d_any_kernel<T, false>, nblocks(total), 256, s, a, (T *)y)));
     }
     return THB_LAUNCH_CHECK("preprocess_s2d_any_kernel");
 }
@@ -1076,7 +1095,7 @@ int thb_minmax_normalized(const float *x, int N, int C, int H, int W, const floa
     if (pieces < 1) pieces = 1;
     while (pieces > 1 && ((HW + pieces - 1) / pieces < 4096 || (HW % (4L * pieces)))) pieces--;
     if (planes * pieces > 0x7fffffffL) return THB_ERR_UNSUPPORTED;
-    minmax_kernel<<<(unsigned)(planes * pieces), 256, 0, (cudaStream_t)s>>>(x, C, HW, pieces, m, sd, minmax2);
+    thb_launch(minmax_kernel, (unsigned)(planes * pieces), 256, s, x, C, HW, pieces, m, sd, minmax2);
     return THB_LAUNCH_CHECK("minmax_kernel");
 }
 
@@ -1087,13 +1106,11 @@ int thb_postprocess_status(const void *x, int dtype, int N, int H, int W, int C,
     if ((long)N * HW * C == 0) return THB_OK;
     if (HW == 1) {
         const long total = (long)N * C;
-        DISPATCH_ANY_DTYPE(dtype, (rows_to_float_kernel<T><<<nblocks(total), 256, 0, (cudaStream_t)s>>>(
-                                      (const T *)x, total, C, x_ld, q_sub, q_invmult, y, status, status_out)));
+        DISPATCH_ANY_DTYPE(dtype, (thb_launch(rows_to_float_kernel<T>, nblocks(total), 256, s, (const T *)x, total, C, x_ld, q_sub, q_invmult, y, status, status_out)));
         return THB_LAUNCH_CHECK("rows_to_float_kernel");
     }
     dim3 grid((HW + 31) / 32, (C + 31) / 32, N), block(32, 8);
-    DISPATCH_ANY_DTYPE(dtype, (nhwc_to_nchw_kernel<T, float><<<grid, block, 0, (cudaStream_t)s>>>(
-                                  (const T *)x, HW, C, x_ld, q_sub, q_invmult, y, status, status_out)));
+    DISPATCH_ANY_DTYPE(dtype, (thb_launch(nhwc_to_nchw_kernel<T, float>, grid, block, s, (const T *)x, HW, C, x_ld, q_sub, q_invmult, y, status, status_out)));
     return THB_LAUNCH_CHECK("nhwc_to_nchw_kernel");
 }
 
@@ -1108,8 +1125,7 @@ int thb_to_nchw(int dtype, const void *x, int N, int H, int W, int C, int x_ld, 
     const int HW = H * W;
     if ((long)N * HW * C == 0) return THB_OK;
     dim3 grid((HW + 31) / 32, (C + 31) / 32, N), block(32, 8);
-    DISPATCH_ANY_DTYPE(dtype, (nhwc_to_nchw_kernel<T, T><<<grid, block, 0, (cudaStream_t)s>>>(
-                                  (const T *)x, HW, C, x_ld, 0.f, 1.f, (T *)y, 0, 0)));
+    DISPATCH_ANY_DTYPE(dtype, (thb_launch(nhwc_to_nchw_kernel<T, T>, grid, block, s, (const T *)x, HW, C, x_ld, 0.f, 1.f, (T *)y, nullptr, nullptr)));
     return THB_LAUNCH_CHECK("nhwc_to_nchw_kernel");
 }
 
@@ -1128,11 +1144,9 @@ int thb_maxpool(int dtype, const void *x, int N, int H, int W, int C, int x_ld, 
         const int nstrips = (oH + strip - 1) / strip;
         const long items = (long)N * nstrips * oW * cvecs;
         if (dtype == THB_F16)
-            maxpool3s2_kernel<__half2><<<nblocks(items), 256, 0, (cudaStream_t)s>>>(
-                (const uint4 *)x, N, H, W, cvecs, x_ld / 8, padH, padW, oH, oW, strip, nstrips, 0xFC00FC00u, (uint4 *)y, y_ld / 8);
+            thb_launch(maxpool3s2_kernel<__half2>, nblocks(items), 256, s, (const uint4 *)x, N, H, W, cvecs, x_ld / 8, padH, padW, oH, oW, strip, nstrips, 0xFC00FC00u, (uint4 *)y, y_ld / 8);
         else
-            maxpool3s2_kernel<__nv_bfloat162><<<nblocks(items), 256, 0, (cudaStream_t)s>>>(
-                (const uint4 *)x, N, H, W, cvecs, x_ld / 8, padH, padW, oH, oW, strip, nstrips, 0xFF80FF80u, (uint4 *)y, y_ld / 8);
+            thb_launch(maxpool3s2_kernel<__nv_bfloat162>, nblocks(items), 256, s, (const uint4 *)x, N, H, W, cvecs, x_ld / 8, padH, padW, oH, oW, strip, nstrips, 0xFF80FF80u, (uint4 *)y, y_ld / 8);
         return THB_LAUNCH_CHECK("maxpool3s2_kernel");
     }
     if (dtype == THB_U8 && kH == 3 && kW == 3 && dH == 2 && dW == 2 && x_ld % 16 == 0 && y_ld % 16 == 0) {
@@ -1142,12 +1156,10 @@ int thb_maxpool(int dtype, const void *x, int N, int H, int W, int C, int x_ld, 
         while (strip > 4 && (long)N * ((oH + strip - 1) / strip) * oW * cvecs < 24L * 148 * 256) strip = (strip + 1) / 2;
         const int nstrips = (oH + strip - 1) / strip;
         const long items = (long)N * nstrips * oW * cvecs;
-        maxpool3s2_kernel<U8x4><<<nblocks(items), 256, 0, (cudaStream_t)s>>>(
-            (const uint4 *)x, N, H, W, cvecs, x_ld / 16, padH, padW, oH, oW, strip, nstrips, 0u, (uint4 *)y, y_ld / 16);
+        thb_launch(maxpool3s2_kernel<U8x4>, nblocks(items), 256, s, (const uint4 *)x, N, H, W, cvecs, x_ld / 16, padH, padW, oH, oW, strip, nstrips, 0u, (uint4 *)y, y_ld / 16);
         return THB_LAUNCH_CHECK("maxpool3s2_kernel");
     }
-    DISPATCH_ANY_DTYPE(dtype, (pool_kernel<T, true><<<nblocks(total), 256, 0, (cudaStream_t)s>>>(
-                                  (const T *)x, N, H, W, C, x_ld, kH, kW, dH, dW, padH, padW, oH, oW, 0, (T *)y, y_ld)));
+    DISPATCH_ANY_DTYPE(dtype, (thb_launch(pool_kernel<T, true>, nblocks(total), 256, s, (const T *)x, N, H, W, C, x_ld, kH, kW, dH, dW, padH, padW, oH, oW, 0, (T *)y, y_ld)));
     return THB_LAUNCH_CHECK("pool_kernel<max>");
 }
 
@@ -1159,11 +1171,10 @@ int thb_avgpool(int dtype, const void *x, int N, int H, int W, int C, int x_ld, 
     if (total == 0) return THB_OK;
     if (kH == H && kW == W && padH == 0 && padW == 0 && oH == 1 && oW == 1 && x_ld % al == 0 && y_ld % al == 0) {
         const dim3 grid((unsigned)N, (unsigned)(((C + al - 1) / al + 31) / 32));
-        DISPATCH_ANY_DTYPE(dtype, (global_avgpool_kernel<T><<<grid, 256, 0, (cudaStream_t)s>>>((const T *)x, H * W, C, x_ld, (T *)y, y_ld)));
+        DISPATCH_ANY_DTYPE(dtype, (thb_launch(global_avgpool_kernel<T>, grid, 256, s, (const T *)x, H * W, C, x_ld, (T *)y, y_ld)));
         return THB_LAUNCH_CHECK("global_avgpool_kernel");
     }
-    DISPATCH_ANY_DTYPE(dtype, (pool_kernel<T, false><<<nblocks(total), 256, 0, (cudaStream_t)s>>>(
-                                    (const T *)x, N, H, W, C, x_ld, kH, kW, dH, dW, padH, padW, oH, oW,
+    DISPATCH_ANY_DTYPE(dtype, (thb_launch(pool_kernel<T, false>, nblocks(total), 256, s, (const T *)x, N, H, W, C, x_ld, kH, kW, dH, dW, padH, padW, oH, oW,
                                     count_include_pad, (T *)y, y_ld)));
     return THB_LAUNCH_CHECK("pool_kernel<avg>");
 }
@@ -1176,8 +1187,7 @@ int thb_affine_act(int dtype, const void *x, long pixels, int C, int x_ld, const
     if (total == 0) return THB_OK;
     thb_act a = {THB_ACT_NONE, 0, 0, 0, nullptr};
     if (act) a = *act;
-    DISPATCH_FLOAT_DTYPE(dtype, (affine_act_kernel<T><<<nblocks(total), 256, 0, (cudaStream_t)s>>>(
-                                    (const T *)x, pixels, C, x_ld, scale, shift, a, (T *)y, y_ld)));
+    DISPATCH_FLOAT_DTYPE(dtype, (thb_launch(affine_act_kernel<T>, nblocks(total), 256, s, (const T *)x, pixels, C, x_ld, scale, shift, a, (T *)y, y_ld)));
     return THB_LAUNCH_CHECK("affine_act_kernel");
 }
 
@@ -1185,7 +1195,7 @@ int thb_u8_threshold(const void *x, long pixels, int C, int x_ld, int thr, int v
 {
     const long total = pixels * ((C + 15) / 16);
     if (total == 0) return THB_OK;
-    u8_threshold_kernel<<<nblocks(total), 256, 0, (cudaStream_t)s>>>((const uint8_t *)x, pixels, C, x_ld, thr, val,
+    thb_launch(u8_threshold_kernel, nblocks(total), 256, s, (const uint8_t *)x, pixels, C, x_ld, thr, val,
                                                                      (uint8_t *)y, y_ld);
     return THB_LAUNCH_CHECK("u8_threshold_kernel");
 }
@@ -1199,7 +1209,7 @@ int thb_u8_combine(const void *a, int a_ld, const void *b, int b_ld, int ca, int
     /* floor(-(ca + cb - 1) * 127.5): +1+1 -> -128, +1-1 -> +127, -1-1 -> +382 */
     const int twice = -(ca + cb - 1) * 255;
     const int addend = twice >= 0 ? twice / 2 : -((-twice + 1) / 2);
-    u8_combine_kernel<<<nblocks(total), 256, 0, (cudaStream_t)s>>>((const uint8_t *)a, a_ld, (const uint8_t *)b, b_ld, ca, cb,
+    thb_launch(u8_combine_kernel, nblocks(total), 256, s, (const uint8_t *)a, a_ld, (const uint8_t *)b, b_ld, ca, cb,
                                                                    addend, thr, val, pixels, C, (uint8_t *)y, y_ld);
     return THB_LAUNCH_CHECK("u8_combine_kernel");
 }
@@ -1218,7 +1228,7 @@ int thb_combine(int dtype, int nin, const void *const *x_host, const int *ld_hos
     const int al = thb_channel_align(dtype);
     const long total = pixels * ((C + al - 1) / al);
     if (total == 0) return THB_OK;
-    DISPATCH_FLOAT_DTYPE(dtype, (combine_kernel<T><<<nblocks(total), 256, 0, (cudaStream_t)s>>>(a, pixels, C, (T *)y, y_ld)));
+    DISPATCH_FLOAT_DTYPE(dtype, (thb_launch(combine_kernel<T>, nblocks(total), 256, s, a, pixels, C, (T *)y, y_ld)));
     return THB_LAUNCH_CHECK("combine_kernel");
 }
 
@@ -1228,16 +1238,14 @@ int thb_copy_channels(int dtype, const void *x, long pixels, int C, int x_ld, vo
     const int cvecs = (C + al - 1) / al;
     const long total = pixels * cvecs;
     if (total == 0) return THB_OK;
-    DISPATCH_ANY_DTYPE(dtype, (copy_channels_kernel<T><<<nblocks(total), 256, 0, (cudaStream_t)s>>>(
-                                  (const T *)x, pixels, cvecs, x_ld, (T *)y, y_ld)));
+    DISPATCH_ANY_DTYPE(dtype, (thb_launch(copy_channels_kernel<T>, nblocks(total), 256, s, (const T *)x, pixels, cvecs, x_ld, (T *)y, y_ld)));
     return THB_LAUNCH_CHECK("copy_channels_kernel");
 }
 
 int thb_softmax(int dtype, const void *x, long pixels, int C, int x_ld, void *y, int y_ld, thb_stream s)
 {
     if (pixels == 0) return THB_OK;
-    DISPATCH_FLOAT_DTYPE(dtype, (softmax_kernel<T><<<nblocks(pixels * 32), 256, 0, (cudaStream_t)s>>>(
-                                    (const T *)x, pixels, C, x_ld, (T *)y, y_ld)));
+    DISPATCH_FLOAT_DTYPE(dtype, (thb_launch(softmax_kernel<T>, nblocks(pixels * 32), 256, s, (const T *)x, pixels, C, x_ld, (T *)y, y_ld)));
     return THB_LAUNCH_CHECK("softmax_kernel");
 }
 
@@ -1251,8 +1259,7 @@ int thb_col2im(int dtype, const void *cols, int N, int H, int W, int Cout, int k
     if (total == 0) return THB_OK;
     thb_act a = {THB_ACT_NONE, 0, 0, 0, nullptr};
     if (act) a = *act;
-    DISPATCH_FLOAT_DTYPE(dtype, (col2im_kernel<T><<<nblocks(total), 256, 0, (cudaStream_t)s>>>(
-                                    (const T *)cols, N, H, W, Cout, kH, kW, dH, dW, padH, padW, oH, oW, cols_ld, Cp, beta,
+    DISPATCH_FLOAT_DTYPE(dtype, (thb_launch(col2im_kernel<T>, nblocks(total), 256, s, (const T *)cols, N, H, W, Cout, kH, kW, dH, dW, padH, padW, oH, oW, cols_ld, Cp, beta,
                                     bias, a, (T *)y, y_ld)));
     return THB_LAUNCH_CHECK("col2im_kernel");
 }
@@ -1267,12 +1274,12 @@ int thb_u8_channel_sum_rows(const void *x, long pixels, int C, int x_ld, int W, 
     if (pixels == 0) return THB_OK;
     if (W < 1 || (row_pitch && row_pitch < pad_left + W)) return THB_ERR_ARG;
     if (!row_pitch && C >= 2048 && pixels <= 65535) {
-        u8_channel_sum_wide_kernel<<<(unsigned)pixels, 256, 0, (cudaStream_t)s>>>((const uint8_t *)x, C, x_ld, csum);
+        thb_launch(u8_channel_sum_wide_kernel, (unsigned)pixels, 256, s, (const uint8_t *)x, C, x_ld, csum);
         return THB_LAUNCH_CHECK("u8_channel_sum_wide_kernel");
     }
     const int chunks = (C + 15) / 16;
 #define CSUM_CASE(G)                                                                                                      \
-    u8_channel_sum_kernel<G><<<nblocks(pixels * G), 256, 0, (cudaStream_t)s>>>((const uint8_t *)x, pixels, C, x_ld, W, row_pitch, pad_left, csum)
+    thb_launch(u8_channel_sum_kernel<G>, nblocks(pixels * G), 256, s, (const uint8_t *)x, pixels, C, x_ld, W, row_pitch, pad_left, csum)
     if (chunks <= 1) CSUM_CASE(1);
     else if (chunks <= 2) CSUM_CASE(2);
     else if (chunks <= 4) CSUM_CASE(4);

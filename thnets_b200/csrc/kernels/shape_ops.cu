@@ -24,6 +24,7 @@ template <typename T>
 __global__ void window_copy_kernel(const T *__restrict__ x, int N, int H, int W, int C, int x_ld, int top, int left, int up2,
                                    int oH, int oW, T *__restrict__ y, int y_ld)
 {
+    pdl_enter();
     const int vec = 16 / (int)sizeof(T), chunks = (C + vec - 1) / vec;
     const long total = (long)N * oH * oW * chunks;
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -48,6 +49,7 @@ __global__ void window_copy_kernel(const T *__restrict__ x, int N, int H, int W,
 template <typename T>
 __global__ void channel_slice_kernel(const T *__restrict__ x, long pixels, int from, int C, int x_ld, T *__restrict__ y, int y_ld, int y_pad)
 {
+    pdl_enter();
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= pixels * y_pad) return;
     const int c = (int)(i % y_pad);
@@ -60,6 +62,7 @@ __global__ void channel_slice_kernel(const T *__restrict__ x, long pixels, int f
 template <typename T>
 __global__ void from_nchw_kernel(const T *__restrict__ x, int x_ld, long images_pixels, long HW, int C, T *__restrict__ y, int y_ld, int y_pad)
 {
+    pdl_enter();
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= images_pixels * y_pad) return;
     const int c = (int)(i % y_pad);
@@ -75,6 +78,7 @@ struct MaxIn {
 template <typename T>
 __global__ void cmax_kernel(MaxIn in, int nin, long pixels, int C, T *__restrict__ y, int y_ld, int y_pad)
 {
+    pdl_enter();
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= pixels * y_pad) return;
     const int c = (int)(i % y_pad);
@@ -97,6 +101,7 @@ __global__ void cmax_kernel(MaxIn in, int nin, long pixels, int C, T *__restrict
 template <typename T>
 __global__ void logsoftmax_kernel(const T *__restrict__ x, long pixels, int C, int x_ld, T *__restrict__ y, int y_ld, int quirk)
 {
+    pdl_enter();
     const long p = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (p >= pixels) return;
@@ -116,6 +121,7 @@ __global__ void logsoftmax_kernel(const T *__restrict__ x, long pixels, int C, i
 template <typename T>
 __global__ void sumsq_rows_kernel(const T *__restrict__ x, long row_len, float *__restrict__ out)
 {
+    pdl_enter();
     __shared__ float part[32];
     const T *row = x + (long)blockIdx.x * row_len;
     float s = 0.f;
@@ -137,6 +143,7 @@ template <typename T>
 __global__ void normalize_scale_kernel(const T *__restrict__ x, long rows, long row_len, const float *__restrict__ sums, int per_row,
                                        T *__restrict__ y)
 {
+    pdl_enter();
     __shared__ float total;
     if (!per_row) {
         if (threadIdx.x == 0) {
@@ -161,6 +168,7 @@ template <typename T>
 __global__ void max_unpool_kernel(const T *__restrict__ v, const T *__restrict__ xin, int N, int H, int W, int C, int x_ld, int v_ld,
                                   int kH, int kW, int dH, int dW, int padH, int padW, int oH, int oW, T *__restrict__ y, int y_ld, int y_pad)
 {
+    pdl_enter();
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const long total = (long)N * H * W * y_pad;
     if (i >= total) return;
@@ -212,7 +220,7 @@ int thb_upsample2x(int dtype, const void *x, int N, int H, int W, int C, int x_l
     if (x_ld % vec || y_ld % vec) return THB_ERR_ARG;
     const long total = (long)N * 2 * H * 2 * W * ((C + vec - 1) / vec);
     if (total == 0) return THB_OK;
-    SHAPE_DISPATCH(dtype, (window_copy_kernel<T><<<nblk(total), 256, 0, (cudaStream_t)s>>>((const T *)x, N, H, W, C, x_ld, 0, 0, 1, 2 * H,
+    SHAPE_DISPATCH(dtype, (thb_launch(window_copy_kernel<T>, nblk(total), 256, s, (const T *)x, N, H, W, C, x_ld, 0, 0, 1, 2 * H,
                                                                                            2 * W, (T *)y, y_ld)));
     return THB_LAUNCH_CHECK("window_copy_kernel (upsample)");
 }
@@ -224,7 +232,7 @@ int thb_zero_pad(int dtype, const void *x, int N, int H, int W, int C, int x_ld,
     const int oH = H + pad_t + pad_b, oW = W + pad_l + pad_r;
     if (x_ld % vec || y_ld % vec || oH < 1 || oW < 1) return THB_ERR_ARG;
     const long total = (long)N * oH * oW * ((C + vec - 1) / vec);
-    SHAPE_DISPATCH(dtype, (window_copy_kernel<T><<<nblk(total), 256, 0, (cudaStream_t)s>>>((const T *)x, N, H, W, C, x_ld, -pad_t, -pad_l, 0,
+    SHAPE_DISPATCH(dtype, (thb_launch(window_copy_kernel<T>, nblk(total), 256, s, (const T *)x, N, H, W, C, x_ld, -pad_t, -pad_l, 0,
                                                                                            oH, oW, (T *)y, y_ld)));
     return THB_LAUNCH_CHECK("window_copy_kernel (zero padding)");
 }
@@ -237,7 +245,7 @@ int thb_reflect_pad(int dtype, const void *x, int N, int H, int W, int C, int x_
     if (x_ld % vec || y_ld % vec || pad_l < 0 || pad_r < 0 || pad_t < 0 || pad_b < 0 || pad_t >= H || pad_b >= H || pad_l >= W || pad_r >= W)
         return THB_ERR_ARG;
     const long total = (long)N * oH * oW * ((C + vec - 1) / vec);
-    SHAPE_DISPATCH(dtype, (window_copy_kernel<T><<<nblk(total), 256, 0, (cudaStream_t)s>>>((const T *)x, N, H, W, C, x_ld, -pad_t, -pad_l, 2,
+    SHAPE_DISPATCH(dtype, (thb_launch(window_copy_kernel<T>, nblk(total), 256, s, (const T *)x, N, H, W, C, x_ld, -pad_t, -pad_l, 2,
                                                                                            oH, oW, (T *)y, y_ld)));
     return THB_LAUNCH_CHECK("window_copy_kernel (reflection padding)");
 }
@@ -247,7 +255,7 @@ int thb_slice_channels(int dtype, const void *x, long pixels, int from, int C, i
     const int al = dtype == THB_F32 ? 4 : 8, y_pad = (C + al - 1) / al * al;
     if (pixels == 0) return THB_OK;
     if (from < 0 || C < 1 || y_pad > y_ld) return THB_ERR_ARG;
-    SHAPE_DISPATCH(dtype, (channel_slice_kernel<T><<<nblk(pixels * y_pad), 256, 0, (cudaStream_t)s>>>((const T *)x, pixels, from, C, x_ld,
+    SHAPE_DISPATCH(dtype, (thb_launch(channel_slice_kernel<T>, nblk(pixels * y_pad), 256, s, (const T *)x, pixels, from, C, x_ld,
                                                                                                       (T *)y, y_ld, y_pad)));
     return THB_LAUNCH_CHECK("channel_slice_kernel");
 }
@@ -257,7 +265,7 @@ int thb_from_nchw(int dtype, const void *x, int N, int H, int W, int C, int x_ld
     const int al = dtype == THB_F32 ? 4 : 8, y_pad = (C + al - 1) / al * al;
     const long HW = (long)H * W;
     if (N < 1 || C < 1 || HW < 1 || y_pad > y_ld || (long)C * HW > x_ld) return THB_ERR_ARG;
-    SHAPE_DISPATCH(dtype, (from_nchw_kernel<T><<<nblk(N * HW * y_pad), 256, 0, (cudaStream_t)s>>>((const T *)x, x_ld, N * HW, HW, C, (T *)y,
+    SHAPE_DISPATCH(dtype, (thb_launch(from_nchw_kernel<T>, nblk(N * HW * y_pad), 256, s, (const T *)x, x_ld, N * HW, HW, C, (T *)y,
                                                                                                  y_ld, y_pad)));
     return THB_LAUNCH_CHECK("from_nchw_kernel");
 }
@@ -269,14 +277,14 @@ int thb_cmax(int dtype, int nin, const void *const *x_host, const int *ld_host, 
     if (pixels == 0) return THB_OK;
     MaxIn in;
     for (int k = 0; k < nin; k++) { in.x[k] = x_host[k]; in.ld[k] = ld_host[k]; }
-    SHAPE_DISPATCH(dtype, (cmax_kernel<T><<<nblk(pixels * y_pad), 256, 0, (cudaStream_t)s>>>(in, nin, pixels, C, (T *)y, y_ld, y_pad)));
+    SHAPE_DISPATCH(dtype, (thb_launch(cmax_kernel<T>, nblk(pixels * y_pad), 256, s, in, nin, pixels, C, (T *)y, y_ld, y_pad)));
     return THB_LAUNCH_CHECK("cmax_kernel");
 }
 
 int thb_logsoftmax(int dtype, const void *x, long pixels, int C, int x_ld, void *y, int y_ld, int first_frame_quirk, thb_stream s)
 {
     if (pixels == 0) return THB_OK;
-    SHAPE_DISPATCH(dtype, (logsoftmax_kernel<T><<<nblk(pixels * 32), 256, 0, (cudaStream_t)s>>>((const T *)x, pixels, C, x_ld, (T *)y, y_ld,
+    SHAPE_DISPATCH(dtype, (thb_launch(logsoftmax_kernel<T>, nblk(pixels * 32), 256, s, (const T *)x, pixels, C, x_ld, (T *)y, y_ld,
                                                                                                 first_frame_quirk)));
     return THB_LAUNCH_CHECK("logsoftmax_kernel");
 }
@@ -284,10 +292,10 @@ int thb_logsoftmax(int dtype, const void *x, long pixels, int C, int x_ld, void 
 int thb_l2_normalize(int dtype, const void *x, long rows, long row_len, int per_row, float *scratch_rows, void *y, thb_stream s)
 {
     if (rows < 1 || row_len < 1) return THB_OK;
-    SHAPE_DISPATCH(dtype, (sumsq_rows_kernel<T><<<(unsigned)rows, 256, 0, (cudaStream_t)s>>>((const T *)x, row_len, scratch_rows)));
+    SHAPE_DISPATCH(dtype, (thb_launch(sumsq_rows_kernel<T>, (unsigned)rows, 256, s, (const T *)x, row_len, scratch_rows)));
     int rc = THB_LAUNCH_CHECK("sumsq_rows_kernel");
     if (rc) return rc;
-    SHAPE_DISPATCH(dtype, (normalize_scale_kernel<T><<<nblk(rows * row_len), 256, 0, (cudaStream_t)s>>>((const T *)x, rows, row_len,
+    SHAPE_DISPATCH(dtype, (thb_launch(normalize_scale_kernel<T>, nblk(rows * row_len), 256, s, (const T *)x, rows, row_len,
                                                                                                         scratch_rows, per_row, (T *)y)));
     return THB_LAUNCH_CHECK("normalize_scale_kernel");
 }
@@ -299,7 +307,7 @@ int thb_max_unpool(int dtype, const void *v, int v_ld, const void *pool_in, int 
     const long total = (long)N * H * W * y_pad;
     if (total == 0) return THB_OK;
     if (kH < 1 || kW < 1 || dH < 1 || dW < 1 || y_pad > y_ld) return THB_ERR_ARG;
-    SHAPE_DISPATCH(dtype, (max_unpool_kernel<T><<<nblk(total), 256, 0, (cudaStream_t)s>>>((const T *)v, (const T *)pool_in, N, H, W, C, x_ld,
+    SHAPE_DISPATCH(dtype, (thb_launch(max_unpool_kernel<T>, nblk(total), 256, s, (const T *)v, (const T *)pool_in, N, H, W, C, x_ld,
                                                                                           v_ld, kH, kW, dH, dW, padH, padW, oH, oW, (T *)y,
                                                                                           y_ld, y_pad)));
     return THB_LAUNCH_CHECK("max_unpool_kernel");
