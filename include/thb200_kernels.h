@@ -141,6 +141,11 @@ int thb_conv_splitk_plan(const thb_conv_desc *d, size_t *scratch_bytes);
  * split that suits this tile count (1: none); thb_conv_few_supported: the kernel of few tiles takes this convolution. */
 int thb_conv_few_splits(const thb_conv_desc *d);
 int thb_conv_few_supported(const thb_conv_desc *d);
+/* A network's last convolution (F16 / BF16) with its result as NCHW fp32, rounded through the 16-bit type, in device or pinned
+ * host memory: the convolution and thb_postprocess_status in one launch.  *status_out: 0 before the call; set when this launch or
+ * one before it (d->status) gave up a wait. */
+int thb_conv_nchw_supported(const thb_conv_desc *d);
+int thb_conv_nchw_fwd(const thb_conv_desc *d, const void *x, float *y_nchw, int *status_out, thb_stream s);
 
 /* Convolution + epilogue as above (no residual) + max pooling with a pk x pk window (2 or 3), stride 2 and padding ppad
  * in ONE launch: the convolution's own output is never written, only the [N][pH][pW][y_ld] pooled tensor.  Replaces

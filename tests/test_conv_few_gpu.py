@@ -87,3 +87,23 @@ def test_few_tiles(lib, case, dtype, monkeypatch):
     finally:
         monkeypatch.undo()
         lib.thb_conv_reload_knobs()
+
+
+@pytest.mark.parametrize("dtype", [K.THB_F16, K.THB_BF16], ids=["fp16", "bf16"])
+@pytest.mark.parametrize("case", [(2, 48, 12, 20, 21, 1, 1, 0), (1, 64, 9, 15, 70, 3, 1, 1), (3, 128, 8, 16, 33, 1, 1, 0)])
+def test_result_as_nchw_floats(lib, case, dtype):
+    """A last convolution that leaves NCHW floats: the bits of the 16-bit result, transposed and widened."""
+    n, cin, h, w, cout, k, s, p = case
+    rng = np.random.default_rng(3)
+    x = rounded(rng.standard_normal((n, cin, h, w)).astype(np.float32), dtype).numpy()
+    wt = rounded((rng.standard_normal((cout, cin, k, k)) * (cin * k * k) ** -0.5).astype(np.float32), dtype).numpy()
+    conv = G.Conv(lib, dtype, x.shape, wt, (s, s), (p, p))
+    conv.set_affine(rng.uniform(0.5, 1.5, cout), rng.standard_normal(cout), host_copies=True)
+    conv.set_act(K.ACT_THRESHOLD)
+    xt, _ = G.to_nhwc(x, dtype)
+    want = G.from_nhwc(conv.run(xt), cout)
+    out, status = torch.zeros(want.shape, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    lib.thb_conv_nchw_fwd.argtypes = [C.c_void_p] * 5
+    assert lib.thb_conv_nchw_fwd(C.byref(conv.d), G.ptr(xt), G.ptr(out), G.ptr(status), None) == 0
+    torch.cuda.synchronize()
+    assert int(status[0]) == 0 and np.array_equal(out.cpu().numpy(), want)

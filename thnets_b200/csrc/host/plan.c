@@ -148,6 +148,7 @@ typedef struct instance {
     /* Sliced start: a large batch is copied in `slices` parts on a stream of its own, and the first `prefix` launches run on
      * each part as it arrives (set up by choose_slices; 0: the launches wait for the whole batch) */
     int prefix, slices;
+    int head; /* the last launch is a convolution that can leave its result as NCHW floats: no boundary kernel out */
     double hidden_us; /* modelled gain */
     cudaStream_t copy_stream;
     cudaEvent_t ev_slice;
@@ -1541,6 +1542,20 @@ static double model_us(const step *s)
     return us > b ? us : b;
 }
 
+/* The network's last launch as one that writes NCHW floats itself (thb_conv_nchw_fwd)?  For maps: a segmentation network's
+ * classifier, whose scores are the largest tensor of the forward, written once instead of three times.  Not where the layer
+ * shares its reduction among CTAs or is a Linear (one position per image: nothing to transpose). */
+static int plan_head(const instance *I)
+{
+    const step *s = I->nsteps ? &I->steps[I->nsteps - 1] : 0;
+    const char *off = getenv("THB200_NO_HEAD");
+    if (!s || (off && atoi(off)) || s->kind != ST_CONV || s->dual || s->pool_k || s->scratch_buf >= 0 || s->conv.splits > 1 ||
+        s->in_off0 || s->out_off0 || s->out_coff || s->out_buf != I->out_val.buf || I->out_val.coff || s->conv.Cout != I->out_val.s.C ||
+        s->conv.oH * s->conv.oW < 32)
+        return 0;
+    return thb_conv_nchw_supported(&s->conv);
+}
+
 /* microseconds of a slice's input on its way to the device (measured: 55 GB/s from pinned memory) */
 static double copy_in_us(const thb_engine *E, const instance *I)
 {
@@ -1566,7 +1581,7 @@ static void choose_slices(thb_engine *E, instance *I)
     for (int m = 2; m <= 8 && m <= I->slice_n / 2; m++) {
         double us = 0;
         int p = 0;
-        while (p < I->nsteps && us < t_in && sliceable(I, &I->steps[p])) {
+        while (p < I->nsteps - I->head && us < t_in && sliceable(I, &I->steps[p])) {
             const double k = model_us(&I->steps[p]);
             if (k > 0 && k < 6 * m) break;
             us += k;
@@ -1662,14 +1677,18 @@ static void instance_free(instance *I)
     memset(I, 0, sizeof(*I));
 }
 
-/* `whole`: the instance computes all of its GPU's images (not one of the pipelined sub-batches of them) */
-static int instance_build(thb_engine *E, instance *I, int device, int slice_off, int slice_n, int whole)
+/* `sub`: -1 when the instance computes all of its GPU's images, else which of the pipelined sub-batches of them.  An earlier
+ * sub-batch's kernels come first where two compete for the SMs: its result can leave while the later ones are computed. */
+static int instance_build(thb_engine *E, instance *I, int device, int slice_off, int slice_n, int sub)
 {
     thb_model *M = E->model;
     memset(I, 0, sizeof(*I));
     I->device = device; I->slice_off = slice_off; I->slice_n = slice_n;
     CU(cudaSetDevice(device));
-    CU(cudaStreamCreateWithFlags(&I->stream, cudaStreamNonBlocking));
+    int prio_lo = 0, prio_hi = 0;
+    CU(cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi));
+    const int prio = sub < 0 ? prio_lo : prio_hi + sub < prio_lo ? prio_hi + sub : prio_lo;
+    CU(cudaStreamCreateWithPriority(&I->stream, cudaStreamNonBlocking, prio));
     CU(cudaEventCreate(&I->ev0));
     CU(cudaEventCreate(&I->ev1));
     I->d_status = dalloc(E, I, sizeof(int));
@@ -1773,7 +1792,8 @@ static int instance_build(thb_engine *E, instance *I, int device, int slice_off,
         I->out_val = P.val[M->output];
         I->out_shape = I->out_val.s;
         I->out_count = (long)I->out_shape.N * I->out_shape.C * I->out_shape.H * I->out_shape.W;
-        if (whole) choose_slices(E, I);
+        I->head = plan_head(I);
+        if (sub < 0) choose_slices(E, I);
         I->arena_bytes = pack_arena(I);
         I->arena = dalloc(E, I, I->arena_bytes);
         size_t in_bytes = (size_t)slice_n * E->cur->C * E->cur->H * E->cur->W * sizeof(float);
@@ -1938,6 +1958,8 @@ static int exec_step(instance *I, int t, int img0, int cnt)
     return rc ? -1 : 0;
 }
 
+static int head_on(const instance *I) { return I->head && !th_profile && !th_minmax; }
+
 static int run_steps_ev(thb_engine *E, instance *I, cudaEvent_t *evs, int from, int to)
 {
     for (int t = from; t < to; t++) {
@@ -1996,11 +2018,11 @@ static int run_steps(thb_engine *E, instance *I, int from)
         for (int t = 0; t < I->nsteps; t++)
             if (I->steps[t].kind == ST_CONV && I->steps[t].dyn_quant) I->graph_from = t + 1;
         if (I->graph_from < I->prefix) I->graph_from = I->prefix;
-        if (I->graph_from < I->nsteps && !(ng && atoi(ng)) && !th_profile && !th_minmax) {
+        if (I->graph_from < I->nsteps - I->head && !(ng && atoi(ng)) && !th_profile && !th_minmax) {
             cudaGraph_t g = 0;
             if (cudaStreamBeginCapture(I->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
                 const int l0 = thb_kernel_launch_count();
-                const int rc = run_steps_ev(E, I, 0, I->graph_from, I->nsteps);
+                const int rc = run_steps_ev(E, I, 0, I->graph_from, I->nsteps - I->head);
                 I->graph_launches = thb_kernel_launch_count() - l0; /* kernels in the graph (its memset nodes are not launches) */
                 thb_count_launches(-I->graph_launches);             /* they have not run yet: the replay below counts them */
                 const cudaError_t ce = cudaStreamEndCapture(I->stream, &g);
@@ -2020,14 +2042,14 @@ static int run_steps(thb_engine *E, instance *I, int from)
         thb_set_error("graph launch failed: %s", cudaGetErrorString(cudaGetLastError()));
         return -1;
     }
-    return run_steps_ev(E, I, 0, from, I->nsteps);
+    return run_steps_ev(E, I, 0, from, I->nsteps - head_on(I));
 }
 
 static int lowp_input_range(thb_engine *E, instance *set, int G, int has_x, int cp, int C, int H, int W, const float *mean,
                             const float *std, float *q_sub, float *q_mult);
 static int boundary_in(thb_engine *E, instance *I, int img0, int n, int has_x, int inplace, int cp, int bgr, int C, int H, int W,
                        const float *mean, const float *std, float q_sub, float q_mult);
-static int boundary_out(thb_engine *E, instance *I, float *dst);
+static int boundary_out(thb_engine *E, instance *I, float *dst, int head);
 
 /* Per-launch device times of one forward on the first GPU from the batch staged by the last THProcess* call (events
  * around every launch on the launching stream, averaged over `iters` passes).  Entry 0 is the boundary kernel in
@@ -2052,7 +2074,7 @@ int thb_engine_profile(thb_engine *E, int iters, int max_steps, int *kinds, floa
         if (!rc) rc = boundary_in(E, I, 0, I->slice_n, E->last_has_x, 0, E->last_cp, E->last_bgr, E->cur->C, E->cur->H, E->cur->W, E->last_mean, E->last_std, q_sub, q_mult);
         cudaEventRecord(evs[1], I->stream);
         if (!rc) rc = run_steps_ev(E, I, evs + 1, 0, I->nsteps);
-        if (!rc) rc = boundary_out(E, I, I->d_out);
+        if (!rc) rc = boundary_out(E, I, I->d_out, 0);
         cudaEventRecord(evs[total], I->stream);
         if (cudaStreamSynchronize(I->stream) != cudaSuccess) rc = -1;
         for (int t = 0; t < n && !rc; t++) {
@@ -2301,7 +2323,7 @@ static int plan_build(thb_engine *E)
     for (int g = 0; g < G; g++) {
         int off, n;
         thb_slice_batch(N, G, g, &off, &n);
-        if (instance_build(E, &E->cur->inst[g], dev0 + g, off, n, 1)) return -1;
+        if (instance_build(E, &E->cur->inst[g], dev0 + g, off, n, -1)) return -1;
     }
     /* gather target: GPU 0 holds the whole result when peer copies are usable */
     if (G > 1 && E->cur->peer_gather) {
@@ -2358,7 +2380,7 @@ static int pipe_build(thb_engine *E, int S)
                 n = (sn * cut[c + 1] + 8) / 16 - off;
             } else
                 thb_slice_sub_batches(E->cur->inst[g].slice_n, S, c, &off, &n);
-            if (instance_build(E, &E->cur->pipe[g * S + c], E->cur->inst[g].device, E->cur->inst[g].slice_off + off, n, 0)) return -1;
+            if (instance_build(E, &E->cur->pipe[g * S + c], E->cur->inst[g].device, E->cur->inst[g].slice_off + off, n, c)) return -1;
         }
     E->cur->pipe_built = G * S;
     E->cur->pipe_chunks = S;
@@ -2451,9 +2473,20 @@ static int boundary_in(thb_engine *E, instance *I, int img0, int n, int has_x, i
     return 0;
 }
 
-/* The boundary kernel out: the network's last tensor -> NCHW fp32 at `dst`. */
-static int boundary_out(thb_engine *E, instance *I, float *dst)
+/* The boundary kernel out: the network's last tensor -> NCHW fp32 at `dst`; `head`: the network's last launch has not run yet
+ * and does it itself. */
+static int boundary_out(thb_engine *E, instance *I, float *dst, int head)
 {
+    if (head) {
+        /* (directly, not from the graph: where the result goes may change from call to call) */
+        step *s = &I->steps[I->nsteps - 1];
+        if (s->nin > 1) s->conv.res = bufptr(I, s->in_buf[1], s->in_coff[1], s->dtype);
+        if (thb_conv_nchw_fwd(&s->conv, bufptr(I, s->in_buf[0], s->in_coff[0], s->dtype), dst, I->h_status, I->stream)) {
+            thb_set_error("the last convolution's launch failed: %s", thb_last_cuda_error());
+            return -1;
+        }
+        return 0;
+    }
     const value *ov = &I->out_val;
     float inv = ov->q_mult ? (float)(1.0 / ov->q_mult) : 0;
     if (thb_postprocess_status(bufptr(I, ov->buf, ov->coff, E->dtype), E->dtype, ov->s.N, ov->s.H, ov->s.W, ov->s.C, ov->ld,
@@ -2483,7 +2516,7 @@ static int device_forward(thb_engine *E, instance *I, int has_x, int inplace, in
     }
     CU(cudaEventRecord(I->ev0, I->stream));
     if (run_steps(E, I, 0)) return -1;
-    return boundary_out(E, I, dst);
+    return boundary_out(E, I, dst, head_on(I));
 }
 
 /* 1 when `p` is ordinary (pageable) host memory: a copy from it is staged by the driver at a fraction of the link rate and
@@ -2596,7 +2629,7 @@ static void stage_planes_normalised(float *dst, float *src, long p0, long p1, in
 }
 
 /* bytes staged per copy to the device, and up to which size a result is written to the host by the kernel that makes it */
-static const size_t STAGE_PIECE = (size_t)4 << 20, DIRECT_RESULT_BYTES = (size_t)2 << 20;
+static const size_t STAGE_PIECE = (size_t)4 << 20, DIRECT_RESULT_BYTES = (size_t)16 << 20;
 
 typedef struct {
     float *x;               /* NCHW floats, or */
@@ -2680,7 +2713,7 @@ int thb_engine_forward(thb_engine *E, float *x, unsigned char **images, int stri
     float *gather = E->cur->built > 1 && peer_gather ? E->cur->inst[0].d_out : 0;
     const int dev0 = E->cur->inst[0].device;
     /* A small result is written by the boundary kernel into the pinned result buffer itself, which saves the copy that would
-     * otherwise start when the kernels have ended (about 6 us for a few kilobytes). */
+     * otherwise start when the kernels have ended (about 6 us for a few kilobytes as for 15 MB). */
     long total = 0;
     for (int g = 0; g < G; g++) total += set[g].out_count;
     const int direct = !gather && (size_t)total * sizeof(float) <= DIRECT_RESULT_BYTES;
@@ -2756,7 +2789,7 @@ int thb_engine_forward(thb_engine *E, float *x, unsigned char **images, int stri
             for (int k = 0; k < g; k++) off += set[k].out_count;
             float *dst = gather && I->device == dev0 ? gather + off : direct ? E->h_out + off : I->d_out;
             if (sliced) {
-                if (run_steps(E, I, I->prefix) || boundary_out(E, I, dst)) return -1;
+                if (run_steps(E, I, I->prefix) || boundary_out(E, I, dst, head_on(I))) return -1;
             } else if (device_forward(E, I, x != 0, inplace, cp, bgr, C, H, W, mean, std, q_sub, q_mult,
                                       x && inplace ? x + (size_t)I->slice_off * img_elems : 0, dst)) return -1;
             CU(cudaEventRecord(I->ev1, I->stream));

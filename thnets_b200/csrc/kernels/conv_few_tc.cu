@@ -32,6 +32,8 @@ constexpr int RECV_BYTES = BM * BN * 4;  // the partial columns a CTA receives, 
 
 struct FewParams {
     uint8_t *y;
+    float *y_nchw;             // not null: the result goes here as NCHW floats (device or pinned host memory) instead of to y
+    const int *prev_status;    // with y_nchw: the status word of the launches before, passed on to `status` when set
     const uint8_t *res;
     const float *scale, *shift, *slope;
     int P, oW, oHW, dH, dW, padH, padW, kW, Cout, out_ld, res_ld, nkb, n_tiles;
@@ -47,6 +49,8 @@ struct FewParams {
     long long wait_limit;
 };
 
+// (a plain store: the word may lie in pinned host memory)
+__device__ __forceinline__ void report(int *status, int code) { *reinterpret_cast<volatile int *>(status) = code; }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ uint32_t cluster_addr(uint32_t smem, uint32_t rank)
@@ -126,6 +130,37 @@ __device__ __forceinline__ void finish_tmem(uint32_t taddr, const uint4 (&rv)[BN
             if (q == j) res = rv[q];
         const uint4 o = finish8<KIND, ACT>(acc, res, j * 8, left - j * 8, k, p);
         if (real && j * 8 < left) *reinterpret_cast<uint4 *>(dst + j * 16) = o;
+    }
+}
+
+// The same for a network's last convolution, whose result leaves as NCHW floats (rounded through the 16-bit type like any
+// other): a warp's lanes are 32 neighbouring pixels of a plane, so every channel is a coalesced 128-byte store.
+template <int KIND, int ACT>
+__device__ __forceinline__ void finish_nchw(uint32_t taddr, const uint4 (&rv)[BN / 8], float *dst, size_t plane, bool real, int left, const Consts &k,
+                                            const FewParams &p)
+{
+#pragma unroll 1
+    for (int j = 0; j < BN / 8 && j * 8 < left; j++) {
+        uint32_t a[8];
+        tmem_ld8(taddr + j * 8, a);
+        tmem_ld_wait();
+        float acc[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) acc[i] = __uint_as_float(a[i]);
+        uint4 res = rv[0];
+#pragma unroll
+        for (int q = 1; q < BN / 8; q++)
+            if (q == j) res = rv[q];
+        const uint4 o = finish8<KIND, ACT>(acc, res, j * 8, left - j * 8, k, p);
+        const uint32_t w[4] = {o.x, o.y, o.z, o.w};
+        if (real) {
+#pragma unroll
+            for (int h = 0; h < 4; h++) {
+                const float2 v = unpack2<KIND>(w[h]);
+                if (j * 8 + 2 * h < left) dst[(j * 8 + 2 * h) * plane] = v.x;
+                if (j * 8 + 2 * h + 1 < left) dst[(j * 8 + 2 * h + 1) * plane] = v.y;
+            }
+        }
     }
 }
 
@@ -216,6 +251,10 @@ __global__ void __launch_bounds__(NTHREADS) conv_few_kernel(const __grid_constan
     const int act = p.act_kind == THB_ACT_NONE ? 0 : p.act_kind == THB_ACT_THRESHOLD && p.act_th == 0.f && p.act_val == 0.f ? 1 : 2;
     bool have = false;
 
+    if (p.prev_status && blockIdx.x == 0 && tid == 0) {
+        const int before = *p.prev_status;
+        if (before) report(p.status, before);
+    }
     if (warp < 4) {
         // the residual of this thread's pixel, asked for before the accumulator is awaited
 #pragma unroll
@@ -226,7 +265,7 @@ __global__ void __launch_bounds__(NTHREADS) conv_few_kernel(const __grid_constan
         }
         have = mbar_wait_bounded(smem_u32(acc_full), 0, p.wait_limit);
         if (!have) {
-            if (lane == 0) atomicExch(p.status, 2);
+            if (lane == 0) report(p.status, 2);
             *abort_flag = 1;
         }
         have = __all_sync(0xffffffffu, have);
@@ -253,7 +292,7 @@ __global__ void __launch_bounds__(NTHREADS) conv_few_kernel(const __grid_constan
             uint32_t ph = 0;
             for (int kb = kb0; kb < kb1; kb++) {
                 if (kb - kb0 >= nst && !mbar_wait_bounded(smem_u32(&empty[s]), ph ^ 1, p.wait_limit)) {
-                    atomicExch(p.status, 3);
+                    report(p.status, 3);
                     *abort_flag = 1;
                     break;
                 }
@@ -282,7 +321,7 @@ __global__ void __launch_bounds__(NTHREADS) conv_few_kernel(const __grid_constan
             uint32_t ph = 0;
             for (int kb = kb0; kb < kb1; kb++) {
                 if (kb - kb0 >= nst && !mbar_wait_bounded(smem_u32(&empty[s]), ph ^ 1, p.wait_limit)) {
-                    atomicExch(p.status, 3);
+                    report(p.status, 3);
                     *abort_flag = 1;
                     break;
                 }
@@ -300,7 +339,7 @@ __global__ void __launch_bounds__(NTHREADS) conv_few_kernel(const __grid_constan
             bool alive = true;
             for (int kb = kb0; kb < kb1; kb++) {
                 if (!mbar_wait_bounded(smem_u32(&full[s]), ph, p.wait_limit)) {
-                    atomicExch(p.status, 4);
+                    report(p.status, 4);
                     *abort_flag = 1;
                     alive = false;
                     break;
@@ -346,6 +385,15 @@ __global__ void __launch_bounds__(NTHREADS) conv_few_kernel(const __grid_constan
             else if (act == 1) finish_parts<KIND, 1>(recv, S, W, rank * W, rv, dst, left, row, consts, p);
             else finish_parts<KIND, 2>(recv, S, W, rank * W, rv, dst, left, row, consts, p);
         }
+    } else if (have && p.y_nchw) {
+        const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16);
+        const bool real = pm < p.P;
+        const int img = pm / p.oHW;
+        float *dst = p.y_nchw + ((size_t)img * p.Cout + n0) * p.oHW + (pm - img * p.oHW);
+        __syncwarp();
+        if (act == 0) finish_nchw<KIND, 0>(taddr, rv, dst, p.oHW, real, p.Cout - n0, consts, p);
+        else if (act == 1) finish_nchw<KIND, 1>(taddr, rv, dst, p.oHW, real, p.Cout - n0, consts, p);
+        else finish_nchw<KIND, 2>(taddr, rv, dst, p.oHW, real, p.Cout - n0, consts, p);
     } else if (have) {
         const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16);
         uint8_t *dst = p.y + ((size_t)pm * p.out_ld + n0) * 2;
@@ -387,12 +435,12 @@ int operand_mode(const thb_conv_desc *d, FewParams &p, int &tmap_mode)
     return thb_im2col_ok(d) && d->Cin_pad % 64 == 0 && d->Ktot_pad == d->kH * d->kW * d->Cin_pad ? 2 : 0;
 }
 
-long tiles_of(const thb_conv_desc *d) { return (((long)d->N * d->oH * d->oW + BM - 1) / BM) * (d->Cout_pad / BN); }
+long tiles_of(const thb_conv_desc *d) { return (((long)d->N * d->oH * d->oW + BM - 1) / BM) * ((d->Cout_pad + BN - 1) / BN); }
 
 bool eligible(const thb_conv_desc *d)
 {
     if (d->dtype != THB_F16 && d->dtype != THB_BF16) return false;
-    if (d->Cout_pad % BN || d->acc_out || d->csum_out || d->splitk_scratch) return false;
+    if ((d->Cout_pad % BN && d->Cout_pad != 32) || d->acc_out || d->csum_out || d->splitk_scratch) return false;
     if (d->in_ld % 8 || d->out_ld % 8 || (d->res && d->res_ld % 8)) return false;
     FewParams p;
     int tm;
@@ -452,7 +500,7 @@ int launch(const CUtensorMap *w, const CUtensorMap *a, const CUtensorMap *a2, co
 extern "C" int thb_conv_few_splits(const thb_conv_desc *d)
 {
     const ThbConvLaunch kn = thb_conv_launch_knobs();
-    if (kn.few_tiles == 0 || !eligible(d)) return 1;
+    if (kn.few_tiles == 0 || !eligible(d) || d->Cout_pad % BN) return 1;
     const long tiles = tiles_of(d);
     const int nkb = d->Ktot_pad / 64;
     int S = 1;
@@ -465,32 +513,34 @@ extern "C" int thb_conv_few_splits(const thb_conv_desc *d)
 // 7.9 / 5.7; 128->512 @28x28, 392: 8.3 / 6.2; 64->256 @56x56, 784: 9.5 / 11.1), and the patch kernel up to one.
 extern "C" int thb_conv_few_supported(const thb_conv_desc *d)
 {
-    if (!eligible(d)) return 0;
+    if (!eligible(d) || d->Cout_pad % BN) return 0;
     if (d->splits > 1) return 1;
     const ThbConvLaunch kn = thb_conv_launch_knobs();
     const long most = kn.few_tiles >= 0 ? kn.few_tiles : (d->kH * d->kW > 1 && thb_conv_patch_supported(d) ? 1 : 4) * (long)kn.sms;
     return tiles_of(d) <= most;
 }
 
-extern "C" int thb_conv_few_fwd(const thb_conv_desc *d, const void *x, void *y, thb_stream s)
+static int few_fwd(const thb_conv_desc *d, const void *x, void *y, float *y_nchw, const int *prev_status, int *status, thb_stream s)
 {
-    if (!d->w || !d->status || !x || !y) return THB_ERR_ARG;
+    if (!d->w || !status || !x || !(y || y_nchw)) return THB_ERR_ARG;
     FewParams p;
     memset(&p, 0, sizeof(p));
     int tmap_mode = 0;
     p.mode = operand_mode(d, p, tmap_mode);
     if (!p.mode || !eligible(d)) return THB_ERR_UNSUPPORTED;
     p.y = (uint8_t *)y;
+    p.y_nchw = y_nchw;
+    p.prev_status = prev_status;
     p.res = (const uint8_t *)d->res; p.res_ld = d->res_ld;
     p.scale = d->scale; p.shift = d->shift; p.slope = d->act.kind == THB_ACT_PRELU ? d->act.slope : nullptr;
     p.P = d->N * d->oH * d->oW; p.oW = d->oW; p.oHW = d->oH * d->oW;
     p.dH = d->dH; p.dW = d->dW; p.padH = d->padH; p.padW = d->padW; p.kW = d->kW;
     p.Cout = d->Cout; p.out_ld = d->out_ld;
     p.nkb = d->Ktot_pad / 64;
-    p.n_tiles = d->Cout_pad / BN;
+    p.n_tiles = (d->Cout_pad + BN - 1) / BN;  // (32 padded channels: the copy fills the missing weight rows with zeros)
     p.self_coef = d->self_coef; p.res_coef = d->res_coef;
     p.act_kind = d->act.kind; p.act_th = d->act.threshold; p.act_val = d->act.value; p.act_alpha = d->act.alpha;
-    p.status = d->status;
+    p.status = status;
     if (p.P <= 0) return THB_OK;
     p.splits = d->splits > 1 ? d->splits : 1;
     if (p.splits != 1 && p.splits != 2 && p.splits != 4 && p.splits != 8) return THB_ERR_ARG;
@@ -529,4 +579,24 @@ extern "C" int thb_conv_few_fwd(const thb_conv_desc *d, const void *x, void *y, 
     const int smem = 1024 + BAR_BYTES + (p.splits > 1 ? RECV_BYTES : 0) + p.stages * STAGE_BYTES;
     cudaStream_t st = (cudaStream_t)s;
     return d->dtype == THB_F16 ? launch<0>(w, a, a2, p, ctas, smem, st) : launch<1>(w, a, a2, p, ctas, smem, st);
+}
+
+extern "C" int thb_conv_few_fwd(const thb_conv_desc *d, const void *x, void *y, thb_stream s)
+{
+    return few_fwd(d, x, y, nullptr, nullptr, d->status, s);
+}
+
+extern "C" int thb_conv_nchw_supported(const thb_conv_desc *d)
+{
+    thb_conv_desc one = *d;
+    one.splits = 0;
+    return eligible(&one) && !d->x2;
+}
+
+extern "C" int thb_conv_nchw_fwd(const thb_conv_desc *d, const void *x, float *y, int *status_out, thb_stream s)
+{
+    if (!thb_conv_nchw_supported(d) || !status_out) return THB_ERR_UNSUPPORTED;
+    thb_conv_desc one = *d;
+    one.splits = 0;
+    return few_fwd(&one, x, nullptr, y, d->status, status_out, s);
 }
