@@ -35,8 +35,26 @@ namespace {
 
 constexpr int BM = 128;                  // pixels per tile (= TMEM lanes)
 constexpr int A_STAGE_BYTES = BM * 128;  // 128 rows of one 128-byte K block
-constexpr int NTHREADS = 480;           // 4 producer/epilogue + 1 TMA + 1 MMA + 2 x 4 epilogue warps + 1 warp of agents
+// 4 producer/epilogue + 1 TMA + 1 MMA + 2 x 4 epilogue warps + 1 warp of agents; uint8 has no agents: that warp and a 16th one
+// are a second TMA and a second MMA warp (ConvTcParams::dual)
+constexpr int nthreads(int kind) { return kind == 2 ? 512 : 480; }
 constexpr int EPI_TILE_BYTES = BM * 128;  // one 128-row x 64-column fp16 tile of the TMA epilogue
+
+// Division of 0 .. 2^31 - 1 by a launch constant: multiply-high, add, shift (the round-up method of Granlund and Montgomery,
+// "Division by invariant integers using multiplication").  The compiler's division by a run-time value is some 25 dependent
+// instructions, and every tile needs three of them before anything else can start.
+struct FastDiv {
+    uint32_t mul, shift;
+    __host__ static FastDiv of(uint32_t d)
+    {
+        FastDiv f;
+        f.shift = 0;
+        while ((1ull << f.shift) < d) f.shift++;
+        f.mul = (uint32_t)((((1ull << f.shift) - d) << 32) / d + 1);
+        return f;
+    }
+    __device__ __forceinline__ int operator()(int n) const { return (int)((__umulhi((uint32_t)n, mul) + (uint32_t)n) >> shift); }
+};
 
 struct ConvTcParams {
     const uint8_t *x;
@@ -44,6 +62,7 @@ struct ConvTcParams {
     const int *kinfo;
     int P, H, W, in_ld, oH, oW, oHW, dH, dW, padH, padW, kH, kW, Cin, Cout, out_ld, nkb, n_kchunks;
     int m_tiles, n_tiles;
+    FastDiv by_ntiles, by_ohw, by_ow;
     const float *scale, *shift, *slope;
     const uint8_t *res;
     int res_ld;
@@ -60,6 +79,10 @@ struct ConvTcParams {
                                // pipeline stage carries both activation tiles and ONE weight tile, and the MMA thread feeds two
                                // accumulators per barrier round: that round costs the thread ~250 cycles whatever it carries,
                                // which a single narrow tile (192-256 tensor cycles per K block) cannot hide.
+    int dual;                  // uint8, TMA modes, BN <= 128: the CTA's even and odd tiles have a TMA warp, an MMA warp and half of
+                               // the stages each.  One tile of a short reduction costs either thread about 0.75 us of its own
+                               // instructions with idle schedulers and over 1.5 us beside three busy epilogue warps, which was
+                               // the whole launch's pace (64->256 1x1 with residual @56x56, 128 images: 42 tiles per SM, 115 us)
     int *csum_out;             // uint8, one column tile: per output pixel the sum of its output bytes (the next layer's channel sums)
     int res_addend;            // uint8 fused residual: the constant of ca*q + cb*r + addend (see thb_u8_combine)
     int u8_classes;            // uint8: > 0 when the border classes of the kernel window ((1 + 2 padH) x (1 + 2 padW) of them)
@@ -230,8 +253,10 @@ struct EpiCursor {
 // the last pixel tile (odd tile count) is a phantom: it is computed from zero-filled loads and never stored.
 template <int BN, bool SPLIT = false> struct TileMap {
     int pair, n_tiles, n_local, last_um, splits, nkb;
+    FastDiv by_ntiles;
     __device__ TileMap(const ConvTcParams &p)
     {
+        by_ntiles = p.by_ntiles;
         pair = p.pair;
         n_tiles = p.n_tiles;
         splits = SPLIT && p.splits > 1 ? p.splits : 1;   // (never with pair mode or a reversed walk)
@@ -253,7 +278,7 @@ template <int BN, bool SPLIT = false> struct TileMap {
     {
         int u = blockIdx.x + (pair ? lt >> 1 : lt) * gridDim.x;
         if (SPLIT && splits > 1) u /= splits;
-        int um = u / n_tiles;
+        int um = by_ntiles(u);
         n0 = (u - um * n_tiles) * BN;
         if (last_um >= 0) um = last_um - um;  // walk the pixel tiles from the end of the tensor
         m0 = (pair ? 2 * um + (lt & 1) : um) * BM;
@@ -532,7 +557,7 @@ __device__ __forceinline__ void epilogue_agent(const ConvTcParams &p, const CUte
 }
 
 template <int KIND, int BN, int STAGES, bool SPLIT>
-__global__ void __launch_bounds__(NTHREADS, 1) conv_tc_kernel(const __grid_constant__ CUtensorMap tmapW, const __grid_constant__ CUtensorMap tmapA,
+__global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid_constant__ CUtensorMap tmapW, const __grid_constant__ CUtensorMap tmapA,
                                                                const __grid_constant__ CUtensorMap tmapY, const __grid_constant__ CUtensorMap tmapR,
                                                                const ConvTcParams p)
 {
@@ -556,7 +581,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) conv_tc_kernel(const __grid_const
     uint8_t *sB = sA + nst * a_stage_bytes;
     uint8_t *stage_buf = sB + nst * B_STAGE_BYTES;
     uint64_t *full = bars, *empty = bars + MAX_STAGES;
-    uint64_t *acc_full = bars + 2 * MAX_STAGES, *acc_empty = acc_full + 4;
+    // uint8: one acc_full barrier per tile modulo 12 (a multiple of the accumulators, of the epilogue groups and of the two MMA
+    // warps).  A group waits on every third tile; on a barrier per accumulator, the tile it finished last would not imply that
+    // the accumulator's previous tile, the OTHER MMA warp's, is complete, and a parity cannot tell that tile's phase from the
+    // one awaited.
+    constexpr int NFULL = KIND == 2 ? 12 : NACC;
+    uint64_t *acc_full = KIND == 2 ? bars + 64 : bars + 2 * MAX_STAGES, *acc_empty = bars + 2 * MAX_STAGES + 4;
     uint64_t *rows_ready = acc_empty + 4, *avail = rows_ready + 9;   // TMA epilogue: a pair per group and tile
     uint64_t *stg_ready = rows_ready, *stg_free = rows_ready + 3;    // staged epilogue: a pair per group
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(avail + 9);
@@ -570,10 +600,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) conv_tc_kernel(const __grid_const
             mbar_init(smem_u32(&full[s]), p.a_tma ? 1 : 128 + 1);
             mbar_init(smem_u32(&empty[s]), 1);
         }
-        for (int b = 0; b < NACC; b++) {
-            mbar_init(smem_u32(&acc_full[b]), 1);
-            mbar_init(smem_u32(&acc_empty[b]), 128);
-        }
+        for (int b = 0; b < NFULL; b++) mbar_init(smem_u32(&acc_full[b]), 1);
+        for (int b = 0; b < NACC; b++) mbar_init(smem_u32(&acc_empty[b]), 128);
         for (int g = 0; g < 9; g++) {
             mbar_init(smem_u32(&rows_ready[g]), 128);
             mbar_init(smem_u32(&avail[g]), 1);
@@ -607,7 +635,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) conv_tc_kernel(const __grid_const
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     }
 
-    if (warp == 14) {
+    if (L::TMA_EPI ? warp == 14 : warp >= 14 && !p.dual) {
         // ================================================================== epilogue agents (TMA epilogue only)
         if constexpr (L::TMA_EPI)
             if (lane < p.epi_groups && !SPLIT)   // (split K: the partial tiles go straight to the fp32 scratch)
@@ -694,16 +722,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) conv_tc_kernel(const __grid_const
         fence_proxy_async_smem();
         if (alive)
             for (int k = (it > LAG ? it - LAG : 0); k < it; k++) mbar_arrive(smem_u32(&full[k % STAGES]));
-    } else if (warp == 4) {
+    } else if (warp == 4 || (KIND == 2 && warp == 14)) {
         // ================================================================== TMA producer: per K block the weight tile
         // and, in the TMA modes, the activation tile (both halves' tiles in pair mode)
         if (lane == 0) {
             const TileMap<BN, SPLIT> map(p);
-            const int halves = pair ? 2 : 1;
-            int ring_s = 0;  // stage and phase in the ring of nst stages
+            const int halves = pair ? 2 : 1, lt_step = KIND == 2 && p.dual ? 2 : halves;
+            const int ring_0 = KIND == 2 && warp == 14 ? nst / 2 : 0, ring_1 = KIND == 2 && p.dual && warp == 4 ? nst / 2 : nst;
+            int ring_s = ring_0;  // stage and phase in this warp's ring of stages
             uint32_t ring_ph = 0;
             bool alive = true;
-            for (int lt = 0; lt < map.n_local && alive; lt += halves) {
+            for (int lt = KIND == 2 && warp == 14 ? 1 : 0; lt < map.n_local && alive; lt += lt_step) {
                 int m0, n0;
                 map.coords(lt, m0, n0);
                 // im2col mode: input position of each half's first output pixel for tap (0, 0)
@@ -711,18 +740,18 @@ __global__ void __launch_bounds__(NTHREADS, 1) conv_tc_kernel(const __grid_const
                 if (p.nkb1 && p.a2_mode == 2)
                     for (int h = 0; h < halves; h++) {   // where the second operand is sampled for each half's first pixel
                         const int m = m0 + h * BM;
-                        in[h] = m / p.oHW;
+                        in[h] = p.by_ohw(m);
                         const int rem = m - in[h] * p.oHW;
-                        const int oh = rem / p.oW;
+                        const int oh = p.by_ow(rem);
                         ih[h] = oh * p.a2_d;
                         iw[h] = (rem - oh * p.oW) * p.a2_d;
                     }
                 if (p.a_tma == 2)
                     for (int h = 0; h < halves; h++) {
                         const int m = m0 + h * BM;
-                        in[h] = m / p.oHW;
+                        in[h] = p.by_ohw(m);
                         const int rem = m - in[h] * p.oHW;
-                        const int oh = rem / p.oW;
+                        const int oh = p.by_ow(rem);
                         ih[h] = oh * p.dH - p.padH;
                         iw[h] = (rem - oh * p.oW) * p.dW - p.tma_padw;
                     }
@@ -740,7 +769,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) conv_tc_kernel(const __grid_const
                 for (int kb = kb0; kb < kb1; kb++) {
                     const int s = ring_s;
                     const uint32_t ph = ring_ph;
-                    if (++ring_s == nst) { ring_s = 0; ring_ph ^= 1; }
+                    if (++ring_s == ring_1) { ring_s = ring_0; ring_ph ^= 1; }
                     if (!mbar_wait_bounded(smem_u32(&empty[s]), ph ^ 1, p.wait_limit)) {
                         atomicExch(p.status, 3);
                         *abort_flag = 1;
@@ -785,15 +814,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) conv_tc_kernel(const __grid_const
             }
         }
         __syncwarp();
-    } else if (warp == 5) {
+    } else if (warp == 5 || (KIND == 2 && warp == 15)) {
         // ================================================================== MMA issuer
         if (lane == 0) {
             const TileMap<BN, SPLIT> map(p);
-            const int halves = pair ? 2 : 1;
-            int ring_s = 0;
+            const int halves = pair ? 2 : 1, lt_step = KIND == 2 && p.dual ? 2 : halves;
+            const int ring_0 = KIND == 2 && warp == 15 ? nst / 2 : 0, ring_1 = KIND == 2 && p.dual && warp == 5 ? nst / 2 : nst;
+            int ring_s = ring_0;
             uint32_t ring_ph = 0;
             bool alive = true;
-            for (int lt = 0; lt < map.n_local && alive; lt += halves) {
+            for (int lt = KIND == 2 && warp == 15 ? 1 : 0; lt < map.n_local && alive; lt += lt_step) {
                 // the accumulators of this unit's local tiles (two in pair mode) must have been drained
                 for (int h = 0; h < halves && alive; h++)
                     if (!mbar_wait_bounded(smem_u32(&acc_empty[(lt + h) % NACC]), (((lt + h) / NACC) & 1) ^ 1, p.wait_limit)) {
@@ -809,7 +839,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) conv_tc_kernel(const __grid_const
                 for (int kb = kb0; kb < kb1; kb++) {
                     const int s = ring_s;
                     const uint32_t ph = ring_ph;
-                    if (++ring_s == nst) { ring_s = 0; ring_ph ^= 1; }
+                    if (++ring_s == ring_1) { ring_s = ring_0; ring_ph ^= 1; }
                     if (!mbar_wait_bounded(smem_u32(&full[s]), ph, p.wait_limit)) {
                         atomicExch(p.status, 4);
                         *abort_flag = 1;
@@ -850,7 +880,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) conv_tc_kernel(const __grid_const
                     tc_commit(smem_u32(&empty[s]));
                 }
                 if (alive)
-                    for (int h = 0; h < halves; h++) tc_commit(smem_u32(&acc_full[(lt + h) % NACC]));
+                    for (int h = 0; h < halves; h++) tc_commit(smem_u32(&acc_full[(lt + h) % NFULL]));
             }
         }
         __syncwarp();
@@ -884,7 +914,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) conv_tc_kernel(const __grid_const
         for (int lt = grp; alive; lt += ngrp) {
             const int tile = blockIdx.x + lt * gridDim.x;
             if (tile >= total_tiles) break;
-            const int m0 = (tile / p.n_tiles) * BM, n0 = (tile % p.n_tiles) * BN;
+            const int tile_m = p.by_ntiles(tile), m0 = tile_m * BM, n0 = (tile - tile_m * p.n_tiles) * BN;
             const int ab = lt % NACC;  // accumulator holding this tile
             const uint32_t lane_addr = lane_base + ab * BN;
             const int pm = m0 + row;
@@ -894,8 +924,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) conv_tc_kernel(const __grid_const
             int corr_pix = 0, r0 = 0, r1 = 0, s0 = 0, s1 = 0, plane_pos = 0;
             bool interior = true;
             if (KIND == 2 && valid) {
-                const int n = pm / p.oHW, rem = pm - n * p.oHW;
-                const int oh = rem / p.oW, ow = rem - oh * p.oW;
+                const int n = p.by_ohw(pm), rem = pm - n * p.oHW;
+                const int oh = p.by_ow(rem), ow = rem - oh * p.oW;
                 plane_pos = rem;
                 const int ihb = oh * p.dH - p.padH, iwb = ow * p.dW - p.padW;
                 r0 = max(0, -ihb); r1 = min(p.kH, p.H - ihb);
@@ -903,8 +933,19 @@ __global__ void __launch_bounds__(NTHREADS, 1) conv_tc_kernel(const __grid_const
                 interior = r0 == 0 && s0 == 0 && r1 == p.kH && s1 == p.kW;
                 int xsum = 0;
                 const int *cs = p.csum + (size_t)n * p.H * p.W;
-                for (int r = r0; r < r1; r++)
-                    for (int s = s0; s < s1; s++) xsum += __ldg(cs + (ihb + r) * p.W + iwb + s);
+                if (p.kH <= 4 && p.kW <= 4) {
+                    // all of the window's sums asked for before any is added (a loop over the window pays a latency per tap)
+                    int v[16];
+#pragma unroll
+                    for (int r = 0; r < 4; r++)
+#pragma unroll
+                        for (int s = 0; s < 4; s++)
+                            v[r * 4 + s] = r >= r0 && r < r1 && s >= s0 && s < s1 ? __ldg(cs + (ihb + r) * p.W + iwb + s) : 0;
+#pragma unroll
+                    for (int i = 0; i < 16; i++) xsum += v[i];
+                } else
+                    for (int r = r0; r < r1; r++)
+                        for (int s = s0; s < s1; s++) xsum += __ldg(cs + (ihb + r) * p.W + iwb + s);
                 const int nvalid = max(0, r1 - r0) * max(0, s1 - s0);
                 corr_pix = p.a_off * (xsum + p.b_off * nvalid * p.Cin);
             }
@@ -985,7 +1026,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) conv_tc_kernel(const __grid_const
                     }
                 }
                 if (!have_acc) {
-                    if (!mbar_wait_bounded(smem_u32(&acc_full[ab]), (lt / NACC) & 1, p.wait_limit)) {
+                    if (!mbar_wait_bounded(smem_u32(&acc_full[lt % NFULL]), (lt / NFULL) & 1, p.wait_limit)) {
                         if (lane == 0) atomicExch(p.status, 2);
                         *abort_flag = 1;
                         alive = false;
@@ -1166,14 +1207,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) conv_tc_kernel(const __grid_const
                 // ---- phase 2: coalesced write-out of the staged block
                 if (KIND == 2) {
                     // the warp's own 32 rows, 16-byte chunks: each instruction stores whole rows' worth of contiguous bytes
-                    constexpr int CPR = SUBN / 16;
+                    constexpr int CPR = SUBN / 16, RPU = 32 / CPR;  // chunks per row, rows per instruction
+                    const int r = quad * 32 + lane / CPR, cg2 = lane % CPR;
+                    if (nsub0 + cg2 * 16 < p.Cout) {
+                        uint8_t *dst = p.y + (size_t)(m0 + r) * p.out_ld + nsub0 + cg2 * 16;
+                        const uint8_t *src = stg + r * (SUBN + 16) + cg2 * 16;
+                        const int rows = p.P - (m0 + r);  // rows from this one to the end of the tensor
 #pragma unroll
-                    for (int u = 0; u < CPR; u++) {
-                        const int idx = lane + u * 32, r = quad * 32 + idx / CPR, cg2 = idx % CPR;
-                        const int pm2 = m0 + r, c0 = nsub0 + cg2 * 16;
-                        if (pm2 < p.P && c0 < p.Cout)
-                            *reinterpret_cast<uint4 *>(p.y + (size_t)pm2 * p.out_ld + c0) =
-                                *reinterpret_cast<const uint4 *>(stg + r * (SUBN + 16) + cg2 * 16);
+                        for (int u = 0; u < CPR; u++)
+                            if (u * RPU < rows)
+                                *reinterpret_cast<uint4 *>(dst + (size_t)(u * RPU) * p.out_ld) =
+                                    *reinterpret_cast<const uint4 *>(src + u * RPU * (SUBN + 16));
                     }
                     __syncwarp();
                 } else if (c0f < p.Cout) {
@@ -1265,7 +1309,7 @@ __global__ void __launch_bounds__(256) splitk_finish_kernel(const ConvTcParams p
 // Diagnostic launcher switches (THB200_* environment variables), read ONCE: a launch costs no getenv call.
 // thb_conv_reload_knobs() re-reads them (the tests change them between cases).  -1 = not set.
 struct ConvKnobs {
-    int pair_min_kb, u8_fast, reverse, epi_groups, epi_bufs, pdl, conv_l1, half_taps, a_tma, test_withhold, few_tiles, few_stages;
+    int pair_min_kb, u8_fast, reverse, epi_groups, epi_bufs, pdl, conv_l1, half_taps, a_tma, test_withhold, few_tiles, few_stages, dual;
     long pair_min_units;
     long long wait_limit;
 };
@@ -1292,6 +1336,7 @@ void read_knobs()
     g_knobs.test_withhold = env_int("THB200_TEST_WITHHOLD", 0);
     g_knobs.few_tiles = env_int("THB200_FEW_TILES", -1);
     g_knobs.few_stages = env_int("THB200_FEW_STAGES", -1);
+    g_knobs.dual = env_int("THB200_U8_DUAL", 1);
     const char *wl = getenv("THB200_WAIT_LIMIT_CYCLES");
     g_knobs.wait_limit = wl && atoll(wl) > 0 ? atoll(wl) : 4000000000ll;
     g_knobs_read = true;
@@ -1370,6 +1415,7 @@ int launch_tc(const ConvTmaps &tm, ConvTcParams p, cudaStream_t st)
     // multiple of the column tiles every CTA stays on one column tile (148 -> 144 CTAs for 8 or 16 column tiles)
     if (KIND == 2 && p.u8_classes > 0 && p.n_tiles > 1 && tiles > grid && grid % p.n_tiles && grid > 2 * p.n_tiles && knobs().u8_fast != 2)
         grid -= grid % p.n_tiles;
+    p.dual = KIND == 2 && p.a_tma && BN <= 128 && kn.dual && (long)p.m_tiles * p.n_tiles >= 2L * num_sms();
     if (!L::TMA_EPI) {
         // staged epilogue: uint8 with nothing to gather runs a third group on warps 0-3 (a fourth accumulator exists below 256 columns)
         p.epi_groups = KIND == 2 && p.a_tma && BN < 256 ? 3 : 2;
@@ -1402,7 +1448,7 @@ int launch_tc(const ConvTmaps &tm, ConvTcParams p, cudaStream_t st)
     p.test_withhold = kn.test_withhold && p.a_tma;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(NTHREADS);
+    cfg.blockDim = dim3(nthreads(KIND));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -1430,7 +1476,7 @@ int dispatch_bn(int BN, const ConvTmaps &tm, const ConvTcParams &p, cudaStream_t
 {
     switch (BN) {
     case 32: return launch_tc<KIND, 32, 6>(tm, p, st);
-    case 64: return launch_tc<KIND, 64, 5>(tm, p, st);
+    case 64: return launch_tc<KIND, 64, KIND == 2 ? 6 : 5>(tm, p, st);
     case 128: return launch_tc<KIND, 128, 4>(tm, p, st);
     case 256: return launch_tc<KIND, 256, 3>(tm, p, st);
     }
@@ -1728,6 +1774,9 @@ extern "C" int thb_conv_fwd_tc(const thb_conv_desc *d, const void *x, void *y, t
     if (p.P <= 0) return THB_OK;
     p.m_tiles = (p.P + BM - 1) / BM;
     p.n_tiles = d->Cout_pad / d->BN;
+    p.by_ntiles = FastDiv::of((uint32_t)p.n_tiles);
+    p.by_ohw = FastDiv::of((uint32_t)p.oHW);
+    p.by_ow = FastDiv::of((uint32_t)p.oW);
     const CUtensorMap &tm = *reinterpret_cast<const CUtensorMap *>(d->tmap);
     const CUtensorMap *ta = &tm;
     // a 1x1 stride-1 unpadded convolution (and every Linear) reads a plain [pixels][Cin] matrix: TMA loads it
