@@ -84,6 +84,7 @@ struct ConvTcParams {
                                // instructions with idle schedulers and over 1.5 us beside three busy epilogue warps, which was
                                // the whole launch's pace (64->256 1x1 with residual @56x56, 128 images: 42 tiles per SM, 115 us)
     int *csum_out;             // uint8, one column tile: per output pixel the sum of its output bytes (the next layer's channel sums)
+    int y_sector;              // uint8: every 32 channels of the output start on a 32-byte boundary
     int res_addend;            // uint8 fused residual: the constant of ca*q + cb*r + addend (see thb_u8_combine)
     int u8_classes;            // uint8: > 0 when the border classes of the kernel window ((1 + 2 padH) x (1 + 2 padW) of them)
                                // fit the epilogue's shared-memory table; 0: every row looks its window up in global memory
@@ -911,6 +912,26 @@ __global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid
         const uint32_t bar_tbl = smem_u32(&rows_ready[6 + grp]);
         int tbl_n0 = -1;
         uint32_t tbl_phase = 0;
+        // uint8: what a tile reads from memory is asked for one step ahead -- the residual bytes of the next 32 columns under the
+        // arithmetic of the current ones, and at a tile's end those of the next tile with its channel sum (1x1 layers, where that
+        // is one word).  Waiting for each where it is used took 5000 of a tile's 13700 cycles.
+        uint4 next0 = make_uint4(0, 0, 0, 0), next1 = next0;
+        int next_xsum = 0;
+        const bool plain_sum = KIND == 2 && p.a_tma == 1;
+        auto fetch_res = [&](int pix, int col) {  // 32 bytes of pixel `pix` from channel `col` on
+            if (p.res && col < p.res_ld) {
+                const uint8_t *r = p.res + (size_t)(pix < p.P ? pix : 0) * p.res_ld + col;
+                next0 = __ldg(reinterpret_cast<const uint4 *>(r));
+                if (col + 16 < p.res_ld) next1 = __ldg(reinterpret_cast<const uint4 *>(r + 16));
+            }
+        };
+        auto fetch_tile = [&](int tile) {
+            if (tile >= total_tiles) return;
+            const int tm = p.by_ntiles(tile), pix = tm * BM + row;
+            fetch_res(pix, (tile - tm * p.n_tiles) * BN);
+            if (plain_sum) next_xsum = pix < p.P ? __ldg(p.csum + pix) : 0;
+        };
+        if (KIND == 2) fetch_tile(blockIdx.x + grp * gridDim.x);
         for (int lt = grp; alive; lt += ngrp) {
             const int tile = blockIdx.x + lt * gridDim.x;
             if (tile >= total_tiles) break;
@@ -933,7 +954,8 @@ __global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid
                 interior = r0 == 0 && s0 == 0 && r1 == p.kH && s1 == p.kW;
                 int xsum = 0;
                 const int *cs = p.csum + (size_t)n * p.H * p.W;
-                if (p.kH <= 4 && p.kW <= 4) {
+                if (plain_sum) xsum = next_xsum;
+                else if (p.kH <= 4 && p.kW <= 4) {
                     // all of the window's sums asked for before any is added (a loop over the window pays a latency per tap)
                     int v[16];
 #pragma unroll
@@ -1066,16 +1088,12 @@ __global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid
                     const int *b2row = tbl + L::TBL_CAP + 256 + sb * (SUBN / 2);
                     // the common case per warp: no tail row, Threshold replaces by its own threshold byte (or none)
                     const bool general = __any_sync(0xffffffffu, e.tailmask != 0) || (p.relu_thr >= 0 && p.relu_val != p.relu_thr);
-                    const uint8_t *rrow = p.res + (size_t)(valid ? pm : 0) * p.res_ld + nsub0;
 #pragma unroll 1
                     for (int cc = 0; cc < SUBN / 32; cc++) {
                         uint32_t acc[32];
-                        uint4 res0 = make_uint4(0, 0, 0, 0), res1 = res0;
-                        if (u8res && nsub0 + cc * 32 < p.res_ld) {
-                            // residual bytes of this row: issued before the accumulator wait
-                            res0 = __ldg(reinterpret_cast<const uint4 *>(rrow + cc * 32));
-                            if (nsub0 + cc * 32 + 16 < p.res_ld) res1 = __ldg(reinterpret_cast<const uint4 *>(rrow + cc * 32 + 16));
-                        }
+                        const uint4 res0 = next0, res1 = next1;
+                        if (sb * SUBN + cc * 32 + 32 < BN) fetch_res(pm, nsub0 + cc * 32 + 32);
+                        else fetch_tile(tile + ngrp * gridDim.x);
                         __syncwarp();
                         tmem_ld32(lane_addr + sb * SUBN + cc * 32, acc);
                         tmem_ld_wait();
@@ -1114,9 +1132,21 @@ __global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid
                         }
 #pragma unroll
                         for (int g4 = 0; g4 < 8; g4++) rowsum = __dp4a(words[g4], 0x01010101u, rowsum);  // (dead code unless csum_out)
-                        uint4 *dst = reinterpret_cast<uint4 *>(stg + row * (SUBN + 16) + cc * 32);
-                        dst[0] = make_uint4(words[0], words[1], words[2], words[3]);
-                        dst[1] = make_uint4(words[4], words[5], words[6], words[7]);
+                        // the thread's 32 bytes are one sector: straight to memory, in one store where they are aligned to it
+                        const int c32 = nsub0 + cc * 32;
+                        if (valid && c32 < p.Cout) {
+                            uint8_t *dst = p.y + (size_t)pm * p.out_ld + c32;
+                            if (c32 + 16 >= p.Cout)
+                                *reinterpret_cast<uint4 *>(dst) = make_uint4(words[0], words[1], words[2], words[3]);
+                            else if (p.y_sector)
+                                asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(words[0]), "r"(words[1]),
+                                             "r"(words[2]), "r"(words[3]), "r"(words[4]), "r"(words[5]), "r"(words[6]), "r"(words[7])
+                                             : "memory");
+                            else {
+                                reinterpret_cast<uint4 *>(dst)[0] = make_uint4(words[0], words[1], words[2], words[3]);
+                                reinterpret_cast<uint4 *>(dst)[1] = make_uint4(words[4], words[5], words[6], words[7]);
+                            }
+                        }
                     }
                 } else if (KIND == 2) {
                     if (p.res && lane == 0) atomicExch(p.status, 9);  // a fused residual exists on the table-driven path only
@@ -1194,6 +1224,7 @@ __global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid
                 }
                 if (KIND == 2) {
                     __syncwarp();
+                    if (fast) continue;  // (stored already)
                 } else {
                     mbar_arrive(bar_ready);
                     if (!mbar_wait_bounded(bar_ready, sub_it & 1, p.wait_limit)) {
@@ -1258,6 +1289,7 @@ __global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid
                 }
                 if (KIND != 2) mbar_arrive(bar_free);
             }
+            if (KIND == 2 && !fast) fetch_tile(tile + ngrp * gridDim.x);
             if (KIND == 2 && alive && p.csum_out && valid) {
                 if (p.n_tiles == 1) p.csum_out[pm] = (int)rowsum;
                 else atomicAdd(p.csum_out + pm, (int)rowsum);  // several column tiles: the buffer was cleared before the launch
@@ -1748,6 +1780,7 @@ extern "C" int thb_conv_fwd_tc(const thb_conv_desc *d, const void *x, void *y, t
     p.act_kind = d->act.kind; p.act_th = d->act.threshold; p.act_val = d->act.value; p.act_alpha = d->act.alpha;
     p.a_off = d->a_offset; p.b_off = d->b_offset; p.c_off = d->c_offset; p.c_mult = d->c_mult; p.c_shift = d->c_shift;
     p.wsat = d->wsat; p.bias_add = d->bias_add; p.csum = d->csum;
+    p.y_sector = (((uintptr_t)y | (uintptr_t)d->out_ld) & 31) == 0;
     if (d->csum_out) {
         if (d->dtype != THB_U8) return THB_ERR_UNSUPPORTED;
         p.csum_out = d->csum_out;
