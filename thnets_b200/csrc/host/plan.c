@@ -74,11 +74,12 @@ typedef struct {
 typedef struct {
     size_t bytes, offset;
     int first, last;
+    int zeroed; /* cleared before every forward, all such buffers at once (they lie at the arena's start) */
 } abuf;
 
 enum step_kind {
     ST_CONV, ST_GEMV, ST_MAXPOOL, ST_AVGPOOL, ST_AFFINE, ST_U8THR, ST_U8COMBINE, ST_COMBINE, ST_COPY, ST_SOFTMAX, ST_COL2IM,
-    ST_CSUM, ST_TO_NCHW, ST_ZERO, ST_UPSAMPLE, ST_ZEROPAD, ST_REFLECTPAD, ST_SLICEC, ST_CMAX, ST_LOGSOFTMAX, ST_NORMALIZE, ST_UNPOOL, ST_FROM_NCHW
+    ST_CSUM, ST_TO_NCHW, ST_UPSAMPLE, ST_ZEROPAD, ST_REFLECTPAD, ST_SLICEC, ST_CMAX, ST_LOGSOFTMAX, ST_NORMALIZE, ST_UNPOOL, ST_FROM_NCHW
 };
 
 typedef struct {
@@ -123,7 +124,7 @@ typedef struct instance {
     void **hostmem; /* host arrays the launches' descriptors point to */
     int nhost, caphost;
     unsigned char *arena;
-    size_t arena_bytes;
+    size_t arena_bytes, zero_bytes; /* the first zero_bytes of the arena are cleared before every forward */
     float *d_in;          /* staged NCHW fp32 input */
     unsigned char *d_img; /* staged u8 HWC images */
     float *d_out;         /* NCHW fp32 result */
@@ -313,6 +314,7 @@ static int new_buf(planner *P, size_t bytes)
     abuf *b = &I->bufs[I->nbufs];
     b->bytes = (bytes + 255) & ~(size_t)255;
     b->offset = 0;
+    b->zeroed = 0;
     b->first = b->last = -1;
     return I->nbufs++;
 }
@@ -896,13 +898,6 @@ static int plan_gemm_group(planner *P, int i)
             if (!is_linear) inw->csum_buf = csum_buf + 1;
         }
     }
-    /* uint8: a place-holder launch in front of the convolution; it becomes the clearing of the output's channel-sum
-     * buffer when the convolution has several column tiles, which then add their partial sums into it */
-    int zero_step = -1;
-    if (dtype == THB_U8 && !is_linear) {
-        new_step(P, ST_ZERO)->pixels = 0;
-        zero_step = P->I->nsteps - 1;
-    }
     step *s = new_step(P, ST_CONV);
     thb_conv_desc *d = &s->conv;
     s->aux_buf = csum_buf;
@@ -1050,14 +1045,12 @@ static int plan_gemm_group(planner *P, int i)
         out->q_sub = out_sub; out->q_mult = out_mult;
         /* one column tile: the epilogue sees every output byte of a pixel and leaves their sum for the next convolution */
         const char *nocs = getenv("THB200_U8_NO_CSUM_OUT");
-        if (!is_linear && zero_step >= 0 && !(nocs && atoi(nocs) == 1) && (d->Cout_pad == d->BN || !(nocs && atoi(nocs) == 2))) {
+        if (!is_linear && !(nocs && atoi(nocs) == 1) && (d->Cout_pad == d->BN || !(nocs && atoi(nocs) == 2))) {
             s->aux2_buf = new_buf(P, sizeof(int) * (size_t)is.N * os.H * os.W);
             out->csum_buf = s->aux2_buf + 1;
-            if (d->Cout_pad != d->BN) {
-                step *z = &P->I->steps[zero_step];
-                z->out_buf = s->aux2_buf;
-                z->pixels = (long)is.N * os.H * os.W;
-            }
+            /* several column tiles add their shares, into a cleared buffer (a clearing launch in front of each of them was a
+             * tenth of a ResNet-50 forward: 2.7 to 6 us, and every one breaks the programmatic launch chain) */
+            P->I->bufs[s->aux2_buf].zeroed = d->Cout_pad != d->BN;
         }
         if (res_node >= 0) {
             const value *rv = &P->val[res_node];
@@ -1521,7 +1514,7 @@ static int sliceable(const instance *I, const step *s)
     switch (s->kind) {
     case ST_CONV: return s->conv.N == I->slice_n && s->scratch_buf < 0 && !s->in_off0 && !s->out_off0;
     case ST_MAXPOOL: return s->N == I->slice_n;
-    case ST_CSUM: case ST_ZERO: return s->pixels % I->slice_n == 0;
+    case ST_CSUM: return s->pixels % I->slice_n == 0;
     default: return 0;
     }
 }
@@ -1632,15 +1625,22 @@ static size_t pack_arena(instance *I)
     if (I->in_val.buf >= 0) I->bufs[I->in_val.buf].first = -1;
     if (I->out_val.buf >= 0) I->bufs[I->out_val.buf].last = I->nsteps;
     size_t top = 0;
+    for (int b = 0; b < I->nbufs; b++)
+        if (I->bufs[b].zeroed) {
+            I->bufs[b].offset = top;
+            top += I->bufs[b].bytes;
+        }
+    I->zero_bytes = top;
     for (int b = 0; b < I->nbufs; b++) {
         abuf *B = &I->bufs[b];
+        if (B->zeroed) continue;
         if (B->last < 0 && b != I->in_val.buf) { B->offset = 0; continue; }
-        size_t off = 0;
+        size_t off = I->zero_bytes;
         for (;;) {
             int moved = 0;
             for (int o = 0; o < b; o++) {
                 abuf *O = &I->bufs[o];
-                if (O->last < 0 && o != I->in_val.buf) continue;
+                if (O->zeroed || (O->last < 0 && o != I->in_val.buf)) continue;
                 int overlap_time = !(O->last < B->first || B->last < O->first);
                 if (overlap_time && off < O->offset + O->bytes && O->offset < off + B->bytes) {
                     off = O->offset + O->bytes;
@@ -1855,9 +1855,9 @@ static int exec_step(instance *I, int t, int img0, int cnt)
             x0 += (size_t)img0 * s->H * s->W * s->in_ld[0] * es;
             y += (size_t)img0 * s->oH * s->oW * s->out_ld * es;
             break;
-        case ST_CSUM: case ST_ZERO: {
+        case ST_CSUM: {
             const long per = s->pixels / I->slice_n;
-            if (s->kind == ST_CSUM) x0 += (size_t)img0 * (s->oW ? per / s->W * s->oW : per) * s->in_ld[0] * es;
+            x0 += (size_t)img0 * (s->oW ? per / s->W * s->oW : per) * s->in_ld[0] * es;
             aux_off = sizeof(int) * (size_t)img0 * per;
             s->pixels = cnt * per;
             break;
@@ -1912,9 +1912,6 @@ static int exec_step(instance *I, int t, int img0, int cnt)
     case ST_COL2IM:
         rc = thb_col2im(dt, x0, s->N, s->H, s->W, s->C, s->kH, s->kW, s->dH, s->dW, s->padH, s->padW, s->oH, s->oW,
                         s->in_ld[0], s->beta, s->bias, &s->act, y, s->out_ld, st);
-        break;
-    case ST_ZERO:
-        if (s->pixels > 0 && cudaMemsetAsync((char *)bufptr(I, s->out_buf, 0, THB_U8) + aux_off, 0, sizeof(int) * (size_t)s->pixels, (cudaStream_t)st) != cudaSuccess) rc = -1;
         break;
     case ST_CSUM:
         rc = thb_u8_channel_sum_rows(x0, s->pixels, s->C, s->in_ld[0], s->W > 0 ? s->W : 1, s->oW, s->padW, (int *)((char *)bufptr(I, s->out_buf, 0, THB_U8) + aux_off), st);
@@ -1971,7 +1968,7 @@ static int run_steps_ev(thb_engine *E, instance *I, cudaEvent_t *evs, int from, 
         if (th_profile) { cudaStreamSynchronize(I->stream); t0 = th_seconds(); }
         if (exec_step(I, t, 0, 0)) return -1;
         if (evs) cudaEventRecord(evs[t + 1], I->stream);
-        if (th_minmax && y && s->out_pixels > 0 && s->out_C > 0 && s->kind != ST_ZERO && s->kind != ST_CSUM) {
+        if (th_minmax && y && s->out_pixels > 0 && s->out_C > 0 && s->kind != ST_CSUM) {
             /* thapi.c:141-154, :197-202: smallest and largest value of every layer's output -- how a caller picks the
              * lowp range.  A diagnostic: the tensor is read back and scanned on the host (uint8 tensors: their bytes). */
             const size_t es = esize_of(dt), bytes = (size_t)s->out_pixels * s->out_ld * es;
@@ -2045,6 +2042,7 @@ static int run_steps(thb_engine *E, instance *I, int from)
     return run_steps_ev(E, I, 0, from, I->nsteps - head_on(I));
 }
 
+static int clear_sums(instance *I);
 static int lowp_input_range(thb_engine *E, instance *set, int G, int has_x, int cp, int C, int H, int W, const float *mean,
                             const float *std, float *q_sub, float *q_mult);
 static int boundary_in(thb_engine *E, instance *I, int img0, int n, int has_x, int inplace, int cp, int bgr, int C, int H, int W,
@@ -2071,6 +2069,7 @@ int thb_engine_profile(thb_engine *E, int iters, int max_steps, int *kinds, floa
         float q_sub = 0, q_mult = 0;
         rc = lowp_input_range(E, E->cur->inst, 1, E->last_has_x, E->last_cp, E->cur->C, E->cur->H, E->cur->W, E->last_mean, E->last_std, &q_sub, &q_mult);
         cudaEventRecord(evs[0], I->stream);
+        if (!rc) rc = clear_sums(I);
         if (!rc) rc = boundary_in(E, I, 0, I->slice_n, E->last_has_x, 0, E->last_cp, E->last_bgr, E->cur->C, E->cur->H, E->cur->W, E->last_mean, E->last_std, q_sub, q_mult);
         cudaEventRecord(evs[1], I->stream);
         if (!rc) rc = run_steps_ev(E, I, evs + 1, 0, I->nsteps);
@@ -2431,6 +2430,13 @@ static int lowp_input_range(thb_engine *E, instance *set, int G, int has_x, int 
     return 0;
 }
 
+/* the buffers the uint8 convolutions add their channel sums into, before a forward's first launch */
+static int clear_sums(instance *I)
+{
+    if (I->zero_bytes) CU(cudaMemsetAsync(I->arena, 0, I->zero_bytes, I->stream));
+    return 0;
+}
+
 /* The boundary kernel in: images [img0, img0 + n) of the staged input (I->d_in: NCHW fp32, or I->d_img: HWC bytes) -> the
  * engine's layout and type. */
 static int boundary_in(thb_engine *E, instance *I, int img0, int n, int has_x, int inplace, int cp, int bgr, int C, int H, int W,
@@ -2501,7 +2507,7 @@ static int boundary_out(thb_engine *E, instance *I, float *dst, int head)
 static int device_forward(thb_engine *E, instance *I, int has_x, int inplace, int cp, int bgr, int C, int H, int W,
                           const float *mean, const float *std, float q_sub, float q_mult, float *writeback, float *dst)
 {
-    if (boundary_in(E, I, 0, I->slice_n, has_x, inplace, cp, bgr, C, H, W, mean, std, q_sub, q_mult)) return -1;
+    if (clear_sums(I) || boundary_in(E, I, 0, I->slice_n, has_x, inplace, cp, bgr, C, H, W, mean, std, q_sub, q_mult)) return -1;
     if (writeback) {
         /* the normalised values go back to the caller on a stream of their own: the link is full duplex and the forward does
          * not wait for them (the caller does, before THProcessFloat returns) */
@@ -2777,6 +2783,7 @@ int thb_engine_forward(thb_engine *E, float *x, unsigned char **images, int stri
                         if (send_images(E, I, &src, i0, cnt, I->copy_stream)) return -1;
                         CU(cudaEventRecord(I->ev_slice, I->copy_stream));
                         CU(cudaStreamWaitEvent(I->stream, I->ev_slice, 0));
+                        if (c == 0 && clear_sums(I)) return -1;
                         if (boundary_in(E, I, i0, cnt, x != 0, 0, cp, bgr, C, H, W, mean, std, q_sub, q_mult)) return -1;
                         if (c == 0) CU(cudaEventRecord(I->ev0, I->stream));
                         for (int t = 0; t < I->prefix; t++)
