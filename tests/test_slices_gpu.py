@@ -54,3 +54,32 @@ def test_sliced_start(th, tmp_path, mode, images, net, batch, size):
     else:
         x = rng.standard_normal((batch, 3, size, size), dtype=np.float32)
     assert np.array_equal(run(th, path, mode, x, images, True), run(th, path, mode, x, images, False))
+
+
+@pytest.mark.parametrize("net,batch,size", [("resnet18", 5, 97), ("resnet18", 66, 224), ("vgg16", 40, 224)])
+@pytest.mark.parametrize("nan", [False, True], ids=["finite", "nan"])
+def test_uint8_range_found_by_the_host(th, tmp_path, net, batch, size, nan):
+    """A uint8 forward of a float batch with the range found by the host's threads (six or more of them) under the copy, its
+    first launches sliced, against the range found by the device after it."""
+    import ctypes
+    omp = ctypes.CDLL("libgomp.so.1")
+    g = fx.vgg16(width=0.25, classes=10, fc=64) if net == "vgg16" else fx.resnet18(width=0.25, size=size, classes=10, fc_bias=0.05)
+    path = str(tmp_path / "n.net")
+    fx.write_pymodel(g, path)
+    x = np.random.default_rng(batch).standard_normal((batch, 3, size, size), dtype=np.float32)
+    if nan:
+        x[batch // 2, 1, 7, 7:11] = np.nan
+    outs = []
+    for threads in (8, 2):
+        omp.omp_set_num_threads(threads)
+        try:
+            h = th.load_network(path)
+            th.set_stats(h, (0.45, 0.4, 0.5), (0.225, 0.25, 0.2))
+            net_h = th.create_lowp_network(h, 8.0)
+            th.free_network(h)
+            outs += [th.process_float(net_h, x)[0] for _ in range(3)]
+            th.free_network(net_h)
+        finally:
+            omp.omp_set_num_threads(4)
+    for o in outs[1:]:
+        assert np.array_equal(o, outs[0])

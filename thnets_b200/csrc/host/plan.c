@@ -152,7 +152,7 @@ typedef struct instance {
     int head; /* the last launch is a convolution that can leave its result as NCHW floats: no boundary kernel out */
     double hidden_us; /* modelled gain */
     cudaStream_t copy_stream;
-    cudaEvent_t ev_slice;
+    cudaEvent_t ev_slice[8];
     int input_s2d; /* the network input is staged space-to-depth by this factor, the stride of the first convolution (0: as it is) */
     int input_neigh; /* uint8 engine, 3x3 / stride 1 / pad 1 first convolution on a three-plane float batch: the boundary kernel
                       * stages every pixel's 27 quantised neighbours as the channels of that pixel (taps outside the image: the
@@ -1507,6 +1507,11 @@ static int plan_node(planner *P, int i)
     return -1;
 }
 
+/* The uint8 engine needs the range of a whole float batch before it can start.  Several host threads read the batch faster than
+ * the link carries it, so they find the range while it is on its way; a few would take longer than the copy and a pass of the
+ * device over it. */
+static int host_scans(void) { return omp_get_max_threads() >= 6; }
+
 /* Can launch `s` run on some of its images?  (The planned convolutions and poolings whose images are independent; what
  * they add is the image offset of every operand, exec_step.) */
 static int sliceable(const instance *I, const step *s)
@@ -1566,7 +1571,7 @@ static double copy_in_us(const thb_engine *E, const instance *I)
 static void choose_slices(thb_engine *E, instance *I)
 {
     I->prefix = I->slices = 0;
-    if ((E->dtype == THB_U8 && !E->cur->cp) || E->cur->cp == 2 || E->whole_batch || I->in_val.buf < 0) return;
+    if ((E->dtype == THB_U8 && !E->cur->cp && !host_scans()) || E->cur->cp == 2 || E->whole_batch || I->in_val.buf < 0) return;
     const char *off = getenv("THB200_NO_SLICES");
     if (off && atoi(off)) return;
     const double t_in = copy_in_us(E, I);
@@ -1670,7 +1675,8 @@ static void instance_free(instance *I)
     if (I->ev_wb) cudaEventDestroy(I->ev_wb);
     if (I->wb_stream) cudaStreamDestroy(I->wb_stream);
     if (I->copy_stream) { cudaStreamSynchronize(I->copy_stream); cudaStreamDestroy(I->copy_stream); }
-    if (I->ev_slice) cudaEventDestroy(I->ev_slice);
+    for (int c = 0; c < 8; c++)
+        if (I->ev_slice[c]) cudaEventDestroy(I->ev_slice[c]);
     if (I->stream) cudaStreamDestroy(I->stream);
     thb_host_free_pinned(I->h_status);
     free(I->allocs); free(I->steps); free(I->bufs);
@@ -1801,10 +1807,10 @@ static int instance_build(thb_engine *E, instance *I, int device, int slice_off,
         I->d_img = dalloc(E, I, (size_t)slice_n * E->cur->H * E->cur->W * 4);
         I->d_out = dalloc(E, I, (size_t)(I->out_count ? I->out_count : 1) * sizeof(float));
         if (!I->arena || !I->d_in || !I->d_out || !I->d_img) rc = -1;
-        if (!rc && I->prefix && (cudaStreamCreateWithFlags(&I->copy_stream, cudaStreamNonBlocking) != cudaSuccess ||
-                                 cudaEventCreateWithFlags(&I->ev_slice, cudaEventDisableTiming) != cudaSuccess)) {
-            thb_set_error("stream creation failed");
-            rc = -1;
+        if (!rc && I->prefix) {
+            int bad = cudaStreamCreateWithFlags(&I->copy_stream, cudaStreamNonBlocking) != cudaSuccess;
+            for (int c = 0; c < I->slices; c++) bad |= cudaEventCreateWithFlags(&I->ev_slice[c], cudaEventDisableTiming) != cudaSuccess;
+            if (bad) { thb_set_error("stream creation failed"); rc = -1; }
         }
         /* padded channels are never read as data, but stale NaN/Inf bit patterns would poison the
          * zero-weight products: start from a clean arena */
@@ -2360,6 +2366,63 @@ static int plan_build(thb_engine *E)
     return 0;
 }
 
+static int stage_threads(void);
+
+/* Smallest and largest normalised value of N images, both seeded with 0 (lowp_basic.c:15-29): the extremes of every channel's
+ * planes as they are, and only those normalised -- a subtraction and a division in fp32 are monotone.  NaNs do not count, as in
+ * the device's pass (thb_minmax_normalized). */
+static void host_range(const float *x, int N, int C, long HW, const float *mean, const float *std, float *lo, float *hi)
+{
+    float mn[4] = {INFINITY, INFINITY, INFINITY, INFINITY}, mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+    const long per = 16384, pieces = (HW + per - 1) / per, items = (long)N * C * pieces;
+#pragma omp parallel num_threads(stage_threads()) if (items > 4)
+    {
+        float tmn[4] = {INFINITY, INFINITY, INFINITY, INFINITY}, tmx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma omp for schedule(static) nowait
+        for (long t = 0; t < items; t++) {
+            const long plane = t / pieces, i0 = (t % pieces) * per, i1 = i0 + per < HW ? i0 + per : HW;
+            const int k = plane % C < 3 ? (int)(plane % C) : 3;
+            const float *p = x + plane * HW;
+            float a = tmn[k], b = tmx[k];
+            long i = i0;
+#ifdef __SSE2__
+            /* (min and max with the running value as second operand keep it when the new one is a NaN) */
+            __m128 a0 = _mm_set1_ps(a), a1 = a0, b0 = _mm_set1_ps(b), b1 = b0;
+            for (; i + 8 <= i1; i += 8) {
+                const __m128 u = _mm_loadu_ps(p + i), v = _mm_loadu_ps(p + i + 4);
+                a0 = _mm_min_ps(u, a0); b0 = _mm_max_ps(u, b0);
+                a1 = _mm_min_ps(v, a1); b1 = _mm_max_ps(v, b1);
+            }
+            float va[8], vb[8];
+            _mm_storeu_ps(va, a0); _mm_storeu_ps(va + 4, a1); _mm_storeu_ps(vb, b0); _mm_storeu_ps(vb + 4, b1);
+            for (int q = 0; q < 8; q++) {
+                if (va[q] < a) a = va[q];
+                if (vb[q] > b) b = vb[q];
+            }
+#endif
+            for (; i < i1; i++) {
+                if (p[i] < a) a = p[i];
+                if (p[i] > b) b = p[i];
+            }
+            tmn[k] = a; tmx[k] = b;
+        }
+#pragma omp critical
+        for (int k = 0; k < 4; k++) {
+            if (tmn[k] < mn[k]) mn[k] = tmn[k];
+            if (tmx[k] > mx[k]) mx[k] = tmx[k];
+        }
+    }
+    *lo = *hi = 0;
+    for (int k = 0; k < 4; k++) {
+        if (!(mn[k] <= mx[k])) continue;
+        float a = mn[k], b = mx[k];
+        if (k < 3) { a = (a - mean[k]) / std[k]; b = (b - mean[k]) / std[k]; }
+        if (a > b) { const float t = a; a = b; b = t; }
+        if (a < *lo) *lo = a;
+        if (b > *hi) *hi = b;
+    }
+}
+
 static int g_chunks_override; /* 0 = the engine's own choice */
 void thb_set_pipeline_chunks(int n) { g_chunks_override = n < 0 ? 0 : n > 4 ? 4 : n; }
 
@@ -2397,6 +2460,14 @@ static void set_dynamic_quant(instance *I, float in_sub, float in_mult)
     }
 }
 
+/* every instance's first convolution gets the parameters that follow from the batch's extremes */
+static void set_input_range(instance *set, int G, float lo, float hi, float *q_sub, float *q_mult)
+{
+    *q_sub = lo;
+    *q_mult = hi - lo > 0 ? (float)(255.0 / (hi - lo)) : 0;
+    for (int g = 0; g < G; g++) set_dynamic_quant(&set[g], *q_sub, *q_mult);
+}
+
 /* The uint8 engine's input range.  A float batch: lowp_basic.c:15-29 takes one range over the WHOLE batch tensor, so
  * the slices' extremes are reduced on the host (one 8-byte read-back per GPU) and every instance's first convolution
  * gets the parameters that follow from it.  Byte images: the loader's range is static (lowp_basic.c:82-131), nothing
@@ -2424,9 +2495,7 @@ static int lowp_input_range(thb_engine *E, instance *set, int G, int has_x, int 
         if (I->h_minmax[0] < lo) lo = I->h_minmax[0];
         if (I->h_minmax[1] > hi) hi = I->h_minmax[1];
     }
-    *q_sub = lo;
-    *q_mult = hi - lo > 0 ? (float)(255.0 / (hi - lo)) : 0;
-    for (int g = 0; g < G; g++) set_dynamic_quant(&set[g], *q_sub, *q_mult);
+    set_input_range(set, G, lo, hi, q_sub, q_mult);
     return 0;
 }
 
@@ -2760,38 +2829,43 @@ int thb_engine_forward(thb_engine *E, float *x, unsigned char **images, int stri
     E->last_has_x = x != 0; E->last_cp = cp; E->last_bgr = bgr;
     for (int k = 0; k < 3; k++) { E->last_mean[k] = mean[k]; E->last_std[k] = std[k]; }
 
-    /* The uint8 engine needs the input range of the whole float batch before any kernel can start: it stages every slice, then
-     * measures, then launches (byte images come with a static range).  The other modes launch a slice's kernels as soon as its copy is queued. */
-    const int two_phase = E->dtype == THB_U8 && x;
+    /* The uint8 engine needs the input range of the whole float batch before any kernel can start: it sends every slice on its
+     * way, then measures, then launches (byte images come with a static range).  The other modes launch a slice's kernels as soon
+     * as its copy is queued. */
+    const int two_phase = E->dtype == THB_U8 && x, scan = two_phase && host_scans();
     cudaEvent_t ev_call = 0;
     if (th_debug > 1 && cudaSetDevice(set[0].device) == cudaSuccess && cudaEventCreate(&ev_call) == cudaSuccess)
         cudaEventRecord(ev_call, set[0].stream);
-    for (int phase = 0; phase < 2; phase++) {
+    for (int phase = 0; phase <= two_phase; phase++) {
         if (phase == 1) {
-            if (!two_phase) break;
-            if (lowp_input_range(E, set, G, x != 0, cp, C, H, W, mean, std, &q_sub, &q_mult)) return -1;
+            if (scan) {
+                float lo, hi;
+                host_range(x, N, C, (long)H * W, mean, std, &lo, &hi);
+                set_input_range(set, G, lo, hi, &q_sub, &q_mult);
+            } else if (lowp_input_range(E, set, G, x != 0, cp, C, H, W, mean, std, &q_sub, &q_mult)) return -1;
         }
         for (int g = 0; g < G; g++) {
             instance *I = &set[g];
             CU(cudaSetDevice(I->device));
-            const int sliced = S == 1 && I->slices && !two_phase && !inplace && !th_profile && !th_minmax;
-            if (phase == 0) {
-                if (sliced) {
-                    for (int c = 0; c < I->slices; c++) {
-                        int i0, cnt;
-                        slice_part(I, c, &i0, &cnt);
-                        if (send_images(E, I, &src, i0, cnt, I->copy_stream)) return -1;
-                        CU(cudaEventRecord(I->ev_slice, I->copy_stream));
-                        CU(cudaStreamWaitEvent(I->stream, I->ev_slice, 0));
-                        if (c == 0 && clear_sums(I)) return -1;
-                        if (boundary_in(E, I, i0, cnt, x != 0, 0, cp, bgr, C, H, W, mean, std, q_sub, q_mult)) return -1;
-                        if (c == 0) CU(cudaEventRecord(I->ev0, I->stream));
-                        for (int t = 0; t < I->prefix; t++)
-                            if (exec_step(I, t, i0, cnt)) return -1;
-                    }
-                } else if (send_images(E, I, &src, 0, I->slice_n, I->stream)) return -1;
-                if (two_phase) continue;
+            const int sliced = S == 1 && I->slices && two_phase == scan && !inplace && !th_profile && !th_minmax;
+            for (int c = 0; sliced && c < I->slices; c++) {
+                int i0, cnt;
+                slice_part(I, c, &i0, &cnt);
+                if (phase == 0) {
+                    if (send_images(E, I, &src, i0, cnt, I->copy_stream)) return -1;
+                    CU(cudaEventRecord(I->ev_slice[c], I->copy_stream));
+                }
+                if (phase == two_phase) {
+                    CU(cudaStreamWaitEvent(I->stream, I->ev_slice[c], 0));
+                    if (c == 0 && clear_sums(I)) return -1;
+                    if (boundary_in(E, I, i0, cnt, x != 0, 0, cp, bgr, C, H, W, mean, std, q_sub, q_mult)) return -1;
+                    if (c == 0) CU(cudaEventRecord(I->ev0, I->stream));
+                    for (int t = 0; t < I->prefix; t++)
+                        if (exec_step(I, t, i0, cnt)) return -1;
+                }
             }
+            if (phase == 0 && !sliced && send_images(E, I, &src, 0, I->slice_n, I->stream)) return -1;
+            if (phase != two_phase) continue;
             long off = 0;
             for (int k = 0; k < g; k++) off += set[k].out_count;
             float *dst = gather && I->device == dev0 ? gather + off : direct ? E->h_out + off : I->d_out;
