@@ -2518,8 +2518,8 @@ static int boundary_in(thb_engine *E, instance *I, int img0, int n, int has_x, i
     float *d_in = I->d_in + (size_t)img0 * C * H * W;
     const unsigned char *d_img = I->d_img + (size_t)img0 * H * W * cp;
     const int f = I->input_s2d, W2 = f ? (W + f - 1) / f : 0, pitch = iv->row_pitch ? iv->row_pitch : W2;
-    /* (even sides and stride 2 in the 16-bit modes have kernels of their own) */
-    if (f && (E->dtype == THB_U8 || f != 2 || ((H | W) & 1))) {
+    /* (float batches with even sides and stride 2 in the 16-bit modes have a kernel of their own) */
+    if (f && (!has_x || E->dtype == THB_U8 || f != 2 || ((H | W) & 1))) {
         rc = thb_preprocess_s2d_any(has_x ? (const void *)d_in : d_img, !has_x, inplace ? d_in : 0, n, C, H, W, f, W * cp, bgr, mean, std,
                                     E->dtype, in_ptr, iv->ld, pitch, iv->pad_left, &q_sub, &q_mult, I->stream);
         if (!has_x && E->dtype == THB_U8) set_dynamic_quant(I, q_sub, q_mult);
@@ -2539,9 +2539,7 @@ static int boundary_in(thb_engine *E, instance *I, int img0, int n, int has_x, i
         rc = thb_preprocess_images_lowp(d_img, n, H, W, W * cp, bgr, mean, std, in_ptr, I->in_val.ld, &q_sub,
                                         &q_mult, I->stream);
         set_dynamic_quant(I, q_sub, q_mult);
-    } else if (f)
-        rc = thb_preprocess_images_s2d(d_img, n, H, W, W * cp, bgr, mean, std, E->dtype, in_ptr, iv->ld, pitch, iv->pad_left, I->stream);
-    else
+    } else
         rc = thb_preprocess_images(d_img, n, H, W, W * cp, cp, bgr, mean, std, E->dtype, in_ptr,
                                    I->in_val.ld, I->stream);
     if (rc) { thb_set_error("preprocess launch failed: %s", thb_last_cuda_error()); return -1; }
