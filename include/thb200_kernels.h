@@ -136,9 +136,10 @@ int thb_conv_make_tmap(const thb_conv_desc *d, thb_tmap *out);
 int thb_conv_fwd(const thb_conv_desc *d, const void *x, void *y, thb_stream s);
 /* the split count that suits a convolution's tile count (1: none) and the scratch bytes it needs; THB200_NO_SPLITK=1: always 1 */
 int thb_conv_splitk_plan(const thb_conv_desc *d, size_t *scratch_bytes);
-/* The other way to share a reduction (F16 / BF16): with splits = 2, 4 or 8 and no splitk_scratch the S CTAs of a cluster work on
+/* The other way to share a reduction (F16 / BF16; U8, where splits = 1 too selects the kernel and csum_out has to be cleared
+ * when Cout_pad > 64 or splits > 1): with splits = 2, 4 or 8 and no splitk_scratch the S CTAs of a cluster work on
  * one tile and add their parts through distributed shared memory, in rank order, in the same launch.  thb_conv_few_splits: the
- * split that suits this tile count (1: none); thb_conv_few_supported: the kernel of few tiles takes this convolution. */
+ * split that suits this tile count (1: none; U8: 0 when the other kernel is the better one); thb_conv_few_supported: the kernel of few tiles takes this convolution. */
 int thb_conv_few_splits(const thb_conv_desc *d);
 int thb_conv_few_supported(const thb_conv_desc *d);
 /* A network's last convolution (F16 / BF16) with its result as NCHW fp32, rounded through the 16-bit type, in device or pinned

@@ -107,3 +107,36 @@ def test_result_as_nchw_floats(lib, case, dtype):
     assert lib.thb_conv_nchw_fwd(C.byref(conv.d), G.ptr(xt), G.ptr(out), G.ptr(status), None) == 0
     torch.cuda.synchronize()
     assert int(status[0]) == 0 and np.array_equal(out.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("net,size,batch", [("resnet18", 64, 1), ("resnet18", 97, 3), ("resnet50", 64, 2), ("resnet50", 161, 1), ("vgg16", 64, 2)])
+@pytest.mark.parametrize("images", [True, False], ids=["bytes", "floats"])
+def test_uint8_networks(lib, tmp_path, monkeypatch, net, size, batch, images):
+    """uint8 networks whose layers are a few tiles each (3x3, 1x1, strided, half-block taps, residuals, Linear layers; clusters
+    of 1 to 8): the bytes of the persistent kernel."""
+    from thnets_b200 import fixtures as fx
+    from thnets_b200.capi import THNets
+    th = THNets()
+    g = fx.vgg16(size=size, classes=37, fc=200) if net == "vgg16" else getattr(fx, net)(size=size, classes=37, fc_bias=0.05)
+    path = str(tmp_path / "n.net")
+    fx.write_pymodel(g, path)
+    rng = np.random.default_rng(size)
+    x = [rng.integers(0, 256, (size, size, 3), dtype=np.uint8) for _ in range(batch)] if images else g.make_input(batch)
+    outs = []
+    try:
+        for few in (None, "0"):
+            if few:
+                monkeypatch.setenv("THB200_FEW_TILES", few)
+            lib.thb_conv_reload_knobs()
+            h = th.load_network(path)
+            th.set_stats(h, (0.45,) * 3, (0.225,) * 3)
+            handle = th.create_lowp_network(h, 20.0)
+            th.free_network(h)
+            outs += [(th.process_images(handle, x) if images else th.process_float(handle, x))[0] for _ in range(3)]
+            th.free_network(handle)
+    finally:
+        monkeypatch.undo()
+        lib.thb_conv_reload_knobs()
+    assert outs[0].std() > 0
+    for o in outs[1:]:
+        assert np.array_equal(o, outs[0])

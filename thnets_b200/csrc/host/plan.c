@@ -991,6 +991,11 @@ static int plan_gemm_group(planner *P, int i)
         d->splits = thb_conv_few_splits(&whole);
         if (d->splits < 2) d->splits = 0;
     }
+    /* (integer sums: any split gives the same bytes) */
+    if (dtype == THB_U8 && is.N == P->I->slice_n) {
+        d->out_ld = ru(d->Cout, al);
+        d->splits = thb_conv_few_splits(d);
+    }
     if (want_split && pool < 0 && dual_conv < 0 && (dtype == THB_F16 || dtype == THB_BF16) && !thb_conv_patch_supported(d)) {
         /* a launch of few tiles: several CTAs share each tile's reduction, through an fp32 scratch that lives for this launch */
         size_t sk_bytes = 0;
@@ -1050,7 +1055,7 @@ static int plan_gemm_group(planner *P, int i)
             out->csum_buf = s->aux2_buf + 1;
             /* several column tiles add their shares, into a cleared buffer (a clearing launch in front of each of them was a
              * tenth of a ResNet-50 forward: 2.7 to 6 us, and every one breaks the programmatic launch chain) */
-            P->I->bufs[s->aux2_buf].zeroed = d->Cout_pad != d->BN;
+            P->I->bufs[s->aux2_buf].zeroed = d->splits ? (d->Cout_pad + 63) / 64 * d->splits > 1 : d->Cout_pad != d->BN;
         }
         if (res_node >= 0) {
             const value *rv = &P->val[res_node];

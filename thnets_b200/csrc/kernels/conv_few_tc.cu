@@ -1,4 +1,4 @@
-// Tensor-core convolution for launches of few tiles (16-bit types): small batches, the late stages of a network.
+// Tensor-core convolution for launches of few tiles (16-bit types, uint8): small batches, the late stages of a network.
 //
 // What bounds such a layer is not arithmetic or bandwidth but the chain of one tile: with 8 images or fewer a ResNet layer
 // is 1 to 100 tiles, the persistent kernel (conv_tc.cu) runs one of them per SM, and a K block costs the SM's copy engine
@@ -43,7 +43,13 @@ struct FewParams {
     int mode;                  // 1: activations are a plain matrix; 2: im2col-mode copies, `slabs` 128-byte slabs per tap
     int slabs, tma_kw, tma_padw;
     int nkb1, a2_mode, a2_d;   // second activation operand from K block nkb1 on (1: plain matrix, 2: sampled every a2_d pixels)
+    int half, ntaps;           // a tap (a kernel row stored with its padding) is half a K block: two copies of 64-byte rows a block
     int splits, stages, pdl;
+    // uint8: zero-point correction, requantisation, bias and Threshold as in the persistent kernel (conv_tc.cu)
+    int H, W, kH, Cin, a_off, b_off, c_off, c_mult, c_shift, tail_start, relu_thr, relu_val, ca, cb, res_addend;
+    int classes, tbl_bytes;    // border classes of the kernel window, and the bytes their table takes
+    const int *wsat, *bias_add, *csum;
+    int *csum_out;
     int test_withhold;         // tests only: the last K block's activations are never delivered
     int *status;
     long long wait_limit;
@@ -188,11 +194,38 @@ __device__ __forceinline__ void finish_parts(const uint8_t *recv, int S, int W, 
     }
 }
 
+// Eight channels of one pixel in uint8: zero-point correction (the border class's table word times c_mult, the row's own term),
+// gemmlowp requantisation, the reference's saturating bias add with its tail quirk, the fused residual and the Threshold -- the
+// integer arithmetic of the persistent kernel's u8_chunk32.
+struct U8Row {
+    uint32_t rc;
+    int tailmask, thr, shift;
+};
+__device__ __forceinline__ uint2 finish8_u8(const int (&acc)[8], const int *t, const int *b, const U8Row &e, const uint2 &rv, int left,
+                                            const FewParams &p)
+{
+    uint32_t ow[2] = {0, 0};
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const int sres = (int)((uint32_t)acc[i] * (uint32_t)p.c_mult + (uint32_t)t[i] + e.rc) >> e.shift;
+        const int q = min(max(sres, 0), 255), t2 = q + b[i];
+        int v = max(min(max(t2, 0), 255), t2 & e.tailmask);
+        if (p.res) {
+            const int r = (int)(((i < 4 ? rv.x : rv.y) >> (8 * (i & 3))) & 255u);
+            v = min(max(p.ca * v + p.cb * r + p.res_addend, 0), 255);
+        }
+        v = v > e.thr ? v : p.relu_val;
+        if (i < left) ow[i >> 2] |= (uint32_t)v << (8 * (i & 3));
+    }
+    return make_uint2(ow[0], ow[1]);
+}
+
 template <int KIND>
 __global__ void __launch_bounds__(NTHREADS) conv_few_kernel(const __grid_constant__ CUtensorMap tmapW, const __grid_constant__ CUtensorMap tmapA,
                                                             const __grid_constant__ CUtensorMap tmapA2, const FewParams p)
 {
-    constexpr uint32_t IDESC = make_idesc(1u, KIND == 1 ? 1u : 0u, BN);
+    constexpr uint32_t IDESC = make_idesc(KIND == 2 ? 2u : 1u, KIND == 1 ? 1u : 0u, BN);
+    constexpr int KE = KIND == 2 ? 128 : 64;  // elements of a K block
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t *full = reinterpret_cast<uint64_t *>(smem), *empty = full + MAX_STAGES, *acc_full = empty + MAX_STAGES;
@@ -203,6 +236,8 @@ __global__ void __launch_bounds__(NTHREADS) conv_few_kernel(const __grid_constan
     // (every CTA of a cluster has the same layout, so an offset into this one's receive buffer fits its peers' too)
     uint8_t *recv = smem + BAR_BYTES;
     uint8_t *ring = recv + (p.splits > 1 ? RECV_BYTES : 0);
+    int *tbl = reinterpret_cast<int *>(ring), *bias = reinterpret_cast<int *>(smem + 192);  // uint8
+    if (KIND == 2) ring += p.tbl_bytes;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int S = p.splits, nst = p.stages;
@@ -220,7 +255,19 @@ __global__ void __launch_bounds__(NTHREADS) conv_few_kernel(const __grid_constan
         fence_barrier_init();
         fence_proxy_async_smem();
     }
-    if (tid < BN) {  // (weights, like the packed matrix: no launch of the forward writes them)
+    if (KIND == 2) {
+        // T[class][channel] = b_off * (sum of the channel's weights over the taps inside the image) * c_mult
+        const int ncc = 1 + 2 * p.padW, satw = p.kW + 1, satn = (p.kH + 1) * satw;
+        for (int i = tid; i < p.classes * BN; i += NTHREADS) {
+            const int k = i / BN, c = min(n0 + i % BN, p.Cout - 1), rc = k / ncc, cc = k - rc * ncc;
+            const int r0 = rc <= p.padH ? rc : 0, r1 = rc > p.padH ? p.kH - (rc - p.padH) : p.kH;
+            const int s0 = cc <= p.padW ? cc : 0, s1 = cc > p.padW ? p.kW - (cc - p.padW) : p.kW;
+            const int *t = p.wsat + (size_t)c * satn;
+            tbl[i] = (int)((uint32_t)(p.b_off * (__ldg(t + r1 * satw + s1) - __ldg(t + r0 * satw + s1) - __ldg(t + r1 * satw + s0) +
+                                                 __ldg(t + r0 * satw + s0))) * (uint32_t)p.c_mult);
+        }
+        if (tid < BN) bias[tid] = p.bias_add ? __ldg(p.bias_add + min(n0 + tid, p.Cout - 1)) : 0;
+    } else if (tid < BN) {  // (weights, like the packed matrix: no launch of the forward writes them)
         const float self = p.res ? p.self_coef : 1.f;
         consts.sc[tid] = (p.scale ? __ldg(p.scale + n0 + tid) : 1.f) * self;
         consts.sh[tid] = (p.shift ? __ldg(p.shift + n0 + tid) : 0.f) * self;
@@ -245,6 +292,9 @@ __global__ void __launch_bounds__(NTHREADS) conv_few_kernel(const __grid_constan
     if (p.pdl && warp != 5) asm volatile("griddepcontrol.wait;" ::: "memory");
 
     uint4 rv[BN / 8];
+    uint2 r8[BN / 8];   // uint8
+    U8Row u8 = {0, 0, -1, 0};
+    const int *trow = tbl;
     const int row = tid;  // epilogue threads: pixel row of the tile = TMEM lane
     const int pm = m0 + row;
     const int wshift = S == 1 ? 6 : S == 2 ? 5 : S == 4 ? 4 : 3, W = 1 << wshift, c_first = n0 + rank * W, cout8 = (p.Cout + 7) & ~7;  // the channels this CTA finishes
@@ -260,8 +310,37 @@ __global__ void __launch_bounds__(NTHREADS) conv_few_kernel(const __grid_constan
 #pragma unroll
         for (int j = 0; j < BN / 8; j++) {
             rv[j] = make_uint4(0, 0, 0, 0);
-            if (p.res && pm < p.P && j * 8 < W && c_first + j * 8 < cout8)
+            if (KIND != 2 && p.res && pm < p.P && j * 8 < W && c_first + j * 8 < cout8)
                 rv[j] = __ldg(reinterpret_cast<const uint4 *>(p.res + ((size_t)pm * p.res_ld + c_first + j * 8) * 2));
+        }
+        if (KIND == 2) {
+#pragma unroll
+            for (int j = 0; j < BN / 8; j++) {
+                r8[j] = make_uint2(0, 0);
+                if (p.res && pm < p.P && j * 8 < W && c_first + j * 8 < cout8)
+                    r8[j] = __ldg(reinterpret_cast<const uint2 *>(p.res + (size_t)pm * p.res_ld + c_first + j * 8));
+            }
+            const int pc = min(pm, p.P - 1), n = pc / p.oHW, rem = pc - n * p.oHW, oh = rem / p.oW, ow = rem - oh * p.oW;
+            const int ihb = oh * p.dH - p.padH, iwb = ow * p.dW - p.padW;
+            const int r0 = max(0, -ihb), r1 = min(p.kH, p.H - ihb), s0 = max(0, -iwb), s1 = min(p.kW, p.W - iwb);
+            const int cb = p.kH - r1, cr = p.kW - s1;  // (clipped on one side at most: the launcher checks)
+            trow = tbl + ((r0 > 0 ? r0 : cb > 0 ? p.padH + cb : 0) * (1 + 2 * p.padW) + (s0 > 0 ? s0 : cr > 0 ? p.padW + cr : 0)) * BN + rank * W;
+            const int *cs = p.csum + ((size_t)n * p.H + ihb) * p.W + iwb;
+            int xsum = 0;
+            if (p.kH <= 4 && p.kW <= 4) {
+#pragma unroll
+                for (int i = 0; i < 16; i++) {
+                    const int r = i >> 2, q = i & 3;
+                    xsum += r >= r0 && r < r1 && q >= s0 && q < s1 ? __ldg(cs + r * p.W + q) : 0;
+                }
+            } else
+                for (int r = r0; r < r1; r++)
+                    for (int q = s0; q < s1; q++) xsum += __ldg(cs + r * p.W + q);
+            const int corr = p.a_off * (xsum + p.b_off * (r1 - r0) * (s1 - s0) * p.Cin);
+            u8.shift = max(p.c_shift, 0);
+            u8.rc = (uint32_t)(corr + p.c_off) * (uint32_t)p.c_mult + (p.c_shift >= 1 ? 1u << (p.c_shift - 1) : 0u);
+            u8.tailmask = rem < p.tail_start ? 0 : 255;
+            u8.thr = p.relu_thr;
         }
         have = mbar_wait_bounded(smem_u32(acc_full), 0, p.wait_limit);
         if (!have) {
@@ -278,8 +357,8 @@ __global__ void __launch_bounds__(NTHREADS) conv_few_kernel(const __grid_constan
                 const int rem = m0 - in * p.oHW, oh = rem / p.oW;
                 ih = oh * p.dH - p.padH;
                 iw = (rem - oh * p.oW) * p.dW - p.tma_padw;
-                const int tap = kb0 / p.slabs;
-                slab = kb0 - tap * p.slabs;
+                const int tap = KIND == 2 && p.half ? 2 * kb0 : kb0 / p.slabs;
+                slab = KIND == 2 && p.half ? 0 : kb0 - tap * p.slabs;
                 tap_h = tap / p.tma_kw;
                 tap_w = tap - tap_h * p.tma_kw;
             } else if (p.a2_mode == 2) {
@@ -298,14 +377,24 @@ __global__ void __launch_bounds__(NTHREADS) conv_few_kernel(const __grid_constan
                 }
                 if (p.test_withhold && kb == kb1 - 1) break;
                 const uint32_t bar = smem_u32(&full[s]), dst = smem_u32(ring + s * STAGE_BYTES);
+                if (KIND == 2 && p.half) {
+                    const int nh = 2 * kb + 1 < p.ntaps ? 2 : 1;
+                    mbar_arrive_expect_tx(bar, (uint32_t)(nh * (A_BYTES / 2)));
+                    for (int h = 0; h < nh; h++) {
+                        tma_load_im2col_4d(dst + h * (A_BYTES / 2), &tmapA, bar, 0, iw, ih, in, (uint16_t)tap_w, (uint16_t)tap_h);
+                        if (++tap_w == p.tma_kw) { tap_w = 0; tap_h++; }
+                    }
+                    if (++s == nst) { s = 0; ph ^= 1; }
+                    continue;
+                }
                 mbar_arrive_expect_tx(bar, A_BYTES);
                 if (p.nkb1 && kb >= p.nkb1) {
-                    if (p.a2_mode == 1) tma_load_2d(dst, &tmapA2, bar, (kb - p.nkb1) * 64, m0);
-                    else tma_load_im2col_4d(dst, &tmapA2, bar, (kb - p.nkb1) * 64, iw, ih, in, 0, 0);
+                    if (p.a2_mode == 1) tma_load_2d(dst, &tmapA2, bar, (kb - p.nkb1) * KE, m0);
+                    else tma_load_im2col_4d(dst, &tmapA2, bar, (kb - p.nkb1) * KE, iw, ih, in, 0, 0);
                 } else if (p.mode == 1) {
-                    tma_load_2d(dst, &tmapA, bar, kb * 64, m0);
+                    tma_load_2d(dst, &tmapA, bar, kb * KE, m0);
                 } else {
-                    tma_load_im2col_4d(dst, &tmapA, bar, slab * 64, iw, ih, in, (uint16_t)tap_w, (uint16_t)tap_h);
+                    tma_load_im2col_4d(dst, &tmapA, bar, slab * KE, iw, ih, in, (uint16_t)tap_w, (uint16_t)tap_h);
                     if (++slab == p.slabs) {
                         slab = 0;
                         if (++tap_w == p.tma_kw) { tap_w = 0; tap_h++; }
@@ -326,8 +415,15 @@ __global__ void __launch_bounds__(NTHREADS) conv_few_kernel(const __grid_constan
                     break;
                 }
                 const uint32_t bar = smem_u32(&full[s]);
-                mbar_arrive_expect_tx(bar, B_BYTES);
-                tma_load_2d(smem_u32(ring + s * STAGE_BYTES + A_BYTES), &tmapW, bar, kb * 64, n0);
+                const uint32_t dst = smem_u32(ring + s * STAGE_BYTES + A_BYTES);
+                if (KIND == 2 && p.half) {
+                    const int nh = 2 * kb + 1 < p.ntaps ? 2 : 1;
+                    mbar_arrive_expect_tx(bar, (uint32_t)(nh * (B_BYTES / 2)));
+                    for (int h = 0; h < nh; h++) tma_load_2d(dst + h * (B_BYTES / 2), &tmapW, bar, (2 * kb + h) * (KE / 2), n0);
+                } else {
+                    mbar_arrive_expect_tx(bar, B_BYTES);
+                    tma_load_2d(dst, &tmapW, bar, kb * KE, n0);
+                }
                 if (++s == nst) { s = 0; ph ^= 1; }
             }
         }
@@ -345,10 +441,25 @@ __global__ void __launch_bounds__(NTHREADS) conv_few_kernel(const __grid_constan
                     break;
                 }
                 tc_fence_after();
-                const uint64_t ad = make_sw128_kmajor_desc(smem_u32(ring + s * STAGE_BYTES));
-                const uint64_t bd = make_sw128_kmajor_desc(smem_u32(ring + s * STAGE_BYTES + A_BYTES));
+                const uint32_t sa = smem_u32(ring + s * STAGE_BYTES), sb = sa + A_BYTES;
+                if (KIND == 2 && p.half) {
+                    const int nh = 2 * kb + 1 < p.ntaps ? 2 : 1;
+                    for (int h = 0; h < nh; h++) {
+                        const uint64_t ad = make_sw64_kmajor_desc(sa + h * (A_BYTES / 2)), bd = make_sw64_kmajor_desc(sb + h * (B_BYTES / 2));
 #pragma unroll
-                for (int k = 0; k < 4; k++) tc_mma_f16(tmem_base, ad + 2 * k, bd + 2 * k, IDESC, ((kb - kb0) | k) != 0);
+                        for (int k = 0; k < 2; k++) {
+                            if (KIND == 2) tc_mma_i8(tmem_base, ad + 2 * k, bd + 2 * k, IDESC, ((kb - kb0) | h | k) != 0);
+                            else tc_mma_f16(tmem_base, ad + 2 * k, bd + 2 * k, IDESC, ((kb - kb0) | h | k) != 0);
+                        }
+                    }
+                } else {
+                    const uint64_t ad = make_sw128_kmajor_desc(sa), bd = make_sw128_kmajor_desc(sb);
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        if (KIND == 2) tc_mma_i8(tmem_base, ad + 2 * k, bd + 2 * k, IDESC, ((kb - kb0) | k) != 0);
+                        else tc_mma_f16(tmem_base, ad + 2 * k, bd + 2 * k, IDESC, ((kb - kb0) | k) != 0);
+                    }
+                }
                 if (kb + nst < kb1) tc_commit(smem_u32(&empty[s]));
                 if (++s == nst) { s = 0; ph ^= 1; }
             }
@@ -378,12 +489,64 @@ __global__ void __launch_bounds__(NTHREADS) conv_few_kernel(const __grid_constan
         __syncwarp();
         cluster_arrive();
         cluster_wait();
-        if (have && pm < p.P) {
+        if constexpr (KIND == 2) {
+            if (have && pm < p.P) {
+                uint32_t rowsum = 0;
+                const int left = p.Cout - c_first, left16 = ((p.Cout + 15) & ~15) - c_first;
+#pragma unroll 1
+                for (int j = 0; j < W / 8 && j * 8 < left16; j++) {
+                    int acc[8];
+#pragma unroll
+                    for (int i = 0; i < 8; i++) acc[i] = 0;
+                    const int4 *part = reinterpret_cast<const int4 *>(recv) + (size_t)(2 * j) * BM + row;
+                    for (int r = 0; r < S; r++, part += (W >> 2) * BM) {
+                        const int4 u = part[0], v = part[BM];
+                        acc[0] += u.x; acc[1] += u.y; acc[2] += u.z; acc[3] += u.w;
+                        acc[4] += v.x; acc[5] += v.y; acc[6] += v.z; acc[7] += v.w;
+                    }
+                    uint2 res = r8[0];
+#pragma unroll
+                    for (int q = 1; q < BN / 16; q++)
+                        if (q == j) res = r8[q];
+                    const uint2 o = finish8_u8(acc, trow + j * 8, bias + rank * W + j * 8, u8, res, left - j * 8, p);
+                    *reinterpret_cast<uint2 *>(p.y + (size_t)pm * p.out_ld + c_first + j * 8) = o;
+                    rowsum = __dp4a(o.x, 0x01010101u, __dp4a(o.y, 0x01010101u, rowsum));
+                }
+                if (p.csum_out && left > 0) atomicAdd(p.csum_out + pm, (int)rowsum);
+            }
+        } else if constexpr (KIND != 2) if (have && pm < p.P) {
             uint8_t *dst = p.y + ((size_t)pm * p.out_ld + c_first) * 2;
             const int left = p.Cout - c_first;
             if (act == 0) finish_parts<KIND, 0>(recv, S, W, rank * W, rv, dst, left, row, consts, p);
             else if (act == 1) finish_parts<KIND, 1>(recv, S, W, rank * W, rv, dst, left, row, consts, p);
             else finish_parts<KIND, 2>(recv, S, W, rank * W, rv, dst, left, row, consts, p);
+        }
+    } else if constexpr (KIND == 2) {
+        if (have) {
+            const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16);
+            uint32_t rowsum = 0;
+            const int left = p.Cout - n0, left16 = ((p.Cout + 15) & ~15) - n0;
+            __syncwarp();
+#pragma unroll 1
+            for (int j = 0; j < BN / 8 && j * 8 < left16; j++) {
+                uint32_t a[8];
+                tmem_ld8(taddr + j * 8, a);
+                tmem_ld_wait();
+                int acc[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++) acc[i] = (int)a[i];
+                uint2 res = r8[0];
+#pragma unroll
+                for (int q = 1; q < BN / 8; q++)
+                    if (q == j) res = r8[q];
+                const uint2 o = finish8_u8(acc, trow + j * 8, bias + j * 8, u8, res, left - j * 8, p);
+                if (pm < p.P) *reinterpret_cast<uint2 *>(p.y + (size_t)pm * p.out_ld + n0 + j * 8) = o;
+                rowsum = __dp4a(o.x, 0x01010101u, __dp4a(o.y, 0x01010101u, rowsum));
+            }
+            if (p.csum_out && pm < p.P) {
+                if (p.n_tiles == 1) p.csum_out[pm] = (int)rowsum;
+                else atomicAdd(p.csum_out + pm, (int)rowsum);  // (the buffer was cleared before the launch)
+            }
         }
     } else if (have && p.y_nchw) {
         const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16);
@@ -419,29 +582,49 @@ __global__ void __launch_bounds__(NTHREADS) conv_few_kernel(const __grid_constan
 int operand_mode(const thb_conv_desc *d, FewParams &p, int &tmap_mode)
 {
     const bool plain = d->kH == 1 && d->kW == 1 && d->dH == 1 && d->dW == 1 && d->padH == 0 && d->padW == 0 && d->oH == d->H && d->oW == d->W;
-    p.slabs = d->Cin_pad / 64;
+    const int bke = d->dtype == THB_U8 ? 128 : 64;
+    p.slabs = d->Cin_pad / bke;
     p.tma_kw = d->kW;
     p.tma_padw = d->padW;
+    p.half = 0;
+    p.ntaps = d->kH * d->kW;
     if (d->in_row_pitch) {
-        if (!thb_im2col_ok(d) || d->dW != 1 || d->kW * d->Cin_pad != 64 || d->Ktot_pad != d->kH * 64) return 0;
+        if (!thb_im2col_ok(d) || d->dW != 1) return 0;
         p.slabs = 1;
         p.tma_kw = 1;
         p.tma_padw = 0;
-        tmap_mode = 3;
-        return 2;
+        p.ntaps = d->kH;
+        if (d->kW * d->Cin_pad == bke && d->Ktot_pad == d->kH * bke) {
+            tmap_mode = 3;
+            return 2;
+        }
+        p.half = 1;
+        tmap_mode = 5;
+        return d->dtype == THB_U8 && d->kW * d->Cin_pad * 2 == bke && d->Ktot_pad == (d->kH + 1) / 2 * bke ? 2 : 0;
     }
     tmap_mode = plain ? 1 : 2;
     if (plain) return 1;
-    return thb_im2col_ok(d) && d->Cin_pad % 64 == 0 && d->Ktot_pad == d->kH * d->kW * d->Cin_pad ? 2 : 0;
+    if (!thb_im2col_ok(d)) return 0;
+    if (d->dtype == THB_U8 && d->Cin_pad * 2 == bke && d->Ktot_pad == (p.ntaps + 1) / 2 * bke) {
+        p.half = 1;
+        tmap_mode = 4;
+        return 2;
+    }
+    return d->Cin_pad % bke == 0 && d->Ktot_pad == d->kH * d->kW * d->Cin_pad ? 2 : 0;
 }
 
 long tiles_of(const thb_conv_desc *d) { return (((long)d->N * d->oH * d->oW + BM - 1) / BM) * ((d->Cout_pad + BN - 1) / BN); }
 
 bool eligible(const thb_conv_desc *d)
 {
-    if (d->dtype != THB_F16 && d->dtype != THB_BF16) return false;
-    if ((d->Cout_pad % BN && d->Cout_pad != 32) || d->acc_out || d->csum_out || d->splitk_scratch) return false;
-    if (d->in_ld % 8 || d->out_ld % 8 || (d->res && d->res_ld % 8)) return false;
+    if (d->dtype == THB_U8) {
+        // (the table of border classes needs windows that are clipped on one side at most, by no more than the padding)
+        if (d->x2 || d->acc_out || d->in_ld % 16 || d->out_ld % 16 || (d->res && d->res_ld % 16)) return false;
+        if (d->H < d->kH || d->W < d->kW || d->padH >= d->kH || d->padW >= d->kW || (1 + 2 * d->padH) * (1 + 2 * d->padW) > 25) return false;
+        if ((d->oH - 1) * d->dH + d->kH - d->H > 2 * d->padH || (d->oW - 1) * d->dW + d->kW - d->W > 2 * d->padW) return false;
+    } else if (d->dtype != THB_F16 && d->dtype != THB_BF16) return false;
+    else if ((d->Cout_pad % BN && d->Cout_pad != 32) || d->acc_out || d->csum_out || d->splitk_scratch) return false;
+    else if (d->in_ld % 8 || d->out_ld % 8 || (d->res && d->res_ld % 8)) return false;
     FewParams p;
     int tm;
     const int mode = operand_mode(d, p, tm), allowed = thb_conv_launch_knobs().a_tma;
@@ -497,12 +680,16 @@ int launch(const CUtensorMap *w, const CUtensorMap *a, const CUtensorMap *a2, co
 //   1x1 512->128 @28x28, 8 images, 98 tiles of 8            8.9 /  6.5 /  7.0
 // So: eight K blocks or more, at least two of them to a CTA, up to one CTA per SM -- two per SM where four K blocks stay, but
 // not in clusters of eight.
+// uint8: the caller says with `splits` (1 included) that this kernel takes the convolution, since it has to clear csum_out when
+// several CTAs add to a pixel's sum; 0 here: it should not.
 extern "C" int thb_conv_few_splits(const thb_conv_desc *d)
 {
     const ThbConvLaunch kn = thb_conv_launch_knobs();
-    if (kn.few_tiles == 0 || !eligible(d) || d->Cout_pad % BN) return 1;
+    const int u8 = d->dtype == THB_U8;
+    if (kn.few_tiles == 0 || !eligible(d) || (!u8 && d->Cout_pad % BN)) return !u8;
     const long tiles = tiles_of(d);
-    const int nkb = d->Ktot_pad / 64;
+    const int nkb = d->Ktot_pad / (u8 ? 128 : 64);
+    if (u8 && tiles > (kn.few_tiles >= 0 ? kn.few_tiles : 4L * kn.sms)) return 0;
     int S = 1;
     while (S < 8 && nkb >= 8 && nkb / (2 * S) >= 2 && tiles * 2 * S <= (S < 4 && nkb / (2 * S) >= 4 ? 2 : 1) * (long)kn.sms) S *= 2;
     return S;
@@ -513,6 +700,7 @@ extern "C" int thb_conv_few_splits(const thb_conv_desc *d)
 // 7.9 / 5.7; 128->512 @28x28, 392: 8.3 / 6.2; 64->256 @56x56, 784: 9.5 / 11.1), and the patch kernel up to one.
 extern "C" int thb_conv_few_supported(const thb_conv_desc *d)
 {
+    if (d->dtype == THB_U8) return d->splits >= 1 && eligible(d);
     if (!eligible(d) || d->Cout_pad % BN) return 0;
     if (d->splits > 1) return 1;
     const ThbConvLaunch kn = thb_conv_launch_knobs();
@@ -536,7 +724,25 @@ static int few_fwd(const thb_conv_desc *d, const void *x, void *y, float *y_nchw
     p.P = d->N * d->oH * d->oW; p.oW = d->oW; p.oHW = d->oH * d->oW;
     p.dH = d->dH; p.dW = d->dW; p.padH = d->padH; p.padW = d->padW; p.kW = d->kW;
     p.Cout = d->Cout; p.out_ld = d->out_ld;
-    p.nkb = d->Ktot_pad / 64;
+    const int u8 = d->dtype == THB_U8;
+    p.nkb = d->Ktot_pad / (u8 ? 128 : 64);
+    p.H = d->H; p.W = d->W; p.kH = d->kH; p.Cin = d->Cin;
+    if (u8) {
+        if (!d->wsat || !d->csum) return THB_ERR_ARG;
+        p.a_off = d->a_offset; p.b_off = d->b_offset; p.c_off = d->c_offset; p.c_mult = d->c_mult; p.c_shift = d->c_shift;
+        p.tail_start = d->tail_start;
+        p.relu_thr = d->relu_thr < 0 ? -1 : d->relu_thr;
+        p.relu_val = d->relu_val;
+        p.wsat = d->wsat; p.bias_add = d->bias_add; p.csum = d->csum; p.csum_out = d->csum_out;
+        p.classes = (1 + 2 * d->padH) * (1 + 2 * d->padW);
+        p.tbl_bytes = (p.classes * BN * 4 + 1023) & ~1023;
+        if (d->res) {
+            p.ca = (int)d->self_coef; p.cb = (int)d->res_coef;
+            if ((p.ca != 1 && p.ca != -1) || (p.cb != 1 && p.cb != -1) || (float)p.ca != d->self_coef || (float)p.cb != d->res_coef) return THB_ERR_UNSUPPORTED;
+            const int twice = -(p.ca + p.cb - 1) * 255;  // floor(-(ca + cb - 1) * 127.5), as thb_u8_combine
+            p.res_addend = twice >= 0 ? twice / 2 : -((-twice + 1) / 2);
+        }
+    }
     p.n_tiles = (d->Cout_pad + BN - 1) / BN;  // (32 padded channels: the copy fills the missing weight rows with zeros)
     p.self_coef = d->self_coef; p.res_coef = d->res_coef;
     p.act_kind = d->act.kind; p.act_th = d->act.threshold; p.act_val = d->act.value; p.act_alpha = d->act.alpha;
@@ -547,7 +753,7 @@ static int few_fwd(const thb_conv_desc *d, const void *x, void *y, float *y_nchw
     if (p.splits > p.nkb) return THB_ERR_ARG;
     const ThbConvLaunch kn = thb_conv_launch_knobs();
     p.pdl = kn.pdl; p.wait_limit = kn.wait_limit; p.test_withhold = kn.test_withhold;
-    const CUtensorMap *w = thb_weights_tmap(d, BN), *a, *a2;
+    const CUtensorMap *w = thb_weights_tmap(d, BN, p.half ? 64 : 128), *a, *a2;
     if (d->x2) {
         const int cin2 = d->Cin - d->cin1;
         if (d->res || p.mode != 1 || d->in_row_pitch || d->cin1 <= 0 || d->cin1 % 64 || cin2 <= 0 || cin2 % 64 || d->x2_d < 1 || d->x2_d > 8 ||
@@ -576,9 +782,9 @@ static int few_fwd(const thb_conv_desc *d, const void *x, void *y, float *y_nchw
     p.stages = kn.few_stages > 0 ? kn.few_stages : p.splits > 1 || ctas > 2 * kn.sms ? 3 : ctas > kn.sms ? 4 : 5;
     if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
     if (p.stages > per) p.stages = per;
-    const int smem = 1024 + BAR_BYTES + (p.splits > 1 ? RECV_BYTES : 0) + p.stages * STAGE_BYTES;
+    const int smem = 1024 + BAR_BYTES + (p.splits > 1 ? RECV_BYTES : 0) + p.tbl_bytes + p.stages * STAGE_BYTES;
     cudaStream_t st = (cudaStream_t)s;
-    return d->dtype == THB_F16 ? launch<0>(w, a, a2, p, ctas, smem, st) : launch<1>(w, a, a2, p, ctas, smem, st);
+    return u8 ? launch<2>(w, a, a2, p, ctas, smem, st) : d->dtype == THB_F16 ? launch<0>(w, a, a2, p, ctas, smem, st) : launch<1>(w, a, a2, p, ctas, smem, st);
 }
 
 extern "C" int thb_conv_few_fwd(const thb_conv_desc *d, const void *x, void *y, thb_stream s)
@@ -590,7 +796,7 @@ extern "C" int thb_conv_nchw_supported(const thb_conv_desc *d)
 {
     thb_conv_desc one = *d;
     one.splits = 0;
-    return eligible(&one) && !d->x2;
+    return d->dtype != THB_U8 && eligible(&one) && !d->x2;
 }
 
 extern "C" int thb_conv_nchw_fwd(const thb_conv_desc *d, const void *x, float *y, int *status_out, thb_stream s)

@@ -8,8 +8,8 @@
 const CUtensorMap *thb_matrix_tmap(const void *x, long rows, int cols, int ld, int dtype, int box_cols);
 // the activation operand: mode 1 plain matrix, 2 im2col, 3 im2col over rows stored with their padding
 const CUtensorMap *thb_activation_tmap(const thb_conv_desc *d, const void *x, int mode);
-// the packed weights in boxes of box_rows output channels x 128 bytes
-const CUtensorMap *thb_weights_tmap(const thb_conv_desc *d, int box_rows);
+// the packed weights in boxes of box_rows output channels x 128 or 64 bytes
+const CUtensorMap *thb_weights_tmap(const thb_conv_desc *d, int box_rows, int box_bytes);
 // a rank-4 im2col descriptor can describe this convolution's input
 bool thb_im2col_ok(const thb_conv_desc *d);
 

@@ -1701,7 +1701,7 @@ const CUtensorMap *thb_matrix_tmap(const void *x, long rows, int cols, int ld, i
     return matrix_tmap(x, rows, cols, ld, dtype, box_cols);
 }
 const CUtensorMap *thb_activation_tmap(const thb_conv_desc *d, const void *x, int mode) { return activation_tmap(d, x, mode); }
-const CUtensorMap *thb_weights_tmap(const thb_conv_desc *d, int box_rows) { return weights_box_tmap(d, box_rows, 128); }
+const CUtensorMap *thb_weights_tmap(const thb_conv_desc *d, int box_rows, int box_bytes) { return weights_box_tmap(d, box_rows, box_bytes); }
 int thb_pdl_enabled() { return knobs().pdl; }
 ThbConvLaunch thb_conv_launch_knobs()
 {
