@@ -141,6 +141,9 @@ int thb_conv_splitk_plan(const thb_conv_desc *d, size_t *scratch_bytes);
  * one tile and add their parts through distributed shared memory, in rank order, in the same launch.  thb_conv_few_splits: the
  * split that suits this tile count (1: none; U8: 0 when the other kernel is the better one); thb_conv_few_supported: the kernel of few tiles takes this convolution. */
 int thb_conv_few_splits(const thb_conv_desc *d);
+/* F32: the number of CTAs that share a tile's reduction.  A launch whose `splits` is 0 takes it; a caller that runs one layer on
+ * parts of a batch gives every part the whole batch's, so that all of them add in the same order. */
+int thb_conv_simt_splits(const thb_conv_desc *d);
 int thb_conv_few_supported(const thb_conv_desc *d);
 /* A network's last convolution (F16 / BF16) with its result as NCHW fp32, rounded through the 16-bit type, in device or pinned
  * host memory: the convolution and thb_postprocess_status in one launch.  *status_out: 0 before the call; set when this launch or

@@ -991,6 +991,7 @@ static int plan_gemm_group(planner *P, int i)
         d->splits = thb_conv_few_splits(&whole);
         if (d->splits < 2) d->splits = 0;
     }
+    if (dtype == THB_F32) d->splits = thb_conv_simt_splits(d); /* (also on parts of the batch: a sliced start changes no sum) */
     /* (integer sums: any split gives the same bytes) */
     if (dtype == THB_U8 && is.N == P->I->slice_n) {
         d->out_ld = ru(d->Cout, al);
@@ -1529,15 +1530,18 @@ static int sliceable(const instance *I, const step *s)
     }
 }
 
-/* Microseconds of a launch on the whole slice, roughly: its share of the arithmetic (at 0.5 PFLOP/s in the 16-bit modes,
- * 0.9 in uint8, 20 TFLOP/s in fp32, what the layers of a large batch reach on average) or of the bytes (4.5 TB/s), whichever
- * is more. */
+/* Microseconds that a launch on the whole slice takes beyond LAUNCH_US, roughly: its share of the arithmetic (at 0.62 PFLOP/s in
+ * the 16-bit modes, 0.75 in uint8, 36 TFLOP/s in fp32, what the layers of a large batch reach on average) or of the bytes
+ * (4.5 TB/s), whichever is more.  LAUNCH_US is every launch's fill, drain and partly filled wave (ResNet-18 and -50 on 1 to 256
+ * images: within a fifth of 7 us a launch plus this). */
+#define LAUNCH_US 7.0
+#define PART_LAUNCH_US 8.5 /* ... of a launch on a part of the batch: issued directly, not from the graph */
 static double model_us(const step *s)
 {
     double elems = (double)s->out_pixels * s->out_C * 2, us = 0;
     if (s->kind == ST_CONV) {
         const thb_conv_desc *d = &s->conv;
-        const double rate = s->dtype == THB_F32 ? 20e6 : s->dtype == THB_U8 ? 0.9e9 : 0.5e9; /* per microsecond */
+        const double rate = s->dtype == THB_F32 ? 36e6 : s->dtype == THB_U8 ? 0.75e9 : 0.62e9; /* per microsecond */
         us = 2.0 * d->N * d->oH * d->oW * (double)d->Cout * d->Cin * d->kH * d->kW / rate;
         elems = (double)d->N * d->H * d->W * d->Cin + elems * (s->nin > 1 ? 1 : 0.5);
     }
@@ -1569,10 +1573,9 @@ static double copy_in_us(const thb_engine *E, const instance *I)
 /* A batch of 256 pictures takes 0.7 ms to arrive, a fifth of a ResNet-50 forward.  The first launches of a network are the
  * ones with the most pixels, which lose nothing on a part of the batch: they follow the copy part by part, and the rest of the
  * network runs on the whole batch.  (Cutting the whole network into sub-batches instead repeats the fill and drain of all its
- * small layers: ResNet-50 on 96 + 160 pictures, 4.35 ms of kernels instead of 3.65.)  Of 2 to 8 parts, the count that hides
- * most of the copy: launches join as long as a part of theirs keeps the chip busy for 6 us, until they take as long as the
- * copy; a launch costs 5 us more on every part (measured: 3 to 7 launches in 4 parts are within 2 % of one another, 9 in 7 parts
- * lose 6 %). */
+ * small layers: ResNet-50 on 96 + 160 pictures, 4.35 ms of kernels instead of 3.65.)  The number of parts and of launches are
+ * those with the earliest end in a model: a part starts when it has arrived and the one before it has been through the launches,
+ * each of which takes PART_LAUNCH_US and its share of model_us on it. */
 static void choose_slices(thb_engine *E, instance *I)
 {
     I->prefix = I->slices = 0;
@@ -1580,22 +1583,26 @@ static void choose_slices(thb_engine *E, instance *I)
     const char *off = getenv("THB200_NO_SLICES");
     if (off && atoi(off)) return;
     const double t_in = copy_in_us(E, I);
-    double best = 20;
+    double all = 0;
+    for (int t = 0; t < I->nsteps; t++) all += LAUNCH_US + model_us(&I->steps[t]);
+    const double whole = t_in + all;
+    double best = whole - 20;
     for (int m = 2; m <= 8 && m <= I->slice_n / 2; m++) {
-        double us = 0;
-        int p = 0;
-        while (p < I->nsteps - I->head && us < t_in && sliceable(I, &I->steps[p])) {
-            const double k = model_us(&I->steps[p]);
-            if (k > 0 && k < 6 * m) break;
-            us += k;
-            p++;
+        double sliced = 0;
+        for (int p = 1; p <= I->nsteps - I->head && sliceable(I, &I->steps[p - 1]); p++) {
+            sliced += model_us(&I->steps[p - 1]);
+            double end = 0;
+            for (int c = 0; c < m; c++) {
+                const double came = t_in * (2 * c + 1) / (2 * m - 1);
+                end = (came > end ? came : end) + p * PART_LAUNCH_US + sliced * (c ? 2 : 1) / (2 * m - 1);
+            }
+            end += all - p * LAUNCH_US - sliced;
+            if (end >= best) continue;
+            best = end;
+            I->prefix = p;
+            I->slices = m;
+            I->hidden_us = whole - end;
         }
-        const double gain = (us < t_in ? us : t_in) * (m - 1) / m - 5.0 * p * m;
-        if (gain <= best) continue;
-        best = gain;
-        I->prefix = p;
-        I->slices = m;
-        I->hidden_us = gain;
     }
 }
 
@@ -2284,8 +2291,8 @@ static const unsigned char sub_batch_cuts[][5] = {
 };
 
 /* Sub-batches per GPU of a host-input forward: the cut with the earliest last result in a model of the three stages a
- * sub-batch goes through -- its copy to the device, its kernels (model_us, and 12 us for each launch's fill and drain however
- * small the sub-batch is), its result's copy back -- each one at a time.  The uint8 engine needs the range of a whole float
+ * sub-batch goes through -- its copy to the device, its kernels (model_us, and LAUNCH_US for each launch however small the
+ * sub-batch is), its result's copy back -- each one at a time.  The uint8 engine needs the range of a whole float
  * batch before any kernel can start; its byte images have a static one. */
 static void choose_sub_batches(thb_engine *E)
 {
@@ -2297,7 +2304,7 @@ static void choose_sub_batches(thb_engine *E)
     const double t_in = copy_in_us(E, I), t_out = 4.0 * I->out_count / 50e3;
     double t_k = 0;
     for (int t = 0; t < I->nsteps; t++) t_k += model_us(&I->steps[t]);
-    const double fixed = I->nsteps * 12.0;
+    const double fixed = I->nsteps * LAUNCH_US;
     double best = 0;
     for (unsigned c = 0; c < sizeof(sub_batch_cuts) / sizeof(sub_batch_cuts[0]); c++) {
         const unsigned char *cut = sub_batch_cuts[c];

@@ -10,7 +10,7 @@
 //     swizzled by XOR so that neither the copies nor the 16-byte reads of four k at a time meet in a bank;
 //   * launches of few tiles: the K blocks of a tile are shared by the S CTAs of a thread-block cluster.  Each leaves its partial tile in its shared memory, and every CTA adds the S parts of its share of
 //     the rows, in rank order, through distributed shared memory (no atomics, the result does not depend on timing).
-// Measured: the table at thb_conv_fwd_simt.
+// Measured: the table at thb_conv_simt_splits.
 #include "common.cuh"
 #include "conv_maps.cuh"
 #include <cooperative_groups.h>
@@ -130,9 +130,15 @@ __global__ void __launch_bounds__(2 * BN, BN == 64 ? 3 : 2) conv_simt_kernel(con
             cp_async16(dst + (r * BN + b_c) * 4, p.w + (size_t)(k < p.Ktot ? k : 0) * p.Cout_pad + n0 + b_c, k < p.Ktot ? 16u : 0u);
         }
     };
-    auto load_a = [&](int kb, int s) {
+    // (the gather word of a K block is read a block ahead: the warps that multiply would wait for it)
+    auto kinfo_of = [&](int kb) {
         const int g = kb * 8 + chunk;
-        const int ki = g < p.n_kchunks ? __ldg(p.kinfo + g) : -1;
+        return g < p.n_kchunks ? __ldg(p.kinfo + g) : -1;
+    };
+    int ki_next = kinfo_of(kb0);
+    auto load_a = [&](int kb, int s) {
+        const int ki = ki_next;
+        ki_next = kinfo_of(kb + 1);
         const int dh = (ki >> 24) & 0x7f, dw = (ki >> 16) & 0xff, coff = (ki & 0xffff) * 4;
         const uint32_t dst = smem_u32(smem + s * STAGE);
 #pragma unroll
@@ -293,6 +299,31 @@ template <int BN, bool SPLIT> int launch_simt(const ConvSimtParams &p, int sms, 
 // (library-internal: thb_conv_reload_knobs() calls it so that a test can switch THB200_NO_SPLITK between cases)
 extern "C" void thb_simt_reload_knobs(void) { g_no_split = -1; }
 
+// Tiles of 64 channels, the reduction split while that leaves at most three CTAs to an SM (what its registers hold); measured,
+// us before / unsplit / split in 2 / 4 / 8 (16 in clusters beyond the portable size):
+//   64->64 3x3 @57x57, 9 images, 229 tiles of 18 K blocks      72 / 65 / 66
+//   128->128 3x3 @29x29, 9 images, 120 of 36                   82 / 70 / 65 / 64
+//   256->256 3x3 @15x15, 9 images, 64 of 72                   144 / 133 / 71 / 63 / 77
+//   512->512 3x3 @8x8, 9 images, 40 of 144                    160 / - / 137 / 120 / 89
+//   64->192 5x5 @27x27, 1 image, 18 of 50                      31 / - / 51 / 28 / 27
+//   384->256 3x3 @13x13, 1 image, 8 of 108                     34 / - / 102 / 53 / 29
+// Large layers: tiles of 128 channels (128->128 3x3 @28x28, 64 images: 401 / 332 with 64, 320 with 128).
+extern "C" int thb_conv_simt_splits(const thb_conv_desc *d)
+{
+    if (g_no_split < 0) {
+        const char *e = getenv("THB200_NO_SPLITK");
+        g_no_split = e && atoi(e) ? 1 : 0;
+    }
+    const int sms = thb_conv_launch_knobs().sms, nkb = (d->Ktot_pad + BK - 1) / BK;
+    const long tiles = (((long)d->N * d->oH * d->oW + BM - 1) / BM) * (d->Cout_pad / 64);
+    int S = 1;
+    if (!g_no_split) {
+        while (S < 8 && tiles * 2 * S <= 3L * sms && nkb >= 2 * S) S *= 2;
+        if (S == 8 && tiles * 16 <= 2L * sms && nkb >= 32) S = 16;
+    }
+    return S;
+}
+
 extern "C" int thb_conv_fwd_simt(const thb_conv_desc *d, const void *x, void *y, thb_stream s)
 {
     if (!d->w || !d->kinfo) return THB_ERR_ARG;
@@ -309,29 +340,11 @@ extern "C" int thb_conv_fwd_simt(const thb_conv_desc *d, const void *x, void *y,
     p.res = (const float *)d->res; p.res_ld = d->res_ld; p.self_coef = d->self_coef; p.res_coef = d->res_coef;
     p.act_kind = d->act.kind; p.act_th = d->act.threshold; p.act_val = d->act.value; p.act_alpha = d->act.alpha;
     if (p.P <= 0) return THB_OK;
-    if (g_no_split < 0) {
-        const char *e = getenv("THB200_NO_SPLITK");
-        g_no_split = e && atoi(e) ? 1 : 0;
-    }
     const ThbConvLaunch kn = thb_conv_launch_knobs();
     p.pdl = kn.pdl;
     const cudaStream_t st = (cudaStream_t)s;
-    // Tiles of 64 channels, the reduction split while that leaves at most three CTAs to an SM (what its registers hold); measured,
-    // us before / unsplit / split in 2 / 4 / 8 (16 in clusters beyond the portable size):
-    //   64->64 3x3 @57x57, 9 images, 229 tiles of 18 K blocks      72 / 65 / 66
-    //   128->128 3x3 @29x29, 9 images, 120 of 36                   82 / 70 / 65 / 64
-    //   256->256 3x3 @15x15, 9 images, 64 of 72                   144 / 133 / 71 / 63 / 77
-    //   512->512 3x3 @8x8, 9 images, 40 of 144                    160 / - / 137 / 120 / 89
-    //   64->192 5x5 @27x27, 1 image, 18 of 50                      31 / - / 51 / 28 / 27
-    //   384->256 3x3 @13x13, 1 image, 8 of 108                     34 / - / 102 / 53 / 29
-    // Large layers: tiles of 128 channels (128->128 3x3 @28x28, 64 images: 401 / 332 with 64, 320 with 128).
     const long tiles = (long)((p.P + BM - 1) / BM) * (d->Cout_pad / 64);
-    const int nkb = (p.Ktot + BK - 1) / BK;
-    p.splits = 1;
-    if (!g_no_split) {
-        while (p.splits < 8 && tiles * 2 * p.splits <= 3L * kn.sms && nkb >= 2 * p.splits) p.splits *= 2;
-        if (p.splits == 8 && tiles * 16 <= 2L * kn.sms && nkb >= 32) p.splits = 16;
-    }
+    p.splits = d->splits > 0 && d->splits <= 16 && !(d->splits & (d->splits - 1)) ? d->splits : thb_conv_simt_splits(d);
     if (p.splits > 1) return launch_simt<64, true>(p, kn.sms, st);
     if (d->Cout_pad % 128 == 0 && tiles >= 200) return launch_simt<128, false>(p, kn.sms, st);
     return launch_simt<64, false>(p, kn.sms, st);
