@@ -83,6 +83,9 @@ struct ConvTcParams {
                                // the stages each.  One tile of a short reduction costs either thread about 0.75 us of its own
                                // instructions with idle schedulers and over 1.5 us beside three busy epilogue warps, which was
                                // the whole launch's pace (64->256 1x1 with residual @56x56, 128 images: 42 tiles per SM, 115 us)
+    int res_w;                 // uint8, TMA modes, the CTA stays on one column tile and its weights fit next to four activation
+                               // stages: they are copied once, ahead of the launch dependency, and stay.  The copy engine works
+                               // at rows per second, and a 64-wide weight tile is a third of a K block's rows
     int *csum_out;             // uint8, one column tile: per output pixel the sum of its output bytes (the next layer's channel sums)
     int y_sector;              // uint8: every 32 channels of the output start on a 32-byte boundary
     int res_addend;            // uint8 fused residual: the constant of ca*q + cb*r + addend (see thb_u8_combine)
@@ -574,13 +577,15 @@ __global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const int nst = L::TMA_EPI ? p.stages : STAGES;  // pipeline stages in use
+    const bool res_w = KIND == 2 && p.res_w;
+    const int nst = L::TMA_EPI || res_w ? p.stages : STAGES;  // pipeline stages in use
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem);
     const bool pair = L::TMA_EPI && p.pair;
     const int a_stage_bytes = pair ? 2 * A_STAGE_BYTES : A_STAGE_BYTES;  // pair mode: both halves' activation tiles
     uint8_t *sA = smem + L::BAR_BYTES;
     uint8_t *sB = sA + nst * a_stage_bytes;
-    uint8_t *stage_buf = sB + nst * B_STAGE_BYTES;
+    uint8_t *stage_buf = L::TMA_EPI ? sB + nst * B_STAGE_BYTES : sA + STAGES * L::STAGE_BYTES;
+    uint64_t *wfull = bars + 80;  // resident weights have arrived
     uint64_t *full = bars, *empty = bars + MAX_STAGES;
     // uint8: one acc_full barrier per tile modulo 12 (a multiple of the accumulators, of the epilogue groups and of the two MMA
     // warps).  A group waits on every third tile; on a barrier per accumulator, the tile it finished last would not imply that
@@ -602,6 +607,7 @@ __global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid
             mbar_init(smem_u32(&empty[s]), 1);
         }
         for (int b = 0; b < NFULL; b++) mbar_init(smem_u32(&acc_full[b]), 1);
+        if (KIND == 2) mbar_init(smem_u32(wfull), 1);
         for (int b = 0; b < NACC; b++) mbar_init(smem_u32(&acc_empty[b]), 128);
         for (int g = 0; g < 9; g++) {
             mbar_init(smem_u32(&rows_ready[g]), 128);
@@ -631,6 +637,18 @@ __global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid
     // still draining, so that the set-up above overlaps its tail.  Nothing before this point touches memory that
     // kernel could write or read; from here on it must have finished.  The next kernel may start its own set-up as
     // soon as this grid's CTAs leave their SMs.
+    if (KIND == 2 && res_w && warp == 4 && lane == 0) {
+        // (weights are written by no launch of a forward)
+        const uint32_t bar = smem_u32(wfull);
+        const int n0 = (int)(blockIdx.x % p.n_tiles) * BN;
+        if (p.half) {
+            mbar_arrive_expect_tx(bar, (uint32_t)(p.ntaps * (B_STAGE_BYTES / 2)));
+            for (int t = 0; t < p.ntaps; t++) tma_load_2d(smem_u32(sB + t * (B_STAGE_BYTES / 2)), &tmapW, bar, t * (BKE / 2), n0);
+        } else {
+            mbar_arrive_expect_tx(bar, (uint32_t)(p.nkb * B_STAGE_BYTES));
+            for (int kb = 0; kb < p.nkb; kb++) tma_load_2d(smem_u32(sB + kb * B_STAGE_BYTES), &tmapW, bar, kb * BKE, n0);
+        }
+    }
     if (p.pdl) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -782,16 +800,16 @@ __global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid
                     const uint32_t bar = smem_u32(&full[s]);
                     if (p.half) {
                         const int nh = 2 * kb + 1 < p.ntaps ? 2 : 1;
-                        mbar_arrive_expect_tx(bar, (uint32_t)(nh * (A_STAGE_BYTES / 2 + B_STAGE_BYTES / 2)));
+                        mbar_arrive_expect_tx(bar, (uint32_t)(nh * (A_STAGE_BYTES / 2 + (res_w ? 0 : B_STAGE_BYTES / 2))));
                         for (int h = 0; h < nh; h++) {
                             tma_load_im2col_4d(smem_u32(sA + s * a_stage_bytes + h * (A_STAGE_BYTES / 2)), &tmapA, bar, 0, iw[0], ih[0],
                                                in[0], (uint16_t)tap_w, (uint16_t)tap_h);
-                            tma_load_2d(smem_u32(sB + s * B_STAGE_BYTES + h * (B_STAGE_BYTES / 2)), &tmapW, bar, (2 * kb + h) * (BKE / 2), n0);
+                            if (!res_w) tma_load_2d(smem_u32(sB + s * B_STAGE_BYTES + h * (B_STAGE_BYTES / 2)), &tmapW, bar, (2 * kb + h) * (BKE / 2), n0);
                             if (++tap_w == p.tma_kw) { tap_w = 0; tap_h++; }
                         }
                         continue;
                     }
-                    mbar_arrive_expect_tx(bar, (uint32_t)(B_STAGE_BYTES + (p.a_tma ? a_stage_bytes : 0)));
+                    mbar_arrive_expect_tx(bar, (uint32_t)((res_w ? 0 : B_STAGE_BYTES) + (p.a_tma ? a_stage_bytes : 0)));
                     if (p.a_tma == 1 && p.nkb1 && kb >= p.nkb1) {
                         for (int h = 0; h < halves; h++) {
                             const uint32_t dst = smem_u32(sA + s * a_stage_bytes + h * A_STAGE_BYTES);
@@ -810,7 +828,7 @@ __global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid
                             if (++tap_w == p.tma_kw) { tap_w = 0; tap_h++; }
                         }
                     }
-                    tma_load_2d(smem_u32(sB + s * B_STAGE_BYTES), &tmapW, bar, kb * BKE, n0);
+                    if (!res_w) tma_load_2d(smem_u32(sB + s * B_STAGE_BYTES), &tmapW, bar, kb * BKE, n0);
                 }
             }
         }
@@ -824,6 +842,11 @@ __global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid
             int ring_s = ring_0;
             uint32_t ring_ph = 0;
             bool alive = true;
+            if (KIND == 2 && res_w && !mbar_wait_bounded(smem_u32(wfull), 0, p.wait_limit)) {
+                atomicExch(p.status, 4);
+                *abort_flag = 1;
+                alive = false;
+            }
             for (int lt = KIND == 2 && warp == 15 ? 1 : 0; lt < map.n_local && alive; lt += lt_step) {
                 // the accumulators of this unit's local tiles (two in pair mode) must have been drained
                 for (int h = 0; h < halves && alive; h++)
@@ -853,7 +876,7 @@ __global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid
                         const int nh = 2 * kb + 1 < p.ntaps ? 2 : 1;
                         for (int h = 0; h < nh; h++) {
                             const uint64_t ad = make_sw64_kmajor_desc(smem_u32(sA + s * a_stage_bytes + h * (A_STAGE_BYTES / 2)));
-                            const uint64_t bd = make_sw64_kmajor_desc(smem_u32(sB + s * B_STAGE_BYTES + h * (B_STAGE_BYTES / 2)));
+                            const uint64_t bd = make_sw64_kmajor_desc(smem_u32(sB + (res_w ? kb : s) * B_STAGE_BYTES + h * (B_STAGE_BYTES / 2)));
 #pragma unroll
                             for (int k = 0; k < 2; k++) {
                                 const uint32_t accum = ((kb - kb0) | h | k) != 0;
@@ -865,7 +888,7 @@ __global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid
                         continue;
                     }
                     const uint64_t adesc = make_sw128_kmajor_desc(smem_u32(sA + s * a_stage_bytes));
-                    const uint64_t bdesc = make_sw128_kmajor_desc(smem_u32(sB + s * B_STAGE_BYTES));
+                    const uint64_t bdesc = make_sw128_kmajor_desc(smem_u32(sB + (res_w ? kb : s) * B_STAGE_BYTES));
 #pragma unroll
                     for (int k = 0; k < 4; k++) {
                         const uint32_t accum = ((kb - kb0) | k) != 0;
@@ -1341,7 +1364,7 @@ __global__ void __launch_bounds__(256) splitk_finish_kernel(const ConvTcParams p
 // Diagnostic launcher switches (THB200_* environment variables), read ONCE: a launch costs no getenv call.
 // thb_conv_reload_knobs() re-reads them (the tests change them between cases).  -1 = not set.
 struct ConvKnobs {
-    int pair_min_kb, u8_fast, reverse, epi_groups, epi_bufs, pdl, conv_l1, half_taps, a_tma, test_withhold, few_tiles, few_stages, dual;
+    int pair_min_kb, u8_fast, reverse, epi_groups, epi_bufs, pdl, conv_l1, half_taps, a_tma, test_withhold, few_tiles, few_stages, dual, u8_res_w;
     long pair_min_units;
     long long wait_limit;
 };
@@ -1369,6 +1392,7 @@ void read_knobs()
     g_knobs.few_tiles = env_int("THB200_FEW_TILES", -1);
     g_knobs.few_stages = env_int("THB200_FEW_STAGES", -1);
     g_knobs.dual = env_int("THB200_U8_DUAL", 1);
+    g_knobs.u8_res_w = env_int("THB200_U8_RES_W", 1);
     const char *wl = getenv("THB200_WAIT_LIMIT_CYCLES");
     g_knobs.wait_limit = wl && atoll(wl) > 0 ? atoll(wl) : 4000000000ll;
     g_knobs_read = true;
@@ -1448,6 +1472,13 @@ int launch_tc(const ConvTmaps &tm, ConvTcParams p, cudaStream_t st)
     if (KIND == 2 && p.u8_classes > 0 && p.n_tiles > 1 && tiles > grid && grid % p.n_tiles && grid > 2 * p.n_tiles && knobs().u8_fast != 2)
         grid -= grid % p.n_tiles;
     p.dual = KIND == 2 && p.a_tma && BN <= 128 && kn.dual && (long)p.m_tiles * p.n_tiles >= 2L * num_sms();
+    if (KIND == 2) {
+        const long room = (long)STAGES * L::STAGE_BYTES - (long)p.nkb * L::B_STAGE_BYTES;
+        int st = (int)(room / A_STAGE_BYTES);
+        if (st > MAX_STAGES) st = MAX_STAGES;
+        p.res_w = p.a_tma && kn.u8_res_w && st >= 4 && grid % p.n_tiles == 0;
+        if (p.res_w) p.stages = st;
+    }
     if (!L::TMA_EPI) {
         // staged epilogue: uint8 with nothing to gather runs a third group on warps 0-3 (a fourth accumulator exists below 256 columns)
         p.epi_groups = KIND == 2 && p.a_tma && BN < 256 ? 3 : 2;
