@@ -2,14 +2,14 @@
 //
 // D[pixel][cout] = sum_k A[pixel][k] * Wk[k][cout], k = tap*Cin_pad + c over NHWC fp32 activations.
 //
-// What bounds it is the FP32 pipe (74 TFLOP/s) once operands reach the registers cheaply, so:
+// What bounds it is the FP32 pipe (61 TFLOP/s measured in a loop without loads) once operands reach the registers cheaply, so:
 //   * a thread owns 8 pixels x 8 channels and multiplies with fma.rn.f32x2, two channels an instruction, which leaves half
 //     of the issue slots to the loads and to the duplication of the pixel operand;
-//   * a CTA's tile is 128 pixels x 64 or 128 channels, the K block 32; both operands arrive by 16-byte cp.async (channel
+//   * a CTA's tile is 128 x 64, 128 x 128 or 64 x 128 (pixels x channels), the K block 32; both operands arrive by 16-byte cp.async (channel
 //     chunks of pixels through the gather table, zeros outside the image) in a ring of three stages, pixel rows of 128 bytes
 //     swizzled by XOR so that neither the copies nor the 16-byte reads of four k at a time meet in a bank;
-//   * launches of few tiles: the K blocks of a tile are shared by the S CTAs of a thread-block cluster.  Each leaves its partial tile in its shared memory, and every CTA adds the S parts of its share of
-//     the rows, in rank order, through distributed shared memory (no atomics, the result does not depend on timing).
+//   * launches of few tiles: the K blocks of a tile are shared by the S CTAs of a thread-block cluster.  Each leaves
+//     its partial tile in its shared memory, and every CTA adds the S parts of its share of the rows, in rank order, through distributed shared memory (no atomics, the result does not depend on timing).
 // Measured: the table at thb_conv_simt_splits.
 #include "common.cuh"
 #include "conv_maps.cuh"
@@ -20,7 +20,7 @@ namespace cg = cooperative_groups;
 
 namespace {
 
-constexpr int BM = 128, BK = 32, STAGES = 3;
+constexpr int BK = 32, STAGES = 3;
 
 struct ConvSimtParams {
     const float *x, *w;
@@ -88,17 +88,17 @@ struct Affine4 {
     }
 };
 
-template <int BN, bool SPLIT>
-__global__ void __launch_bounds__(2 * BN, BN == 64 ? 3 : 2) conv_simt_kernel(const ConvSimtParams p)
+template <int BM, int BN, bool SPLIT>
+__global__ void __launch_bounds__(BM * BN / 64, BM * BN == 128 * 64 ? 3 : 2) conv_simt_kernel(const ConvSimtParams p)
 {
-    constexpr int NT = 2 * BN, A_BYTES = BM * 128, B_BYTES = BK * BN * 4, STAGE = A_BYTES + B_BYTES;
+    constexpr int NT = BM * BN / 64, A_BYTES = BM * 128, B_BYTES = BK * BN * 4, STAGE = A_BYTES + B_BYTES;
     constexpr int A_ROWS = BM * 8 / NT, B_ROWS = BK * (BN / 4) / NT;
     extern __shared__ __align__(1024) uint8_t smem[];
 
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int tx = lane & 7, ty = lane >> 3;
     const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-    const int wm = (warp & 3) * 32, wn = (warp >> 2) * 64;  // this warp's 32 pixels x 64 channels
+    const int wm = (warp % (BM / 32)) * 32, wn = (warp / (BM / 32)) * 64;  // this warp's 32 pixels x 64 channels
 
     // this thread's share of the copies: one 16-byte chunk of K of A_ROWS pixel rows, B_ROWS chunks of weight rows
     const int chunk = t & 7;
@@ -253,9 +253,9 @@ __global__ void __launch_bounds__(2 * BN, BN == 64 ? 3 : 2) conv_simt_kernel(con
     cluster.sync();  // the parts must outlive the reads above
 }
 
-template <int BN, bool SPLIT> int launch_simt(const ConvSimtParams &p, int sms, cudaStream_t st)
+template <int BM, int BN, bool SPLIT> int launch_simt(const ConvSimtParams &p, int sms, cudaStream_t st)
 {
-    auto kern = conv_simt_kernel<BN, SPLIT>;
+    auto kern = conv_simt_kernel<BM, BN, SPLIT>;
     constexpr int need = STAGES * (BM * 128 + BK * BN * 4);
     static bool set[64];
     int dev = 0;
@@ -272,7 +272,7 @@ template <int BN, bool SPLIT> int launch_simt(const ConvSimtParams &p, int sms, 
     const int smem = ctas > sms && ctas <= 2L * sms && need < 115712 ? 115712 : need;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((p.P + BM - 1) / BM, p.Cout_pad / BN, p.splits);
-    cfg.blockDim = dim3(2 * BN);
+    cfg.blockDim = dim3(BM * BN / 64);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
@@ -299,6 +299,12 @@ template <int BN, bool SPLIT> int launch_simt(const ConvSimtParams &p, int sms, 
 // (library-internal: thb_conv_reload_knobs() calls it so that a test can switch THB200_NO_SPLITK between cases)
 extern "C" void thb_simt_reload_knobs(void) { g_no_split = -1; }
 
+// A split launch works on tiles of 64 pixels x 128 channels where it can: fewer wasted rows (49 pixels of a 7 x 7 map, 169 of a
+// 13 x 13 one), and 2 to 5 % where the rows come out even.  us, 128 x 64 / 64 x 128: 3x3 512->512 @7x7, 1 image 32.1 / 19.2;
+// 384->256 @13x13, 1 image 26.2 / 15.9; 256->256 @14x14, 2 images 29.9 / 20.3, 8 images 61.6 / 58.3; 128->128 @29x29, 9 images
+// 62.9 / 61.4.
+static bool low_tiles(const thb_conv_desc *d) { return d->Cout_pad % 128 == 0; }
+
 // Tiles of 64 channels, the reduction split while that leaves at most three CTAs to an SM (what its registers hold); measured,
 // us before / unsplit / split in 2 / 4 / 8 (16 in clusters beyond the portable size):
 //   64->64 3x3 @57x57, 9 images, 229 tiles of 18 K blocks      72 / 65 / 66
@@ -315,7 +321,8 @@ extern "C" int thb_conv_simt_splits(const thb_conv_desc *d)
         g_no_split = e && atoi(e) ? 1 : 0;
     }
     const int sms = thb_conv_launch_knobs().sms, nkb = (d->Ktot_pad + BK - 1) / BK;
-    const long tiles = (((long)d->N * d->oH * d->oW + BM - 1) / BM) * (d->Cout_pad / 64);
+    const long P = (long)d->N * d->oH * d->oW;
+    const long tiles = low_tiles(d) ? (P + 63) / 64 * (d->Cout_pad / 128) : (P + 127) / 128 * (d->Cout_pad / 64);
     int S = 1;
     if (!g_no_split) {
         while (S < 8 && tiles * 2 * S <= 3L * sms && nkb >= 2 * S) S *= 2;
@@ -343,9 +350,10 @@ extern "C" int thb_conv_fwd_simt(const thb_conv_desc *d, const void *x, void *y,
     const ThbConvLaunch kn = thb_conv_launch_knobs();
     p.pdl = kn.pdl;
     const cudaStream_t st = (cudaStream_t)s;
-    const long tiles = (long)((p.P + BM - 1) / BM) * (d->Cout_pad / 64);
+    const long tiles = (long)((p.P + 127) / 128) * (d->Cout_pad / 64);
     p.splits = d->splits > 0 && d->splits <= 16 && !(d->splits & (d->splits - 1)) ? d->splits : thb_conv_simt_splits(d);
-    if (p.splits > 1) return launch_simt<64, true>(p, kn.sms, st);
-    if (d->Cout_pad % 128 == 0 && tiles >= 200) return launch_simt<128, false>(p, kn.sms, st);
-    return launch_simt<64, false>(p, kn.sms, st);
+    // (64 x 128 tiles give the same sums as 128 x 64 ones)
+    if (p.splits > 1) return low_tiles(d) ? launch_simt<64, 128, true>(p, kn.sms, st) : launch_simt<128, 64, true>(p, kn.sms, st);
+    if (d->Cout_pad % 128 == 0 && tiles >= 200) return launch_simt<128, 128, false>(p, kn.sms, st);
+    return launch_simt<128, 64, false>(p, kn.sms, st);
 }
