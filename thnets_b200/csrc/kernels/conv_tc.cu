@@ -560,6 +560,114 @@ __device__ __forceinline__ void epilogue_agent(const ConvTcParams &p, const CUte
         for (int k = q; k < q_pre; k++) mbar_wait_bounded(smem_u32(&avail[k % nbuf]), (k / nbuf) & 1, p.wait_limit);
 }
 
+// The copy thread's loop for whole 128-byte K blocks (no split, no 64-byte taps).  Its instructions pace a long reduction: a
+// round of the general loop, which asks in every K block what kind of layer this is, took some 1000 cycles beside busy epilogue
+// warps where the multiplies take 512, and a dozen more instructions in it cost a fifth of the layer.  Here every address is
+// stepped and everything that depends on the layer only is decided outside (3x3 256->256 @14x14, 256 images: 64 -> 59 us, 512->512 @7x7: 74 -> 67 us).
+struct CopyRing {
+    uint32_t a, b, full, empty;           // this stage: activation and weight tiles, barriers
+    uint32_t a_first, b_first, full_first, empty_first;
+    uint32_t a_step, b_step, parity;
+    int s, first, last;
+    __device__ CopyRing(uint32_t a0, uint32_t as, uint32_t b0, uint32_t bs, uint32_t f0, uint32_t e0, int ring_0, int ring_1)
+    {
+        first = s = ring_0;
+        last = ring_1;
+        a_step = as; b_step = bs;
+        a = a_first = a0 + ring_0 * as;
+        b = b_first = b0 + ring_0 * bs;
+        full = full_first = f0 + 8 * ring_0;
+        empty = empty_first = e0 + 8 * ring_0;
+        parity = 1;
+    }
+    __device__ __forceinline__ void next()
+    {
+        a += a_step; b += b_step; full += 8; empty += 8;
+        if (++s == last) {
+            s = first;
+            a = a_first; b = b_first; full = full_first; empty = empty_first;
+            parity ^= 1;
+        }
+    }
+};
+template <int KIND, int BN, bool PAIR>
+__device__ __forceinline__ void copy_tiles(const ConvTcParams &p, const CUtensorMap *tmA, const CUtensorMap *tmW, const CUtensorMap *tmR,
+                                           CopyRing ring, int lt, int lt_step, bool load_w, volatile int *abort_flag)
+{
+    constexpr int BKE = 128 / kind_traits<KIND>::esize;
+    const TileMap<BN> map(p);
+    const uint32_t bytes = (PAIR ? 2 : 1) * A_STAGE_BYTES + (load_w ? BN * 128 : 0);
+    const int nk1 = p.nkb1 ? p.nkb1 * BKE : p.nkb * BKE, nk = p.nkb * BKE;
+    const bool withhold = p.test_withhold != 0;
+    const long long limit = p.wait_limit;
+    auto wait = [&]() {
+        if (mbar_try_wait(ring.empty, ring.parity) || mbar_wait_bounded(ring.empty, ring.parity, limit)) return true;
+        atomicExch(p.status, 3);
+        *abort_flag = 1;
+        return false;
+    };
+    for (; lt < map.n_local; lt += lt_step) {
+        int m0, n0, k = 0;
+        map.coords(lt, m0, n0);
+        const bool last_unit = withhold && lt + (PAIR ? 2 : 1) >= map.n_local;
+        int iw[2] = {0, 0}, ih[2] = {0, 0}, in[2] = {0, 0};
+        if (p.a_tma == 2 || p.a2_mode == 2) {
+            // input position of each half's first output pixel: for tap (0, 0), or as the second operand is sampled
+            const int dh = p.a_tma == 2 ? p.dH : p.a2_d, dw = p.a_tma == 2 ? p.dW : p.a2_d;
+            const int ph = p.a_tma == 2 ? p.padH : 0, pw = p.a_tma == 2 ? p.tma_padw : 0;
+#pragma unroll
+            for (int h = 0; h < (PAIR ? 2 : 1); h++) {
+                const int m = m0 + h * BM, n = p.by_ohw(m), rem = m - n * p.oHW, oh = p.by_ow(rem);
+                in[h] = n;
+                ih[h] = oh * dh - ph;
+                iw[h] = (rem - oh * p.oW) * dw - pw;
+            }
+        }
+        if (p.a_tma == 2) {
+            const int slab_end = p.slabs * BKE;
+            for (int th = 0; k < nk; th++)
+                for (int tw = 0; tw < p.tma_kw; tw++)
+#pragma unroll 1
+                    for (int c = 0; c < slab_end; c += BKE) {
+                        if (!wait()) return;
+                        if (last_unit && k + BKE >= nk) return;
+                        mbar_arrive_expect_tx(ring.full, bytes);
+                        tma_load_im2col_4d(ring.a, tmA, ring.full, c, iw[0], ih[0], in[0], (uint16_t)tw, (uint16_t)th);
+                        if (PAIR) tma_load_im2col_4d(ring.a + A_STAGE_BYTES, tmA, ring.full, c, iw[1], ih[1], in[1], (uint16_t)tw, (uint16_t)th);
+                        if (load_w) tma_load_2d(ring.b, tmW, ring.full, k, n0);
+                        k += BKE;
+                        ring.next();
+                    }
+            continue;
+        }
+#pragma unroll 1
+        for (; k < nk1; k += BKE) {
+            if (!wait()) return;
+            if (last_unit && k + BKE >= nk) return;
+            mbar_arrive_expect_tx(ring.full, bytes);
+            tma_load_2d(ring.a, tmA, ring.full, k, m0);
+            if (PAIR) tma_load_2d(ring.a + A_STAGE_BYTES, tmA, ring.full, k, m0 + BM);
+            if (load_w) tma_load_2d(ring.b, tmW, ring.full, k, n0);
+            ring.next();
+        }
+#pragma unroll 1
+        for (; k < nk; k += BKE) {  // the second activation operand
+            if (!wait()) return;
+            if (last_unit && k + BKE >= nk) return;
+            mbar_arrive_expect_tx(ring.full, bytes);
+            if (p.a2_mode == 1) {
+                tma_load_2d(ring.a, tmR, ring.full, k - nk1, m0);
+                if (PAIR) tma_load_2d(ring.a + A_STAGE_BYTES, tmR, ring.full, k - nk1, m0 + BM);
+            } else {
+                tma_load_im2col_4d(ring.a, tmR, ring.full, k - nk1, iw[0], ih[0], in[0], 0, 0);
+                if (PAIR) tma_load_im2col_4d(ring.a + A_STAGE_BYTES, tmR, ring.full, k - nk1, iw[1], ih[1], in[1], 0, 0);
+            }
+            if (load_w) tma_load_2d(ring.b, tmW, ring.full, k, n0);
+            ring.next();
+        }
+    }
+}
+
 template <int KIND, int BN, int STAGES, bool SPLIT>
 __global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid_constant__ CUtensorMap tmapW, const __grid_constant__ CUtensorMap tmapA,
                                                                const __grid_constant__ CUtensorMap tmapY, const __grid_constant__ CUtensorMap tmapR,
@@ -744,7 +852,14 @@ __global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid
     } else if (warp == 4 || (KIND == 2 && warp == 14)) {
         // ================================================================== TMA producer: per K block the weight tile
         // and, in the TMA modes, the activation tile (both halves' tiles in pair mode)
-        if (lane == 0) {
+        if (!SPLIT && p.a_tma && !p.half) {
+            if (lane == 0) {
+                const int ring_0 = KIND == 2 && warp == 14 ? nst / 2 : 0, ring_1 = KIND == 2 && p.dual && warp == 4 ? nst / 2 : nst;
+                const CopyRing ring(smem_u32(sA), a_stage_bytes, smem_u32(sB), B_STAGE_BYTES, smem_u32(full), smem_u32(empty), ring_0, ring_1);
+                if (L::TMA_EPI && BN <= 128 && pair) copy_tiles<KIND, BN, true>(p, &tmapA, &tmapW, &tmapR, ring, 0, 2, true, abort_flag);
+                else copy_tiles<KIND, BN, false>(p, &tmapA, &tmapW, &tmapR, ring, KIND == 2 && warp == 14 ? 1 : 0, KIND == 2 && p.dual ? 2 : 1, !res_w, abort_flag);
+            }
+        } else if (lane == 0) {
             const TileMap<BN, SPLIT> map(p);
             const int halves = pair ? 2 : 1, lt_step = KIND == 2 && p.dual ? 2 : halves;
             const int ring_0 = KIND == 2 && warp == 14 ? nst / 2 : 0, ring_1 = KIND == 2 && p.dual && warp == 4 ? nst / 2 : nst;
@@ -842,6 +957,8 @@ __global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid
             int ring_s = ring_0;
             uint32_t ring_ph = 0;
             bool alive = true;
+            const uint64_t a_desc = make_sw128_kmajor_desc(smem_u32(sA)), b_desc = make_sw128_kmajor_desc(smem_u32(sB));
+            const uint32_t a_dstep = (uint32_t)a_stage_bytes >> 4;
             if (KIND == 2 && res_w && !mbar_wait_bounded(smem_u32(wfull), 0, p.wait_limit)) {
                 atomicExch(p.status, 4);
                 *abort_flag = 1;
@@ -860,6 +977,32 @@ __global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid
                 const uint32_t d0 = tmem_base + (lt % NACC) * BN, d1 = tmem_base + ((lt + 1) % NACC) * BN;
                 int kb0 = 0, kb1 = p.nkb;
                 if (SPLIT) map.kblocks(lt, kb0, kb1);
+                if (!SPLIT && p.a_tma && !p.half) {
+                    // whole K blocks brought by the copy engine: nothing to decide per block (and no writes of this proxy to fence)
+#pragma unroll 1
+                    for (int kb = 0; kb < kb1; kb++) {
+                        const uint32_t bar = smem_u32(&full[ring_s]);
+                        if (!mbar_try_wait(bar, ring_ph) && !mbar_wait_bounded(bar, ring_ph, p.wait_limit)) {
+                            atomicExch(p.status, 4);
+                            *abort_flag = 1;
+                            alive = false;
+                            break;
+                        }
+                        tc_fence_after();
+                        const uint64_t ad = a_desc + (uint32_t)ring_s * a_dstep, bd = b_desc + (uint32_t)(res_w ? kb : ring_s) * (B_STAGE_BYTES >> 4);
+#pragma unroll
+                        for (int k = 0; k < 4; k++) {
+                            if (KIND == 2) tc_mma_i8(d0, ad + 2 * k, bd + 2 * k, IDESC, (kb | k) != 0);
+                            else tc_mma_f16(d0, ad + 2 * k, bd + 2 * k, IDESC, (kb | k) != 0);
+                        }
+                        if (pair) {
+#pragma unroll
+                            for (int k = 0; k < 4; k++) tc_mma_f16(d1, ad + (A_STAGE_BYTES >> 4) + 2 * k, bd + 2 * k, IDESC, (kb | k) != 0);
+                        }
+                        tc_commit(smem_u32(&empty[ring_s]));
+                        if (++ring_s == ring_1) { ring_s = ring_0; ring_ph ^= 1; }
+                    }
+                } else
                 for (int kb = kb0; kb < kb1; kb++) {
                     const int s = ring_s;
                     const uint32_t ph = ring_ph;
