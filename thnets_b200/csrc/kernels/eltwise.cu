@@ -140,10 +140,9 @@ __global__ void preprocess_kernel(const float *x, float *x_inplace, int N, int C
 // a row is written here, the padding as zeros.
 template <typename T>
 __global__ void preprocess_s2d_kernel(const float *x, float *x_inplace, int N, int C, int H, int W, float3 mean,
-                                      float3 std_, T *y, int y_ld, int row_pitch, int pad_left, float q_min, float q_mult)
+                                      float3 std_, T *y, int y_ld, int row_pitch, int pad_left)
 {
     pdl_enter();
-    const float zr = roundf(q_min * q_mult);  // uint8 only: the quantisation of preprocess_kernel
     constexpr int VN = Vec<T>::N;
     const int H2 = H / 2, W2 = W / 2;
     const long pix = (long)blockIdx.x * blockDim.x + threadIdx.x;  // over the stored (padded) pixels
@@ -169,7 +168,6 @@ __global__ void preprocess_s2d_kernel(const float *x, float *x_inplace, int N, i
                     val = x[idx];
                     if (c < 3) val = __fdiv_rn(__fsub_rn(val, m[c]), sd[c]);
                     if (x_inplace) x_inplace[idx] = val;
-                    if (sizeof(T) == 1) val = (float)(((int)(roundf(val * q_mult) - zr)) & 255);
                 }
                 v[i] = val;
             }
@@ -192,10 +190,6 @@ __global__ void preprocess_s2d_kernel(const float *x, float *x_inplace, int N, i
                     v.y = __fdiv_rn(__fsub_rn(v.y, m[c]), sd[c]);
                 }
                 if (x_inplace) *reinterpret_cast<float2 *>(x_inplace + idx) = v;
-                if (sizeof(T) == 1) {
-                    v.x = (float)(((int)(roundf(v.x * q_mult) - zr)) & 255);
-                    v.y = (float)(((int)(roundf(v.y * q_mult) - zr)) & 255);
-                }
                 // channel (ph*2 + pw)*3 + c of the regrouped pixel
                 vals[(ph * 2) * 3 + c] = v.x;
                 vals[(ph * 2 + 1) * 3 + c] = v.y;
@@ -418,40 +412,6 @@ __global__ void preprocess_images_kernel(const uint8_t *img, int N, int H, int W
 #pragma unroll
     for (int i = 0; i < VN; i++) v[i] = 0.f;
     for (int c0 = VN; c0 < y_ld; c0 += VN) Vec<T>::store(y + pix * y_ld + c0, v);
-}
-
-// u8 HWC RGB images -> normalised space-to-depth NHWC T: the layout preprocess_s2d_kernel writes (channel (ph*2 + pw)*3 + c
-// of block (bh, bw) = pixel (2bh + ph, 2bw + pw), rows row_pitch pixels apart with pad_left zero pixels in front), with the
-// arithmetic of the image loader (thapi.c:20-46)
-template <typename T>
-__global__ void preprocess_images_s2d_kernel(const uint8_t *img, int N, int H, int W, int stride, int bgr, float3 mean, float3 istd,
-                                             T *y, int y_ld, int row_pitch, int pad_left)
-{
-    pdl_enter();
-    constexpr int VN = Vec<T>::N;
-    const int H2 = H / 2, W2 = W / 2;
-    const long pix = (long)blockIdx.x * blockDim.x + threadIdx.x;  // over the stored (padded) pixels
-    if (pix >= (long)N * H2 * row_pitch) return;
-    const long n = pix / ((long)H2 * row_pitch);
-    const int rem = (int)(pix - n * (long)H2 * row_pitch), bh = rem / row_pitch, bw = rem - bh * row_pitch - pad_left;
-    const bool real = bw >= 0 && bw < W2;
-    const float m[3] = {mean.x, mean.y, mean.z}, is[3] = {istd.x, istd.y, istd.z};
-    constexpr int Cs = 12, Cpad = (Cs + VN - 1) / VN * VN;
-    for (int c0 = 0; c0 < Cpad; c0 += VN) {
-        float v[VN];
-#pragma unroll
-        for (int i = 0; i < VN; i++) {
-            const int cs = c0 + i;
-            float val = 0.f;
-            if (real && cs < Cs) {
-                const int blk = cs / 3, c = cs - blk * 3;
-                const uint8_t *src = img + ((size_t)n * H + 2 * bh + (blk >> 1)) * stride + (size_t)(2 * bw + (blk & 1)) * 3;
-                val = __fmul_rn(__fsub_rn(__fmul_rn((float)src[bgr ? 2 - c : c], 0.003921568f), m[c]), is[c]);
-            }
-            v[i] = val;
-        }
-        Vec<T>::store(y + pix * y_ld + c0, v);
-    }
 }
 
 // One YUYV frame (Y0 U Y1 V per pixel pair) -> normalised NHWC T with three channels, the arithmetic of the reference's
@@ -1073,7 +1033,7 @@ int thb_preprocess_s2d_padded(const float *x, float *x_inplace, int N, int C, in
     const long pix = (long)N * (H / 2) * row_pitch;
     if (pix == 0) return THB_OK;
     float3 m = make_float3(mean3[0], mean3[1], mean3[2]), sd = make_float3(std3[0], std3[1], std3[2]);
-    DISPATCH_FLOAT_DTYPE(dtype, (thb_launch(preprocess_s2d_kernel<T>, nblocks(pix), 256, s, x, x_inplace, N, C, H, W, m, sd, (T *)y, y_ld, row_pitch, pad_left, 0.f, 0.f)));
+    DISPATCH_FLOAT_DTYPE(dtype, (thb_launch(preprocess_s2d_kernel<T>, nblocks(pix), 256, s, x, x_inplace, N, C, H, W, m, sd, (T *)y, y_ld, row_pitch, pad_left)));
     return THB_LAUNCH_CHECK("preprocess_s2d_kernel");
 }
 
@@ -1081,12 +1041,7 @@ int thb_preprocess_s2d_u8(const float *x, float *x_inplace, int N, int C, int H,
                           void *y, int y_ld, float q_sub, float q_mult, thb_stream s)
 {
     if ((H | W) & 1) return THB_ERR_ARG;
-    const long pix = (long)N * (H / 2) * (W / 2);
-    if (pix == 0) return THB_OK;
-    float3 m = make_float3(mean3[0], mean3[1], mean3[2]), sd = make_float3(std3[0], std3[1], std3[2]);
-    thb_launch(preprocess_s2d_kernel<uint8_t>, nblocks(pix), 256, s, x, x_inplace, N, C, H, W, m, sd, (uint8_t *)y, y_ld,
-                                                                              W / 2, 0, q_sub, q_mult);
-    return THB_LAUNCH_CHECK("preprocess_s2d_kernel<u8>");
+    return thb_preprocess_s2d_any(x, 0, x_inplace, N, C, H, W, 2, 0, 0, mean3, std3, THB_U8, y, y_ld, W / 2, 0, &q_sub, &q_mult, s);
 }
 
 int thb_preprocess_neigh_u8(const float *x, float *x_inplace, int N, int H, int W, const float *mean3, const float *std3, void *y,
@@ -1142,14 +1097,10 @@ int thb_preprocess_yuyv(const unsigned char *frame, int H, int W, const float *m
 int thb_preprocess_images_s2d(const unsigned char *img, int N, int H, int W, int stride, int bgr, const float *mean3, const float *std3,
                               int dtype, void *y, int y_ld, int row_pitch, int pad_left, thb_stream s)
 {
-    if (((H | W) & 1) || pad_left < 0 || row_pitch < pad_left + W / 2 || y_ld < 12) return THB_ERR_ARG;
+    if (((H | W) & 1) || y_ld < 12) return THB_ERR_ARG;
     if (dtype != THB_F16 && dtype != THB_BF16) return THB_ERR_UNSUPPORTED;
-    const long pix = (long)N * (H / 2) * row_pitch;
-    if (pix == 0) return THB_OK;
-    float3 m = make_float3(mean3[0], mean3[1], mean3[2]);
-    float3 is = make_float3(1 / std3[0], 1 / std3[1], 1 / std3[2]);
-    DISPATCH_FLOAT_DTYPE(dtype, (thb_launch(preprocess_images_s2d_kernel<T>, nblocks(pix), 256, s, img, N, H, W, stride, bgr, m, is, (T *)y, y_ld, row_pitch, pad_left)));
-    return THB_LAUNCH_CHECK("preprocess_images_s2d_kernel");
+    float q_sub = 0, q_mult = 0;
+    return thb_preprocess_s2d_any(img, 1, 0, N, 3, H, W, 2, stride, bgr, mean3, std3, dtype, y, y_ld, row_pitch, pad_left, &q_sub, &q_mult, s);
 }
 
 int thb_preprocess_images_lowp(const unsigned char *img, int N, int H, int W, int stride, int bgr, const float *mean3,
