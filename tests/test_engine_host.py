@@ -1,0 +1,116 @@
+"""The host side of a forward -- plans kept and dropped, sub-batches, where the uint8 input range comes from -- without a GPU: the
+host library's own sources on a CUDA runtime and kernel launchers that compute nothing (fake_cuda.c).  Every test runs in a process
+of its own, so that the fakes meet no other library."""
+import os
+import shutil
+import subprocess
+import sys
+
+import pytest
+
+from thnets_b200.capi import DEFAULT_LIB
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CUDA = os.environ.get("CUDA", "/usr/local/cuda")
+
+pytestmark = [
+    pytest.mark.skipif(not os.path.exists(DEFAULT_LIB), reason="libthnets.so not built"),
+    pytest.mark.skipif(shutil.which("gcc") is None or not os.path.exists(os.path.join(CUDA, "include")), reason="needs gcc and CUDA's headers"),
+]
+
+
+@pytest.fixture(scope="module")
+def engine(tmp_path_factory):
+    """Runs a test's code on the faked engine: `th` the binding, `lib` the library, `fake` its variables by name."""
+    so = str(tmp_path_factory.mktemp("engine") / "libengine.so")
+    csrc = os.path.join(ROOT, "thnets_b200", "csrc")
+    host = [os.path.join(csrc, "host", f) for f in sorted(os.listdir(os.path.join(csrc, "host"))) if f.endswith(".c")]
+    subprocess.check_call(["gcc", "-O1", "-w", "-std=gnu11", "-shared", "-fPIC", "-ffp-contract=off", "-fopenmp", "-I", os.path.join(ROOT, "include"),
+                           "-I", os.path.join(csrc, "host"), "-I", os.path.join(csrc, "kernels"), "-I", os.path.join(CUDA, "include"), "-o", so]
+                          + host + [os.path.join(ROOT, "tests", "fake_cuda.c"), DEFAULT_LIB, "-lm", "-Wl,-rpath," + os.path.dirname(DEFAULT_LIB)])
+    head = f"""
+import ctypes as C, os, sys
+sys.path.insert(0, {ROOT!r})
+os.environ["THB200_NO_EXIT"] = "1"
+import numpy as np
+from thnets_b200 import fixtures as fx
+from thnets_b200.capi import THNets
+th = THNets({so!r})
+lib = th.lib
+class Fake:
+    kinds = dict(budget=C.c_size_t, live=C.c_size_t, q_sub=C.c_float, q_mult=C.c_float)
+    def var(self, name):
+        return self.kinds.get(name, C.c_int).in_dll(lib, "fake_" + name)
+    def __getattr__(self, name):
+        return self.var(name).value
+    def __setattr__(self, name, v):
+        self.var(name).value = v
+fake = Fake()
+def network(g, mode, path="net"):
+    fx.write_pymodel(g, path)
+    src = th.load_network(path)
+    if mode == 3:
+        net = th.create_lowp_network(src, 8.0)
+    else:
+        lib.THB200_SetPrecision(mode)
+        net = lib.THCreateCudaNetwork(src)
+    assert net
+    th.free_network(src)
+    return net
+def pinned(shape):
+    p = lib.THB200_HostAlloc(4 * int(np.prod(shape)))
+    return np.ctypeslib.as_array(C.cast(p, C.POINTER(C.c_float)), shape=shape)
+def call(net, x, fn=None):
+    res, ow, oh = C.POINTER(C.c_float)(), C.c_int(), C.c_int()
+    n, c, h, w = x.shape
+    return (fn or lib.THB200_ProcessFloatConst)(net, x.ctypes.data, n, w, h, c, C.byref(res), C.byref(ow), C.byref(oh))
+"""
+
+    def run(code, tmp_path, threads=4):
+        env = dict(os.environ, OMP_NUM_THREADS=str(threads))
+        r = subprocess.run([sys.executable, "-c", head + code], capture_output=True, text=True, env=env, cwd=tmp_path)
+        assert r.returncode == 0, r.stdout + r.stderr
+
+    return run
+
+
+@pytest.mark.parametrize("threads", [1, 4, 16])
+@pytest.mark.parametrize("size", [64, 225])
+def test_uint8_input_range(engine, tmp_path, threads, size):
+    """A uint8 forward of a float batch takes its range from one pass: the host's staging of a pageable batch, a pass of the host's
+    threads over a small page-locked one, the devices' pass over a large one -- and only there is the devices' pass launched, whatever
+    the number of threads.  Where the host finds the range it is that of the normalised values, NaNs left out."""
+    engine(f"""
+size, threads = {size}, {threads}
+g = fx.resnet18(width=0.25, size=size, classes=10, fc_bias=0.05)
+net = network(g, 3)
+mean, std = np.float32([0.45, 0.4, 0.5]), np.float32([0.225, 0.25, 0.2])
+th.set_stats(net, mean, std)
+def expected(x):
+    v = (x - mean[None, :, None, None]) / std[None, :, None, None]
+    lo, hi = min(0, np.nanmin(v)), max(0, np.nanmax(v))
+    return np.float32(lo), np.float32(255.0 / float(hi - lo))
+rng = np.random.default_rng(size)
+for n in (1, 5, 67):
+    for where in ("const", "inplace", "pinned"):
+        x = (pinned if where == "pinned" else np.empty)((n, 3, size, size))
+        x = x.astype(np.float32, copy=False)
+        x[...] = rng.standard_normal(x.shape, dtype=np.float32)
+        x[n // 2, 1, 7, 7:11] = np.nan
+        x[n - 1, n % 3, size - 1, size - 1] = 9 + n  # the batch's very last values count
+        x[0, 2, 0, 0] = -7 - n
+        want, fake.minmax = expected(x), 0
+        copy = x.copy()
+        assert call(net, x, lib.THProcessFloat if where == "inplace" else None) > 0
+        small = x.nbytes <= min(threads, 8) * 300 * 1024
+        if where == "pinned" and not small:
+            assert fake.minmax == 1, (n, where)
+        else:
+            assert fake.minmax == 0, (n, where)
+            assert (np.float32(fake.q_sub), np.float32(fake.q_mult)) == want, (n, where, fake.q_sub, fake.q_mult, want)
+        if where == "inplace":
+            assert np.array_equal(x, (copy - mean[None, :, None, None]) / std[None, :, None, None], equal_nan=True)
+        else:
+            assert np.array_equal(x, copy, equal_nan=True)
+assert fake.empty == 0
+""", tmp_path, threads)

@@ -59,16 +59,21 @@ def test_sliced_start(th, tmp_path, mode, images, net, batch, size):
 @pytest.mark.parametrize("net,batch,size", [("resnet18", 5, 97), ("resnet18", 66, 224), ("vgg16", 40, 224)])
 @pytest.mark.parametrize("nan", [False, True], ids=["finite", "nan"])
 def test_uint8_range_found_by_the_host(th, tmp_path, net, batch, size, nan):
-    """A uint8 forward of a float batch with the range found by the host's threads (six or more of them) under the copy, its
-    first launches sliced, against the range found by the device after it."""
+    """A uint8 forward of a float batch with the range found wherever it is found -- by the host's threads while they stage a
+    pageable batch, as it is or normalising it in place, by a pass of theirs over a small page-locked one, by the device's pass
+    over a large one -- and with many threads or few: the same bytes."""
     import ctypes
     omp = ctypes.CDLL("libgomp.so.1")
+    threads_before = omp.omp_get_max_threads()
     g = fx.vgg16(width=0.25, classes=10, fc=64) if net == "vgg16" else fx.resnet18(width=0.25, size=size, classes=10, fc_bias=0.05)
     path = str(tmp_path / "n.net")
     fx.write_pymodel(g, path)
     x = np.random.default_rng(batch).standard_normal((batch, 3, size, size), dtype=np.float32)
     if nan:
         x[batch // 2, 1, 7, 7:11] = np.nan
+    p = th.lib.THB200_HostAlloc(x.nbytes)
+    pinned = np.ctypeslib.as_array(ctypes.cast(p, ctypes.POINTER(ctypes.c_float)), shape=x.shape)
+    pinned[...] = x
     outs = []
     for threads in (8, 2):
         omp.omp_set_num_threads(threads)
@@ -77,9 +82,11 @@ def test_uint8_range_found_by_the_host(th, tmp_path, net, batch, size, nan):
             th.set_stats(h, (0.45, 0.4, 0.5), (0.225, 0.25, 0.2))
             net_h = th.create_lowp_network(h, 8.0)
             th.free_network(h)
-            outs += [th.process_float(net_h, x)[0] for _ in range(3)]
+            outs += [th.process_float(net_h, b)[0] for b in (x, x, pinned, x, pinned)]
+            outs.append(th.process_float(net_h, x.copy(), copy_input=False)[0])
             th.free_network(net_h)
         finally:
-            omp.omp_set_num_threads(4)
+            omp.omp_set_num_threads(threads_before)
+    th.lib.THB200_HostFree(p)
     for o in outs[1:]:
         assert np.array_equal(o, outs[0])

@@ -1513,11 +1513,6 @@ static int plan_node(planner *P, int i)
     return -1;
 }
 
-/* The uint8 engine needs the range of a whole float batch before it can start.  Several host threads read the batch faster than
- * the link carries it, so they find the range while it is on its way; a few would take longer than the copy and a pass of the
- * device over it. */
-static int host_scans(void) { return omp_get_max_threads() >= 6; }
-
 /* Can launch `s` run on some of its images?  (The planned convolutions and poolings whose images are independent; what
  * they add is the image offset of every operand, exec_step.) */
 static int sliceable(const instance *I, const step *s)
@@ -1579,7 +1574,8 @@ static double copy_in_us(const thb_engine *E, const instance *I)
 static void choose_slices(thb_engine *E, instance *I)
 {
     I->prefix = I->slices = 0;
-    if ((E->dtype == THB_U8 && !E->cur->cp && !host_scans()) || E->cur->cp == 2 || E->whole_batch || I->in_val.buf < 0) return;
+    /* (a uint8 float batch: its range is known when the last of it has been staged, scanned or copied, and nothing starts before) */
+    if ((E->dtype == THB_U8 && !E->cur->cp) || E->cur->cp == 2 || E->whole_batch || I->in_val.buf < 0) return;
     const char *off = getenv("THB200_NO_SLICES");
     if (off && atoi(off)) return;
     const double t_in = copy_in_us(E, I);
@@ -2378,63 +2374,6 @@ static int plan_build(thb_engine *E)
     return 0;
 }
 
-static int stage_threads(void);
-
-/* Smallest and largest normalised value of N images, both seeded with 0 (lowp_basic.c:15-29): the extremes of every channel's
- * planes as they are, and only those normalised -- a subtraction and a division in fp32 are monotone.  NaNs do not count, as in
- * the device's pass (thb_minmax_normalized). */
-static void host_range(const float *x, int N, int C, long HW, const float *mean, const float *std, float *lo, float *hi)
-{
-    float mn[4] = {INFINITY, INFINITY, INFINITY, INFINITY}, mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-    const long per = 16384, pieces = (HW + per - 1) / per, items = (long)N * C * pieces;
-#pragma omp parallel num_threads(stage_threads()) if (items > 4)
-    {
-        float tmn[4] = {INFINITY, INFINITY, INFINITY, INFINITY}, tmx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma omp for schedule(static) nowait
-        for (long t = 0; t < items; t++) {
-            const long plane = t / pieces, i0 = (t % pieces) * per, i1 = i0 + per < HW ? i0 + per : HW;
-            const int k = plane % C < 3 ? (int)(plane % C) : 3;
-            const float *p = x + plane * HW;
-            float a = tmn[k], b = tmx[k];
-            long i = i0;
-#ifdef __SSE2__
-            /* (min and max with the running value as second operand keep it when the new one is a NaN) */
-            __m128 a0 = _mm_set1_ps(a), a1 = a0, b0 = _mm_set1_ps(b), b1 = b0;
-            for (; i + 8 <= i1; i += 8) {
-                const __m128 u = _mm_loadu_ps(p + i), v = _mm_loadu_ps(p + i + 4);
-                a0 = _mm_min_ps(u, a0); b0 = _mm_max_ps(u, b0);
-                a1 = _mm_min_ps(v, a1); b1 = _mm_max_ps(v, b1);
-            }
-            float va[8], vb[8];
-            _mm_storeu_ps(va, a0); _mm_storeu_ps(va + 4, a1); _mm_storeu_ps(vb, b0); _mm_storeu_ps(vb + 4, b1);
-            for (int q = 0; q < 8; q++) {
-                if (va[q] < a) a = va[q];
-                if (vb[q] > b) b = vb[q];
-            }
-#endif
-            for (; i < i1; i++) {
-                if (p[i] < a) a = p[i];
-                if (p[i] > b) b = p[i];
-            }
-            tmn[k] = a; tmx[k] = b;
-        }
-#pragma omp critical
-        for (int k = 0; k < 4; k++) {
-            if (tmn[k] < mn[k]) mn[k] = tmn[k];
-            if (tmx[k] > mx[k]) mx[k] = tmx[k];
-        }
-    }
-    *lo = *hi = 0;
-    for (int k = 0; k < 4; k++) {
-        if (!(mn[k] <= mx[k])) continue;
-        float a = mn[k], b = mx[k];
-        if (k < 3) { a = (a - mean[k]) / std[k]; b = (b - mean[k]) / std[k]; }
-        if (a > b) { const float t = a; a = b; b = t; }
-        if (a < *lo) *lo = a;
-        if (b > *hi) *hi = b;
-    }
-}
-
 static int g_chunks_override; /* 0 = the engine's own choice */
 void thb_set_pipeline_chunks(int n) { g_chunks_override = n < 0 ? 0 : n > 4 ? 4 : n; }
 
@@ -2604,13 +2543,14 @@ static int device_forward(thb_engine *E, instance *I, int has_x, int inplace, in
     return boundary_out(E, I, dst, head_on(I));
 }
 
-/* 1 when `p` is ordinary (pageable) host memory: a copy from it is staged by the driver at a fraction of the link rate and
- * blocks the calling thread */
-static int host_is_pageable(const void *p)
+/* What the caller's batch lies in.  A copy from ordinary (pageable) memory is staged by the driver at a fraction of the link rate
+ * and blocks the calling thread; only page-locked memory is known to be at hand for the host's threads too. */
+enum host_memory { MEM_PAGEABLE, MEM_PINNED, MEM_OTHER };
+static enum host_memory host_memory_of(const void *p)
 {
     struct cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return 0; }
-    return a.type == cudaMemoryTypeUnregistered;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return MEM_OTHER; }
+    return a.type == cudaMemoryTypeUnregistered ? MEM_PAGEABLE : a.type == cudaMemoryTypeHost ? MEM_PINNED : MEM_OTHER;
 }
 
 /* Copy into the pinned staging buffer past the caches.  The device reads the buffer next and the host never does: lines left
@@ -2661,6 +2601,123 @@ static void parallel_copy(void *dst, const void *src, size_t bytes)
     }
 }
 
+/* Smallest and largest value of a float batch's planes, by what is subtracted from them: channels 0, 1 and 2, and the others.
+ * Empty classes are (INFINITY, -INFINITY); NaNs do not count, as in the device's pass (thb_minmax_normalized). */
+typedef struct {
+    float mn[4], mx[4];
+} extremes;
+static const extremes NO_EXTREMES = {{INFINITY, INFINITY, INFINITY, INFINITY}, {-INFINITY, -INFINITY, -INFINITY, -INFINITY}};
+
+static void extremes_join(extremes *e, const extremes *t)
+{
+#pragma omp critical(thb_extremes)
+    for (int k = 0; k < 4; k++) {
+        if (t->mn[k] < e->mn[k]) e->mn[k] = t->mn[k];
+        if (t->mx[k] > e->mx[k]) e->mx[k] = t->mx[k];
+    }
+}
+
+#ifdef __SSE2__
+/* four values into the running extremes (min and max with the running value as second operand keep it when the new one is a NaN) */
+#define EXTREMES4(v, lo, hi) ((lo) = _mm_min_ps(v, lo), (hi) = _mm_max_ps(v, hi))
+static void extremes_of4(__m128 lo, __m128 hi, float *mn, float *mx)
+{
+    float a[4], b[4];
+    _mm_storeu_ps(a, lo);
+    _mm_storeu_ps(b, hi);
+    for (int q = 0; q < 4; q++) {
+        if (a[q] < *mn) *mn = a[q];
+        if (b[q] > *mx) *mx = b[q];
+    }
+}
+#endif
+
+/* The extremes of n values joined to *mn and *mx and, with `d`, the values copied there past the caches, in one pass over them. */
+static void scan_values(float *d, const float *s, long n, float *mn, float *mx)
+{
+    float a = *mn, b = *mx;
+    long i = 0;
+#ifdef __SSE2__
+    long head = d ? (long)((64 - ((size_t)d & 63)) & 63) / 4 : 0; /* whole lines from there on */
+    if (head > n) head = n;
+    for (; i < head; i++) {
+        const float v = d[i] = s[i];
+        if (v < a) a = v;
+        if (v > b) b = v;
+    }
+    __m128 a0 = _mm_set1_ps(a), a1 = a0, b0 = _mm_set1_ps(b), b1 = b0;
+    for (; i + 16 <= n; i += 16) {
+        const __m128 t = _mm_loadu_ps(s + i), u = _mm_loadu_ps(s + i + 4), v = _mm_loadu_ps(s + i + 8), w = _mm_loadu_ps(s + i + 12);
+        EXTREMES4(t, a0, b0);
+        EXTREMES4(u, a1, b1);
+        EXTREMES4(v, a0, b0);
+        EXTREMES4(w, a1, b1);
+        if (d) {
+            _mm_stream_ps(d + i, t);
+            _mm_stream_ps(d + i + 4, u);
+            _mm_stream_ps(d + i + 8, v);
+            _mm_stream_ps(d + i + 12, w);
+        }
+    }
+    extremes_of4(a0, b0, &a, &b);
+    extremes_of4(a1, b1, &a, &b);
+    if (d) _mm_sfence();
+#endif
+    for (; i < n; i++) {
+        const float v = s[i];
+        if (d) d[i] = v;
+        if (v < a) a = v;
+        if (v > b) b = v;
+    }
+    *mn = a;
+    *mx = b;
+}
+
+/* The same for planes [p0, p1) of an NCHW float batch (plane p = image p / C, channel p % C, HW floats), by several threads. */
+static void scan_planes(float *dst, const float *x, long p0, long p1, int C, long HW, extremes *e)
+{
+    const long pieces = (HW + 16383) / 16384, per = ((HW + pieces - 1) / pieces + 15) & ~15L, items = (p1 - p0) * pieces;
+#pragma omp parallel num_threads(stage_threads()) if (items > 4)
+    {
+        extremes t = NO_EXTREMES;
+#pragma omp for schedule(static) nowait
+        for (long q = 0; q < items; q++) {
+            const long p = p0 + q / pieces, i0 = q % pieces * per, i1 = i0 + per < HW ? i0 + per : HW;
+            const int k = p % C < 3 ? (int)(p % C) : 3;
+            if (i0 < i1) scan_values(dst ? dst + p * HW + i0 : 0, x + p * HW + i0, i1 - i0, &t.mn[k], &t.mx[k]);
+        }
+        extremes_join(e, &t);
+    }
+}
+
+/* Smallest and largest normalised value of the batch, both seeded with 0 (lowp_basic.c:15-29): only the extremes are normalised --
+ * a subtraction and a division in fp32 are monotone. */
+static void extremes_range(const extremes *e, const float *mean, const float *std, float *lo, float *hi)
+{
+    *lo = *hi = 0;
+    for (int k = 0; k < 4; k++) {
+        if (!(e->mn[k] <= e->mx[k])) continue;
+        float a = e->mn[k], b = e->mx[k];
+        if (k < 3) { a = (a - mean[k]) / std[k]; b = (b - mean[k]) / std[k]; }
+        if (a > b) { const float t = a; a = b; b = t; }
+        if (a < *lo) *lo = a;
+        if (b > *hi) *hi = b;
+    }
+}
+
+/* Does a pass of the host's threads over a page-locked batch, under its copy, end before the devices' pass after it?  What it can
+ * save is that pass and the wait for its result: 20 to 25 us, whatever the size.  But a thread reads 6 GB/s of a batch that is in
+ * no cache, several slow one another and the copy down, and the link carries 55 GB/s: from some size on, the more the longer, the
+ * call waits for the host.  ResNet-18 uint8, microseconds a call with the devices' pass / the host's, batches read from memory
+ * (in brackets: from the cache):
+ *     threads      1               2               4               8
+ *     0.6 MB   225 / 252 (208)  224 / 212 (200)  225 / 212 (200)  225 / 203 (200)
+ *     1.2 MB   246 / 323 (254)  247 / 262 (218)  247 / 233 (219)  247 / 229 (218)
+ *     2.4 MB   286 / 473 (317)  286 / 348 (273)  285 / 285 (259)  285 / 282 (260)
+ *     4.8 MB   356 / 757 (434)  356 / 511 (365)  358 / 384 (337)  356 / 384 (345)
+ *     9.6 MB   506 / 1315 (672) 506 / 829 (557)  505 / 581 (534)  507 / 579 (503) */
+static int host_scan_pays(size_t bytes) { return bytes <= (size_t)stage_threads() * 300 << 10; }
+
 /* Byte images, each wherever the caller has it, to one tightly packed array.  The threads share blocks of rows, so that
  * one large image is spread over them as well as a batch of small ones. */
 static void stage_images(unsigned char *dst, unsigned char *const *images, int n, int H, size_t row, size_t stride)
@@ -2679,37 +2736,52 @@ static void stage_images(unsigned char *dst, unsigned char *const *images, int n
     }
 }
 
-/* The same for planes [p0, p1) of an NCHW float batch (plane p = image p / C, channel p % C, HW floats), normalising the
- * first three channels on the way exactly as the boundary kernels do -- (x - mean) / std, a subtraction and a division in
- * fp32 -- and writing the normalised values back over the caller's planes: THProcessFloat's in-place side effect
- * (thapi.c:396-403) done where the reference does it, on the host, instead of a 12-bytes-per-pixel copy back from the
- * device. */
-static void stage_planes_normalised(float *dst, float *src, long p0, long p1, int C, long HW, const float *mean, const float *std)
+/* The copy of planes [p0, p1) of an NCHW float batch into the staging buffer, normalising the first three channels on the way
+ * exactly as the boundary kernels do -- (x - mean) / std, a subtraction and a division in fp32 -- and writing the normalised
+ * values back over the caller's planes: THProcessFloat's in-place side effect (thapi.c:396-403) done where the reference does
+ * it, on the host, instead of a 12-bytes-per-pixel copy back from the device.  `e`: the extremes of what is staged, or NULL. */
+static void stage_planes_normalised(float *dst, float *src, long p0, long p1, int C, long HW, const float *mean, const float *std,
+                                    extremes *e)
 {
-#pragma omp parallel for schedule(static) if ((p1 - p0) * HW > 65536) num_threads(stage_threads())
-    for (long p = p0; p < p1; p++) {
-        const int c = (int)(p % C);
-        float *s = src + p * HW, *d = dst + p * HW;
-        if (c < 3) {
-            const float m = mean[c], sd = std[c];
-            long i = 0;
+#pragma omp parallel if ((p1 - p0) * HW > 65536) num_threads(stage_threads())
+    {
+        extremes t = NO_EXTREMES;
+#pragma omp for schedule(static) nowait
+        for (long p = p0; p < p1; p++) {
+            const int c = (int)(p % C);
+            float *s = src + p * HW, *d = dst + p * HW;
+            if (c < 3) {
+                const float m = mean[c], sd = std[c];
+                float a = t.mn[c], b = t.mx[c];
+                long i = 0;
 #ifdef __SSE2__
-            const __m128 vm = _mm_set1_ps(m), vs = _mm_set1_ps(sd);
-            if (((size_t)d & 15) == 0)
-                for (; i + 4 <= HW; i += 4) {
-                    const __m128 v = _mm_div_ps(_mm_sub_ps(_mm_loadu_ps(s + i), vm), vs);
-                    _mm_storeu_ps(s + i, v);
-                    _mm_stream_ps(d + i, v);
-                }
-            _mm_sfence();
+                const __m128 vm = _mm_set1_ps(m), vs = _mm_set1_ps(sd);
+                __m128 lo = _mm_set1_ps(a), hi = _mm_set1_ps(b);
+                if (((size_t)d & 15) == 0)
+                    for (; i + 4 <= HW; i += 4) {
+                        const __m128 v = _mm_div_ps(_mm_sub_ps(_mm_loadu_ps(s + i), vm), vs);
+                        _mm_storeu_ps(s + i, v);
+                        _mm_stream_ps(d + i, v);
+                        if (e) EXTREMES4(v, lo, hi);
+                    }
+                _mm_sfence();
+                extremes_of4(lo, hi, &a, &b);
 #endif
-            for (; i < HW; i++) {
-                const float v = (s[i] - m) / sd;
-                s[i] = v;
-                d[i] = v;
-            }
-        } else
-            copy_past_caches(d, s, (size_t)HW * sizeof(float));
+                for (; i < HW; i++) {
+                    const float v = (s[i] - m) / sd;
+                    s[i] = v;
+                    d[i] = v;
+                    if (v < a) a = v;
+                    if (v > b) b = v;
+                }
+                t.mn[c] = a;
+                t.mx[c] = b;
+            } else if (e)
+                scan_values(d, s, HW, &t.mn[3], &t.mx[3]);
+            else
+                copy_past_caches(d, s, (size_t)HW * sizeof(float));
+        }
+        if (e) extremes_join(e, &t);
     }
 }
 
@@ -2724,6 +2796,7 @@ typedef struct {
     int staged;    /* by way of the engine's pinned buffer */
     int host_norm; /* normalised in place on the way, with these statistics */
     const float *mean, *std;
+    extremes *range; /* of a staged float batch whose extremes are wanted: found on the way, or NULL */
 } input_batch;
 
 /* Images [i0, i0 + cnt) of an instance's slice to its input buffer, by copies on stream `st`. */
@@ -2744,7 +2817,8 @@ static int send_images(thb_engine *E, instance *I, const input_batch *in, int i0
         for (long p0 = 0; p0 < planes; p0 += per_piece) {
             const long p1 = p0 + per_piece < planes ? p0 + per_piece : planes;
             const size_t o = (size_t)p0 * HW, n = (size_t)(p1 - p0) * HW;
-            if (in->host_norm) stage_planes_normalised(stage, xs, p0, p1, in->C, HW, in->mean, in->std);
+            if (in->host_norm) stage_planes_normalised(stage, xs, p0, p1, in->C, HW, in->mean, in->std, in->range);
+            else if (in->range) scan_planes(stage, xs, p0, p1, in->C, HW, in->range);
             else parallel_copy(stage + o, xs + o, n * sizeof(float));
             CU(cudaMemcpyAsync(dst + o, stage + o, n * sizeof(float), cudaMemcpyHostToDevice, st));
         }
@@ -2818,7 +2892,8 @@ int thb_engine_forward(thb_engine *E, float *x, unsigned char **images, int stri
      * call.  (THB200_NO_STAGING=1: hand the caller's pointers to the driver as they are.) */
     int staged = 0;
     const size_t in_bytes = x ? (size_t)N * img_elems * sizeof(float) : (size_t)N * H * W * cp;
-    if (host_is_pageable(x ? (const void *)x : images[0])) {
+    const enum host_memory mem = host_memory_of(x ? (const void *)x : images[0]);
+    if (mem == MEM_PAGEABLE) {
         const char *ns = getenv("THB200_NO_STAGING");
         staged = !(ns && atoi(ns));
         if (staged && in_bytes > E->h_stage_bytes) {
@@ -2834,45 +2909,45 @@ int thb_engine_forward(thb_engine *E, float *x, unsigned char **images, int stri
     const float *host_mean = mean, *host_std = std;
     const int host_norm = staged && x && inplace;
     if (host_norm) { mean = zero3; std = one3; inplace = 0; }
-    const input_batch src = {x, images, (size_t)stride, cp, C, H, W, staged, host_norm, host_mean, host_std};
+    /* The uint8 engine needs the input range of the whole float batch before any kernel can start: it sends every slice on its
+     * way, then has the range, then launches (byte images come with a static range).  The range comes from the host's threads
+     * while they stage the batch, from a pass of theirs over a page-locked one while it is on its way, or from the GPUs' pass
+     * over what has arrived.  The other modes launch a slice's kernels as soon as its copy is queued. */
+    const int two_phase = E->dtype == THB_U8 && x;
+    const int scan = two_phase && mem == MEM_PINNED && host_scan_pays(in_bytes);
+    extremes range = NO_EXTREMES;
+    const input_batch src = {x, images, (size_t)stride, cp, C, H, W, staged, host_norm, host_mean, host_std, two_phase && staged ? &range : 0};
     /* what the device-resident timing loop needs to repeat this forward from the staged input */
     E->last_has_x = x != 0; E->last_cp = cp; E->last_bgr = bgr;
     for (int k = 0; k < 3; k++) { E->last_mean[k] = mean[k]; E->last_std[k] = std[k]; }
 
-    /* The uint8 engine needs the input range of the whole float batch before any kernel can start: it sends every slice on its
-     * way, then measures, then launches (byte images come with a static range).  The other modes launch a slice's kernels as soon
-     * as its copy is queued. */
-    const int two_phase = E->dtype == THB_U8 && x, scan = two_phase && host_scans();
     cudaEvent_t ev_call = 0;
     if (th_debug > 1 && cudaSetDevice(set[0].device) == cudaSuccess && cudaEventCreate(&ev_call) == cudaSuccess)
         cudaEventRecord(ev_call, set[0].stream);
     for (int phase = 0; phase <= two_phase; phase++) {
         if (phase == 1) {
-            if (scan) {
+            if (scan) scan_planes(0, x, 0, (long)N * C, C, (long)H * W, &range);
+            if (scan || staged) {
                 float lo, hi;
-                host_range(x, N, C, (long)H * W, mean, std, &lo, &hi);
+                extremes_range(&range, mean, std, &lo, &hi);
                 set_input_range(set, G, lo, hi, &q_sub, &q_mult);
             } else if (lowp_input_range(E, set, G, x != 0, cp, C, H, W, mean, std, &q_sub, &q_mult)) return -1;
         }
         for (int g = 0; g < G; g++) {
             instance *I = &set[g];
             CU(cudaSetDevice(I->device));
-            const int sliced = S == 1 && I->slices && two_phase == scan && !inplace && !th_profile && !th_minmax;
+            const int sliced = S == 1 && I->slices && !two_phase && !inplace && !th_profile && !th_minmax;
             for (int c = 0; sliced && c < I->slices; c++) {
                 int i0, cnt;
                 slice_part(I, c, &i0, &cnt);
-                if (phase == 0) {
-                    if (send_images(E, I, &src, i0, cnt, I->copy_stream)) return -1;
-                    CU(cudaEventRecord(I->ev_slice[c], I->copy_stream));
-                }
-                if (phase == two_phase) {
-                    CU(cudaStreamWaitEvent(I->stream, I->ev_slice[c], 0));
-                    if (c == 0 && clear_sums(I)) return -1;
-                    if (boundary_in(E, I, i0, cnt, x != 0, 0, cp, bgr, C, H, W, mean, std, q_sub, q_mult)) return -1;
-                    if (c == 0) CU(cudaEventRecord(I->ev0, I->stream));
-                    for (int t = 0; t < I->prefix; t++)
-                        if (exec_step(I, t, i0, cnt)) return -1;
-                }
+                if (send_images(E, I, &src, i0, cnt, I->copy_stream)) return -1;
+                CU(cudaEventRecord(I->ev_slice[c], I->copy_stream));
+                CU(cudaStreamWaitEvent(I->stream, I->ev_slice[c], 0));
+                if (c == 0 && clear_sums(I)) return -1;
+                if (boundary_in(E, I, i0, cnt, x != 0, 0, cp, bgr, C, H, W, mean, std, q_sub, q_mult)) return -1;
+                if (c == 0) CU(cudaEventRecord(I->ev0, I->stream));
+                for (int t = 0; t < I->prefix; t++)
+                    if (exec_step(I, t, i0, cnt)) return -1;
             }
             if (phase == 0 && !sliced && send_images(E, I, &src, 0, I->slice_n, I->stream)) return -1;
             if (phase != two_phase) continue;
