@@ -114,3 +114,38 @@ for n in (1, 5, 67):
             assert np.array_equal(x, copy, equal_nan=True)
 assert fake.empty == 0
 """, tmp_path, threads)
+
+
+def test_sub_batches_make_room(engine, tmp_path):
+    """A shape whose sub-batch plans do not fit beside the plans of earlier shapes makes those give way, as a shape's own plan does;
+    when nothing is left to give way the call fails and a smaller one still works."""
+    engine("""
+g = fx.resnet18(width=0.25, size=64, classes=10)
+x = {n: pinned((n, 3, 64, 64)) for n in (1, 8, 16)}
+def sizes():
+    net = network(g, 1)
+    lib.THB200_SetPipelineChunks(1)
+    assert call(net, x[8]) > 0
+    whole = fake.live
+    lib.THB200_SetPipelineChunks(2)
+    assert call(net, x[8]) > 0
+    both = fake.live
+    th.free_network(net)
+    assert fake.live == 0
+    return whole, both
+whole, both = sizes()
+net = network(g, 1)
+lib.THB200_SetPipelineChunks(1)
+assert call(net, x[16]) > 0
+assert call(net, x[1]) > 0
+fake.budget = fake.live + whole // 2 + (both - whole) // 2
+assert both <= fake.budget
+lib.THB200_SetPipelineChunks(2)
+for _ in range(3):
+    assert call(net, x[8]) > 0, lib.THB200_LastErrorString()
+assert fake.live >= both
+fake.budget = 1000
+assert call(net, x[16]) <= 0
+fake.budget = 1 << 50
+assert call(net, x[16]) > 0
+""", tmp_path)

@@ -2238,6 +2238,15 @@ static int plan_oldest(thb_engine *E, const shape_plan *keep)
     return v;
 }
 
+/* After a plan that did not fit on the device: one other shape's plan makes way.  0: that was not the reason, or there is none. */
+static int plans_make_way(thb_engine *E)
+{
+    const int v = E->out_of_memory ? plan_oldest(E, E->cur) : -1;
+    if (v < 0) return 0;
+    plan_drop(E, v);
+    return 1;
+}
+
 static int plan_build(thb_engine *E);
 
 /* Make the plan of this input shape the current one, building it when it is not kept. */
@@ -2263,10 +2272,7 @@ static int select_plan(thb_engine *E, int N, int C, int H, int W, int rank, int 
         p->used = E->clock;
         if (!plan_build(E)) break;
         plan_drop(E, slot);
-        /* no room on the device: the other shapes' plans make way, one at a time */
-        const int v = E->out_of_memory ? plan_oldest(E, 0) : -1;
-        if (v < 0) return -1;
-        plan_drop(E, v);
+        if (!plans_make_way(E)) return -1;
     }
     size_t total = 0;
     for (int i = 0; i < MAX_PLANS; i++)
@@ -2377,12 +2383,16 @@ static int plan_build(thb_engine *E)
 static int g_chunks_override; /* 0 = the engine's own choice */
 void thb_set_pipeline_chunks(int n) { g_chunks_override = n < 0 ? 0 : n > 4 ? 4 : n; }
 
-/* plan instances of the sub-batches (first pipelined forward of this shape with S sub-batches per GPU) */
-static int pipe_build(thb_engine *E, int S)
+static void pipe_free(shape_plan *p)
+{
+    for (int g = 0; g < 32; g++) instance_free(&p->pipe[g]);
+    p->pipe_built = 0;
+}
+
+static int pipe_instances(thb_engine *E, int S)
 {
     const int G = E->cur->built;
-    for (int g = 0; g < 32; g++) instance_free(&E->cur->pipe[g]);
-    E->cur->pipe_built = 0;
+    E->out_of_memory = 0;
     for (int g = 0; g < G; g++)
         for (int c = 0; c < S; c++) {
             int off, n;
@@ -2397,6 +2407,17 @@ static int pipe_build(thb_engine *E, int S)
         }
     E->cur->pipe_built = G * S;
     E->cur->pipe_chunks = S;
+    return 0;
+}
+
+/* plan instances of the sub-batches (first pipelined forward of this shape with S sub-batches per GPU) */
+static int pipe_build(thb_engine *E, int S)
+{
+    pipe_free(E->cur);
+    while (pipe_instances(E, S)) {
+        pipe_free(E->cur);
+        if (!plans_make_way(E)) return -1;
+    }
     return 0;
 }
 
