@@ -149,3 +149,25 @@ assert call(net, x[16]) <= 0
 fake.budget = 1 << 50
 assert call(net, x[16]) > 0
 """, tmp_path)
+
+
+def test_plan_memory_bound(engine, tmp_path):
+    """The plans an engine keeps stay within their bound in bytes, their sub-batches included, the one in use is never dropped, and
+    dropped shapes are planned again."""
+    engine("""
+LIMIT = 12 << 30
+net = network(fx.segnet(), 1)
+lib.THB200_SetPipelineChunks(2)
+x = pinned((23, 3, 512, 512))
+assert call(net, x[:1]) > 0
+weights = fake.live  # (an upper bound: with the smallest plan)
+seen = set()
+for n in (20, 21, 22, 23, 20, 1, 22):
+    before = fake.live
+    assert call(net, x[:n]) > 0, lib.THB200_LastErrorString()
+    assert fake.live <= LIMIT + weights, (n, fake.live / 2**30)
+    seen.add(fake.live < before)
+assert fake.live > LIMIT // 4 and len(seen) == 2, "some plans were kept and some dropped"
+th.free_network(net)
+assert fake.live == 0
+""", tmp_path)

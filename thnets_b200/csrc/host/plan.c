@@ -2247,6 +2247,18 @@ static int plans_make_way(thb_engine *E)
     return 1;
 }
 
+/* Plans beyond MAX_PLAN_BYTES are dropped, the least recently used first and the current one never. */
+static void plans_bound(thb_engine *E)
+{
+    size_t total = 0;
+    for (int i = 0; i < MAX_PLANS; i++)
+        if (E->plans[i]) total += plan_bytes(E->plans[i]);
+    for (int v; total > MAX_PLAN_BYTES && (v = plan_oldest(E, E->cur)) >= 0;) {
+        total -= plan_bytes(E->plans[v]);
+        plan_drop(E, v);
+    }
+}
+
 static int plan_build(thb_engine *E);
 
 /* Make the plan of this input shape the current one, building it when it is not kept. */
@@ -2274,13 +2286,7 @@ static int select_plan(thb_engine *E, int N, int C, int H, int W, int rank, int 
         plan_drop(E, slot);
         if (!plans_make_way(E)) return -1;
     }
-    size_t total = 0;
-    for (int i = 0; i < MAX_PLANS; i++)
-        if (E->plans[i]) total += plan_bytes(E->plans[i]);
-    for (int v; total > MAX_PLAN_BYTES && (v = plan_oldest(E, E->cur)) >= 0;) {
-        total -= plan_bytes(E->plans[v]);
-        plan_drop(E, v);
-    }
+    plans_bound(E);
     return 0;
 }
 
@@ -2418,6 +2424,7 @@ static int pipe_build(thb_engine *E, int S)
         pipe_free(E->cur);
         if (!plans_make_way(E)) return -1;
     }
+    plans_bound(E);
     return 0;
 }
 
