@@ -171,3 +171,21 @@ assert fake.live > LIMIT // 4 and len(seen) == 2, "some plans were kept and some
 th.free_network(net)
 assert fake.live == 0
 """, tmp_path)
+
+
+def test_a_plan_that_does_not_fit_leaves_nothing_behind(engine, tmp_path):
+    """whatever allocation a plan fails at, its streams and memory are given back"""
+    engine("""
+g = fx.resnet18(width=0.25, size=64, classes=10)
+net = network(g, 1)
+x = pinned((8, 3, 64, 64))
+assert call(net, x[:1]) > 0
+for room in (0, 8, 64, 1 << 10, 1 << 17, 1 << 18, 1 << 20):
+    th.free_network(net)
+    assert fake.streams == 0 and fake.live == 0
+    net = network(g, 1)
+    fake.budget = room
+    assert call(net, x) <= 0
+    assert fake.streams == 0, room
+    fake.budget = 1 << 50
+""", tmp_path)

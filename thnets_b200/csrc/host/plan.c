@@ -1670,7 +1670,7 @@ static size_t pack_arena(instance *I)
 
 static void instance_free(instance *I)
 {
-    if (!I->allocs && !I->steps) return;
+    if (!I->stream) return; /* (the first thing an instance has) */
     for (int i = 0; i < I->nhost; i++) free(I->hostmem[i]);
     free(I->hostmem);
     cudaSetDevice(I->device);
