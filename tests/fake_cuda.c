@@ -9,11 +9,13 @@
 size_t fake_budget = (size_t)1 << 50, fake_live; /* device bytes */
 int fake_devices = 1, fake_streams;              /* GPUs; streams alive */
 int fake_minmax, fake_boundaries, fake_empty;    /* launches: of the device's range pass, of boundary kernels in, of those on nothing */
+int fake_images;                                 /* that boundary kernels in were launched on */
 float fake_q_sub, fake_q_mult;                   /* the input quantisation of the last boundary kernel in */
 
 static void boundary(int n, float q_sub, float q_mult)
 {
     fake_boundaries++;
+    fake_images += n;
     if (n < 1) fake_empty++;
     fake_q_sub = q_sub;
     fake_q_mult = q_mult;

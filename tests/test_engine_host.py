@@ -189,3 +189,30 @@ for room in (0, 8, 64, 1 << 10, 1 << 17, 1 << 18, 1 << 20):
     assert fake.streams == 0, room
     fake.budget = 1 << 50
 """, tmp_path)
+
+
+def test_no_empty_sub_batch(engine, tmp_path):
+    """Every sub-batch of every GPU's slice has an image, whether the engine cuts the batch by its model or on request, and all of
+    the images are computed.  (The network's first launch is none that could start on a part of the batch, so that the model cuts.)"""
+    engine("""
+fake.devices = 2
+cut = 0
+for gpus in (1, 2):
+    lib.THB200_SetDevices(gpus)
+    for side in (512, 1024, 2048):
+        g = fx.Graph()
+        t = g.conv(g.relu(g.conv(g.bn(0, 3), 3, 64, 3, pad=1)), 64, 64, 3, pad=1)
+        g.linear(g.view(g.avgpool(t, side), 64), 64, 5)
+        net = network(g, 1)
+        x = pinned((17, 3, side, side))
+        for chunks in (0, 2, 3, 4):
+            lib.THB200_SetPipelineChunks(chunks)
+            for n in range(2, 18):
+                fake.boundaries = fake.images = 0
+                assert call(net, x[:n]) > 0
+                assert fake.empty == 0, (gpus, side, chunks, n)
+                assert fake.images == n
+                cut += chunks == 0 and fake.boundaries > gpus
+        th.free_network(net)
+assert cut > 40, "the model cut some of the batches"
+""", tmp_path)

@@ -2298,6 +2298,13 @@ static const unsigned char sub_batch_cuts[][5] = {
     {0, 1, 3, 7, 16}, {0, 2, 6, 11, 16}, {0, 4, 8, 12, 16}, {0, 5, 10, 14, 16},
 };
 
+/* sub-batch c of a slice of n images under a cut */
+static void cut_at(int n, const unsigned char *cut, int c, int *offset, int *count)
+{
+    *offset = (n * cut[c] + 8) / 16;
+    *count = (n * cut[c + 1] + 8) / 16 - *offset;
+}
+
 /* Sub-batches per GPU of a host-input forward: the cut with the earliest last result in a model of the three stages a
  * sub-batch goes through -- its copy to the device, its kernels (model_us, and LAUNCH_US for each launch however small the
  * sub-batch is), its result's copy back -- each one at a time.  The uint8 engine needs the range of a whole float
@@ -2320,7 +2327,12 @@ static void choose_sub_batches(thb_engine *E)
         int S = 0, ok = 1;
         do {
             const double f = (cut[S + 1] - cut[S]) / 16.0;
-            if (cut[S + 1] < 16 && I->slice_n * (cut[S + 1] - cut[S]) < 16) ok = 0; /* (every sub-batch at least an image) */
+            if (cut[S + 1] < 16 && I->slice_n * (cut[S + 1] - cut[S]) < 16) ok = 0;
+            /* every sub-batch at least an image, also where the boundaries are rounded and on the GPU with the fewest images */
+            int off, n, n_least;
+            cut_at(I->slice_n, cut, S, &off, &n);
+            cut_at(p->inst[p->built - 1].slice_n, cut, S, &off, &n_least);
+            if (n < 1 || n_least < 1) ok = 0;
             in += f * t_in;
             k = (in > k ? in : k) + f * t_k + fixed;
             out = (k > out ? k : out) + f * t_out;
@@ -2402,13 +2414,8 @@ static int pipe_instances(thb_engine *E, int S)
     for (int g = 0; g < G; g++)
         for (int c = 0; c < S; c++) {
             int off, n;
-            if (E->cur->cut && S == E->cur->chunks) {
-                const unsigned char *cut = E->cur->cut;
-                const int sn = E->cur->inst[g].slice_n;
-                off = (sn * cut[c] + 8) / 16;
-                n = (sn * cut[c + 1] + 8) / 16 - off;
-            } else
-                thb_slice_sub_batches(E->cur->inst[g].slice_n, S, c, &off, &n);
+            if (E->cur->cut && S == E->cur->chunks) cut_at(E->cur->inst[g].slice_n, E->cur->cut, c, &off, &n);
+            else thb_slice_sub_batches(E->cur->inst[g].slice_n, S, c, &off, &n);
             if (instance_build(E, &E->cur->pipe[g * S + c], E->cur->inst[g].device, E->cur->inst[g].slice_off + off, n, c)) return -1;
         }
     E->cur->pipe_built = G * S;
@@ -2888,7 +2895,7 @@ int thb_engine_forward(thb_engine *E, float *x, unsigned char **images, int stri
     int G = E->cur->built;
     const int peer_gather = E->cur->peer_gather;
     int S = g_chunks_override ? g_chunks_override : E->cur->chunks;
-    if ((E->dtype == THB_U8 && x) || S > E->cur->inst[0].slice_n || E->whole_batch) S = 1;
+    if ((E->dtype == THB_U8 && x) || S > E->cur->inst[G - 1].slice_n || E->whole_batch) S = 1;
     if (S > 1) {
         if ((!E->cur->pipe_built || E->cur->pipe_chunks != S) && pipe_build(E, S)) return -1;
         set = E->cur->pipe;
