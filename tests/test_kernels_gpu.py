@@ -729,6 +729,28 @@ def test_softmax(lib, G, oracle, dtype):
 
 
 @pytest.mark.parametrize("dtype", [K.THB_F32, K.THB_F16])
+@pytest.mark.parametrize("C", [21, 64, 65, 250, 1000, 1024, 1025])
+def test_softmax_of_few_and_many_pixels(lib, G, oracle, dtype, C):
+    """a pixel's scores are the same bits whether it is launched among few pixels or among many; every form against the oracle"""
+    rng = np.random.default_rng(C)
+    rows, ld = 2 * 8 * 148 + 3, (C + 7) // 8 * 8
+    x = np.zeros((rows, ld), np.float32)
+    x[:, :C] = rng.standard_normal((rows, C)) * 4
+    if dtype == K.THB_F16:
+        x = x.astype(np.float16).astype(np.float32)
+    ref = oracle.softmax(np.ascontiguousarray(x[:40, :C]))
+    xt = G.dev(x).to(torch.float32 if dtype == K.THB_F32 else torch.float16)
+    out = []
+    for n in (rows, rows - 3, 40):
+        y = torch.zeros_like(xt)
+        assert lib.thb_softmax(dtype, G.ptr(xt), n, C, ld, G.ptr(y), ld, None) == 0
+        out.append(y.float().cpu().numpy())
+        assert not out[-1][n:].any() and not out[-1][:, C:].any()
+    assert np.array_equal(out[0][:rows - 3], out[1][:rows - 3]) and np.array_equal(out[0][:40], out[2][:40])
+    assert G.rel_err(out[2][:40, :C], ref) < (1e-5 if dtype == K.THB_F32 else 2e-3)
+
+
+@pytest.mark.parametrize("dtype", [K.THB_F32, K.THB_F16])
 @pytest.mark.parametrize("with_bias", [False, True])
 def test_fullconv_gemm_col2im(lib, G, oracle, dtype, with_bias):
     """SpatialFullConvolution = 1x1 convolution to the column matrix, then the col2im gather;

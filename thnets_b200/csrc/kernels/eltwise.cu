@@ -844,12 +844,15 @@ __global__ void softmax_kernel(const T *x, long pixels, int C, int x_ld, T *y, i
 }
 
 // The same with a block per pixel, for few pixels of many channels (a classifier's scores), and each exponential evaluated once: a
-// warp's 32 evaluations per lane, twice, were 11 us for one pixel of 1000 channels and 18 us for 126.
+// warp's 32 evaluations per lane, twice, were 11 us for one pixel of 1000 channels and 18 us for 126.  Every warp then adds the
+// exponentials up by itself, in softmax_kernel's order: a pixel's bits must not depend on how many pixels are in the launch, which
+// differs with the sub-batches and GPUs that a batch is cut into.  (softmax_kernel in the order of a sum by blocks instead: 43 us
+// for 50000 pixels of 65 channels, where it takes 31.)
 template <typename T>
 __global__ void __launch_bounds__(256) softmax_block_kernel(const T *x, int C, int x_ld, T *y, int y_ld)
 {
     constexpr int PER = 4;  // channels a thread keeps (the launcher sends C <= 1024 here)
-    __shared__ float part[8];
+    __shared__ float part[8], ex[256 * PER];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     pdl_enter();
     const T *xp = x + (size_t)blockIdx.x * x_ld;
@@ -864,19 +867,16 @@ __global__ void __launch_bounds__(256) softmax_block_kernel(const T *x, int C, i
     __syncthreads();
 #pragma unroll
     for (int w = 0; w < 8; w++) mx = fmaxf(mx, part[w]);
-    float sum = 0.f;
 #pragma unroll
     for (int i = 0; i < PER; i++) {
         v[i] = t + i * 256 < C ? exp_minus_approx(mx - v[i]) : 0.f;
-        sum += v[i];
+        ex[t + i * 256] = v[i];
     }
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     __syncthreads();
-    if (lane == 0) part[warp] = sum;
-    __syncthreads();
-    sum = 0.f;
+    float sum = 0.f;
 #pragma unroll
-    for (int w = 0; w < 8; w++) sum += part[w];
+    for (int c = 0; c < 256 * PER; c += 32) sum += ex[c + lane];  // (zeros from C on)
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     const float inv = 1 / sum;
 #pragma unroll
     for (int i = 0; i < PER; i++)
@@ -1323,7 +1323,8 @@ int thb_copy_channels(int dtype, const void *x, long pixels, int C, int x_ld, vo
 int thb_softmax(int dtype, const void *x, long pixels, int C, int x_ld, void *y, int y_ld, thb_stream s)
 {
     if (pixels == 0) return THB_OK;
-    if (C > 64 && C <= 1024 && pixels <= 148 * 16) {  // up to two waves of blocks; beyond, a warp per pixel fills the chip
+    // up to two waves of eight blocks on each of 148 SMs; beyond, a warp per pixel fills the chip (both compute the same bits)
+    if (C > 64 && C <= 1024 && pixels <= 2 * 8 * 148) {
         DISPATCH_FLOAT_DTYPE(dtype, (thb_launch(softmax_block_kernel<T>, (unsigned)pixels, 256, s, (const T *)x, C, x_ld, (T *)y, y_ld)));
         return THB_LAUNCH_CHECK("softmax_block_kernel");
     }
