@@ -219,6 +219,7 @@ struct S2dArgs {
     int3 q_sub;         // uint8 bytes (lowp_images.c)
     float3 q_mul;
     int q_zero;         // uint8: the byte of 0.0
+    int words;          // bytes: every pixel pair starts at an even address
 };
 template <typename T, bool BYTES>
 __global__ void preprocess_s2d_any_kernel(const S2dArgs a, T *y)
@@ -328,7 +329,7 @@ __global__ void normalize_kernel(float *x, long total, long HW, float3 mean, flo
 }
 
 // Space-to-depth by two of RGB bytes (any sides): one thread per stored pixel, its twelve bytes as three 2-byte words a row where
-// the rows allow it, everything unrolled.  (preprocess_s2d_any_kernel, which steps through channels and blocks of any size, took
+// the address and the row pitch allow it, everything unrolled.  (preprocess_s2d_any_kernel, which steps through channels and blocks of any size, took
 // 123 us in uint8 for 256 pictures of 224 x 224, 89 MB.)
 template <typename T>
 __global__ void __launch_bounds__(256) preprocess_s2d_bytes_kernel(const S2dArgs a, T *y)
@@ -352,7 +353,7 @@ __global__ void __launch_bounds__(256) preprocess_s2d_bytes_kernel(const S2dArgs
             const uint8_t *row = reinterpret_cast<const uint8_t *>(a.src) + ((size_t)n * a.H + h) * a.stride + 6 * (size_t)bw;
             const bool in_h = h < a.H, two = 2 * bw + 1 < a.W;
             uint32_t b[6];
-            if (in_h && two && !(a.stride & 1)) {
+            if (in_h && two && a.words) {
 #pragma unroll
                 for (int k = 0; k < 3; k++) {
                     const uint32_t u = __ldg(reinterpret_cast<const uint16_t *>(row) + k);
@@ -1130,6 +1131,7 @@ int thb_preprocess_s2d_any(const void *src, int bytes, float *x_inplace, int N, 
     a.mean = make_float3(mean3[0], mean3[1], mean3[2]);
     a.std_ = bytes ? make_float3(1 / std3[0], 1 / std3[1], 1 / std3[2]) : make_float3(std3[0], std3[1], std3[2]);
     a.y_ld = y_ld; a.row_pitch = row_pitch; a.pad_left = pad_left;
+    a.words = bytes && !((reinterpret_cast<uintptr_t>(src) | (unsigned)stride) & 1);
     a.q_mult = a.zr = 0; a.q_sub = make_int3(0, 0, 0); a.q_mul = make_float3(0, 0, 0); a.q_zero = 0;
     if (dtype == THB_U8) {
         if (bytes) {
