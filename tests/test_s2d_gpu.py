@@ -124,3 +124,22 @@ def test_float_space_to_depth_entry_points():
         else:
             assert lib.thb_preprocess_s2d(G.ptr(x), None, n, 3, h, w, *st, dtype, G.ptr(b), ld, None) == 0
         assert torch.equal(a, b) and a.float().std() > 0
+
+
+@pytest.mark.parametrize("inplace", [False, True])
+def test_float_space_to_depth_at_any_float_address(inplace):
+    """planes that start at an odd float, whose pixel pairs are not 8-byte aligned, give what aligned ones give"""
+    lib, (n, h, w), mean, std = K.load(), (2, 6, 10), np.float32([0.45, 0.4, 0.5]), np.float32([0.225, 0.25, 0.2])
+    raw = np.random.default_rng(6).standard_normal(n * 3 * h * w).astype(np.float32)
+    st = (mean.ctypes.data_as(C.c_void_p), std.ctypes.data_as(C.c_void_p))
+    outs = []
+    for lead in (0, 1):
+        x = G.dev(np.concatenate([np.zeros(lead, np.float32), raw]))
+        at = C.c_void_p(x.data_ptr() + 4 * lead)
+        y = torch.full((n, h // 2, w // 2 + 3, 16), 7, dtype=torch.float16, device="cuda")
+        assert lib.thb_preprocess_s2d_padded(at, at if inplace else None, n, 3, h, w, *st, K.THB_F16, G.ptr(y), 16, w // 2 + 3, 2, None) == 0
+        outs.append((y.cpu(), x[lead:].cpu()))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+    assert torch.equal(outs[0][1], torch.from_numpy(raw)) != inplace
+    frame = torch.zeros(64, dtype=torch.uint8, device="cuda")
+    assert lib.thb_preprocess_yuyv(C.c_void_p(frame.data_ptr() + 2), 2, 4, *st, K.THB_F16, G.ptr(y), 16, None) != 0

@@ -1031,6 +1031,11 @@ int thb_preprocess_s2d_padded(const float *x, float *x_inplace, int N, int C, in
                               const float *std3, int dtype, void *y, int y_ld, int row_pitch, int pad_left, thb_stream s)
 {
     if (((H | W) & 1) || pad_left < 0 || row_pitch < pad_left + W / 2) return THB_ERR_ARG;
+    if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(x_inplace)) & 7) {  // the kernel moves pairs of floats
+        float q_sub = 0, q_mult = 0;
+        if (dtype == THB_U8) return THB_ERR_UNSUPPORTED;
+        return thb_preprocess_s2d_any(x, 0, x_inplace, N, C, H, W, 2, 0, 0, mean3, std3, dtype, y, y_ld, row_pitch, pad_left, &q_sub, &q_mult, s);
+    }
     const long pix = (long)N * (H / 2) * row_pitch;
     if (pix == 0) return THB_OK;
     float3 m = make_float3(mean3[0], mean3[1], mean3[2]), sd = make_float3(std3[0], std3[1], std3[2]);
@@ -1086,7 +1091,7 @@ int thb_preprocess_images(const unsigned char *img, int N, int H, int W, int str
 int thb_preprocess_yuyv(const unsigned char *frame, int H, int W, const float *mean3, const float *std3, int dtype, void *y,
                         int y_ld, thb_stream s)
 {
-    if (H < 1 || W < 2 || (W & 1) || y_ld < 3) return THB_ERR_ARG;
+    if (H < 1 || W < 2 || (W & 1) || y_ld < 3 || (reinterpret_cast<uintptr_t>(frame) & 3)) return THB_ERR_ARG;
     if (dtype == THB_U8) return THB_ERR_UNSUPPORTED;  // (the reference refuses this entry point on its lowp engine)
     const long pairs = (long)H * (W / 2);
     float3 m = make_float3(mean3[0], mean3[1], mean3[2]);
