@@ -532,3 +532,13 @@ def test_loaders_accept_the_remaining_operators(th, tmp_path):
     lines = describe(th, h)
     assert any("upsample" in l.lower() for l in lines), lines
     th.free_network(h)
+
+
+@pytest.mark.skipif(shutil.which("make") is None, reason="needs make")
+def test_a_changed_kernel_header_rebuilds_every_kernel():
+    """the layouts in kernels/*.cuh are shared by the kernels' objects: none may be left as it was when one of them changes"""
+    csrc = os.path.join(ROOT, "thnets_b200", "csrc")
+    kernels = [f for f in os.listdir(os.path.join(csrc, "kernels")) if f.endswith(".cu")]
+    for header in (f for f in os.listdir(os.path.join(csrc, "kernels")) if f.endswith(".cuh")):
+        plan = subprocess.check_output(["make", "-n", "-C", csrc, "-W", "kernels/" + header], text=True)
+        assert not [k for k in kernels if "-c kernels/%s " % k not in plan], header
