@@ -18,8 +18,9 @@
 //   warps 6-13 two epilogue groups; a thread owns one pixel row (TMEM lane): it reads 64 accumulator
 //              columns with tcgen05.ld, applies bias/BN scale-shift, residual and activation, and leaves the
 //              fp16/bf16 row in a swizzled shared-memory tile.  It never waits on global memory or on the
-//              other threads of its group.  The uint8 path (exact lowp requantisation) and BN = 32 stage
-//              through shared memory and write out with plain stores;
+//              other threads of its group.  The uint8 path (exact lowp requantisation) stores 32 channels of
+//              a row straight from registers; BN = 32, and uint8 rows outside the table-driven path
+//              (ConvTcParams::u8_classes), stage through shared memory and write out with plain stores;
 //   warp 14    epilogue agents, one thread per group: TMA load of the fused residual tile into the group's
 //              shared-memory tile, TMA store of the finished tile, recycling of the tile.
 // No im2col buffer exists anywhere.  Every wait is bounded: a wait that runs out records a code in
@@ -41,8 +42,8 @@ constexpr int nthreads(int kind) { return kind == 2 ? 512 : 480; }
 constexpr int EPI_TILE_BYTES = BM * 128;  // one 128-row x 64-column fp16 tile of the TMA epilogue
 
 // Division of 0 .. 2^31 - 1 by a launch constant: multiply-high, add, shift (the round-up method of Granlund and Montgomery,
-// "Division by invariant integers using multiplication").  The compiler's division by a run-time value is some 25 dependent
-// instructions, and every tile needs three of them before anything else can start.
+// "Division by invariant integers using multiplication").  Every tile needs three divisions before anything else can start, and a
+// division by a run-time value is a long chain of dependent instructions.
 struct FastDiv {
     uint32_t mul, shift;
     __host__ static FastDiv of(uint32_t d)
@@ -860,8 +861,10 @@ __global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid
                 else copy_tiles<KIND, BN, false>(p, &tmapA, &tmapW, &tmapR, ring, KIND == 2 && warp == 14 ? 1 : 0, KIND == 2 && p.dual ? 2 : 1, !res_w, abort_flag);
             }
         } else if (lane == 0) {
+            // what is left: gathered activations (the copy engine brings the weights only), 64-byte taps, and splits -- one tile at
+            // a time, one activation operand; resident weights with the 64-byte taps only
             const TileMap<BN, SPLIT> map(p);
-            const int halves = pair ? 2 : 1, lt_step = KIND == 2 && p.dual ? 2 : halves;
+            const int lt_step = KIND == 2 && p.dual ? 2 : 1;
             const int ring_0 = KIND == 2 && warp == 14 ? nst / 2 : 0, ring_1 = KIND == 2 && p.dual && warp == 4 ? nst / 2 : nst;
             int ring_s = ring_0;  // stage and phase in this warp's ring of stages
             uint32_t ring_ph = 0;
@@ -869,26 +872,14 @@ __global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid
             for (int lt = KIND == 2 && warp == 14 ? 1 : 0; lt < map.n_local && alive; lt += lt_step) {
                 int m0, n0;
                 map.coords(lt, m0, n0);
-                // im2col mode: input position of each half's first output pixel for tap (0, 0)
-                int iw[2] = {0, 0}, ih[2] = {0, 0}, in[2] = {0, 0}, tap_w = 0, tap_h = 0, slab = 0;
-                if (p.nkb1 && p.a2_mode == 2)
-                    for (int h = 0; h < halves; h++) {   // where the second operand is sampled for each half's first pixel
-                        const int m = m0 + h * BM;
-                        in[h] = p.by_ohw(m);
-                        const int rem = m - in[h] * p.oHW;
-                        const int oh = p.by_ow(rem);
-                        ih[h] = oh * p.a2_d;
-                        iw[h] = (rem - oh * p.oW) * p.a2_d;
-                    }
-                if (p.a_tma == 2)
-                    for (int h = 0; h < halves; h++) {
-                        const int m = m0 + h * BM;
-                        in[h] = p.by_ohw(m);
-                        const int rem = m - in[h] * p.oHW;
-                        const int oh = p.by_ow(rem);
-                        ih[h] = oh * p.dH - p.padH;
-                        iw[h] = (rem - oh * p.oW) * p.dW - p.tma_padw;
-                    }
+                // im2col mode: input position of the first output pixel for tap (0, 0)
+                int iw = 0, ih = 0, in = 0, tap_w = 0, tap_h = 0, slab = 0;
+                if (p.a_tma == 2) {
+                    in = p.by_ohw(m0);
+                    const int rem = m0 - in * p.oHW, oh = p.by_ow(rem);
+                    ih = oh * p.dH - p.padH;
+                    iw = (rem - oh * p.oW) * p.dW - p.tma_padw;
+                }
                 // split K: this unit covers the K blocks [kb0, kb1) of its tile, starting at the tap and slab of kb0
                 int kb0 = 0, kb1 = p.nkb;
                 if (SPLIT) {
@@ -911,39 +902,31 @@ __global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid
                         break;
                     }
                     // (tests of the give-up path: every earlier copy has been consumed by then, nothing is in flight)
-                    if (p.test_withhold && kb == kb1 - 1 && lt + halves >= map.n_local) break;
+                    if (p.test_withhold && kb == kb1 - 1 && lt + 1 >= map.n_local) break;
                     const uint32_t bar = smem_u32(&full[s]);
                     if (p.half) {
                         const int nh = 2 * kb + 1 < p.ntaps ? 2 : 1;
                         mbar_arrive_expect_tx(bar, (uint32_t)(nh * (A_STAGE_BYTES / 2 + (res_w ? 0 : B_STAGE_BYTES / 2))));
                         for (int h = 0; h < nh; h++) {
-                            tma_load_im2col_4d(smem_u32(sA + s * a_stage_bytes + h * (A_STAGE_BYTES / 2)), &tmapA, bar, 0, iw[0], ih[0],
-                                               in[0], (uint16_t)tap_w, (uint16_t)tap_h);
+                            tma_load_im2col_4d(smem_u32(sA + s * A_STAGE_BYTES + h * (A_STAGE_BYTES / 2)), &tmapA, bar, 0, iw, ih, in,
+                                               (uint16_t)tap_w, (uint16_t)tap_h);
                             if (!res_w) tma_load_2d(smem_u32(sB + s * B_STAGE_BYTES + h * (B_STAGE_BYTES / 2)), &tmapW, bar, (2 * kb + h) * (BKE / 2), n0);
                             if (++tap_w == p.tma_kw) { tap_w = 0; tap_h++; }
                         }
                         continue;
                     }
-                    mbar_arrive_expect_tx(bar, (uint32_t)((res_w ? 0 : B_STAGE_BYTES) + (p.a_tma ? a_stage_bytes : 0)));
-                    if (p.a_tma == 1 && p.nkb1 && kb >= p.nkb1) {
-                        for (int h = 0; h < halves; h++) {
-                            const uint32_t dst = smem_u32(sA + s * a_stage_bytes + h * A_STAGE_BYTES);
-                            if (p.a2_mode == 1) tma_load_2d(dst, &tmapR, bar, (kb - p.nkb1) * BKE, m0 + h * BM);
-                            else tma_load_im2col_4d(dst, &tmapR, bar, (kb - p.nkb1) * BKE, iw[h], ih[h], in[h], 0, 0);
-                        }
-                    } else if (p.a_tma == 1) {
-                        for (int h = 0; h < halves; h++)
-                            tma_load_2d(smem_u32(sA + s * a_stage_bytes + h * A_STAGE_BYTES), &tmapA, bar, kb * BKE, m0 + h * BM);
-                    } else if (p.a_tma == 2) {
-                        for (int h = 0; h < halves; h++)
-                            tma_load_im2col_4d(smem_u32(sA + s * a_stage_bytes + h * A_STAGE_BYTES), &tmapA, bar, slab * BKE, iw[h],
-                                               ih[h], in[h], (uint16_t)tap_w, (uint16_t)tap_h);
+                    mbar_arrive_expect_tx(bar, (uint32_t)(B_STAGE_BYTES + (p.a_tma ? A_STAGE_BYTES : 0)));
+                    if (p.a_tma == 1)
+                        tma_load_2d(smem_u32(sA + s * A_STAGE_BYTES), &tmapA, bar, kb * BKE, m0);
+                    else if (p.a_tma == 2) {
+                        tma_load_im2col_4d(smem_u32(sA + s * A_STAGE_BYTES), &tmapA, bar, slab * BKE, iw, ih, in, (uint16_t)tap_w,
+                                           (uint16_t)tap_h);
                         if (++slab == p.slabs) {
                             slab = 0;
                             if (++tap_w == p.tma_kw) { tap_w = 0; tap_h++; }
                         }
                     }
-                    if (!res_w) tma_load_2d(smem_u32(sB + s * B_STAGE_BYTES), &tmapW, bar, kb * BKE, n0);
+                    tma_load_2d(smem_u32(sB + s * B_STAGE_BYTES), &tmapW, bar, kb * BKE, n0);
                 }
             }
         }
@@ -995,7 +978,7 @@ __global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid
                             if (KIND == 2) tc_mma_i8(d0, ad + 2 * k, bd + 2 * k, IDESC, (kb | k) != 0);
                             else tc_mma_f16(d0, ad + 2 * k, bd + 2 * k, IDESC, (kb | k) != 0);
                         }
-                        if (pair) {
+                        if (pair) {  // (the second half's tile lies A_STAGE_BYTES further on)
 #pragma unroll
                             for (int k = 0; k < 4; k++) tc_mma_f16(d1, ad + (A_STAGE_BYTES >> 4) + 2 * k, bd + 2 * k, IDESC, (kb | k) != 0);
                         }
@@ -1018,7 +1001,7 @@ __global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid
                     if (p.half) {
                         const int nh = 2 * kb + 1 < p.ntaps ? 2 : 1;
                         for (int h = 0; h < nh; h++) {
-                            const uint64_t ad = make_sw64_kmajor_desc(smem_u32(sA + s * a_stage_bytes + h * (A_STAGE_BYTES / 2)));
+                            const uint64_t ad = make_sw64_kmajor_desc(smem_u32(sA + s * A_STAGE_BYTES + h * (A_STAGE_BYTES / 2)));
                             const uint64_t bd = make_sw64_kmajor_desc(smem_u32(sB + (res_w ? kb : s) * B_STAGE_BYTES + h * (B_STAGE_BYTES / 2)));
 #pragma unroll
                             for (int k = 0; k < 2; k++) {
@@ -1030,19 +1013,13 @@ __global__ void __launch_bounds__(nthreads(KIND), 1) conv_tc_kernel(const __grid
                         tc_commit(smem_u32(&empty[s]));
                         continue;
                     }
-                    const uint64_t adesc = make_sw128_kmajor_desc(smem_u32(sA + s * a_stage_bytes));
-                    const uint64_t bdesc = make_sw128_kmajor_desc(smem_u32(sB + (res_w ? kb : s) * B_STAGE_BYTES));
+                    const uint64_t adesc = make_sw128_kmajor_desc(smem_u32(sA + s * A_STAGE_BYTES));
+                    const uint64_t bdesc = make_sw128_kmajor_desc(smem_u32(sB + s * B_STAGE_BYTES));
 #pragma unroll
                     for (int k = 0; k < 4; k++) {
                         const uint32_t accum = ((kb - kb0) | k) != 0;
                         if (KIND == 2) tc_mma_i8(d0, adesc + 2 * k, bdesc + 2 * k, IDESC, accum);
                         else tc_mma_f16(d0, adesc + 2 * k, bdesc + 2 * k, IDESC, accum);
-                    }
-                    if (pair) {
-                        // the second half's tile lies A_STAGE_BYTES further on (1024 in the descriptor's 16-byte units)
-#pragma unroll
-                        for (int k = 0; k < 4; k++)
-                            tc_mma_f16(d1, adesc + (A_STAGE_BYTES >> 4) + 2 * k, bdesc + 2 * k, IDESC, (uint32_t)((kb | k) != 0));
                     }
                     tc_commit(smem_u32(&empty[s]));
                 }
