@@ -5,11 +5,12 @@
 // What bounds it is the FP32 pipe (61 TFLOP/s measured in a loop without loads) once operands reach the registers cheaply, so:
 //   * a thread owns 8 pixels x 8 channels and multiplies with fma.rn.f32x2, two channels an instruction, which leaves half
 //     of the issue slots to the loads and to the duplication of the pixel operand;
-//   * a CTA's tile is 128 x 64, 128 x 128 or 64 x 128 (pixels x channels), the K block 32; both operands arrive by 16-byte cp.async (channel
-//     chunks of pixels through the gather table, zeros outside the image) in a ring of three stages, pixel rows of 128 bytes
-//     swizzled by XOR so that neither the copies nor the 16-byte reads of four k at a time meet in a bank;
-//   * launches of few tiles: the K blocks of a tile are shared by the S CTAs of a thread-block cluster.  Each leaves
-//     its partial tile in its shared memory, and every CTA adds the S parts of its share of the rows, in rank order, through distributed shared memory (no atomics, the result does not depend on timing).
+//   * a CTA's tile is 128 x 64, 128 x 128 or 64 x 128 (pixels x channels), the K block 32; both operands arrive by 16-byte
+//     cp.async (channel chunks of pixels through the gather table, zeros outside the image) in a ring of three stages, pixel
+//     rows of 128 bytes swizzled by XOR so that neither the copies nor the 16-byte reads of four k at a time meet in a bank;
+//   * launches of few tiles: the K blocks of a tile are shared by the S CTAs of a thread-block cluster.  Each leaves its
+//     partial tile in its shared memory, and every CTA adds the S parts of its share of the rows, in rank order, through
+//     distributed shared memory (no atomics, the result does not depend on timing).
 // Measured: the table at thb_conv_simt_splits.
 #include "common.cuh"
 #include "conv_maps.cuh"
@@ -305,15 +306,18 @@ extern "C" void thb_simt_reload_knobs(void) { g_no_split = -1; }
 // 62.9 / 61.4.
 static bool low_tiles(const thb_conv_desc *d) { return d->Cout_pad % 128 == 0; }
 
-// Tiles of 64 channels, the reduction split while that leaves at most three CTAs to an SM (what its registers hold); measured,
-// us before / unsplit / split in 2 / 4 / 8 (16 in clusters beyond the portable size):
-//   64->64 3x3 @57x57, 9 images, 229 tiles of 18 K blocks      72 / 65 / 66
-//   128->128 3x3 @29x29, 9 images, 120 of 36                   82 / 70 / 65 / 64
-//   256->256 3x3 @15x15, 9 images, 64 of 72                   144 / 133 / 71 / 63 / 77
-//   512->512 3x3 @8x8, 9 images, 40 of 144                    160 / - / 137 / 120 / 89
-//   64->192 5x5 @27x27, 1 image, 18 of 50                      31 / - / 51 / 28 / 27
-//   384->256 3x3 @13x13, 1 image, 8 of 108                     34 / - / 102 / 53 / 29
-// Large layers: tiles of 128 channels (128->128 3x3 @28x28, 64 images: 401 / 332 with 64, 320 with 128).
+// The reduction split while that leaves at most three CTAs to an SM (what its registers hold), in 16 parts where that leaves two at
+// most.  Tiles are those of a split launch (low_tiles): 64 x 128 for 128, 256 and 512 output channels, 128 x 64 for 64 and 192.
+// Measured, us in 1 / 2 / 4 / 8 / 16 parts (16 in clusters beyond the portable size); * the rule's choice:
+//   64->64 3x3 @57x57, 9 images, 229 tiles of 18 K blocks      61* / 65 / 66 / 80 / 132
+//   128->128 3x3 @29x29, 9 images, 119 of 36                   65 / 62* / 60 / 68 / 89
+//   256->256 3x3 @15x15, 9 images, 64 of 72                   126 / 67 / 60* / 73 / 83
+//   512->512 3x3 @8x8, 9 images, 36 of 144                    252 / 128 / 115 / 88* / 87
+//   64->192 5x5 @27x27, 1 image, 18 of 50                      89 / 49 / 28 / 27 / 27*
+//   256->256 3x3 @14x14, 2 images, 14 of 72                   124 / 67 / 35 / 20 / 21*
+//   384->256 3x3 @13x13, 1 image, 6 of 108                    188 / 97 / 50 / 28 / 17*
+//   512->512 3x3 @7x7, 1 image, 4 of 144                      250 / 127 / 65 / 35 / 20*
+// Unsplit large layers: tiles of 128 channels (128->128 3x3 @28x28, 64 images: 332 with 64, 320 with 128).
 extern "C" int thb_conv_simt_splits(const thb_conv_desc *d)
 {
     if (g_no_split < 0) {
