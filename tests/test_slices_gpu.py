@@ -56,6 +56,40 @@ def test_sliced_start(th, tmp_path, mode, images, net, batch, size):
     assert np.array_equal(run(th, path, mode, x, images, True), run(th, path, mode, x, images, False))
 
 
+@pytest.mark.parametrize("mode", [0, 1], ids=["fp32", "fp16"])
+def test_sliced_start_in_place(th, tmp_path, monkeypatch, mode):
+    """A page-locked float batch that is normalised in place: sliced or whole, the same scores, and in the caller's buffer exactly
+    the normalised values."""
+    import ctypes
+    batch, size, mean, std = 67, 225, np.float32([0.45, 0.4, 0.5]), np.float32([0.225, 0.25, 0.2])
+    path = str(tmp_path / "n.net")
+    fx.write_pymodel(fx.resnet18(width=0.25, size=size, classes=10, fc_bias=0.05), path)
+    x = np.random.default_rng(3).standard_normal((batch, 3, size, size), dtype=np.float32)
+    p = th.lib.THB200_HostAlloc(x.nbytes)
+    pinned = np.ctypeslib.as_array(ctypes.cast(p, ctypes.POINTER(ctypes.c_float)), shape=x.shape)
+    th.lib.THB200_SetPipelineChunks(1)
+    outs = []
+    try:
+        for off in ("0", "1"):
+            monkeypatch.setenv("THB200_NO_SLICES", off)
+            h = th.load_network(path)
+            th.set_stats(h, mean, std)
+            th.lib.THB200_SetPrecision(mode)
+            net = th.lib.THCreateCudaNetwork(h)
+            th.lib.THB200_SetPrecision(0)
+            th.free_network(h)
+            for _ in range(3):
+                pinned[...] = x
+                outs.append(th.process_float(net, pinned, copy_input=False)[0])
+                assert np.array_equal(pinned, (x - mean[:, None, None]) / std[:, None, None])
+            th.free_network(net)
+    finally:
+        th.lib.THB200_SetPipelineChunks(0)
+        th.lib.THB200_HostFree(p)
+    for o in outs[1:]:
+        assert np.array_equal(o, outs[0])
+
+
 @pytest.mark.parametrize("net,batch,size", [("resnet18", 5, 97), ("resnet18", 66, 224), ("vgg16", 40, 224)])
 @pytest.mark.parametrize("nan", [False, True], ids=["finite", "nan"])
 def test_uint8_range_found_by_the_host(th, tmp_path, net, batch, size, nan):

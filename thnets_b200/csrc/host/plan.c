@@ -2553,6 +2553,21 @@ static int boundary_out(thb_engine *E, instance *I, float *dst, int head)
     return 0;
 }
 
+/* The normalised values [off, off + n) of the instance's slice go back to the caller's slice on a stream of their own: the link is
+ * full duplex and the forward does not wait for them (the caller does, before THProcessFloat returns). */
+static int write_back(instance *I, float *slice, size_t off, size_t n)
+{
+    if (!I->wb_stream) {
+        CU(cudaStreamCreateWithFlags(&I->wb_stream, cudaStreamNonBlocking));
+        CU(cudaEventCreateWithFlags(&I->ev_wb, cudaEventDisableTiming));
+    }
+    CU(cudaEventRecord(I->ev_wb, I->stream));
+    CU(cudaStreamWaitEvent(I->wb_stream, I->ev_wb, 0));
+    CU(cudaMemcpyAsync(slice + off, I->d_in + off, n * sizeof(float), cudaMemcpyDeviceToHost, I->wb_stream));
+    I->wb_pending = 1;
+    return 0;
+}
+
 /* Everything one GPU does between its staged input and its NCHW fp32 result, on the instance's stream: the boundary
  * kernel in, the planned launches, the boundary kernel out.  ev0 marks the start of the planned launches.
  * `writeback`: host address the normalised input slice is copied back to (THProcessFloat's in-place side effect), or
@@ -2561,18 +2576,7 @@ static int device_forward(thb_engine *E, instance *I, int has_x, int inplace, in
                           const float *mean, const float *std, float q_sub, float q_mult, float *writeback, float *dst)
 {
     if (clear_sums(I) || boundary_in(E, I, 0, I->slice_n, has_x, inplace, cp, bgr, C, H, W, mean, std, q_sub, q_mult)) return -1;
-    if (writeback) {
-        /* the normalised values go back to the caller on a stream of their own: the link is full duplex and the forward does
-         * not wait for them (the caller does, before THProcessFloat returns) */
-        if (!I->wb_stream) {
-            CU(cudaStreamCreateWithFlags(&I->wb_stream, cudaStreamNonBlocking));
-            CU(cudaEventCreateWithFlags(&I->ev_wb, cudaEventDisableTiming));
-        }
-        CU(cudaEventRecord(I->ev_wb, I->stream));
-        CU(cudaStreamWaitEvent(I->wb_stream, I->ev_wb, 0));
-        CU(cudaMemcpyAsync(writeback, I->d_in, (size_t)I->slice_n * C * H * W * sizeof(float), cudaMemcpyDeviceToHost, I->wb_stream));
-        I->wb_pending = 1;
-    }
+    if (writeback && write_back(I, writeback, 0, (size_t)I->slice_n * C * H * W)) return -1;
     CU(cudaEventRecord(I->ev0, I->stream));
     if (run_steps(E, I, 0)) return -1;
     return boundary_out(E, I, dst, head_on(I));
@@ -2971,7 +2975,9 @@ int thb_engine_forward(thb_engine *E, float *x, unsigned char **images, int stri
         for (int g = 0; g < G; g++) {
             instance *I = &set[g];
             CU(cudaSetDevice(I->device));
-            const int sliced = S == 1 && I->slices && !two_phase && !inplace && !th_profile && !th_minmax;
+            float *back = x && inplace ? x + (size_t)I->slice_off * img_elems : 0;
+            /* (values on their way back to memory that is not page-locked would hold the calling thread up between the parts) */
+            const int sliced = S == 1 && I->slices && !two_phase && (!back || mem == MEM_PINNED) && !th_profile && !th_minmax;
             for (int c = 0; sliced && c < I->slices; c++) {
                 int i0, cnt;
                 slice_part(I, c, &i0, &cnt);
@@ -2979,7 +2985,8 @@ int thb_engine_forward(thb_engine *E, float *x, unsigned char **images, int stri
                 CU(cudaEventRecord(I->ev_slice[c], I->copy_stream));
                 CU(cudaStreamWaitEvent(I->stream, I->ev_slice[c], 0));
                 if (c == 0 && clear_sums(I)) return -1;
-                if (boundary_in(E, I, i0, cnt, x != 0, 0, cp, bgr, C, H, W, mean, std, q_sub, q_mult)) return -1;
+                if (boundary_in(E, I, i0, cnt, x != 0, inplace, cp, bgr, C, H, W, mean, std, q_sub, q_mult)) return -1;
+                if (back && write_back(I, back, i0 * img_elems, cnt * img_elems)) return -1;
                 if (c == 0) CU(cudaEventRecord(I->ev0, I->stream));
                 for (int t = 0; t < I->prefix; t++)
                     if (exec_step(I, t, i0, cnt)) return -1;
@@ -2991,8 +2998,7 @@ int thb_engine_forward(thb_engine *E, float *x, unsigned char **images, int stri
             float *dst = gather && I->device == dev0 ? gather + off : direct ? E->h_out + off : I->d_out;
             if (sliced) {
                 if (run_steps(E, I, I->prefix) || boundary_out(E, I, dst, head_on(I))) return -1;
-            } else if (device_forward(E, I, x != 0, inplace, cp, bgr, C, H, W, mean, std, q_sub, q_mult,
-                                      x && inplace ? x + (size_t)I->slice_off * img_elems : 0, dst)) return -1;
+            } else if (device_forward(E, I, x != 0, inplace, cp, bgr, C, H, W, mean, std, q_sub, q_mult, back, dst)) return -1;
             CU(cudaEventRecord(I->ev1, I->stream));
             if (gather) {
                 if (I->device != dev0)
