@@ -221,7 +221,7 @@ assert cut > 40, "the model cut some of the batches"
 def test_sliced_start_of_a_batch_normalised_in_place(engine, tmp_path):
     """a large page-locked batch starts part by part whether or not its normalised values go back to the caller"""
     engine("""
-net = network(fx.resnet18(width=0.25, size=224, classes=10), 1)
+net = network(fx.resnet18(size=224, classes=10), 1)
 th.set_stats(net, (0.45,) * 3, (0.225,) * 3)
 x = pinned((67, 3, 224, 224))
 lib.THB200_SetPipelineChunks(1)
