@@ -60,9 +60,8 @@ LOWP_RANGE = 20.0
 
 
 # dram__bytes_read.sum + dram__bytes_write.sum of the convolution launches of ONE forward, from the ncu capture whose
-# summary is profiles/conv_resnet50_fp16_b128_dram_tensor.md (captured at batch 128: 4.423 GB, of which 0.051 GB are
-# weights; activations scaled to batch 256, weights counted once); None for workloads without a capture
-NCU_DRAM_BYTES_PER_STEP = {("resnet50", "fp16", 256): 8.80e9}
+# summary is profiles/conv_resnet50_fp16_b256_dram.md; None for workloads without a capture
+NCU_DRAM_BYTES_PER_STEP = {("resnet50", "fp16", 256): 9.92e9}
 
 
 def read_peaks():

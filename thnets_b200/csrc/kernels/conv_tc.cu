@@ -2,7 +2,8 @@
 //
 // GEMM view: D[pixel][cout] = sum_k A[pixel][k] * Wt[cout][k], k = tap*Cin_pad + c.
 // One PERSISTENT CTA per SM walks output tiles of 128 consecutive pixels (flat over n, oh, ow: tiles
-// may span rows and images, so small feature maps waste nothing) x BN output channels.  Fifteen warps:
+// may span rows and images, so small feature maps waste nothing) x BN output channels.  Fifteen
+// warps, in uint8 sixteen (ConvTcParams::dual):
 //   warp  4    TMA producer: packed weights (K-major, SWIZZLE_128B, no multicast) and -- whenever a K block is
 //              one whole 128-byte channel slab of one tap -- the activation operand too: a plain 2-D load for
 //              1x1 stride-1 convolutions, an im2col-mode load (the copy engine walks the 128 output pixels,
