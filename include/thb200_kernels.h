@@ -145,6 +145,16 @@ int thb_conv_few_splits(const thb_conv_desc *d);
  * parts of a batch gives every part the whole batch's, so that all of them add in the same order. */
 int thb_conv_simt_splits(const thb_conv_desc *d);
 int thb_conv_few_supported(const thb_conv_desc *d);
+/* F32 on the tensor cores: the convolution of thb_conv_fwd from a second copy of the weights, each value as three bf16 parts
+ * (w_split: split_bytes of device memory, filled from d->w by split_weights on the stream).  d->w and d->kinfo stay in use (sums
+ * that are not finite are computed from them), d->status has to be set, and d->splits is the number of CTAs that share a tile's
+ * reduction (1, 2, 4 or 8; 0: thb_conv_f32_splits).  supported: up to 16 padded input channels, or a
+ * multiple of 32 of them, and at least 64 products to a sum. */
+int thb_conv_f32_supported(const thb_conv_desc *d);
+size_t thb_conv_f32_split_bytes(const thb_conv_desc *d);
+int thb_conv_f32_split_weights(const thb_conv_desc *d, void *w_split, thb_stream s);
+int thb_conv_f32_splits(const thb_conv_desc *d);
+int thb_conv_f32_fwd(const thb_conv_desc *d, const void *w_split, const void *x, void *y, thb_stream s);
 /* A network's last convolution (F16 / BF16) with its result as NCHW fp32, rounded through the 16-bit type, in device or pinned
  * host memory: the convolution and thb_postprocess_status in one launch.  *status_out: 0 before the call; set when this launch or
  * one before it (d->status) gave up a wait. */

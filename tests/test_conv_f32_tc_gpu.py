@@ -1,0 +1,146 @@
+"""The fp32 convolution on the tensor cores: edges of its tiles (128 pixels, 64 and 128 channels, K blocks of 32), every split of
+the reduction, every way its activations are loaded, against a double-precision convolution and against the FFMA kernel."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+import torch  # noqa: E402
+
+from thnets_b200 import kernels_abi as K  # noqa: E402
+from tests import gpu_util as G  # noqa: E402
+
+
+@pytest.fixture(scope="module")
+def lib():
+    return K.load()
+
+
+class Split:
+    """A convolution with its weights' parts."""
+
+    def __init__(self, lib, x, wt, stride, pad):
+        self.lib, self.x = lib, x
+        self.conv = G.Conv(lib, K.THB_F32, x.shape, wt, (stride, stride), (pad, pad))
+        d = C.byref(self.conv.d)
+        assert lib.thb_conv_f32_supported(d)
+        self.parts = G.dzeros(lib.thb_conv_f32_split_bytes(d))
+        assert lib.thb_conv_f32_split_weights(d, self.parts.data_ptr(), None) == 0
+        self.xt, self.conv.d.in_ld = G.to_nhwc(x, K.THB_F32)
+
+    def run(self, splits, pad=0):
+        d = self.conv.d
+        d.splits, d.out_ld = splits, G.ru(d.Cout, 4) + pad
+        y = torch.full((d.N, d.oH, d.oW, d.out_ld), 3.0, device="cuda")
+        rc = self.lib.thb_conv_f32_fwd(C.byref(d), self.parts.data_ptr(), self.xt.data_ptr(), y.data_ptr(), None)
+        torch.cuda.synchronize()
+        assert rc == 0, (rc, self.lib.thb_last_cuda_error())
+        assert int(self.conv.keep[3].cpu()[0]) == 0, "a bounded wait gave up"
+        assert pad == 0 or bool((y[..., -pad:] == 3.0).all()), "wrote beyond its channels"
+        return G.from_nhwc(y, d.Cout)
+
+    def ffma(self):
+        d = self.conv.d
+        d.splits, d.out_ld = 0, G.ru(d.Cout, 4)
+        return G.from_nhwc(self.conv.run(self.xt), d.Cout)
+
+
+def double(x, wt, s, p):
+    return torch.nn.functional.conv2d(torch.from_numpy(x).double().cuda(), torch.from_numpy(wt).double().cuda(), stride=s, padding=p).cpu().numpy()
+
+
+CASES = [  # n, cin, h, w, cout, k, stride, pad
+    (1, 3, 43, 31, 64, 7, 2, 3),        # gathered, 22 x 16 pixels, K = 196: the last K block a sixth full
+    (2, 3, 67, 67, 128, 11, 4, 2),      # gathered, wide tiles
+    (1, 16, 9, 9, 64, 3, 1, 1),         # gathered, 16 channels
+    (1, 64, 127, 1, 64, 1, 1, 0),       # 127 pixels, a plain matrix of two K blocks: narrow tiles
+    (1, 64, 16, 8, 130, 1, 1, 0),       # 128 pixels, channels beyond a tile
+    (1, 128, 43, 3, 256, 1, 1, 0),      # 129 pixels, four K blocks: wide tiles
+    (3, 64, 9, 5, 200, 3, 2, 1),        # im2col, stride 2, 256 padded channels of 200
+    (1, 32, 7, 7, 21, 3, 1, 1),         # im2col, one slab, few channels
+    (9, 512, 1, 1, 1000, 1, 1, 0),      # rows of a Linear
+    (20, 64, 40, 41, 128, 3, 1, 1),     # more tiles than SMs
+    (1, 256, 5, 13, 64, 5, 1, 2),       # 200 K blocks: every ring wraps many times
+]
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_tiles_and_splits(lib, case):
+    n, cin, h, w, cout, k, s, p = case
+    rng = np.random.default_rng(cin + k)
+    x = rng.standard_normal((n, cin, h, w)).astype(np.float32)
+    wt = (rng.standard_normal((cout, cin, k, k)) * (cin * k * k) ** -0.5).astype(np.float32)
+    ref = double(x, wt, s, p)
+    c = Split(lib, x, wt, s, p)
+    err = lambda y: np.linalg.norm(y - ref) / np.linalg.norm(ref)  # noqa: E731
+    before = err(c.ffma())
+    for splits in (0, 1, 2, 4, 8):
+        y = c.run(splits, pad=4)
+        # half an ulp of a result (3e-8 of it on average), and what a truncated sum of 32 loses on the way (4e-8)
+        assert err(y) <= max(before, 1.2e-7), splits
+        assert G.rel_err(y, ref) < 1e-6, splits
+        assert np.array_equal(y, c.run(splits)), splits
+    # residual, scale, shift and the activations
+    scale, shift = rng.uniform(0.5, 1.5, cout).astype(np.float32), rng.standard_normal(cout).astype(np.float32)
+    res = rng.standard_normal(ref.shape).astype(np.float32)
+    c.conv.set_affine(scale, shift)
+    rt, rld = G.to_nhwc(res, K.THB_F32)
+    c.conv.set_residual(rt, rld, 1.0, -1.0)
+    want = ref * scale[None, :, None, None] + shift[None, :, None, None] - res
+    slope = rng.uniform(0.1, 0.5, cout).astype(np.float32)
+    for kind, kw, f in ((K.ACT_THRESHOLD, dict(threshold=0.1, value=-1.0), lambda v: np.where(v > 0.1, v, -1.0)),
+                        (K.ACT_PRELU, dict(slope=slope), lambda v: np.where(v > 0, v, v * slope[None, :, None, None]))):
+        c.conv.set_act(kind, **kw)
+        for splits in (1, 4):
+            y, keep = c.run(splits), np.abs(want - 0.1) > 1e-5  # (a value at the threshold may fall on either side)
+            assert G.rel_err(np.where(keep, y, 0), np.where(keep, f(want), 0)) < 1e-6, (kind, splits)
+
+
+def test_values_the_parts_cannot_hold(lib):
+    """Infinities, NaN and values near the end of fp32's range come out as the FFMA kernel has them; small values keep their bits."""
+    rng = np.random.default_rng(5)
+    x = rng.standard_normal((1, 64, 12, 12)).astype(np.float32)
+    wt = (rng.standard_normal((64, 64, 3, 3)) * 0.1).astype(np.float32)
+    wt[:, 1] = 0.5      # parts beyond the first are zero: infinity times them would be NaN
+    wt[:, 2] = 0.0      # 0 x infinity is NaN in the reference's order of operations as well
+    x[0, 1, 2, 2], x[0, 1, 8, 8], x[0, 3, 2, 9], x[0, 2, 9, 2] = np.inf, -np.inf, np.nan, np.inf
+    x[0, 4, 5, 5] = 3.4e38  # rounds to an infinite bf16
+    wt[:, 4] = 0.25
+    c = Split(lib, x, wt, 1, 1)
+    a = c.ffma()
+    assert np.isinf(a).any() and np.isnan(a).any() and np.isfinite(a).any() and (np.abs(a[np.isfinite(a)]) > 1e37).any()
+    for splits in (1, 2, 8):
+        b = c.run(splits)
+        assert np.array_equal(np.isnan(a), np.isnan(b)) and np.array_equal(np.isinf(a), np.isinf(b)), splits
+        same = np.isinf(a)
+        assert np.array_equal(a[same], b[same])
+        fin = np.isfinite(a)
+        assert np.abs(a[fin] / b[fin] - 1).max() < 1e-3 and G.rel_err(b[fin], a[fin]) < 1e-6
+    tiny = Split(lib, (x := rng.standard_normal((1, 64, 12, 12)).astype(np.float32) * 1e-30), wt, 1, 1)
+    assert G.rel_err(tiny.run(1), double(x, wt, 1, 1)) < 1e-6
+
+
+def test_bounded_wait(lib, monkeypatch):
+    """A copy that is never made: the launch ends, reports, and the next one is right."""
+    rng = np.random.default_rng(6)
+    x = rng.standard_normal((1, 64, 10, 10)).astype(np.float32)
+    wt = rng.standard_normal((64, 64, 3, 3)).astype(np.float32)
+    c = Split(lib, x, wt, 1, 1)
+    good = c.run(2)
+    monkeypatch.setenv("THB200_TEST_WITHHOLD", "1")
+    monkeypatch.setenv("THB200_WAIT_LIMIT_CYCLES", "20000000")
+    lib.thb_conv_reload_knobs()
+    try:
+        y = torch.zeros((1, 10, 10, 64), device="cuda")
+        for splits in (1, 2):
+            c.conv.d.splits = splits
+            assert lib.thb_conv_f32_fwd(C.byref(c.conv.d), c.parts.data_ptr(), c.xt.data_ptr(), y.data_ptr(), None) == 0
+            torch.cuda.synchronize()
+            assert int(c.conv.keep[3].cpu()[0]) != 0
+            c.conv.keep[3].zero_()
+    finally:
+        monkeypatch.undo()
+        lib.thb_conv_reload_knobs()
+    assert np.array_equal(c.run(2), good)

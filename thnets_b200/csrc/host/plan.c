@@ -99,6 +99,7 @@ typedef struct {
     thb_conv_desc conv;
     thb_tmap *tmap;
     const void *w; /* gemv weights */
+    const void *w_split; /* conv fp32: the weights' parts for the tensor-core kernel (NULL: the kernel on the FP32 units) */
     int K, M;
     int dyn_quant; /* conv u8 whose input scale is only known per forward (first layer) */
     /* u8 conv constants needed to derive the per-forward parameters */
@@ -250,7 +251,7 @@ static void host_keep(instance *I, void *p)
 }
 
 /* ---- weights and constants, owned by the engine ---- */
-enum blob_tag { BL_SCALE = 1, BL_SHIFT, BL_SLOPE, BL_BIAS, BL_FACTOR, BL_ADDEND, BL_GEMV, BL_CONV, BL_KINFO, BL_WSAT };
+enum blob_tag { BL_SCALE = 1, BL_SHIFT, BL_SLOPE, BL_BIAS, BL_FACTOR, BL_ADDEND, BL_GEMV, BL_CONV, BL_KINFO, BL_WSAT, BL_SPLIT };
 enum { BLOB_KEY = sizeof(((wblob *)0)->key) / sizeof(int) };
 
 static wblob *blob_find(thb_engine *E, int device, const int *key)
@@ -259,12 +260,12 @@ static wblob *blob_find(thb_engine *E, int device, const int *key)
         if (E->blobs[i].device == device && !memcmp(E->blobs[i].key, key, sizeof(E->blobs[i].key))) return &E->blobs[i];
     return 0;
 }
-/* upload `bytes` and keep them under `key` (on the instance's device, which is current) */
+/* upload `bytes` (host NULL: only room for them) and keep them under `key` (on the instance's device, which is current) */
 static wblob *blob_add(thb_engine *E, int device, const int *key, const void *host, size_t bytes)
 {
     void *p = 0;
     const cudaError_t e = cudaMalloc(&p, bytes ? bytes : 16);
-    if (e != cudaSuccess || cudaMemcpy(p, host, bytes, cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (e != cudaSuccess || (host && cudaMemcpy(p, host, bytes, cudaMemcpyHostToDevice) != cudaSuccess)) {
         E->out_of_memory = e == cudaErrorMemoryAllocation;
         cudaGetLastError();
         if (p) cudaFree(p);
@@ -584,6 +585,31 @@ static float *weights_oihw(const thb_model *M, const thb_conv_desc *d, const wso
     return w;
 }
 
+/* The second copy of an fp32 convolution's weights, which sends it to the tensor cores; none, and so the kernel on the FP32 units,
+ * where that one does not take the layer, where the device has no room for the copy and with THB200_NO_F32_TC=1. */
+static const void *conv_split_weights(planner *P, const thb_conv_desc *d, const int *conv_key)
+{
+    thb_engine *E = P->E;
+    const char *off = getenv("THB200_NO_F32_TC");
+    if ((off && atoi(off)) || !thb_conv_f32_supported(d)) return 0;
+    int key[BLOB_KEY];
+    memcpy(key, conv_key, sizeof(key));
+    key[1] = BL_SPLIT;
+    wblob *w = blob_find(E, P->I->device, key);
+    if (w) return w->ptr;
+    w = blob_add(E, P->I->device, key, 0, thb_conv_f32_split_bytes(d));
+    if (!w) {
+        E->out_of_memory = 0;
+        return 0;
+    }
+    if (thb_conv_f32_split_weights(d, w->ptr, 0) || cudaStreamSynchronize(0) != cudaSuccess) {
+        cudaFree(w->ptr);
+        E->nblobs--;
+        return 0;
+    }
+    return w->ptr;
+}
+
 /* Packed weights and gather table of a planned convolution: the engine's, when a plan with the same layout made them
  * before (another batch or image size nearly always has it), else packed here and uploaded. */
 static int conv_weights(planner *P, step *s, thb_conv_desc *d, const wsource *ws)
@@ -634,6 +660,10 @@ static int conv_weights(planner *P, step *s, thb_conv_desc *d, const wsource *ws
     d->kinfo = blob_find(E, dev, key)->ptr;
     key[1] = BL_WSAT;
     d->wsat = u8 ? blob_find(E, dev, key)->ptr : 0;
+    if (d->dtype == THB_F32) {
+        s->w_split = conv_split_weights(P, d, key);
+        d->splits = s->w_split ? thb_conv_f32_splits(d) : thb_conv_simt_splits(d); /* (also on parts of the batch: a sliced start changes no sum) */
+    }
     return 0;
 }
 
@@ -991,7 +1021,6 @@ static int plan_gemm_group(planner *P, int i)
         d->splits = thb_conv_few_splits(&whole);
         if (d->splits < 2) d->splits = 0;
     }
-    if (dtype == THB_F32) d->splits = thb_conv_simt_splits(d); /* (also on parts of the batch: a sliced start changes no sum) */
     /* (integer sums: any split gives the same bytes) */
     if (dtype == THB_U8 && is.N == P->I->slice_n) {
         d->out_ld = ru(d->Cout, al);
@@ -1887,7 +1916,8 @@ static int exec_step(instance *I, int t, int img0, int cnt)
         if (s->aux2_buf >= 0) d->csum_out = (int *)((char *)bufptr(I, s->aux2_buf, 0, THB_U8) + aux2_off);
         if (s->scratch_buf >= 0) d->splitk_scratch = (float *)bufptr(I, s->scratch_buf, 0, THB_U8);
         rc = s->pool_k ? thb_conv_maxpool_fwd(d, s->pool_k, 2, s->pool_pad, s->pool_oH, s->pool_oW, x0, y, s->out_ld, st)
-                       : thb_conv_fwd(d, x0, y, st);
+             : s->w_split ? thb_conv_f32_fwd(d, s->w_split, x0, y, st)
+                          : thb_conv_fwd(d, x0, y, st);
         break;
     }
     case ST_GEMV:

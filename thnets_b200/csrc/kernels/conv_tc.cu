@@ -1701,6 +1701,13 @@ encode_im2col_fn get_encode_im2col_fn()
     return fn;
 }
 
+size_t tmap_esize(int dtype) { return dtype == THB_F32 ? 4 : dtype == THB_U8 ? 1 : 2; }
+CUtensorMapDataType tmap_type(int dtype)
+{
+    return dtype == THB_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : dtype == THB_U8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8
+           : dtype == THB_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+}
+
 // TMA descriptors of plain row-major matrices [rows][cols] with a row pitch (activation operand of a 1x1
 // convolution, output and residual tensors), keyed by what they encode and built once per buffer and shape.
 struct MTmapEntry {
@@ -1721,9 +1728,8 @@ const CUtensorMap *matrix_tmap(const void *x, long rows, int cols, int ld, int d
     if (!enc) return nullptr;
     MTmapEntry &e = cache[used < 1024 ? used++ : (next++ % 1024)];
     e.x = nullptr;
-    const int es = dtype == THB_U8 ? 1 : 2;
-    CUtensorMapDataType t = dtype == THB_U8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8
-                            : dtype == THB_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+    const size_t es = tmap_esize(dtype);
+    const CUtensorMapDataType t = tmap_type(dtype);
     cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
     cuuint64_t strides[1] = {(cuuint64_t)ld * es};
     cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)BM};
@@ -1745,7 +1751,7 @@ struct ATmapEntry {
 const CUtensorMap *activation_tmap(const thb_conv_desc *d, const void *x, int mode)
 {
     if (mode == 1)
-        return matrix_tmap(x, (long)d->N * d->H * d->W, d->Cin_pad, d->in_ld, d->dtype, d->dtype == THB_U8 ? 128 : 64);
+        return matrix_tmap(x, (long)d->N * d->H * d->W, d->Cin_pad, d->in_ld, d->dtype, (int)(128 / tmap_esize(d->dtype)));
     static ATmapEntry cache[512];
     static int used = 0, next = 0;
     const int geom[8] = {d->kH, d->kW, d->dH, d->dW, d->padH, mode == 3 || mode == 5 ? d->in_row_pitch : d->padW, d->oH, d->oW};
@@ -1757,9 +1763,8 @@ const CUtensorMap *activation_tmap(const thb_conv_desc *d, const void *x, int mo
     }
     ATmapEntry &e = cache[used < 512 ? used++ : (next++ % 512)];
     e.x = nullptr;
-    const int es = d->dtype == THB_U8 ? 1 : 2;
-    CUtensorMapDataType t = d->dtype == THB_U8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8
-                            : d->dtype == THB_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+    const size_t es = tmap_esize(d->dtype);
+    const CUtensorMapDataType t = tmap_type(d->dtype);
     {
         encode_im2col_fn enc = get_encode_im2col_fn();
         if (!enc) return nullptr;

@@ -76,6 +76,11 @@ def load(libpath: str | None = None):
     lib.thb_conv_pack_weights_host.argtypes = [C.POINTER(ConvDesc), vp, vp, vp, vp, vp]
     lib.thb_conv_make_tmap.argtypes = [C.POINTER(ConvDesc), C.POINTER(TMap)]
     lib.thb_conv_fwd.argtypes = [C.POINTER(ConvDesc), vp, vp, vp]
+    lib.thb_conv_f32_supported.argtypes = lib.thb_conv_f32_splits.argtypes = [C.POINTER(ConvDesc)]
+    lib.thb_conv_f32_split_bytes.argtypes = [C.POINTER(ConvDesc)]
+    lib.thb_conv_f32_split_bytes.restype = C.c_size_t
+    lib.thb_conv_f32_split_weights.argtypes = [C.POINTER(ConvDesc), vp, vp]
+    lib.thb_conv_f32_fwd.argtypes = [C.POINTER(ConvDesc), vp, vp, vp, vp]
     lib.thb_gemv_fwd.argtypes = [ci, vp, ci, ci, ci, vp, ci, vp, vp, C.POINTER(Act), vp, ci, vp]
     lib.thb_preprocess.argtypes = [vp, vp, ci, ci, ci, ci, vp, vp, ci, vp, ci, cf, cf, vp]
     lib.thb_preprocess_images.argtypes = [vp, ci, ci, ci, ci, ci, ci, vp, vp, ci, vp, ci, vp]
