@@ -28,8 +28,12 @@
 namespace {
 
 constexpr int PT_THREADS = 640;        // warps: 0 copy producer, 1-2 MMA issuers, 3 idle, 4-19 epilogue
+constexpr int PT_GROUPS = 3;            // with pooling: at most three epilogue groups of eight warps, a patch each
 constexpr int PT_MAX_STAGES = 4;
-constexpr int PT_NACC = 2;              // accumulator pairs in TMEM: the MMA issuers run one patch ahead of the epilogue (four measured no faster)
+constexpr int PT_NACC_MAX = 4;
+// accumulator pairs in TMEM: without pooling the MMA issuers run one patch ahead of the epilogue (four measured no faster)
+__host__ __device__ constexpr int pt_nacc(int kp) { return kp ? 4 : 2; }
+__host__ __device__ constexpr int pt_threads(int kp) { return kp ? (4 + 8 * PT_GROUPS) * 32 : PT_THREADS; }
 constexpr int PT_CT_BYTES = 256 * 128;  // activated outputs of one patch, one 128-byte row each
 constexpr int PT_PT_BYTES = 64 * 128;   // pooled tile (at most 64 pooled pixels)
 constexpr size_t PT_SMEM_MAX = 232448;
@@ -44,6 +48,7 @@ struct PatchParams {
     int stage_bytes, nst;   // raw patch buffers
     int w_bytes;            // resident weights: kH*kW tiles of 64 rows x px_bytes
     int ct_bufs;            // output tiles without pooling: 2, or 1 when shared memory is short
+    int eg;                 // with pooling: epilogue groups of eight warps, an output tile and a pooled tile each; 1: all 16 warps on one patch
     int Cout;
     int kp, pp, PR, PC;     // max pooling fused behind the convolution (kp = 0: none): window, padding, pooled tile
     const float *slope;
@@ -69,6 +74,14 @@ __device__ __forceinline__ void tma_store_4d(const void *tmap, uint32_t src, int
     asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(tmap), "r"(src),
                  "r"(c0), "r"(c1), "r"(c2), "r"(c3)
                  : "memory");
+}
+// barrier among the 256 threads of one epilogue group; true on all of them when `bad` is on one
+__device__ __forceinline__ bool group_bar(int g, bool bad)
+{
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %2, 0;\n\tbar.red.or.pred q, %1, 256, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(r) : "r"(g + 2), "r"((uint32_t)bad) : "memory");
+    return r != 0;
 }
 // barrier among the 512 epilogue threads only
 __device__ __forceinline__ void epi_bar_sync() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
@@ -126,43 +139,26 @@ __device__ __forceinline__ Unit unit_of(const PatchParams &p, int u)
     return q;
 }
 
-// All tcgen05.mma of ONE tap into one accumulator (KSTEPS instructions of K = 16 elements), descriptors given as
-// (low word, high word).  An issuing thread is a single thread whose instruction latency is the kernel's critical
-// path: the low word (the 14-bit start-address field, in 16-byte units) is advanced with adds, nothing else is
-// recomputed, and the statement carries no memory clobber so that the compiler may fetch the next tap's offset early
-// (the operands were made visible by the mbarrier wait and the fence before the loop).
-template <int KSTEPS>
-__device__ __forceinline__ void mma_tap(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t accumulate)
-{
-    if (KSTEPS == 1) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
-            "setp.ne.b32 p, %5, 0;\n\t"
-            "mov.b64 da, {%1, %3};\n\t"
-            "mov.b64 db, {%2, %3};\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}" ::"r"(d_tmem),
-            "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate));
-    } else {
-        // four K steps along a 128-byte row: 32 bytes = 2 address units each; `hi` is never zero, so q is always true
-        asm volatile(
-            "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
-            "setp.ne.b32 p, %5, 0;\n\t"
-            "setp.ne.b32 q, %3, 0;\n\t"
-            "mov.b64 da, {%1, %3};\n\t"
-            "mov.b64 db, {%2, %3};\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t"
-            "add.s64 da, da, 2;\n\t"
-            "add.s64 db, db, 2;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, q;\n\t"
-            "add.s64 da, da, 2;\n\t"
-            "add.s64 db, db, 2;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, q;\n\t"
-            "add.s64 da, da, 2;\n\t"
-            "add.s64 db, db, 2;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, q;\n\t}" ::"r"(d_tmem),
-            "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate));
+// Every `step`-th unit from `first` on, without a division per unit (two of them took 390 cycles of a patch's epilogue).
+struct UnitWalk {
+    int n, tr, tc, dn, dtr, dtc;
+    __device__ UnitWalk(const PatchParams &p, int first, int step)
+    {
+        const int per_img = p.tiles_r * p.tiles_c;
+        n = first / per_img; tr = (first - n * per_img) / p.tiles_c; tc = first - n * per_img - tr * p.tiles_c;
+        dn = step / per_img; dtr = (step - dn * per_img) / p.tiles_c; dtc = step - dn * per_img - dtr * p.tiles_c;
     }
-}
+    __device__ __forceinline__ void next(const PatchParams &p)
+    {
+        tc += dtc;
+        int c = 0;
+        if (tc >= p.tiles_c) { tc -= p.tiles_c; c = 1; }
+        tr += dtr + c;
+        c = 0;
+        if (tr >= p.tiles_r) { tr -= p.tiles_r; c = 1; }
+        n += dn + c;
+    }
+};
 
 // One thread's 32 accumulator columns (channels CH*32 .. CH*32+31 of its output pixel) -> four 16-byte chunks:
 // y = act(acc * scale[c] + shift[c]).  CH is a template argument so that every index into the constants is known at
@@ -226,19 +222,20 @@ __device__ __forceinline__ void activate_half_res(const uint32_t (&acc)[32], con
 
 // PX: bytes per input pixel in shared memory (32 or 128); KP: pooling window fused behind the convolution (0: none)
 template <int PX, int KP>
-__global__ void __launch_bounds__(PT_THREADS, 1)
+__global__ void __launch_bounds__(pt_threads(KP), 1)
 conv_patch_tc_kernel(const __grid_constant__ CUtensorMap tmapW, const __grid_constant__ CUtensorMap tmapA,
                      const __grid_constant__ CUtensorMap tmapY, const __grid_constant__ CUtensorMap tmapR, const PatchParams p)
 {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t *full = reinterpret_cast<uint64_t *>(smem), *empty = full + PT_MAX_STAGES;
-    uint64_t *acc_full = empty + PT_MAX_STAGES, *acc_empty = acc_full + PT_NACC, *w_full = acc_empty + PT_NACC;
+    constexpr int PT_NACC = pt_nacc(KP);
+    uint64_t *acc_full = empty + PT_MAX_STAGES, *acc_empty = acc_full + PT_NACC_MAX, *w_full = acc_empty + PT_NACC_MAX;
     uint64_t *res_full = w_full + 1;                    // residual tile landed in output tile 0 / 1
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(res_full + 2);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     // header of 2048 bytes: [0, 256) mbarriers, the TMEM slot and the abort flag; [512, 768) PReLU slopes
-    static_assert((2 * PT_MAX_STAGES + 2 * PT_NACC + 1 + 2) * 8 + 8 <= 256, "the barriers outgrow their part of the header");
+    static_assert((2 * PT_MAX_STAGES + 2 * PT_NACC_MAX + 1 + 2) * 8 + 8 <= 256, "the barriers outgrow their part of the header");
     float *s_slope = reinterpret_cast<float *>(smem + 512);
     uint8_t *sW = smem + 2048;                          // resident weights: tap t at sW + t * 64 * PX
     uint8_t *sP = sW + p.w_bytes;                       // raw patch buffers
@@ -258,7 +255,7 @@ conv_patch_tc_kernel(const __grid_constant__ CUtensorMap tmapW, const __grid_con
         }
         for (int b = 0; b < PT_NACC; b++) {
             mbar_init(smem_u32(&acc_full[b]), 2);          // one commit per MMA issuer
-            mbar_init(smem_u32(&acc_empty[b]), 16);        // one arrival per epilogue warp
+            mbar_init(smem_u32(&acc_empty[b]), KP && p.eg > 1 ? 8 : 16);  // one arrival per epilogue warp
         }
         mbar_init(smem_u32(w_full), 1);
         mbar_init(smem_u32(&res_full[0]), 1);
@@ -322,59 +319,143 @@ conv_patch_tc_kernel(const __grid_constant__ CUtensorMap tmapW, const __grid_con
         // ================================================================== MMA issuers: warp 1 feeds the accumulator of GEMM
         // rows 0..127, warp 2 that of rows 128..255 (an instruction of N = 64 takes the tensor pipe 48 cycles, which
         // one issuing thread cannot sustain)
-        if (lane == 0 && mine > 0) {
+        if (mine > 0) {
             constexpr uint32_t IDESC_F16 = make_idesc(1u, 0u, 64), IDESC_BF16 = make_idesc(1u, 1u, 64);
             const uint32_t idesc = p.kind == 1 ? IDESC_BF16 : IDESC_F16;
             constexpr int KSTEPS = PX / 32;      // tcgen05.mma of K = 16 elements per tap
             constexpr uint32_t HALF = 128u * PX / 16, BSTEP = 64u * PX / 16;   // descriptor steps: second accumulator's rows, next tap's weights
             constexpr uint32_t PXU = PX / 16;
-            const int hsel = warp - 1, kW = p.kW;
-            const uint32_t rowstep = (uint32_t)(p.P - p.kW + 1) * PXU;
-            const uint64_t proto = make_rows_desc(0u, PX);
-            const uint32_t hi = (uint32_t)(proto >> 32), lo_flags = (uint32_t)proto;
-            const uint32_t b_lo0 = lo_flags | ((smem_u32(sW) >> 4) & 0x3FFFu);
-            const int ntaps = taps;
+            const int hsel = warp - 1, kW = p.kW, kH = p.kH;
+            const uint32_t rowstep = (uint32_t)p.P * PXU;
+            const uint64_t b0 = make_rows_desc(smem_u32(sW), PX);
+            // The whole warp walks the taps and one elected thread issues: addresses stay in uniform registers, where the
+            // instruction wants them.
+            const bool leader = elect_one();
             int ring_s = 0;
             uint32_t ring_ph = 0;
-            bool alive = mbar_wait_bounded(smem_u32(w_full), 0);
-            if (!alive) {
+            bool alive = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(w_full), 0));
+            if (!alive && leader) {
                 atomicExch(p.status, 10);
                 *abort_flag = 1;
             }
             for (int u = 0; u < mine && alive; u++) {
                 const int ab = u % PT_NACC;
-                if (!mbar_wait_bounded(smem_u32(&acc_empty[ab]), ((u / PT_NACC) & 1) ^ 1)) {
-                    atomicExch(p.status, 6);
-                    *abort_flag = 1;
+                if (!__all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&acc_empty[ab]), ((u / PT_NACC) & 1) ^ 1))) {
+                    if (leader) {
+                        atomicExch(p.status, 6);
+                        *abort_flag = 1;
+                    }
                     break;
                 }
                 const int s = ring_s;
                 const uint32_t ph = ring_ph;
                 if (++ring_s == p.nst) { ring_s = 0; ring_ph ^= 1; }
-                if (!mbar_wait_bounded(smem_u32(&full[s]), ph)) {
-                    atomicExch(p.status, 4);
-                    *abort_flag = 1;
+                if (!__all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&full[s]), ph))) {
+                    if (leader) {
+                        atomicExch(p.status, 4);
+                        *abort_flag = 1;
+                    }
                     break;
                 }
                 tc_fence_after();
                 const uint32_t d = tmem_base + ab * 128 + hsel * 64;
-                const uint32_t a_lo0 = (lo_flags | ((smem_u32(sP + s * p.stage_bytes) >> 4) & 0x3FFFu)) + hsel * HALF;
-                // tap (r, s) reads the patch from pixel row r*P + s on: one pixel (PXU address units) further per tap, and
-                // P - kW + 1 pixels further at the end of a kernel row -- all in registers, the loop touches no memory
-                uint32_t b_lo = b_lo0, a_lo = a_lo0;
-                int sx = 1;
-                mma_tap<KSTEPS>(d, a_lo, b_lo, hi, idesc, 0u);   // first tap: the accumulator starts from zero
-#pragma unroll 4
-                for (int t = 1; t < ntaps; t++) {
-                    b_lo += BSTEP;
-                    if (sx == kW) { sx = 1; a_lo += rowstep; } else { sx++; a_lo += PXU; }
-                    mma_tap<KSTEPS>(d, a_lo, b_lo, hi, idesc, 1u);
+                // tap (r, s) reads the patch from pixel row r*P + s on
+                uint64_t a_row = make_rows_desc(smem_u32(sP + s * p.stage_bytes) + hsel * HALF * 16, PX), b = b0;
+                uint32_t accumulate = 0;
+                for (int r = 0; r < kH; r++, a_row += rowstep) {
+                    uint64_t a = a_row;
+                    for (int t = 0; t < kW; t++, a += PXU, b += BSTEP) {
+                        if (leader) {
+#pragma unroll
+                            for (int k = 0; k < KSTEPS; k++) tc_mma_f16(d, a + 2 * k, b + 2 * k, idesc, k ? 1u : accumulate);
+                        }
+                        accumulate = 1;
+                    }
                 }
-                tc_commit(smem_u32(&empty[s]));
-                tc_commit(smem_u32(&acc_full[ab]));
+                if (leader) {
+                    tc_commit(smem_u32(&empty[s]));
+                    tc_commit(smem_u32(&acc_full[ab]));
+                }
+                __syncwarp();
             }
         }
         __syncwarp();
+    } else if (KP && p.eg > 1 && warp >= 4) {
+        // ================================================================== epilogue with pooling: `eg` groups of eight warps, a
+        // patch each.  What bounds a patch is not its instructions but the chain of them -- accumulator, activation, barrier,
+        // pooling, barrier, store: with all 16 warps on one patch 4200 cycles of it against 1800 of multiplies -- so several are
+        // under way.  Outputs outside the map go to shared memory as the smallest value: the pooling asks nothing.
+        if constexpr (KP > 0) {
+            const int g = (warp - 4) >> 3, et = tid - 128 - g * 256, quad = warp & 3, half = ((warp - 4) >> 2) & 1;
+            const int m = half * 128 + quad * 32 + lane, cr = m / p.P, cc = m - cr * p.P, ci = cr * p.CC + cc;
+            const bool valid = cr < p.CR && cc < p.CC;
+            const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + half * 64;
+            const int act_mode = p.act_kind == THB_ACT_NONE ? 0
+                                 : p.act_kind != THB_ACT_THRESHOLD ? 2
+                                 : (p.act_th == 0.f && p.act_val == 0.f) ? 3 : 1;
+            const uint32_t neg_inf2 = p.kind == 0 ? 0xFC00FC00u : 0xFF80FF80u;
+            const int kind = p.kind, items = p.PR * p.PC * 8, j = et & 7;
+            uint8_t *tile = ct + g * PT_CT_BYTES, *ptile = pt + g * PT_PT_BYTES, *row_smem = tile + ci * 128;
+            UnitWalk walk(p, blockIdx.x + g * gridDim.x, p.eg * gridDim.x);
+            for (int u = g; u < mine; u += p.eg, walk.next(p)) {
+                const int ab = u % PT_NACC, r0 = 2 * walk.tr * p.PR - p.pp, c0 = 2 * walk.tc * p.PC - p.pp;
+                const bool have = mbar_wait_bounded(smem_u32(&acc_full[ab]), (u / PT_NACC) & 1);
+                if (!have) {
+                    if (lane == 0) atomicExch(p.status, 2);
+                    *abort_flag = 1;
+                }
+                tc_fence_after();
+                const bool inside = (unsigned)(r0 + cr) < (unsigned)p.oH && (unsigned)(c0 + cc) < (unsigned)p.oW;
+#pragma unroll
+                for (int ch = 0; ch < 2; ch++) {
+                    uint32_t acc[32];
+                    uint4 o[4];
+                    __syncwarp();
+                    tmem_ld32(lane_addr + ab * 128 + ch * 32, acc);
+                    tmem_ld_wait();
+                    if (ch == 1) {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(smem_u32(&acc_empty[ab]));
+                    }
+                    if (ch == 0) activate_half<0>(acc, p, act_mode, s_slope, o);
+                    else activate_half<1>(acc, p, act_mode, s_slope, o);
+                    if (valid) {
+#pragma unroll
+                        for (int cj = 0; cj < 4; cj++)
+                            *reinterpret_cast<uint4 *>(row_smem + (((ch * 4 + cj) ^ (ci & 7)) << 4)) =
+                                inside ? o[cj] : make_uint4(neg_inf2, neg_inf2, neg_inf2, neg_inf2);
+                    }
+                }
+                if (et == 0) bulk_wait_group_read<0>();       // the pooled tile has left
+                if (group_bar(g, !have || *abort_flag)) break;  // the activated patch is complete
+                for (int it = et; it < items; it += 256) {
+                    const int px = it >> 3, pr = px / p.PC, m00 = 2 * pr * p.CC + 2 * (px - pr * p.PC);
+                    uint4 v[KP * KP];
+#pragma unroll
+                    for (int k = 0; k < KP * KP; k++) {
+                        const int mm = m00 + (k / KP) * p.CC + k % KP;
+                        v[k] = *reinterpret_cast<const uint4 *>(tile + mm * 128 + ((j ^ (mm & 7)) << 4));
+                    }
+                    uint4 mx = make_uint4(neg_inf2, neg_inf2, neg_inf2, neg_inf2);
+#pragma unroll
+                    for (int k = 0; k < KP * KP; k++) {
+                        mx.x = max_pair(mx.x, v[k].x, kind);
+                        mx.y = max_pair(mx.y, v[k].y, kind);
+                        mx.z = max_pair(mx.z, v[k].z, kind);
+                        mx.w = max_pair(mx.w, v[k].w, kind);
+                    }
+                    *reinterpret_cast<uint4 *>(ptile + px * 128 + j * 16) = mx;
+                }
+                fence_proxy_async_smem();
+                group_bar(g, false);                          // pooled tile complete; the patch tile may be overwritten
+                if (et == 0) {
+                    tma_store_4d(&tmapY, smem_u32(ptile), 0, walk.tc * p.PC, walk.tr * p.PR, walk.n);  // clips pooled pixels beyond the map
+                    bulk_commit_group();
+                }
+            }
+            if (et == 0) bulk_wait_group<0>();
+        }
     } else if (warp >= 4) {
         // ================================================================== epilogue: activate, (pool,) store
         // 16 warps: a thread owns one GEMM row (TMEM lane) and 32 of its 64 output channels
@@ -536,7 +617,7 @@ encode_tiled_fn pt_encode_fn()
 
 struct Geometry {
     int CR, CC, P, tiles_r, tiles_c, PR, PC;
-    int stage_bytes, nst, ct_bufs, w_bytes;
+    int stage_bytes, nst, ct_bufs, eg, w_bytes;
     size_t smem;
 };
 
@@ -547,9 +628,24 @@ bool plan_smem(int kH, int kW, int px_bytes, int kp, bool two_tiles, Geometry *g
     // a patch buffer holds the copied pixels and whatever the 256 GEMM rows of the last tap reach beyond them
     const int box_px = (g->CR + kH - 1) * g->P, reach_px = (kH - 1) * g->P + kW - 1 + 256;
     g->stage_bytes = ((box_px > reach_px ? box_px : reach_px) * px_bytes + 1023) & ~1023;
+    if (kp) {
+        // as many epilogue groups as leave three patches in flight, then as leave two; one group: 16 warps and a pair of pooled tiles
+        for (int want = 3; want >= 2; want--)
+            for (g->eg = PT_GROUPS; g->eg >= 1; g->eg--) {
+                if (g->eg == 1 && want == 3) continue;
+                g->ct_bufs = g->eg;
+                const size_t fixed = 1024 + 2048 + (size_t)g->w_bytes + (size_t)g->eg * PT_CT_BYTES + (size_t)(g->eg > 1 ? g->eg : 2) * PT_PT_BYTES;
+                if (fixed + (size_t)want * g->stage_bytes > PT_SMEM_MAX) continue;
+                g->nst = (int)((PT_SMEM_MAX - fixed) / g->stage_bytes);
+                if (g->nst > PT_MAX_STAGES) g->nst = PT_MAX_STAGES;
+                g->smem = fixed + (size_t)g->nst * g->stage_bytes;
+                return true;
+            }
+        return false;
+    }
     // without pooling the output tile is the source of an asynchronous store: two of them when room allows
-    for (g->ct_bufs = kp ? 1 : 2; g->ct_bufs >= 1; g->ct_bufs--) {
-        const size_t fixed = 1024 + 2048 + (size_t)g->w_bytes + (size_t)g->ct_bufs * PT_CT_BYTES + (kp ? 2 * PT_PT_BYTES : 0);
+    for (g->ct_bufs = 2; g->ct_bufs >= 1; g->ct_bufs--) {
+        const size_t fixed = 1024 + 2048 + (size_t)g->w_bytes + (size_t)g->ct_bufs * PT_CT_BYTES;
         if (fixed + 2 * (size_t)g->stage_bytes > PT_SMEM_MAX) continue;
         g->nst = (int)((PT_SMEM_MAX - fixed) / g->stage_bytes);
         if (g->nst > PT_MAX_STAGES) g->nst = PT_MAX_STAGES;
@@ -642,7 +738,7 @@ int patch_launch(const thb_conv_desc *d, int pk, int ppad, int pH, int pW, const
     p.act_kind = d->act.kind; p.act_th = d->act.threshold; p.act_val = d->act.value; p.act_alpha = d->act.alpha;
     p.kind = d->dtype == THB_BF16 ? 1 : 0;
     p.status = d->status;
-    p.w_bytes = g.w_bytes; p.stage_bytes = g.stage_bytes; p.nst = g.nst; p.ct_bufs = g.ct_bufs;
+    p.w_bytes = g.w_bytes; p.stage_bytes = g.stage_bytes; p.nst = g.nst; p.ct_bufs = g.ct_bufs; p.eg = g.eg;
     const size_t smem = g.smem;
 
     // tensor maps of the weights (one tap per box), the input (patch box) and the output (tile box), cached by buffer and shape
@@ -750,7 +846,7 @@ int patch_launch(const thb_conv_desc *d, int pk, int ppad, int pH, int pW, const
     p.pdl = use_pdl;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(PT_THREADS);
+    cfg.blockDim = dim3(pk && p.eg > 1 ? (4 + 8 * p.eg) * 32 : PT_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = (cudaStream_t)s;
     cudaLaunchAttribute attr[1];
