@@ -33,6 +33,7 @@ CASES = [  # n, cin, h, w, cout, k, stride, pad
     (1, 256, 5, 6, 66, 5, 1, 2),
     (9, 192, 1, 1, 1000, 1, 1, 0),    # a Linear
     (2, 64, 57, 31, 64, 3, 1, 1),
+    (20, 64, 45, 43, 72, 1, 1, 0),    # 606 tiles: the form with four epilogue warps
 ]
 
 
@@ -84,6 +85,39 @@ def test_few_tiles(lib, case, dtype, monkeypatch):
                     assert np.array_equal(out, run(kind, 0, few=False)), kind
                 else:
                     assert np.array_equal(out, run(kind, splits)), (kind, splits)
+    finally:
+        monkeypatch.undo()
+        lib.thb_conv_reload_knobs()
+
+
+@pytest.mark.parametrize("splits", [1, 4])
+def test_bounded_wait(lib, splits, monkeypatch):
+    """A copy that is never made: the launch ends (the peers of the CTA that lacks it give up their own waits), reports, and the next
+    one is right."""
+    rng = np.random.default_rng(6)
+    conv = G.Conv(lib, K.THB_F16, (1, 64, 10, 10), rng.standard_normal((64, 64, 3, 3)).astype(np.float32), (1, 1), (1, 1))
+    conv.d.splits = splits
+    xt, _ = G.to_nhwc(rng.standard_normal((1, 64, 10, 10)).astype(np.float32), K.THB_F16)
+    monkeypatch.setenv("THB200_FEW_TILES", "100000")
+    monkeypatch.setenv("THB200_NO_PATCH", "1")
+    try:
+        lib.thb_conv_reload_knobs()
+        good = conv.run(xt)
+        monkeypatch.setenv("THB200_TEST_WITHHOLD", "1")
+        monkeypatch.setenv("THB200_WAIT_LIMIT_CYCLES", "20000000")
+        lib.thb_conv_reload_knobs()
+        y = torch.zeros_like(good)
+        assert lib.thb_conv_fwd(C.byref(conv.d), G.ptr(xt), G.ptr(y), None) == 0
+        torch.cuda.synchronize()
+        assert int(conv.keep[3].cpu()[0]) != 0
+        conv.keep[3].zero_()
+    finally:
+        monkeypatch.undo()
+        lib.thb_conv_reload_knobs()
+    monkeypatch.setenv("THB200_FEW_TILES", "100000")
+    lib.thb_conv_reload_knobs()
+    try:
+        assert torch.equal(conv.run(xt), good)
     finally:
         monkeypatch.undo()
         lib.thb_conv_reload_knobs()

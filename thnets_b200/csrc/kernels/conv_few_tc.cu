@@ -6,16 +6,19 @@
 // Here
 //   * a tile is 128 pixels x 64 channels, one CTA works on one tile only, and two CTAs fit an SM;
 //   * the K blocks of a tile are shared by the S = 1, 2, 4 or 8 CTAs of a thread-block cluster.  Each pushes the columns of
-//     its fp32 partial tile to the CTA that owns them, through distributed shared memory, and every owner adds the S parts
-//     in rank order and finishes its 64 / S channels (no atomics, no scratch in global memory, no second launch);
+//     its fp32 partial tile to the CTA that owns them, through distributed shared memory (stores that the owner's barrier
+//     counts: a cluster barrier behind them took 1100 to 2900 cycles), and every owner adds the S parts in rank order and
+//     finishes its 64 / S channels (no atomics, no scratch in global memory, no second launch);
 //   * weights and activations are loaded by two different warps, and since weights do not depend on the kernel before, their
-//     loads start ahead of griddepcontrol.wait, under that kernel's tail;
-//   * the epilogue goes from registers to global memory.
-// Measured: the tables at thb_conv_few_splits and thb_conv_few_supported.  ResNet-18, 1 image: 305 -> 155 us of kernels;
-// ResNet-50, 8 images: 727 -> 480 us.
+//     loads start ahead of griddepcontrol.wait, under that kernel's tail, as does everything that is worked out from parameters;
+//   * the epilogue passes the accumulator through shared memory to a thread per row and eight channels, whose constants stay in
+//     registers and whose rows leave and arrive whole (a thread per row took 3900 cycles a tile, 1600 now).
+// Measured: the tables at thb_conv_few_splits and thb_conv_few_supported.  Calls: ResNet-18 fp16, 1 image 179 -> 160 us; ResNet-50
+// fp16, 8 images 537 -> 510; ResNet-18 uint8, 1 image 206 -> 184.  What is left of a launch's 4 to 6 us: 2 us from the last store to
+// the next launch's first load, 0.5 us to its first K block, the K blocks, 1.5 us of exchange and epilogue.
 //
 // Every mbarrier wait is bounded; one that runs out records a code in *status and the CTA drains (all its threads still
-// reach both cluster barriers, so that its peers end too).
+// reach both cluster barriers; its peers' waits for its part run out like any other).
 #include <cuda.h>
 #include <string.h>
 #include "common.cuh"
@@ -24,11 +27,16 @@
 namespace {
 
 constexpr int BM = 128, BN = 64;
-constexpr int NTHREADS = 224;  // 4 epilogue warps, activation producer, weight producer, MMA issuer
+// EW epilogue warps (4 or 8), an activation producer, a weight producer, an MMA issuer
+constexpr int nthreads(int ew) { return (ew + 3) * 32; }
 constexpr int A_BYTES = BM * 128, B_BYTES = BN * 128, STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int MAX_STAGES = 8;
-constexpr int BAR_BYTES = 1024;
-constexpr int RECV_BYTES = BM * BN * 4;  // the partial columns a CTA receives, its own included
+// ahead of the tiles: barriers, from 192 on the per-channel constants; uint8: bias addends, per-row terms from 448 on, then the table
+constexpr int U8_ROWS = 448, U8_TABLE = U8_ROWS + BM * 8;
+__host__ __device__ constexpr int header_bytes(bool u8, int tbl_bytes) { return u8 ? (U8_TABLE + tbl_bytes + 1023) & ~1023 : 1024; }
+// Partial sums by way of shared memory: groups of four columns, the rows of a group after one another and one row of padding, so
+// that neither a warp's 32 rows of a group nor its reads of several groups meet in a bank.
+constexpr int RECV_ROWS = BM + 1, RECV_BYTES = (BN / 4) * RECV_ROWS * 16;
 
 struct FewParams {
     uint8_t *y;
@@ -58,6 +66,7 @@ struct FewParams {
 // (a plain store: the word may lie in pinned host memory)
 __device__ __forceinline__ void report(int *status, int code) { *reinterpret_cast<volatile int *>(status) = code; }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ uint32_t cluster_addr(uint32_t smem, uint32_t rank)
 {
@@ -65,10 +74,14 @@ __device__ __forceinline__ uint32_t cluster_addr(uint32_t smem, uint32_t rank)
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem), "r"(rank));
     return a;
 }
-__device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d)
+// 16 bytes into the shared memory of a CTA of the cluster, counted by a barrier there
+__device__ __forceinline__ void st_async_v4(uint32_t addr, uint32_t bar, uint32_t a, uint32_t b, uint32_t c, uint32_t d)
 {
-    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%2, %3, %4, %5}, [%1];" ::"r"(addr), "r"(bar), "r"(a),
+                 "r"(b), "r"(c), "r"(d)
+                 : "memory");
 }
+template <int EW> __device__ __forceinline__ void epi_bar_sync() { asm volatile("bar.sync 1, %0;" ::"n"(EW * 32) : "memory"); }
 
 template <int KIND> __device__ __forceinline__ uint32_t pack2(float a, float b)
 {
@@ -90,12 +103,11 @@ struct Consts {
     float sc[BN], sh[BN], sl[BN];
 };
 
-// Eight channels of one pixel, the first of them channel c of the tile: y = act(acc * scale + shift + res_coef * residual),
-// channels >= Cout zero.  The operations and their order are those of the persistent kernel's epilogue: the same bits.
-// ACT: 0 none, 1 plain ReLU, 2 anything.  The variant is chosen once per tile: with the general activation inlined in every
-// chunk the epilogue was bound by instruction fetch (0.8 us per chunk of eight channels).
+// Eight channels of one pixel: y = act(acc * scale + shift + res_coef * residual), channels >= Cout zero.  The operations and
+// their order are those of the persistent kernel's epilogue: the same bits.  ACT: 0 none, 1 plain ReLU, 2 anything.
 template <int KIND, int ACT>
-__device__ __forceinline__ uint4 finish8(const float (&acc)[8], const uint4 &rv, int c, int left, const Consts &k, const FewParams &p)
+__device__ __forceinline__ uint4 finish8(const float (&acc)[8], const uint4 &rv, const float (&sc)[8], const float (&sh)[8], const float *sl, int left,
+                                         const FewParams &p)
 {
     const uint32_t rw[4] = {rv.x, rv.y, rv.z, rv.w};
     uint32_t ow[4];
@@ -106,10 +118,10 @@ __device__ __forceinline__ uint4 finish8(const float (&acc)[8], const uint4 &rv,
 #pragma unroll
         for (int e = 0; e < 2; e++) {
             const int i = 2 * h + e;
-            v[e] = fmaf(acc[i], k.sc[c + i], k.sh[c + i]);
+            v[e] = fmaf(acc[i], sc[i], sh[i]);
             if (p.res) v[e] = fmaf(p.res_coef, e ? rr.y : rr.x, v[e]);
             if (ACT == 1) v[e] = fmaxf(v[e], 0.f);
-            if (ACT == 2) v[e] = thb_apply_act(v[e], p.act_kind, p.act_th, p.act_val, p.act_alpha, k.sl[c + i]);
+            if (ACT == 2) v[e] = thb_apply_act(v[e], p.act_kind, p.act_th, p.act_val, p.act_alpha, sl[i]);
             if (i >= left) v[e] = 0.f;
         }
         ow[h] = pack2<KIND>(v[0], v[1]);
@@ -117,47 +129,28 @@ __device__ __forceinline__ uint4 finish8(const float (&acc)[8], const uint4 &rv,
     return make_uint4(ow[0], ow[1], ow[2], ow[3]);
 }
 
-// The thread's pixel, straight from its TMEM lane (no split): 64 channels.
+// A network's last convolution, whose result leaves as NCHW floats (rounded through the 16-bit type like any other), straight
+// from the thread's TMEM lane: a warp's lanes are 32 neighbouring pixels of a plane, so every channel is a coalesced 128-byte
+// store.  Two groups of four warps take every other eight channels.
 template <int KIND, int ACT>
-__device__ __forceinline__ void finish_tmem(uint32_t taddr, const uint4 (&rv)[BN / 8], uint8_t *dst, bool real, int left, const Consts &k,
-                                            const FewParams &p)
-{
-#pragma unroll(ACT == 2 ? 1 : 8)
-    for (int j = 0; j < BN / 8; j++) {
-        uint32_t a[8];
-        tmem_ld8(taddr + j * 8, a);
-        tmem_ld_wait();
-        float acc[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++) acc[i] = __uint_as_float(a[i]);
-        uint4 res = rv[0];
-#pragma unroll
-        for (int q = 1; q < BN / 8; q++)  // (constant indices keep the residual in registers)
-            if (q == j) res = rv[q];
-        const uint4 o = finish8<KIND, ACT>(acc, res, j * 8, left - j * 8, k, p);
-        if (real && j * 8 < left) *reinterpret_cast<uint4 *>(dst + j * 16) = o;
-    }
-}
-
-// The same for a network's last convolution, whose result leaves as NCHW floats (rounded through the 16-bit type like any
-// other): a warp's lanes are 32 neighbouring pixels of a plane, so every channel is a coalesced 128-byte store.
-template <int KIND, int ACT>
-__device__ __forceinline__ void finish_nchw(uint32_t taddr, const uint4 (&rv)[BN / 8], float *dst, size_t plane, bool real, int left, const Consts &k,
-                                            const FewParams &p)
+__device__ __forceinline__ void finish_nchw(uint32_t taddr, const uint8_t *res, float *dst, size_t plane, bool real, int left, const Consts &k,
+                                            int first, int step, const FewParams &p)
 {
 #pragma unroll 1
-    for (int j = 0; j < BN / 8 && j * 8 < left; j++) {
+    for (int j = first; j < BN / 8 && j * 8 < left; j += step) {
         uint32_t a[8];
         tmem_ld8(taddr + j * 8, a);
         tmem_ld_wait();
-        float acc[8];
+        float acc[8], sc[8], sh[8];
 #pragma unroll
-        for (int i = 0; i < 8; i++) acc[i] = __uint_as_float(a[i]);
-        uint4 res = rv[0];
-#pragma unroll
-        for (int q = 1; q < BN / 8; q++)
-            if (q == j) res = rv[q];
-        const uint4 o = finish8<KIND, ACT>(acc, res, j * 8, left - j * 8, k, p);
+        for (int i = 0; i < 8; i++) {
+            acc[i] = __uint_as_float(a[i]);
+            sc[i] = k.sc[j * 8 + i];
+            sh[i] = k.sh[j * 8 + i];
+        }
+        uint4 rv = make_uint4(0, 0, 0, 0);
+        if (p.res && real) rv = __ldg(reinterpret_cast<const uint4 *>(res + j * 16));
+        const uint4 o = finish8<KIND, ACT>(acc, rv, sc, sh, k.sl + j * 8, left - j * 8, p);
         const uint32_t w[4] = {o.x, o.y, o.z, o.w};
         if (real) {
 #pragma unroll
@@ -170,27 +163,48 @@ __device__ __forceinline__ void finish_nchw(uint32_t taddr, const uint4 (&rv)[BN
     }
 }
 
-// The same for the W = 64 / S channels this CTA owns, summing the S parts its peers (and itself) left in `recv`.
-template <int KIND, int ACT>
-__device__ __forceinline__ void finish_parts(const uint8_t *recv, int S, int W, int c_local, const uint4 (&rv)[BN / 8], uint8_t *dst, int left,
-                                             int row, const Consts &k, const FewParams &p)
+// Eight columns of one row, the sum of the S parts in rank order: `part` points at the first part's first group of four.
+template <typename T> struct vec4;
+template <> struct vec4<float> { typedef float4 type; };
+template <> struct vec4<int> { typedef int4 type; };
+template <typename T> __device__ __forceinline__ void sum_parts(const uint8_t *part, int S, int stride, T (&acc)[8])
 {
+    typedef typename vec4<T>::type V;
+    const V u0 = *reinterpret_cast<const V *>(part), v0 = *reinterpret_cast<const V *>(part + RECV_ROWS * 16);
+    acc[0] = u0.x; acc[1] = u0.y; acc[2] = u0.z; acc[3] = u0.w;
+    acc[4] = v0.x; acc[5] = v0.y; acc[6] = v0.z; acc[7] = v0.w;
+    for (int r = 1; r < S; r++) {
+        part += stride;
+        const V u = *reinterpret_cast<const V *>(part), v = *reinterpret_cast<const V *>(part + RECV_ROWS * 16);
+        acc[0] += u.x; acc[1] += u.y; acc[2] += u.z; acc[3] += u.w;
+        acc[4] += v.x; acc[5] += v.y; acc[6] += v.z; acc[7] += v.w;
+    }
+}
+
+// The items (row, eight channels) of an epilogue thread: eight channels of those this CTA finishes, rows r0, r0 + rows, ...  The
+// residual of the first four is there already.
+template <int KIND, int ACT>
+__device__ __forceinline__ void finish_rows(const uint8_t *part, int S, int stride, int r0, int rows, uint4 (&rv)[4], int m0, const float *sc_, const float *sh_,
+                                            const float *sl, int left, const uint8_t *res, uint8_t *dst, const FewParams &p)
+{
+    float sc[8], sh[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) { sc[i] = sc_[i]; sh[i] = sh_[i]; }
 #pragma unroll 1
-    for (int j = 0; j < W / 8 && j * 8 < left; j++) {
-        float acc[8];
+    for (int r = r0; r < BM;) {
 #pragma unroll
-        for (int i = 0; i < 8; i++) acc[i] = 0.f;
-        const float4 *part = reinterpret_cast<const float4 *>(recv) + (size_t)(2 * j) * BM + row;
-        for (int r = 0; r < S; r++, part += (W >> 2) * BM) {
-            const float4 u = part[0], v = part[BM];
-            acc[0] += u.x; acc[1] += u.y; acc[2] += u.z; acc[3] += u.w;
-            acc[4] += v.x; acc[5] += v.y; acc[6] += v.z; acc[7] += v.w;
+        for (int i = 0; i < 4; i++, r += rows) {
+            if (r >= BM || m0 + r >= p.P) return;
+            float acc[8];
+            sum_parts(part, S, stride, acc);
+            part += rows * 16;
+            *reinterpret_cast<uint4 *>(dst + (size_t)r * p.out_ld * 2) = finish8<KIND, ACT>(acc, rv[i], sc, sh, sl, left, p);
         }
-        uint4 res = rv[0];
+        if (p.res) {
 #pragma unroll
-        for (int q = 1; q < BN / 16; q++)  // (W <= 32 here)
-            if (q == j) res = rv[q];
-        *reinterpret_cast<uint4 *>(dst + j * 16) = finish8<KIND, ACT>(acc, res, c_local + j * 8, left - j * 8, k, p);
+            for (int i = 0; i < 4; i++)
+                if (r + i * rows < BM && m0 + r + i * rows < p.P) rv[i] = __ldg(reinterpret_cast<const uint4 *>(res + (size_t)(r + i * rows) * p.res_ld * 2));
+        }
     }
 }
 
@@ -199,45 +213,51 @@ __device__ __forceinline__ void finish_parts(const uint8_t *recv, int S, int W, 
 // integer arithmetic of the persistent kernel's u8_chunk32.
 struct U8Row {
     uint32_t rc;
-    int tailmask, thr, shift;
+    int trow;  // the border class's row of the table, its sign bit set where the reference's tail quirk does not apply
 };
-__device__ __forceinline__ uint2 finish8_u8(const int (&acc)[8], const int *t, const int *b, const U8Row &e, const uint2 &rv, int left,
+__device__ __forceinline__ uint2 finish8_u8(const int (&acc)[8], const int *tbl, const int (&b)[8], const U8Row &e, int shift, int thr, const uint2 &rv, int left,
                                             const FewParams &p)
 {
+    const int tailmask = e.trow < 0 ? 0 : 255;
+    const int4 *t4 = reinterpret_cast<const int4 *>(tbl + (e.trow & 0x7fffffff));
+    const int4 ta = t4[0], tb = t4[1];
+    const int t[8] = {ta.x, ta.y, ta.z, ta.w, tb.x, tb.y, tb.z, tb.w};
     uint32_t ow[2] = {0, 0};
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-        const int sres = (int)((uint32_t)acc[i] * (uint32_t)p.c_mult + (uint32_t)t[i] + e.rc) >> e.shift;
+        const int sres = (int)((uint32_t)acc[i] * (uint32_t)p.c_mult + (uint32_t)t[i] + e.rc) >> shift;
         const int q = min(max(sres, 0), 255), t2 = q + b[i];
-        int v = max(min(max(t2, 0), 255), t2 & e.tailmask);
+        int v = max(min(max(t2, 0), 255), t2 & tailmask);
         if (p.res) {
             const int r = (int)(((i < 4 ? rv.x : rv.y) >> (8 * (i & 3))) & 255u);
             v = min(max(p.ca * v + p.cb * r + p.res_addend, 0), 255);
         }
-        v = v > e.thr ? v : p.relu_val;
+        v = v > thr ? v : p.relu_val;
         if (i < left) ow[i >> 2] |= (uint32_t)v << (8 * (i & 3));
     }
     return make_uint2(ow[0], ow[1]);
 }
 
-template <int KIND>
-__global__ void __launch_bounds__(NTHREADS) conv_few_kernel(const __grid_constant__ CUtensorMap tmapW, const __grid_constant__ CUtensorMap tmapA,
-                                                            const __grid_constant__ CUtensorMap tmapA2, const FewParams p)
+template <int KIND, int EW>
+__global__ void __launch_bounds__(nthreads(EW), EW == 8 ? 2 : 3) conv_few_kernel(const __grid_constant__ CUtensorMap tmapW, const __grid_constant__ CUtensorMap tmapA,
+                                                               const __grid_constant__ CUtensorMap tmapA2, const __grid_constant__ FewParams p)
 {
     constexpr uint32_t IDESC = make_idesc(KIND == 2 ? 2u : 1u, KIND == 1 ? 1u : 0u, BN);
     constexpr int KE = KIND == 2 ? 128 : 64;  // elements of a K block
+    constexpr int EPI = EW * 32, NT = EPI + 96, W_A = EW, W_B = EW + 1, W_MMA = EW + 2;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t *full = reinterpret_cast<uint64_t *>(smem), *empty = full + MAX_STAGES, *acc_full = empty + MAX_STAGES;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 1);
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem), *empty = full + MAX_STAGES, *acc_full = empty + MAX_STAGES, *recv_full = acc_full + 1;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(recv_full + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     Consts &consts = *reinterpret_cast<Consts *>(smem + 192);
-    static_assert(192 + sizeof(Consts) <= BAR_BYTES, "barriers and constants share the first kilobyte");
-    // (every CTA of a cluster has the same layout, so an offset into this one's receive buffer fits its peers' too)
-    uint8_t *recv = smem + BAR_BYTES;
-    uint8_t *ring = recv + (p.splits > 1 ? RECV_BYTES : 0);
-    int *tbl = reinterpret_cast<int *>(ring), *bias = reinterpret_cast<int *>(smem + 192);  // uint8
-    if (KIND == 2) ring += p.tbl_bytes;
+    static_assert((2 * MAX_STAGES + 2) * 8 + 8 <= 192 && 192 + sizeof(Consts) <= 1024, "barriers and constants share the first kilobyte");
+    U8Row *row_terms = reinterpret_cast<U8Row *>(smem + U8_ROWS);  // uint8
+    // (every CTA of a cluster has the same layout, so an offset into this one's receive buffer fits its peers' too; unsplit, the
+    // sums of the CTA itself take the place of its stages, which are free by then)
+    uint8_t *recv = smem + header_bytes(KIND == 2, p.tbl_bytes);
+    int *tbl = reinterpret_cast<int *>(smem + U8_TABLE), *bias = reinterpret_cast<int *>(smem + 192);  // uint8
+    uint8_t *ring = recv + (p.splits > 1 ? (RECV_BYTES + 1023) / 1024 * 1024 : 0);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int S = p.splits, nst = p.stages;
@@ -251,14 +271,16 @@ __global__ void __launch_bounds__(NTHREADS) conv_few_kernel(const __grid_constan
             mbar_init(smem_u32(&empty[s]), 1);
         }
         mbar_init(smem_u32(acc_full), 1);
+        mbar_init(smem_u32(recv_full), 1);
         *abort_flag = 0;
         fence_barrier_init();
         fence_proxy_async_smem();
+        if (S > 1) mbar_arrive_expect_tx(smem_u32(recv_full), min(BM, p.P - m0) * BN * 4);  // what the S CTAs push: the tile's real rows
     }
     if (KIND == 2) {
         // T[class][channel] = b_off * (sum of the channel's weights over the taps inside the image) * c_mult
         const int ncc = 1 + 2 * p.padW, satw = p.kW + 1, satn = (p.kH + 1) * satw;
-        for (int i = tid; i < p.classes * BN; i += NTHREADS) {
+        for (int i = tid; i < p.classes * BN; i += NT) {
             const int k = i / BN, c = min(n0 + i % BN, p.Cout - 1), rc = k / ncc, cc = k - rc * ncc;
             const int r0 = rc <= p.padH ? rc : 0, r1 = rc > p.padH ? p.kH - (rc - p.padH) : p.kH;
             const int s0 = cc <= p.padW ? cc : 0, s1 = cc > p.padW ? p.kW - (cc - p.padW) : p.kW;
@@ -273,12 +295,12 @@ __global__ void __launch_bounds__(NTHREADS) conv_few_kernel(const __grid_constan
         consts.sh[tid] = (p.shift ? __ldg(p.shift + n0 + tid) : 0.f) * self;
         consts.sl[tid] = p.slope ? __ldg(p.slope + n0 + tid) : 0.f;
     }
-    if (warp == 4 && lane == 0) {
+    if (warp == W_A && lane == 0) {
         tma_prefetch_desc(&tmapA);
         if (p.nkb1) tma_prefetch_desc(&tmapA2);
     }
-    if (warp == 5 && lane == 0) tma_prefetch_desc(&tmapW);
-    if (warp == 6) {
+    if (warp == W_B && lane == 0) tma_prefetch_desc(&tmapW);
+    if (warp == W_MMA) {
         tmem_alloc(smem_u32(tmem_slot), BN);
         tmem_relinquish();
     }
@@ -288,155 +310,104 @@ __global__ void __launch_bounds__(NTHREADS) conv_few_kernel(const __grid_constan
     const uint32_t tmem_base = *tmem_slot;
     if (S > 1) cluster_arrive();  // (the wait is ahead of the first store to a peer)
     if (p.pdl) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    // weights are not written by any launch of the forward: their producer does not wait for the kernel before
-    if (p.pdl && warp != 5) asm volatile("griddepcontrol.wait;" ::: "memory");
+    // weights are not written by any launch of the forward: their producer does not wait for the kernel before; the others do once
+    // they have worked out what they need
+    auto launch_wait = [&]() { if (p.pdl) asm volatile("griddepcontrol.wait;" ::: "memory"); };
 
-    uint4 rv[BN / 8];
-    uint2 r8[BN / 8];   // uint8
-    U8Row u8 = {0, 0, -1, 0};
-    const int *trow = tbl;
-    const int row = tid;  // epilogue threads: pixel row of the tile = TMEM lane
-    const int pm = m0 + row;
-    const int wshift = S == 1 ? 6 : S == 2 ? 5 : S == 4 ? 4 : 3, W = 1 << wshift, c_first = n0 + rank * W, cout8 = (p.Cout + 7) & ~7;  // the channels this CTA finishes
-    const int act = p.act_kind == THB_ACT_NONE ? 0 : p.act_kind == THB_ACT_THRESHOLD && p.act_th == 0.f && p.act_val == 0.f ? 1 : 2;
-    bool have = false;
-
-    if (p.prev_status && blockIdx.x == 0 && tid == 0) {
-        const int before = *p.prev_status;
-        if (before) report(p.status, before);
-    }
-    if (warp < 4) {
-        // the residual of this thread's pixel, asked for before the accumulator is awaited
-#pragma unroll
-        for (int j = 0; j < BN / 8; j++) {
-            rv[j] = make_uint4(0, 0, 0, 0);
-            if (KIND != 2 && p.res && pm < p.P && j * 8 < W && c_first + j * 8 < cout8)
-                rv[j] = __ldg(reinterpret_cast<const uint4 *>(p.res + ((size_t)pm * p.res_ld + c_first + j * 8) * 2));
-        }
-        if (KIND == 2) {
-#pragma unroll
-            for (int j = 0; j < BN / 8; j++) {
-                r8[j] = make_uint2(0, 0);
-                if (p.res && pm < p.P && j * 8 < W && c_first + j * 8 < cout8)
-                    r8[j] = __ldg(reinterpret_cast<const uint2 *>(p.res + (size_t)pm * p.res_ld + c_first + j * 8));
-            }
-            const int pc = min(pm, p.P - 1), n = pc / p.oHW, rem = pc - n * p.oHW, oh = rem / p.oW, ow = rem - oh * p.oW;
-            const int ihb = oh * p.dH - p.padH, iwb = ow * p.dW - p.padW;
-            const int r0 = max(0, -ihb), r1 = min(p.kH, p.H - ihb), s0 = max(0, -iwb), s1 = min(p.kW, p.W - iwb);
-            const int cb = p.kH - r1, cr = p.kW - s1;  // (clipped on one side at most: the launcher checks)
-            trow = tbl + ((r0 > 0 ? r0 : cb > 0 ? p.padH + cb : 0) * (1 + 2 * p.padW) + (s0 > 0 ? s0 : cr > 0 ? p.padW + cr : 0)) * BN + rank * W;
-            const int *cs = p.csum + ((size_t)n * p.H + ihb) * p.W + iwb;
-            int xsum = 0;
-            if (p.kH <= 4 && p.kW <= 4) {
-#pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    const int r = i >> 2, q = i & 3;
-                    xsum += r >= r0 && r < r1 && q >= s0 && q < s1 ? __ldg(cs + r * p.W + q) : 0;
+    if (warp >= W_A) {
+        if (warp == W_A) {
+            if (lane == 0) {
+                int iw = 0, ih = 0, in = 0, tap_w = 0, tap_h = 0, slab = 0;
+                if (p.mode == 2) {
+                    in = m0 / p.oHW;
+                    const int rem = m0 - in * p.oHW, oh = rem / p.oW;
+                    ih = oh * p.dH - p.padH;
+                    iw = (rem - oh * p.oW) * p.dW - p.tma_padw;
+                    const int tap = KIND == 2 && p.half ? 2 * kb0 : kb0 / p.slabs;
+                    slab = KIND == 2 && p.half ? 0 : kb0 - tap * p.slabs;
+                    tap_h = tap / p.tma_kw;
+                    tap_w = tap - tap_h * p.tma_kw;
+                } else if (p.a2_mode == 2) {
+                    in = m0 / p.oHW;
+                    const int rem = m0 - in * p.oHW, oh = rem / p.oW;
+                    ih = oh * p.a2_d;
+                    iw = (rem - oh * p.oW) * p.a2_d;
                 }
-            } else
-                for (int r = r0; r < r1; r++)
-                    for (int q = s0; q < s1; q++) xsum += __ldg(cs + r * p.W + q);
-            const int corr = p.a_off * (xsum + p.b_off * (r1 - r0) * (s1 - s0) * p.Cin);
-            u8.shift = max(p.c_shift, 0);
-            u8.rc = (uint32_t)(corr + p.c_off) * (uint32_t)p.c_mult + (p.c_shift >= 1 ? 1u << (p.c_shift - 1) : 0u);
-            u8.tailmask = rem < p.tail_start ? 0 : 255;
-            u8.thr = p.relu_thr;
-        }
-        have = mbar_wait_bounded(smem_u32(acc_full), 0, p.wait_limit);
-        if (!have) {
-            if (lane == 0) report(p.status, 2);
-            *abort_flag = 1;
-        }
-        have = __all_sync(0xffffffffu, have);
-        tc_fence_after();
-    } else if (warp == 4) {
-        if (lane == 0) {
-            int iw = 0, ih = 0, in = 0, tap_w = 0, tap_h = 0, slab = 0;
-            if (p.mode == 2) {
-                in = m0 / p.oHW;
-                const int rem = m0 - in * p.oHW, oh = rem / p.oW;
-                ih = oh * p.dH - p.padH;
-                iw = (rem - oh * p.oW) * p.dW - p.tma_padw;
-                const int tap = KIND == 2 && p.half ? 2 * kb0 : kb0 / p.slabs;
-                slab = KIND == 2 && p.half ? 0 : kb0 - tap * p.slabs;
-                tap_h = tap / p.tma_kw;
-                tap_w = tap - tap_h * p.tma_kw;
-            } else if (p.a2_mode == 2) {
-                in = m0 / p.oHW;
-                const int rem = m0 - in * p.oHW, oh = rem / p.oW;
-                ih = oh * p.a2_d;
-                iw = (rem - oh * p.oW) * p.a2_d;
-            }
-            int s = 0;
-            uint32_t ph = 0;
-            for (int kb = kb0; kb < kb1; kb++) {
-                if (kb - kb0 >= nst && !mbar_wait_bounded(smem_u32(&empty[s]), ph ^ 1, p.wait_limit)) {
-                    report(p.status, 3);
-                    *abort_flag = 1;
-                    break;
-                }
-                if (p.test_withhold && kb == kb1 - 1) break;
-                const uint32_t bar = smem_u32(&full[s]), dst = smem_u32(ring + s * STAGE_BYTES);
-                if (KIND == 2 && p.half) {
-                    const int nh = 2 * kb + 1 < p.ntaps ? 2 : 1;
-                    mbar_arrive_expect_tx(bar, (uint32_t)(nh * (A_BYTES / 2)));
-                    for (int h = 0; h < nh; h++) {
-                        tma_load_im2col_4d(dst + h * (A_BYTES / 2), &tmapA, bar, 0, iw, ih, in, (uint16_t)tap_w, (uint16_t)tap_h);
-                        if (++tap_w == p.tma_kw) { tap_w = 0; tap_h++; }
+                launch_wait();
+                int s = 0;
+                uint32_t ph = 0;
+                for (int kb = kb0; kb < kb1; kb++) {
+                    if (kb - kb0 >= nst && !mbar_wait_bounded(smem_u32(&empty[s]), ph ^ 1, p.wait_limit)) {
+                        report(p.status, 3);
+                        *abort_flag = 1;
+                        break;
+                    }
+                    if (p.test_withhold && kb == kb1 - 1) break;
+                    const uint32_t bar = smem_u32(&full[s]), dst = smem_u32(ring + s * STAGE_BYTES);
+                    if (KIND == 2 && p.half) {
+                        const int nh = 2 * kb + 1 < p.ntaps ? 2 : 1;
+                        mbar_arrive_expect_tx(bar, (uint32_t)(nh * (A_BYTES / 2)));
+                        for (int h = 0; h < nh; h++) {
+                            tma_load_im2col_4d(dst + h * (A_BYTES / 2), &tmapA, bar, 0, iw, ih, in, (uint16_t)tap_w, (uint16_t)tap_h);
+                            if (++tap_w == p.tma_kw) { tap_w = 0; tap_h++; }
+                        }
+                        if (++s == nst) { s = 0; ph ^= 1; }
+                        continue;
+                    }
+                    mbar_arrive_expect_tx(bar, A_BYTES);
+                    if (p.nkb1 && kb >= p.nkb1) {
+                        if (p.a2_mode == 1) tma_load_2d(dst, &tmapA2, bar, (kb - p.nkb1) * KE, m0);
+                        else tma_load_im2col_4d(dst, &tmapA2, bar, (kb - p.nkb1) * KE, iw, ih, in, 0, 0);
+                    } else if (p.mode == 1) {
+                        tma_load_2d(dst, &tmapA, bar, kb * KE, m0);
+                    } else {
+                        tma_load_im2col_4d(dst, &tmapA, bar, slab * KE, iw, ih, in, (uint16_t)tap_w, (uint16_t)tap_h);
+                        if (++slab == p.slabs) {
+                            slab = 0;
+                            if (++tap_w == p.tma_kw) { tap_w = 0; tap_h++; }
+                        }
                     }
                     if (++s == nst) { s = 0; ph ^= 1; }
-                    continue;
                 }
-                mbar_arrive_expect_tx(bar, A_BYTES);
-                if (p.nkb1 && kb >= p.nkb1) {
-                    if (p.a2_mode == 1) tma_load_2d(dst, &tmapA2, bar, (kb - p.nkb1) * KE, m0);
-                    else tma_load_im2col_4d(dst, &tmapA2, bar, (kb - p.nkb1) * KE, iw, ih, in, 0, 0);
-                } else if (p.mode == 1) {
-                    tma_load_2d(dst, &tmapA, bar, kb * KE, m0);
-                } else {
-                    tma_load_im2col_4d(dst, &tmapA, bar, slab * KE, iw, ih, in, (uint16_t)tap_w, (uint16_t)tap_h);
-                    if (++slab == p.slabs) {
-                        slab = 0;
-                        if (++tap_w == p.tma_kw) { tap_w = 0; tap_h++; }
+            }
+            __syncwarp();
+        } else if (warp == W_B) {
+            if (lane == 0) {
+                int s = 0;
+                uint32_t ph = 0;
+                for (int kb = kb0; kb < kb1; kb++) {
+                    if (kb - kb0 >= nst && !mbar_wait_bounded(smem_u32(&empty[s]), ph ^ 1, p.wait_limit)) {
+                        report(p.status, 3);
+                        *abort_flag = 1;
+                        break;
                     }
+                    const uint32_t bar = smem_u32(&full[s]);
+                    const uint32_t dst = smem_u32(ring + s * STAGE_BYTES + A_BYTES);
+                    if (KIND == 2 && p.half) {
+                        const int nh = 2 * kb + 1 < p.ntaps ? 2 : 1;
+                        mbar_arrive_expect_tx(bar, (uint32_t)(nh * (B_BYTES / 2)));
+                        for (int h = 0; h < nh; h++) tma_load_2d(dst + h * (B_BYTES / 2), &tmapW, bar, (2 * kb + h) * (KE / 2), n0);
+                    } else {
+                        mbar_arrive_expect_tx(bar, B_BYTES);
+                        tma_load_2d(dst, &tmapW, bar, kb * KE, n0);
+                    }
+                    if (++s == nst) { s = 0; ph ^= 1; }
                 }
-                if (++s == nst) { s = 0; ph ^= 1; }
             }
-        }
-        __syncwarp();
-    } else if (warp == 5) {
-        if (lane == 0) {
-            int s = 0;
-            uint32_t ph = 0;
-            for (int kb = kb0; kb < kb1; kb++) {
-                if (kb - kb0 >= nst && !mbar_wait_bounded(smem_u32(&empty[s]), ph ^ 1, p.wait_limit)) {
-                    report(p.status, 3);
-                    *abort_flag = 1;
-                    break;
-                }
-                const uint32_t bar = smem_u32(&full[s]);
-                const uint32_t dst = smem_u32(ring + s * STAGE_BYTES + A_BYTES);
-                if (KIND == 2 && p.half) {
-                    const int nh = 2 * kb + 1 < p.ntaps ? 2 : 1;
-                    mbar_arrive_expect_tx(bar, (uint32_t)(nh * (B_BYTES / 2)));
-                    for (int h = 0; h < nh; h++) tma_load_2d(dst + h * (B_BYTES / 2), &tmapW, bar, (2 * kb + h) * (KE / 2), n0);
-                } else {
-                    mbar_arrive_expect_tx(bar, B_BYTES);
-                    tma_load_2d(dst, &tmapW, bar, kb * KE, n0);
-                }
-                if (++s == nst) { s = 0; ph ^= 1; }
-            }
-        }
-        __syncwarp();
-    } else {
-        if (lane == 0) {
+            __syncwarp();
+        } else {
+            // (the whole warp waits and steps, one elected thread issues: addresses stay in uniform registers)
+            const bool leader = elect_one();
+            launch_wait();
             int s = 0;
             uint32_t ph = 0;
             bool alive = true;
             for (int kb = kb0; kb < kb1; kb++) {
-                if (!mbar_wait_bounded(smem_u32(&full[s]), ph, p.wait_limit)) {
-                    report(p.status, 4);
-                    *abort_flag = 1;
+                if (!__all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&full[s]), ph, p.wait_limit))) {
+                    if (leader) {
+                        report(p.status, 4);
+                        *abort_flag = 1;
+                    }
                     alive = false;
                     break;
                 }
@@ -444,138 +415,193 @@ __global__ void __launch_bounds__(NTHREADS) conv_few_kernel(const __grid_constan
                 const uint32_t sa = smem_u32(ring + s * STAGE_BYTES), sb = sa + A_BYTES;
                 if (KIND == 2 && p.half) {
                     const int nh = 2 * kb + 1 < p.ntaps ? 2 : 1;
-                    for (int h = 0; h < nh; h++) {
-                        const uint64_t ad = make_sw64_kmajor_desc(sa + h * (A_BYTES / 2)), bd = make_sw64_kmajor_desc(sb + h * (B_BYTES / 2));
+                    if (leader) {
+                        for (int h = 0; h < nh; h++) {
+                            const uint64_t ad = make_sw64_kmajor_desc(sa + h * (A_BYTES / 2)), bd = make_sw64_kmajor_desc(sb + h * (B_BYTES / 2));
 #pragma unroll
-                        for (int k = 0; k < 2; k++) {
-                            if (KIND == 2) tc_mma_i8(tmem_base, ad + 2 * k, bd + 2 * k, IDESC, ((kb - kb0) | h | k) != 0);
-                            else tc_mma_f16(tmem_base, ad + 2 * k, bd + 2 * k, IDESC, ((kb - kb0) | h | k) != 0);
+                            for (int k = 0; k < 2; k++) {
+                                if (KIND == 2) tc_mma_i8(tmem_base, ad + 2 * k, bd + 2 * k, IDESC, ((kb - kb0) | h | k) != 0);
+                                else tc_mma_f16(tmem_base, ad + 2 * k, bd + 2 * k, IDESC, ((kb - kb0) | h | k) != 0);
+                            }
                         }
                     }
                 } else {
                     const uint64_t ad = make_sw128_kmajor_desc(sa), bd = make_sw128_kmajor_desc(sb);
+                    if (leader) {
 #pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        if (KIND == 2) tc_mma_i8(tmem_base, ad + 2 * k, bd + 2 * k, IDESC, ((kb - kb0) | k) != 0);
-                        else tc_mma_f16(tmem_base, ad + 2 * k, bd + 2 * k, IDESC, ((kb - kb0) | k) != 0);
+                        for (int k = 0; k < 4; k++) {
+                            if (KIND == 2) tc_mma_i8(tmem_base, ad + 2 * k, bd + 2 * k, IDESC, ((kb - kb0) | k) != 0);
+                            else tc_mma_f16(tmem_base, ad + 2 * k, bd + 2 * k, IDESC, ((kb - kb0) | k) != 0);
+                        }
                     }
                 }
-                if (kb + nst < kb1) tc_commit(smem_u32(&empty[s]));
+                if (leader && kb + nst < kb1) tc_commit(smem_u32(&empty[s]));
+                __syncwarp();
                 if (++s == nst) { s = 0; ph ^= 1; }
             }
-            if (alive) tc_commit(smem_u32(acc_full));
-        }
-        __syncwarp();
-    }
-    if (S > 1) {
-        __syncwarp();
-        cluster_wait();  // every CTA of the cluster has started
-        if (have) {
-#pragma unroll
-            for (int half = 0; half < BN; half += 32) {
-                uint32_t a[32];
-                __syncwarp();
-                tmem_ld32(tmem_base + ((uint32_t)(warp * 32) << 16) + half, a);
-                tmem_ld_wait();
-#pragma unroll
-                for (int q = 0; q < 8; q++) {
-                    // columns half + 4q .. + 3 belong to CTA `owner`; slot [rank][column group][row] of its buffer
-                    const int c = half + 4 * q, owner = c >> wshift, g = (c & (W - 1)) >> 2;
-                    const uint32_t at = smem_u32(recv + (size_t)((rank * (W >> 2) + g) * BM + row) * 16);
-                    st_cluster_v4(cluster_addr(at, owner), a[4 * q], a[4 * q + 1], a[4 * q + 2], a[4 * q + 3]);
-                }
-            }
-        }
-        __syncwarp();
-        cluster_arrive();
-        cluster_wait();
-        if constexpr (KIND == 2) {
-            if (have && pm < p.P) {
-                uint32_t rowsum = 0;
-                const int left = p.Cout - c_first, left16 = ((p.Cout + 15) & ~15) - c_first;
-#pragma unroll 1
-                for (int j = 0; j < W / 8 && j * 8 < left16; j++) {
-                    int acc[8];
-#pragma unroll
-                    for (int i = 0; i < 8; i++) acc[i] = 0;
-                    const int4 *part = reinterpret_cast<const int4 *>(recv) + (size_t)(2 * j) * BM + row;
-                    for (int r = 0; r < S; r++, part += (W >> 2) * BM) {
-                        const int4 u = part[0], v = part[BM];
-                        acc[0] += u.x; acc[1] += u.y; acc[2] += u.z; acc[3] += u.w;
-                        acc[4] += v.x; acc[5] += v.y; acc[6] += v.z; acc[7] += v.w;
-                    }
-                    uint2 res = r8[0];
-#pragma unroll
-                    for (int q = 1; q < BN / 16; q++)
-                        if (q == j) res = r8[q];
-                    const uint2 o = finish8_u8(acc, trow + j * 8, bias + rank * W + j * 8, u8, res, left - j * 8, p);
-                    *reinterpret_cast<uint2 *>(p.y + (size_t)pm * p.out_ld + c_first + j * 8) = o;
-                    rowsum = __dp4a(o.x, 0x01010101u, __dp4a(o.y, 0x01010101u, rowsum));
-                }
-                if (p.csum_out && left > 0) atomicAdd(p.csum_out + pm, (int)rowsum);
-            }
-        } else if constexpr (KIND != 2) if (have && pm < p.P) {
-            uint8_t *dst = p.y + ((size_t)pm * p.out_ld + c_first) * 2;
-            const int left = p.Cout - c_first;
-            if (act == 0) finish_parts<KIND, 0>(recv, S, W, rank * W, rv, dst, left, row, consts, p);
-            else if (act == 1) finish_parts<KIND, 1>(recv, S, W, rank * W, rv, dst, left, row, consts, p);
-            else finish_parts<KIND, 2>(recv, S, W, rank * W, rv, dst, left, row, consts, p);
-        }
-    } else if constexpr (KIND == 2) {
-        if (have) {
-            const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16);
-            uint32_t rowsum = 0;
-            const int left = p.Cout - n0, left16 = ((p.Cout + 15) & ~15) - n0;
+            if (alive && leader) tc_commit(smem_u32(acc_full));
             __syncwarp();
-#pragma unroll 1
-            for (int j = 0; j < BN / 8 && j * 8 < left16; j++) {
-                uint32_t a[8];
-                tmem_ld8(taddr + j * 8, a);
-                tmem_ld_wait();
-                int acc[8];
+        }
+        if (S > 1) {
+            cluster_wait();
+            cluster_arrive_relaxed();
+        }
+    } else {
+        // ---- epilogue: the accumulator by way of shared memory to the CTA that finishes its columns, there a thread per row and
+        // eight channels, so that residual and result pass in whole rows (the thread that owns a row used to finish all of its
+        // channels: 3900 cycles of instructions and scattered 16-byte stores against 1600 now) ----
+        const int row = tid & 127, grp = warp >> 2;  // TMEM lane; eight warps: columns 32 grp .. + 31, four: all
+        // this CTA finishes W = 64 / S channels, 1 << cshift items a row
+        const int sshift = S == 1 ? 0 : S == 2 ? 1 : S == 4 ? 2 : 3, wshift = 6 - sshift, W = 1 << wshift, cshift = 3 - sshift;
+        const int c_local = rank * W + (tid & ((1 << cshift) - 1)) * 8, c_first = n0 + c_local, cout8 = (p.Cout + 7) & ~7;
+        const int r0 = tid >> cshift, rows = EPI >> cshift;
+        const int act = p.act_kind == THB_ACT_NONE ? 0 : p.act_kind == THB_ACT_THRESHOLD && p.act_th == 0.f && p.act_val == 0.f ? 1 : 2;
+        launch_wait();
+        if (p.prev_status && blockIdx.x == 0 && tid == 0) {
+            const int before = *p.prev_status;
+            if (before) report(p.status, before);
+        }
+        // the residual of this thread's items, asked for before the accumulator is awaited
+        uint4 rv[4];
+        uint2 r8[32 / EW];   // uint8
+        const uint8_t *res = p.res + ((size_t)m0 * p.res_ld + c_first) * (KIND == 2 ? 1 : 2);
 #pragma unroll
-                for (int i = 0; i < 8; i++) acc[i] = (int)a[i];
-                uint2 res = r8[0];
+        for (int i = 0; i < (KIND == 2 ? 32 / EW : 4); i++) {
+            const int r = r0 + i * rows;
+            const bool real = p.res && !p.y_nchw && r < BM && m0 + r < p.P && c_first < cout8;
+            if (KIND == 2) r8[i] = real ? __ldg(reinterpret_cast<const uint2 *>(res + (size_t)r * p.res_ld)) : make_uint2(0, 0);
+            else rv[i] = real ? __ldg(reinterpret_cast<const uint4 *>(res + (size_t)r * p.res_ld * 2)) : make_uint4(0, 0, 0, 0);
+        }
+        if (KIND == 2 && grp == 0) {
+            const int pc = min(m0 + row, p.P - 1), n = pc / p.oHW, rem = pc - n * p.oHW, oh = rem / p.oW, ow = rem - oh * p.oW;
+            const int ihb = oh * p.dH - p.padH, iwb = ow * p.dW - p.padW;
+            const int w0 = max(0, -ihb), w1 = min(p.kH, p.H - ihb), s0 = max(0, -iwb), s1 = min(p.kW, p.W - iwb);
+            const int cb = p.kH - w1, cr = p.kW - s1;  // (clipped on one side at most: the launcher checks)
+            const int *cs = p.csum + ((size_t)n * p.H + ihb) * p.W + iwb;
+            int xsum = 0;
+            if (p.kH <= 4 && p.kW <= 4) {
 #pragma unroll
-                for (int q = 1; q < BN / 8; q++)
-                    if (q == j) res = r8[q];
-                const uint2 o = finish8_u8(acc, trow + j * 8, bias + j * 8, u8, res, left - j * 8, p);
-                if (pm < p.P) *reinterpret_cast<uint2 *>(p.y + (size_t)pm * p.out_ld + n0 + j * 8) = o;
-                rowsum = __dp4a(o.x, 0x01010101u, __dp4a(o.y, 0x01010101u, rowsum));
+                for (int i = 0; i < 16; i++) {
+                    const int r = i >> 2, q = i & 3;
+                    xsum += r >= w0 && r < w1 && q >= s0 && q < s1 ? __ldg(cs + r * p.W + q) : 0;
+                }
+            } else
+                for (int r = w0; r < w1; r++)
+                    for (int q = s0; q < s1; q++) xsum += __ldg(cs + r * p.W + q);
+            const int corr = p.a_off * (xsum + p.b_off * (w1 - w0) * (s1 - s0) * p.Cin);
+            U8Row t;
+            t.rc = (uint32_t)(corr + p.c_off) * (uint32_t)p.c_mult + (p.c_shift >= 1 ? 1u << (p.c_shift - 1) : 0u);
+            t.trow = ((w0 > 0 ? w0 : cb > 0 ? p.padH + cb : 0) * (1 + 2 * p.padW) + (s0 > 0 ? s0 : cr > 0 ? p.padW + cr : 0)) * BN;
+            if (rem < p.tail_start) t.trow |= (int)0x80000000u;
+            row_terms[row] = t;
+        }
+        bool have = mbar_wait_bounded(smem_u32(acc_full), 0, p.wait_limit);
+        if (!have) {
+            if (lane == 0) report(p.status, 2);
+            *abort_flag = 1;
+        }
+        have = __all_sync(0xffffffffu, have);
+        tc_fence_after();
+        const uint32_t taddr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
+        const bool nchw = KIND != 2 && p.y_nchw;  // (never split)
+        if (nchw) {
+            if constexpr (KIND != 2) if (have) {
+                const int pm = m0 + row, img = pm / p.oHW;
+                const bool real = pm < p.P;
+                float *dst = p.y_nchw + ((size_t)img * p.Cout + n0) * p.oHW + (pm - img * p.oHW);
+                const uint8_t *nres = p.res + ((size_t)pm * p.res_ld + n0) * 2;
+                if (act == 0) finish_nchw<KIND, 0>(taddr, nres, dst, p.oHW, real, p.Cout - n0, consts, grp, EW / 4, p);
+                else if (act == 1) finish_nchw<KIND, 1>(taddr, nres, dst, p.oHW, real, p.Cout - n0, consts, grp, EW / 4, p);
+                else finish_nchw<KIND, 2>(taddr, nres, dst, p.oHW, real, p.Cout - n0, consts, grp, EW / 4, p);
             }
-            if (p.csum_out && pm < p.P) {
-                if (p.n_tiles == 1) p.csum_out[pm] = (int)rowsum;
-                else atomicAdd(p.csum_out + pm, (int)rowsum);  // (the buffer was cleared before the launch)
+        } else {
+            if (S > 1) cluster_wait();  // every CTA of the cluster has started
+            if (have) {
+                uint8_t *at = recv + (size_t)row * 16;
+                const uint32_t bar = smem_u32(recv_full);
+#pragma unroll 1
+                for (int c0 = EW == 8 ? grp * 32 : 0; c0 < (EW == 8 ? grp * 32 + 32 : 64); c0 += 32) {
+                    uint32_t a[32];
+                    tmem_ld32(taddr + c0, a);
+                    tmem_ld_wait();
+                    if (S == 1) {
+#pragma unroll
+                        for (int q = 0; q < 8; q++)
+                            *reinterpret_cast<uint4 *>(at + (c0 / 4 + q) * RECV_ROWS * 16) = make_uint4(a[4 * q], a[4 * q + 1], a[4 * q + 2], a[4 * q + 3]);
+                    } else if (m0 + row < p.P) {
+                        // columns c .. c + 3 belong to CTA c / W; slot [rank][column group][row] of its buffer
+#pragma unroll
+                        for (int q = 0; q < 8; q++) {
+                            const int c = c0 + 4 * q, owner = c >> wshift, g = (c & (W - 1)) >> 2;
+                            st_async_v4(cluster_addr(smem_u32(at + (rank * (W >> 2) + g) * RECV_ROWS * 16), owner), cluster_addr(bar, owner), a[4 * q],
+                                        a[4 * q + 1], a[4 * q + 2], a[4 * q + 3]);
+                        }
+                    }
+                }
+            }
+            __syncwarp();
+            if (S > 1) {
+                cluster_arrive_relaxed();  // (waited for at the end: no CTA leaves while a peer may still write to it)
+                if (have && !mbar_wait_bounded(smem_u32(recv_full), 0, p.wait_limit)) {
+                    report(p.status, 5);
+                    *abort_flag = 1;
+                    have = false;
+                }
+                have = __all_sync(0xffffffffu, have);
+            }
+            if (S == 1 || KIND == 2) epi_bar_sync<EW>();
+            if constexpr (KIND == 2) {
+                if (have) {
+                    const int left = p.Cout - c_first, shift = max(p.c_shift, 0), thr = p.relu_thr;
+                    const bool write = c_first < ((p.Cout + 15) & ~15);
+                    const uint8_t *part = recv + (size_t)(2 * (tid & ((1 << cshift) - 1)) * RECV_ROWS + r0) * 16;
+                    int b[8];
+#pragma unroll
+                    for (int i = 0; i < 8; i++) b[i] = bias[c_local + i];
+#pragma unroll
+                    for (int i = 0; i < 32 / EW; i++) {
+                        const int r = r0 + i * rows, pm = m0 + r;
+                        if (r >= BM) break;  // (the same for a whole warp)
+                        int acc[8];  // (rows beyond the last pixel: whatever lies there, never stored)
+                        sum_parts(part + i * rows * 16, S, (2 << cshift) * RECV_ROWS * 16, acc);
+                        const U8Row t = row_terms[r];
+                        const uint2 o = finish8_u8(acc, tbl + c_local, b, t, shift, thr, r8[i], left, p);
+                        if (write && pm < p.P) *reinterpret_cast<uint2 *>(p.y + (size_t)pm * p.out_ld + c_first) = o;
+                        if (p.csum_out) {
+                            // the lanes of a row add up its bytes
+                            int sum = (int)__dp4a(o.x, 0x01010101u, __dp4a(o.y, 0x01010101u, 0u));
+                            for (int d = 1; d < 1 << cshift; d <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+                            if (pm < p.P && !(tid & ((1 << cshift) - 1))) {
+                                if (p.n_tiles == 1 && S == 1) p.csum_out[pm] = sum;
+                                else atomicAdd(p.csum_out + pm, sum);  // (the buffer was cleared before the launch)
+                            }
+                        }
+                    }
+                }
+            } else {
+                if (have && c_first < cout8) {
+                    const int left = p.Cout - c_first, stride = (2 << cshift) * RECV_ROWS * 16;
+                    const uint8_t *part = recv + (size_t)(2 * (tid & ((1 << cshift) - 1)) * RECV_ROWS + r0) * 16;
+                    uint8_t *dst = p.y + ((size_t)m0 * p.out_ld + c_first) * 2;
+                    const float *sc = consts.sc + c_local, *sh = consts.sh + c_local, *sl = consts.sl + c_local;
+                    if (act == 0) finish_rows<KIND, 0>(part, S, stride, r0, rows, rv, m0, sc, sh, sl, left, res, dst, p);
+                    else if (act == 1) finish_rows<KIND, 1>(part, S, stride, r0, rows, rv, m0, sc, sh, sl, left, res, dst, p);
+                    else finish_rows<KIND, 2>(part, S, stride, r0, rows, rv, m0, sc, sh, sl, left, res, dst, p);
+                }
             }
         }
-    } else if (have && p.y_nchw) {
-        const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16);
-        const bool real = pm < p.P;
-        const int img = pm / p.oHW;
-        float *dst = p.y_nchw + ((size_t)img * p.Cout + n0) * p.oHW + (pm - img * p.oHW);
-        __syncwarp();
-        if (act == 0) finish_nchw<KIND, 0>(taddr, rv, dst, p.oHW, real, p.Cout - n0, consts, p);
-        else if (act == 1) finish_nchw<KIND, 1>(taddr, rv, dst, p.oHW, real, p.Cout - n0, consts, p);
-        else finish_nchw<KIND, 2>(taddr, rv, dst, p.oHW, real, p.Cout - n0, consts, p);
-    } else if (have) {
-        const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16);
-        uint8_t *dst = p.y + ((size_t)pm * p.out_ld + n0) * 2;
-        const bool real = pm < p.P;
-        __syncwarp();
-        if (act == 0) finish_tmem<KIND, 0>(taddr, rv, dst, real, p.Cout - n0, consts, p);
-        else if (act == 1) finish_tmem<KIND, 1>(taddr, rv, dst, real, p.Cout - n0, consts, p);
-        else finish_tmem<KIND, 2>(taddr, rv, dst, real, p.Cout - n0, consts, p);
     }
+    if (S > 1) cluster_wait();
     tc_fence_before();
     __syncthreads();
-    if (*abort_flag && warp == 4 && lane == 0) {
+    if (*abort_flag && warp == W_A && lane == 0) {
         // a wait ran out: copies still on their way must land before the CTA may leave
         const int n = kb1 - kb0 < nst ? kb1 - kb0 : nst;
         for (int s = 0; s < n; s++) mbar_wait_bounded(smem_u32(&full[s]), ((kb1 - kb0 - 1 - s) / nst) & 1, p.wait_limit);
     }
     __syncthreads();
     tc_fence_after();
-    if (warp == 6) tmem_dealloc(tmem_base, BN);
+    if (warp == W_MMA) tmem_dealloc(tmem_base, BN);
 }
 
 // How the activation operand is loaded: 0 not at all (a gather would be needed), else FewParams.mode and its companions.
@@ -631,13 +657,13 @@ bool eligible(const thb_conv_desc *d)
     return mode != 0 && (allowed < 0 || allowed == 2 || mode <= allowed);
 }
 
-template <int KIND>
+template <int KIND, int EW>
 int launch(const CUtensorMap *w, const CUtensorMap *a, const CUtensorMap *a2, const FewParams &p, int ctas, int smem, cudaStream_t st)
 {
     static bool set[64];
     int dev = 0;
     cudaGetDevice(&dev);
-    auto kern = conv_few_kernel<KIND>;
+    const auto kern = conv_few_kernel<KIND, EW>;
     if (dev >= 0 && dev < 64 && !set[dev]) {
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
         if (e != cudaSuccess) return thb_note_launch(e, "conv_few_kernel attributes");
@@ -645,7 +671,7 @@ int launch(const CUtensorMap *w, const CUtensorMap *a, const CUtensorMap *a2, co
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ctas);
-    cfg.blockDim = dim3(NTHREADS);
+    cfg.blockDim = dim3(nthreads(EW));
     cfg.dynamicSmemBytes = (size_t)smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
@@ -670,16 +696,23 @@ int launch(const CUtensorMap *w, const CUtensorMap *a, const CUtensorMap *a2, co
 }  // namespace
 
 // How many CTAs should share the reduction of each tile of this convolution in conv_few_kernel (1: none need to).  Measured, us
-// per launch in a chain of launches (the persistent kernel / no split / split in 2 / 4 / 8):
-//   3x3 512->512 @7x7,  1 image,  8 tiles of 72 K blocks   28.9 / 25.4 / 15.2 / 9.6 / 7.3
-//   3x3 256->256 @14x14, 1 image, 8 tiles of 36            17.0 / 14.4 /  9.8 / 7.1 / 5.7
-//   1x1 1024->256 @14x14, 1 image, 8 tiles of 16           10.0 /  8.0 /  6.5 / 5.2 / 4.8
-//   1x1 256->1024 @14x14, 1 image, 32 tiles of 4            6.3 /  4.7 /  4.9 / 6.1
-//   3x3 256->256 @14x14, 8 images, 52 tiles of 36          17.3 / 15.6 / 11.2 / 9.0 / 15.0
-//   3x3 128->128 @28x28, 8 images, 98 tiles of 18          12.9 / 10.0 /  8.7 / 14.1
-//   1x1 512->128 @28x28, 8 images, 98 tiles of 8            8.9 /  6.5 /  7.0
-// So: eight K blocks or more, at least two of them to a CTA, up to one CTA per SM -- two per SM where four K blocks stay, but
-// not in clusters of eight.
+// per launch in a chain of launches (the persistent kernel / no split / split in 2 / 4 / 8; * the rule's choice):
+//   3x3 512->512 @7x7,  1 image,  8 tiles of 72 K blocks   25.2 / 22.7 / 13.4 / 8.6 / 6.2*
+//   3x3 256->256 @14x14, 1 image, 8 tiles of 36            14.8 / 13.3 /  9.3 / 6.8 / 5.7*
+//   3x3 128->128 @28x28, 1 image, 14 tiles of 18            9.8 /  8.6 /  7.0 / 5.8* / 6.4
+//   1x1 1024->256 @14x14, 1 image, 8 tiles of 16            8.9 /  7.3 /  6.3 / 5.3* / 5.2
+//   1x1 512->2048 @7x7, 1 image, 32 tiles of 8              6.7 /  5.3 /  4.5* / 4.9 / 6.1
+//   1x1 256->1024 @14x14, 1 image, 32 tiles of 4            5.6 /  4.4* / 5.5 / 6.2
+//   3x3 256->256 @14x14, 4 images, 28 tiles of 36          15.1 / 13.6 / 10.1 / 8.8 / 7.6*
+//   3x3 256->256 @14x14, 8 images, 52 tiles of 36          15.2 / 13.7 / 10.6 / 9.3* / 14.0
+//   3x3 512->512 @7x7,  8 images, 32 tiles of 72           25.6 / 23.6 / 15.4 / 11.4 / 9.4*
+//   3x3 128->128 @28x28, 8 images, 98 tiles of 18          11.1 /  9.0 /  8.5* / 13.5
+//   1x1 1024->256 @14x14, 8 images, 52 tiles of 16          9.2 /  7.7 /  7.5* / 7.7
+//   1x1 512->128 @28x28, 8 images, 98 tiles of 8            7.5 /  5.8* / 6.9
+//   uint8 3x3 256->256 @14x14, 1 image, 8 tiles of 18      10.0 / 10.4 /  7.9 / 5.9 / 5.4*
+//   uint8 1x1 2048->512 @7x7, 16 images, 56 tiles of 16     9.7 /  9.5 /  8.9 / 7.7* / 13.2
+// So: four K blocks to a CTA (uint8 two), eight (four) where two CTAs share an SM -- four in clusters of eight, of which there are
+// never more than the SMs hold at once.
 // uint8: the caller says with `splits` (1 included) that this kernel takes the convolution, since it has to clear csum_out when
 // several CTAs add to a pixel's sum; 0 here: it should not.
 extern "C" int thb_conv_few_splits(const thb_conv_desc *d)
@@ -689,22 +722,28 @@ extern "C" int thb_conv_few_splits(const thb_conv_desc *d)
     if (kn.few_tiles == 0 || !eligible(d) || (!u8 && d->Cout_pad % BN)) return !u8;
     const long tiles = tiles_of(d);
     const int nkb = d->Ktot_pad / (u8 ? 128 : 64);
-    if (u8 && tiles > (kn.few_tiles >= 0 ? kn.few_tiles : 4L * kn.sms)) return 0;
+    if (u8 && tiles > (kn.few_tiles >= 0 ? kn.few_tiles : 2L * kn.sms)) return 0;
     int S = 1;
-    while (S < 8 && nkb >= 8 && nkb / (2 * S) >= 2 && tiles * 2 * S <= (S < 4 && nkb / (2 * S) >= 4 ? 2 : 1) * (long)kn.sms) S *= 2;
+    while (S < 8) {
+        const long ctas = tiles * 2 * S;
+        const int part = nkb / (2 * S);  // K blocks left to a CTA
+        if (part < (u8 ? 2 : 4) || ctas > (S == 4 ? 7 * (long)kn.sms / 4 : 2 * (long)kn.sms) || (ctas > kn.sms && part < (u8 || S == 4 ? 4 : 8))) break;
+        S *= 2;
+    }
     return S;
 }
 
-// Does this convolution belong to conv_few_kernel?  A split one does.  Otherwise small CTAs beat the persistent kernel up to
-// about four of them per SM (8 images, tiles / persistent / here: 1x1 512->2048 @7x7, 128: 9.0 / 7.0; 256->1024 @14x14, 208:
-// 7.9 / 5.7; 128->512 @28x28, 392: 8.3 / 6.2; 64->256 @56x56, 784: 9.5 / 11.1), and the patch kernel up to one.
+// Does this convolution belong to conv_few_kernel?  A split one does.  Otherwise small CTAs beat the persistent kernel while all of
+// them are resident, three to an SM (tiles / persistent / here, us: 1x1 512->128 @28x28, 392: 11.1 / 9.7; 3x3 256->256 @14x14, 392:
+// 28.5 / 20.7; 3x3 128->128 @28x28, 454: 18.1 / 22.3; 3x3 256->256 @14x14, 588: 30.1 / 35.5), and the patch kernel up to one.
+// uint8 (thb_conv_few_splits): two to an SM (3x3 256->256 @14x14, 296: 14.1 / 13.9; 256->1024, 400: 9.7 / 11.0).
 extern "C" int thb_conv_few_supported(const thb_conv_desc *d)
 {
     if (d->dtype == THB_U8) return d->splits >= 1 && eligible(d);
     if (!eligible(d) || d->Cout_pad % BN) return 0;
     if (d->splits > 1) return 1;
     const ThbConvLaunch kn = thb_conv_launch_knobs();
-    const long most = kn.few_tiles >= 0 ? kn.few_tiles : (d->kH * d->kW > 1 && thb_conv_patch_supported(d) ? 1 : 4) * (long)kn.sms;
+    const long most = kn.few_tiles >= 0 ? kn.few_tiles : (d->kH * d->kW > 1 && thb_conv_patch_supported(d) ? 1 : 3) * (long)kn.sms;
     return tiles_of(d) <= most;
 }
 
@@ -735,7 +774,7 @@ static int few_fwd(const thb_conv_desc *d, const void *x, void *y, float *y_nchw
         p.relu_val = d->relu_val;
         p.wsat = d->wsat; p.bias_add = d->bias_add; p.csum = d->csum; p.csum_out = d->csum_out;
         p.classes = (1 + 2 * d->padH) * (1 + 2 * d->padW);
-        p.tbl_bytes = (p.classes * BN * 4 + 1023) & ~1023;
+        p.tbl_bytes = p.classes * BN * 4;
         if (d->res) {
             p.ca = (int)d->self_coef; p.cb = (int)d->res_coef;
             if ((p.ca != 1 && p.ca != -1) || (p.cb != 1 && p.cb != -1) || (float)p.ca != d->self_coef || (float)p.cb != d->res_coef) return THB_ERR_UNSUPPORTED;
@@ -782,9 +821,13 @@ static int few_fwd(const thb_conv_desc *d, const void *x, void *y, float *y_nchw
     p.stages = kn.few_stages > 0 ? kn.few_stages : p.splits > 1 || ctas > 2 * kn.sms ? 3 : ctas > kn.sms ? 4 : 5;
     if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
     if (p.stages > per) p.stages = per;
-    const int smem = 1024 + BAR_BYTES + (p.splits > 1 ? RECV_BYTES : 0) + p.tbl_bytes + p.stages * STAGE_BYTES;
+    const int recv = (RECV_BYTES + 1023) / 1024 * 1024, room = p.stages * STAGE_BYTES;
+    const int smem = 1024 + header_bytes(u8, p.tbl_bytes) + (p.splits > 1 ? recv + room : room > recv ? room : recv);
     cudaStream_t st = (cudaStream_t)s;
-    return u8 ? launch<2>(w, a, a2, p, ctas, smem, st) : d->dtype == THB_F16 ? launch<0>(w, a, a2, p, ctas, smem, st) : launch<1>(w, a, a2, p, ctas, smem, st);
+    // eight epilogue warps where one tile's chain is the launch; four where three CTAs share an SM and overlap
+    if (p.splits > 1 || ctas <= 2 * kn.sms)
+        return u8 ? launch<2, 8>(w, a, a2, p, ctas, smem, st) : d->dtype == THB_F16 ? launch<0, 8>(w, a, a2, p, ctas, smem, st) : launch<1, 8>(w, a, a2, p, ctas, smem, st);
+    return u8 ? launch<2, 4>(w, a, a2, p, ctas, smem, st) : d->dtype == THB_F16 ? launch<0, 4>(w, a, a2, p, ctas, smem, st) : launch<1, 4>(w, a, a2, p, ctas, smem, st);
 }
 
 extern "C" int thb_conv_few_fwd(const thb_conv_desc *d, const void *x, void *y, thb_stream s)
