@@ -1555,7 +1555,7 @@ static int sliceable(const instance *I, const step *s)
 }
 
 /* Microseconds that a launch on the whole slice takes beyond LAUNCH_US, roughly: its share of the arithmetic (at 0.62 PFLOP/s in
- * the 16-bit modes, 0.75 in uint8, 36 TFLOP/s in fp32, what the layers of a large batch reach on average) or of the bytes
+ * the 16-bit modes, 0.75 in uint8, 100 TFLOP/s in fp32 on the tensor cores and 36 on the FP32 units, what the layers of a large batch reach on average) or of the bytes
  * (4.5 TB/s), whichever is more.  LAUNCH_US is every launch's fill, drain and partly filled wave (ResNet-18 and -50 on 1 to 256
  * images: within a fifth of 7 us a launch plus this). */
 #define LAUNCH_US 7.0
@@ -1565,7 +1565,7 @@ static double model_us(const step *s)
     double elems = (double)s->out_pixels * s->out_C * 2, us = 0;
     if (s->kind == ST_CONV) {
         const thb_conv_desc *d = &s->conv;
-        const double rate = s->dtype == THB_F32 ? 36e6 : s->dtype == THB_U8 ? 0.75e9 : 0.62e9; /* per microsecond */
+        const double rate = s->dtype == THB_F32 ? (s->w_split ? 100e6 : 36e6) : s->dtype == THB_U8 ? 0.75e9 : 0.62e9; /* per microsecond */
         us = 2.0 * d->N * d->oH * d->oW * (double)d->Cout * d->Cin * d->kH * d->kW / rate;
         elems = (double)d->N * d->H * d->W * d->Cin + elems * (s->nin > 1 ? 1 : 0.5);
     }
