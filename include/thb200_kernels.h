@@ -245,6 +245,11 @@ int thb_postprocess_status(const void *x, int dtype, int N, int H, int W, int C,
 /* ---- pooling: SpatialMaxPooling.c:74-247, SpatialAveragePooling.c:71-207, lowp_SpatialMaxPooling.c ---- */
 int thb_maxpool(int dtype, const void *x, int N, int H, int W, int C, int x_ld, int kH, int kW, int dH, int dW,
                 int padH, int padW, int oH, int oW, void *y, int y_ld, thb_stream s);
+/* the same in uint8, which also leaves per output pixel the sum of its bytes (what thb_u8_channel_sum gives for the next
+ * convolution): windows of 2 x 2 or 3 x 3, a power of two of 16-channel groups up to 32 (thb_maxpool_sums_supported) */
+int thb_maxpool_sums_supported(int C, int kH, int kW, int x_ld, int y_ld);
+int thb_maxpool_sums(int dtype, const void *x, int N, int H, int W, int C, int x_ld, int kH, int kW, int dH, int dW, int padH, int padW,
+                     int oH, int oW, void *y, int y_ld, int *csum, thb_stream s);
 int thb_avgpool(int dtype, const void *x, int N, int H, int W, int C, int x_ld, int kH, int kW, int dH, int dW,
                 int padH, int padW, int oH, int oW, int count_include_pad, void *y, int y_ld, thb_stream s);
 

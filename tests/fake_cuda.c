@@ -132,4 +132,5 @@ NOTHING(thb_conv_make_tmap) NOTHING(thb_conv_maxpool_fwd) NOTHING(thb_conv_nchw_
 NOTHING(thb_gemv_fwd) NOTHING(thb_l2_normalize) NOTHING(thb_logsoftmax) NOTHING(thb_max_unpool) NOTHING(thb_maxpool)
 NOTHING(thb_postprocess_status) NOTHING(thb_preprocess_images) NOTHING(thb_preprocess_images_lowp) NOTHING(thb_preprocess_yuyv)
 NOTHING(thb_reflect_pad) NOTHING(thb_slice_channels) NOTHING(thb_softmax) NOTHING(thb_to_nchw) NOTHING(thb_u8_channel_sum_rows)
+NOTHING(thb_conv_f32_fwd) NOTHING(thb_conv_f32_split_weights) NOTHING(thb_conv_f32_supported) NOTHING(thb_maxpool_sums) NOTHING(thb_maxpool_sums_supported)
 NOTHING(thb_u8_combine) NOTHING(thb_u8_threshold) NOTHING(thb_upsample2x) NOTHING(thb_zero_pad)

@@ -1228,6 +1228,11 @@ static int plan_node(planner *P, int i)
         step_in(s, in); step_out(s, out);
         s->N = in->s.N; s->H = in->s.H; s->W = in->s.W; s->C = in->s.C; s->kH = kH; s->kW = kW; s->dH = n->dH; s->dW = n->dW;
         s->padH = n->padH; s->padW = n->padW; s->oH = os.H; s->oW = os.W; s->flag = n->count_include_pad;
+        if (dtype == THB_U8 && n->op == OP_MAXPOOL && thb_maxpool_sums_supported(in->s.C, kH, kW, in->ld, out->ld)) {
+            /* the pixels' channel sums for the convolution behind it, from the values in hand */
+            s->aux2_buf = new_buf(P, sizeof(int) * (size_t)os.N * os.H * os.W);
+            out->csum_buf = s->aux2_buf + 1;
+        }
         return 0;
     }
     case OP_COMBINE: {
@@ -1897,6 +1902,7 @@ static int exec_step(instance *I, int t, int img0, int cnt)
             s->N = cnt;
             x0 += (size_t)img0 * s->H * s->W * s->in_ld[0] * es;
             y += (size_t)img0 * s->oH * s->oW * s->out_ld * es;
+            aux2_off = sizeof(int) * (size_t)img0 * s->oH * s->oW;
             break;
         case ST_CSUM: {
             const long per = s->pixels / I->slice_n;
@@ -1924,8 +1930,10 @@ static int exec_step(instance *I, int t, int img0, int cnt)
         rc = thb_gemv_fwd(dt, x0, s->N, s->K, s->in_ld[0], s->w, s->M, s->scale, s->shift, &s->act, y, s->out_ld, st);
         break;
     case ST_MAXPOOL:
-        rc = thb_maxpool(dt, x0, s->N, s->H, s->W, s->C, s->in_ld[0], s->kH, s->kW, s->dH, s->dW, s->padH, s->padW, s->oH,
-                         s->oW, y, s->out_ld, st);
+        rc = s->aux2_buf >= 0 ? thb_maxpool_sums(dt, x0, s->N, s->H, s->W, s->C, s->in_ld[0], s->kH, s->kW, s->dH, s->dW, s->padH, s->padW, s->oH, s->oW,
+                                                 y, s->out_ld, (int *)((char *)bufptr(I, s->aux2_buf, 0, THB_U8) + aux2_off), st)
+                              : thb_maxpool(dt, x0, s->N, s->H, s->W, s->C, s->in_ld[0], s->kH, s->kW, s->dH, s->dW, s->padH, s->padW, s->oH, s->oW,
+                                            y, s->out_ld, st);
         break;
     case ST_AVGPOOL:
         rc = thb_avgpool(dt, x0, s->N, s->H, s->W, s->C, s->in_ld[0], s->kH, s->kW, s->dH, s->dW, s->padH, s->padW, s->oH,

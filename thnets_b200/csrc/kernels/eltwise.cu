@@ -644,11 +644,7 @@ __global__ void __launch_bounds__(256) global_avgpool_kernel(const T *x, int HW,
     }
 }
 
-// 3x3 stride-2 max pooling of a 16-bit type, without a conversion and with each input row reduced once: a thread owns one
-// output column of one 8-channel group and walks down a strip of output rows; of the three input rows of a window the
-// first is the last one of the window above, so every step reads two new rows of three pixels, takes their
-// horizontal maxima, and combines them with the carried one.  Neighbouring threads read neighbouring pixels, so the
-// shared column of adjacent windows is served by L1.
+// maxima of 16-byte vectors without a conversion
 template <typename T2> __device__ __forceinline__ uint4 max8(const uint4 &a, const uint4 &b)
 {
     uint4 r;
@@ -663,40 +659,49 @@ template <> __device__ __forceinline__ uint4 max8<U8x4>(const uint4 &a, const ui
 {
     return make_uint4(__vmaxu4(a.x, b.x), __vmaxu4(a.y, b.y), __vmaxu4(a.z, b.z), __vmaxu4(a.w, b.w));
 }
-template <typename T2>
-__global__ void maxpool3s2_kernel(const uint4 *__restrict__ x, int N, int H, int W, int cvecs, int x_ld8, int padH, int padW,
-                                  int oH, int oW, int strip, int nstrips, uint32_t neg_inf2, uint4 *__restrict__ y, int y_ld8)
+// four floats; the comparison of the general kernel, so that NaN and signed zeros come out as there
+template <> __device__ __forceinline__ uint4 max8<float>(const uint4 &a, const uint4 &b)
+{
+    auto m = [](uint32_t p, uint32_t q) { return __uint_as_float(q) > __uint_as_float(p) ? q : p; };
+    return make_uint4(m(a.x, b.x), m(a.y, b.y), m(a.z, b.z), m(a.w, b.w));
+}
+// uint8: the sum of a pixel's bytes (channels beyond the real ones are zero), what the next convolution's zero-point correction
+// needs.  Its vectors lie in `cvecs` neighbouring lanes, a power of two up to 32; all of them call.
+__device__ __forceinline__ void pixel_sum(const uint4 &v, int cvecs, bool write, int *csum)
+{
+    const int lane = threadIdx.x & 31;
+    const uint32_t group = (cvecs == 32 ? 0xffffffffu : (1u << cvecs) - 1u) << (lane & ~(cvecs - 1));
+    int sum = (int)__dp4a(v.w, 0x01010101u, __dp4a(v.z, 0x01010101u, __dp4a(v.y, 0x01010101u, __dp4a(v.x, 0x01010101u, 0u))));
+    for (int d = 1; d < cvecs; d <<= 1) sum += __shfl_xor_sync(group, sum, d);
+    if (write && (lane & (cvecs - 1)) == 0) *csum = sum;
+}
+
+// K x K max pooling, any stride and padding: a thread owns one 16-byte vector of an output pixel, a block a piece of an output
+// row, so that a pixel costs one division; all of its loads are on their way before the first maximum.  HBM-bound.  3x3 stride 2,
+// fp16, 112x112x64: 1 image 6.9 -> 6.4 us, 32 images 16.3 -> 12.4, 256 images 127 -> 104 against threads that walked down strips of
+// rows and carried the row two windows share (uint8: 8.8 -> 6.2, 16.5 -> 11.5, 75 -> 79).  VGG-16's five 2x2 poolings in uint8, 32 images, with the sums of the pooled
+// pixels for the next layers: 77 us (28.6 for the first, 129 MB: 4.5 TB/s) against 119 for the general kernel and 41 for passes of
+// their own over its results.
+template <typename T2, int K>
+__global__ void __launch_bounds__(256) maxpool_kernel(const uint4 *__restrict__ x, int H, int W, int cvecs, int x_ld, int dH, int dW, int padH, int padW,
+                                                      int oH, int oW, uint32_t lowest, uint4 *__restrict__ y, int y_ld, int *csum)
 {
     pdl_enter();
-    const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (long)N * nstrips * oW * cvecs) return;
-    const int cv = (int)(idx % cvecs);
-    long r = idx / cvecs;
-    const int ow = (int)(r % oW);
-    r /= oW;
-    const int st = (int)(r % nstrips);
-    const long n = r / nstrips;
-    const uint4 ninf = make_uint4(neg_inf2, neg_inf2, neg_inf2, neg_inf2);
-    const int iw0 = ow * 2 - padW;
-    const uint4 *img = x + (size_t)n * H * W * x_ld8 + cv;
-    auto hrow = [&](int ih) {
-        uint4 m = ninf;
-        if ((unsigned)ih < (unsigned)H) {
-            const uint4 *row = img + (size_t)ih * W * x_ld8;
+    const int n = blockIdx.x / oH, ih0 = (blockIdx.x - n * oH) * dH - padH;
+    const int it = blockIdx.y * 256 + threadIdx.x, ow = it / cvecs, cv = it - ow * cvecs, iw0 = ow * dW - padW;
+    const bool real = ow < oW;
+    const uint4 *img = x + (size_t)n * H * W * x_ld + cv;
+    uint4 v[K * K], m = make_uint4(lowest, lowest, lowest, lowest);
 #pragma unroll
-            for (int k = 0; k < 3; k++)
-                if ((unsigned)(iw0 + k) < (unsigned)W) m = max8<T2>(m, __ldg(row + (size_t)(iw0 + k) * x_ld8));
-        }
-        return m;
-    };
-    const int oh0 = st * strip, oh1 = min(oH, oh0 + strip);
-    uint4 carried = hrow(oh0 * 2 - padH);
-    uint4 *out = y + ((size_t)n * oH * oW + ow) * y_ld8 + cv;
-    for (int oh = oh0; oh < oh1; oh++) {
-        const uint4 r1 = hrow(oh * 2 - padH + 1), r2 = hrow(oh * 2 - padH + 2);
-        out[(size_t)oh * oW * y_ld8] = max8<T2>(max8<T2>(carried, r1), r2);
-        carried = r2;
+    for (int k = 0; k < K * K; k++) {
+        const int ih = ih0 + k / K, iw = iw0 + k % K;
+        v[k] = real && (unsigned)ih < (unsigned)H && (unsigned)iw < (unsigned)W ? __ldg(img + ((size_t)ih * W + iw) * x_ld) : m;
     }
+#pragma unroll
+    for (int k = 0; k < K * K; k++) m = max8<T2>(m, v[k]);
+    const size_t pix = (size_t)blockIdx.x * oW + ow;
+    if (real) y[pix * y_ld + cv] = m;
+    if (csum) pixel_sum(m, cvecs, real, csum + pix);
 }
 
 // ---- y = act(x*scale[c] + shift[c]) ----------------------------------------------------------------------
@@ -1217,32 +1222,34 @@ int thb_to_nchw(int dtype, const void *x, int N, int H, int W, int C, int x_ld, 
 int thb_maxpool(int dtype, const void *x, int N, int H, int W, int C, int x_ld, int kH, int kW, int dH, int dW, int padH,
                 int padW, int oH, int oW, void *y, int y_ld, thb_stream s)
 {
+    return thb_maxpool_sums(dtype, x, N, H, W, C, x_ld, kH, kW, dH, dW, padH, padW, oH, oW, y, y_ld, 0, s);
+}
+
+int thb_maxpool_sums_supported(int C, int kH, int kW, int x_ld, int y_ld)
+{
+    const int cvecs = (C + 15) / 16;
+    return kH == kW && (kH == 2 || kH == 3) && cvecs <= 32 && !(cvecs & (cvecs - 1)) && x_ld % 16 == 0 && y_ld % 16 == 0;
+}
+
+int thb_maxpool_sums(int dtype, const void *x, int N, int H, int W, int C, int x_ld, int kH, int kW, int dH, int dW, int padH, int padW,
+                     int oH, int oW, void *y, int y_ld, int *csum, thb_stream s)
+{
     const int al = thb_channel_align(dtype);
+    if (csum && (dtype != THB_U8 || !thb_maxpool_sums_supported(C, kH, kW, x_ld, y_ld))) return THB_ERR_UNSUPPORTED;
     const long total = (long)N * oH * oW * ((C + al - 1) / al);
     if (total == 0) return THB_OK;
-    if ((dtype == THB_F16 || dtype == THB_BF16) && kH == 3 && kW == 3 && dH == 2 && dW == 2 && x_ld % 8 == 0 && y_ld % 8 == 0) {
-        const int cvecs = (C + 7) / 8;
-        // strips of output rows: long enough to amortise the carried row, short enough for several waves of CTAs (measured:
-        // strips of 4-7 rows are 7 % faster than 14 on the 112x112 ResNet stem output)
-        int strip = oH;
-        while (strip > 4 && (long)N * ((oH + strip - 1) / strip) * oW * cvecs < 24L * 148 * 256) strip = (strip + 1) / 2;
-        const int nstrips = (oH + strip - 1) / strip;
-        const long items = (long)N * nstrips * oW * cvecs;
-        if (dtype == THB_F16)
-            thb_launch(maxpool3s2_kernel<__half2>, nblocks(items), 256, s, (const uint4 *)x, N, H, W, cvecs, x_ld / 8, padH, padW, oH, oW, strip, nstrips, 0xFC00FC00u, (uint4 *)y, y_ld / 8);
-        else
-            thb_launch(maxpool3s2_kernel<__nv_bfloat162>, nblocks(items), 256, s, (const uint4 *)x, N, H, W, cvecs, x_ld / 8, padH, padW, oH, oW, strip, nstrips, 0xFF80FF80u, (uint4 *)y, y_ld / 8);
-        return THB_LAUNCH_CHECK("maxpool3s2_kernel");
-    }
-    if (dtype == THB_U8 && kH == 3 && kW == 3 && dH == 2 && dW == 2 && x_ld % 16 == 0 && y_ld % 16 == 0) {
-        // the same kernel on 16-channel vectors; the maximum starts from byte 0 as lowp_SpatialMaxPooling.c does
-        const int cvecs = (C + 15) / 16;
-        int strip = oH;
-        while (strip > 4 && (long)N * ((oH + strip - 1) / strip) * oW * cvecs < 24L * 148 * 256) strip = (strip + 1) / 2;
-        const int nstrips = (oH + strip - 1) / strip;
-        const long items = (long)N * nstrips * oW * cvecs;
-        thb_launch(maxpool3s2_kernel<U8x4>, nblocks(items), 256, s, (const uint4 *)x, N, H, W, cvecs, x_ld / 16, padH, padW, oH, oW, strip, nstrips, 0u, (uint4 *)y, y_ld / 16);
-        return THB_LAUNCH_CHECK("maxpool3s2_kernel");
+    const int cvecs = (C + al - 1) / al;
+    const bool vectors = x_ld % al == 0 && y_ld % al == 0 && (((uintptr_t)x | (uintptr_t)y) & 15) == 0;
+    // (uint8: the maximum starts from byte 0 as lowp_SpatialMaxPooling.c does; fp32: from the smallest finite value)
+    const uint32_t lowest = dtype == THB_F16 ? 0xFC00FC00u : dtype == THB_BF16 ? 0xFF80FF80u : dtype == THB_U8 ? 0u : 0xFF7FFFFFu;
+    if (kH == kW && (kH == 2 || kH == 3) && vectors && (long)N * oH <= 0x7fffffffL && ((long)oW * cvecs + 255) / 256 <= 65535) {
+        const dim3 grid((unsigned)(N * oH), (unsigned)((oW * cvecs + 255) / 256));
+#define MAXPOOL_KERNEL(K) \
+    (dtype == THB_F16 ? maxpool_kernel<__half2, K> : dtype == THB_BF16 ? maxpool_kernel<__nv_bfloat162, K> : dtype == THB_U8 ? maxpool_kernel<U8x4, K> : maxpool_kernel<float, K>)
+        const auto kern = kH == 2 ? MAXPOOL_KERNEL(2) : MAXPOOL_KERNEL(3);
+#undef MAXPOOL_KERNEL
+        thb_launch(kern, grid, 256, s, (const uint4 *)x, H, W, cvecs, x_ld / al, dH, dW, padH, padW, oH, oW, lowest, (uint4 *)y, y_ld / al, csum);
+        return THB_LAUNCH_CHECK("maxpool_kernel");
     }
     DISPATCH_ANY_DTYPE(dtype, (thb_launch(pool_kernel<T, true>, nblocks(total), 256, s, (const T *)x, N, H, W, C, x_ld, kH, kW, dH, dW, padH, padW, oH, oW, 0, (T *)y, y_ld)));
     return THB_LAUNCH_CHECK("pool_kernel<max>");
