@@ -144,3 +144,15 @@ def test_bounded_wait(lib, monkeypatch):
         monkeypatch.undo()
         lib.thb_conv_reload_knobs()
     assert np.array_equal(c.run(2), good)
+
+
+def test_cold_activations(lib):
+    """Activations from memory, of which some K blocks arrive late and out of order: every launch gives the same bits."""
+    rng = np.random.default_rng(3)
+    x = rng.standard_normal((16, 1024, 14, 14)).astype(np.float32)
+    c = Split(lib, x, (rng.standard_normal((256, 1024, 1, 1)) / 32).astype(np.float32), 1, 0)
+    big = torch.empty(160 << 20, dtype=torch.uint8, device="cuda")
+    first = c.run(0)
+    for i in range(60):
+        big.fill_(i)
+        assert np.array_equal(c.run(0), first), i

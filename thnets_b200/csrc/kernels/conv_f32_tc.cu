@@ -40,7 +40,10 @@ constexpr int RECV_ROWS = BM + 1;  // (padded: a warp's reads of several column 
 // NT = 1 (layers of 64 channels): two CTAs to an SM, each half of the tensor memory.  GATHER: the activations do not come by TMA.
 template <int NT, bool GATHER> struct Cfg {
     static constexpr int BN = 64 * NT, BPART = BN * BK * 2, B_BYTES = 3 * BPART;
-    static constexpr int RA = NT == 2 && !GATHER ? 5 : 4;  // stages of raw activations (gather: two a group)
+    // Stages of raw activations (gather: two a group), an even number: a stage then belongs to one of the two splitting groups, which
+    // sees every phase of its barrier.  With an odd one a group sees every other phase, all of one parity, and passes a stage whose
+    // copy for the OTHER group has not landed yet (copies land out of order: a later one had).
+    static constexpr int RA = 4;
     // Stages of weight parts, an even number: a barrier of the ring then serves the K blocks of one parity only, and the other
     // parity's multiplies cannot carry it a phase further than someone still waits for.
     static constexpr int RB = NT == 2 ? 6 : 4;
@@ -50,7 +53,7 @@ template <int NT, bool GATHER> struct Cfg {
     static constexpr int RECV_BYTES = (BN / 4) * RECV_ROWS * 16;
     static constexpr int SMEM = 1024 + RA * A_BYTES + RB * B_BYTES;
     static_assert(RECV_BYTES <= RB * B_BYTES, "the partial sums take the place of the weight stages");
-    static_assert(RB % 2 == 0 && RB >= NA && SMEM <= 227 * 1024, "stages");
+    static_assert(RA % 2 == 0 && RB % 2 == 0 && RB >= NA && SMEM <= 227 * 1024, "stages");
     static_assert(NT == 2 || (2 * (SMEM + 1024) <= 228 * 1024 && 3 * (SMEM + 1024) > 228 * 1024), "two CTAs to an SM, not three");
     static_assert(A_COL + 64 * NA <= TMEM_COLS, "tensor memory");
 };
