@@ -156,3 +156,28 @@ def test_cold_activations(lib):
     for i in range(60):
         big.fill_(i)
         assert np.array_equal(c.run(0), first), i
+
+
+@pytest.mark.parametrize("cin,h,w,cout,k,s,p", [(3, 67, 67, 128, 11, 4, 2), (128, 43, 3, 256, 1, 1, 0), (64, 9, 9, 128, 3, 1, 1), (64, 9, 9, 200, 5, 1, 2)])
+def test_half_tiles(lib, cin, h, w, cout, k, s, p):
+    """Layers of 128 channels a tile: few tiles go to CTAs of 64 channels, which read halves of the weights' stages.  The K blocks and
+    their order are the same, so an image gives the same bits in a launch of either kind."""
+    rng = np.random.default_rng(cout + k)
+    x = rng.standard_normal((1, cin, h, w)).astype(np.float32)
+    wt = (rng.standard_normal((cout, cin, k, k)) * (cin * k * k) ** -0.5).astype(np.float32)
+    one = Split(lib, x, wt, s, p)
+    d = one.conv.d
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    tiles = -(-d.oH * d.oW // 128) * (d.Cout_pad // 64)
+    assert d.Cout_pad % 128 == 0 and tiles * 16 <= sms
+    n = -(-(sms + 1) * 64 * 128 // (d.Cout_pad * d.oH * d.oW)) + 1
+    many = Split(lib, np.repeat(x, n, 0), wt, s, p)
+    ref = double(x, wt, s, p)
+    err = lambda y: np.linalg.norm(y - ref) / np.linalg.norm(ref)  # noqa: E731
+    # the bound of test_tiles_and_splits: 1.2e-7, and for long reductions (each K block is one more rounded addition) the FFMA chain's
+    bound = max(err(one.ffma()), 1.2e-7)
+    for splits in (1, 2, 4, 8):
+        y = one.run(splits, pad=4)
+        assert err(y) <= bound, splits
+        wide = many.run(splits)
+        assert np.array_equal(wide[:1], y) and np.array_equal(wide[-1:], y), splits

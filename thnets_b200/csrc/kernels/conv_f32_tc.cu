@@ -36,8 +36,8 @@ constexpr int BM = 128, BK = 32;
 constexpr int A_BYTES = BM * BK * 4;
 constexpr int RECV_ROWS = BM + 1;  // (padded: a warp's reads of several column groups meet in no bank)
 
-// A tile is 128 pixels x 64 NT channels.  NT = 2: one CTA to an SM, a multiply of 128 columns takes hardly longer than one of 64.
-// NT = 1 (layers of 64 channels): two CTAs to an SM, each half of the tensor memory.  GATHER: the activations do not come by TMA.
+// A tile is 128 pixels x 64 NT channels.  NT = 2: one CTA to an SM, a multiply of 128 columns takes little longer than one of 64.
+// NT = 1 (layers of 64 channels, launches of few tiles): two CTAs to an SM, each half of the tensor memory.  GATHER: the activations do not come by TMA.
 template <int NT, bool GATHER> struct Cfg {
     static constexpr int BN = 64 * NT, BPART = BN * BK * 2, B_BYTES = 3 * BPART;
     // Stages of raw activations (gather: two a group), an even number: a stage then belongs to one of the two splitting groups, which
@@ -70,6 +70,7 @@ struct F32Params {
     float act_th, act_val, act_alpha;
     int mode, slabs;   // 0: gathered; 1: activations are a plain matrix; 2: im2col-mode copies, `slabs` slabs of 32 channels per tap
     int splits, pdl, test_withhold;
+    int halves;        // NT = 1 on weights laid out for 128 channels: a tile's parts are halves of theirs
     const uint8_t *parts;  // the weights' parts, one stage after another: [column tile][K block][part][64 rows of 64 bytes, swizzled]
     int *status;
     long long wait_limit;
@@ -345,7 +346,10 @@ __global__ void __launch_bounds__(Cfg<NT, GATHER>::NTHREADS, 3 - NT) conv_f32_ke
             __syncwarp();
         } else if (warp == W_B) {
             if (lane == 0) {
-                const uint8_t *src = p.parts + ((size_t)(tile % p.n_tiles) * p.nkb + kb0) * B_BYTES;
+                const int ct = tile % p.n_tiles;
+                const bool halves = NT == 1 && p.halves;
+                const uint8_t *src = halves ? p.parts + ((size_t)(ct >> 1) * p.nkb + kb0) * (2 * B_BYTES) + (ct & 1) * BPART
+                                            : p.parts + ((size_t)ct * p.nkb + kb0) * B_BYTES;
                 int s = 0;
                 uint32_t ph = 0;
                 for (int i = 0; i < nkb; i++) {
@@ -355,7 +359,10 @@ __global__ void __launch_bounds__(Cfg<NT, GATHER>::NTHREADS, 3 - NT) conv_f32_ke
                     }
                     const uint32_t bar = smem_u32(&go[s]), dst = smem_u32(ringB + s * B_BYTES);
                     mbar_arrive_expect_tx(bar, B_BYTES);
-                    bulk_load(dst, src + (size_t)i * B_BYTES, B_BYTES, bar);
+                    if (halves)
+                        for (int part = 0; part < 3; part++) bulk_load(dst + part * BPART, src + (size_t)i * (2 * B_BYTES) + part * (2 * BPART), BPART, bar);
+                    else
+                        bulk_load(dst, src + (size_t)i * B_BYTES, B_BYTES, bar);
                     issued[1] = i + 1;
                     if (++s == RB) { s = 0; ph ^= 1; }
                 }
@@ -549,10 +556,21 @@ int operand_mode(const thb_conv_desc *d)
 
 int k_blocks(const thb_conv_desc *d) { return (d->Ktot_pad + BK - 1) / BK; }
 
-// Channels of a tile (a property of the layer, not of the batch: the weights are laid out by it).  Reductions of fewer than four K
+// Channels of a tile as the weights are laid out (a property of the layer, not of the batch).  Reductions of fewer than four K
 // blocks are mostly prologue and epilogue, which two small CTAs on an SM overlap: 1x1 64->256 @56x56, 16 images 45 -> 37 us, 64->512
 // @28x28 25 -> 20; from 128 channels on it is even (128->512: 25.5 / 25.5), 3x3 128->128 of 64 images 95 -> 70 with 128.
 int tile_n(const thb_conv_desc *d) { return d->Cout_pad % 128 == 0 && k_blocks(d) >= 4 ? 128 : 64; }
+
+// Channels of a launch's tiles.  Where CTAs of 64 channels, as many parts a tile, take half of the SMs at most, a CTA takes half of a
+// tile the weights are laid out for: a K block's multiplies take 540 cycles instead of 768, and beside its 113 KB of shared memory and
+// half of the tensor memory the next launch of the chain sets itself up.  us of kernels, tiles of 128 / this / 64 up to all SMs:
+// AlexNet, 1 image 117 / 115 / 112, 2 images 133 / 133 / 142; ResNet-50, 1 image 579 / 566 / 557, 4 images 658 / 658 / 668; ResNet-18,
+// 3 images 267 / 263 / 276.
+int launch_n(const thb_conv_desc *d, int splits, long sms)
+{
+    const long tiles = ((long)d->N * d->oH * d->oW + BM - 1) / BM * (d->Cout_pad / 64);
+    return tile_n(d) == 128 && tiles * splits * 2 > sms ? 128 : 64;
+}
 
 template <int NT, bool GATHER> int launch(const CUtensorMap *a, const F32Params &p, cudaStream_t st)
 {
@@ -609,7 +627,9 @@ extern "C" int thb_conv_f32_split_weights(const thb_conv_desc *d, void *w_split,
     return THB_LAUNCH_CHECK("split_weights_kernel");
 }
 
-// The reduction split while that leaves at most one CTA of 128 columns or two of 64 to an SM and at least four K blocks to a CTA.
+// The reduction split while that leaves at most one CTA to an SM and at least four K blocks to a CTA; tiles of 64 channels (two CTAs fit
+// an SM) once more where at least eight are left.  (Split on to two CTAs an SM at four K blocks each, us of kernels before / now:
+// AlexNet, 2 images 137 / 133; ResNet-18, 3 images 292 / 263; ResNet-50, 3 images 634 / 604.  Never on to two: AlexNet, 8 images 232.)
 // Measured, us in 1 / 2 / 4 / 8 parts (* the rule's choice; before: the FFMA kernel's own rule) and the relative error (2-norm,
 // against double precision) of the choice / of the FFMA kernel:
 //   7x7/2 3->64 @225x225, 9 images            52*                      before  85    7.5e-8 / 1.5e-7
@@ -620,7 +640,7 @@ extern "C" int thb_conv_f32_split_weights(const thb_conv_desc *d, void *w_split,
 //   1x1/2 64->128 @57x57, 9 images           6.4* / 7.9                before  9.5   6.0e-8 / 8.0e-8
 //   1x1 64->256 @56x56, 16 images             37* / 75                 before  48    6.4e-8 / 1.4e-7
 //   1x1 256->1024 @14x14, 16 images           21* / 28                 before  53    8.0e-8 / 2.9e-7
-//   11x11/4 3->64 @224x224, 1 image           18 / 14 / 12 / 12*       before  12    8.3e-8 / 1.1e-7
+//   11x11/4 3->64 @224x224, 1 image           18 / 14 / 12* / 12       before  12    8.3e-8 / 1.1e-7
 //   5x5 64->192 @27x27, 1 image               29 / 18 / 13 / 13*       before  27    9.4e-8 / 2.0e-7
 //   3x3 384->256 @13x13, 1 image              53 / 31 / 20 / 15*       before  17    1.1e-7 / 2.7e-7
 //   3x3 512->512 @7x7, 1 image                67 / 38 / 23 / 16*       before  20    1.1e-7 / 2.3e-7
@@ -631,8 +651,7 @@ extern "C" int thb_conv_f32_splits(const thb_conv_desc *d)
     const long sms = thb_conv_launch_knobs().sms, tiles = ((long)d->N * d->oH * d->oW + BM - 1) / BM * (d->Cout_pad / tile_n(d));
     const int nkb = k_blocks(d);
     int S = 1;
-    const long most = (tile_n(d) == 128 ? 1 : 2) * sms;
-    while (S < 8 && tiles * 2 * S <= most && nkb >= 4 * S) S *= 2;
+    while (S < 8 && (tiles * 2 * S <= sms ? nkb >= 4 * S : tile_n(d) == 64 && tiles * S <= sms && nkb >= 16 * S)) S *= 2;
     return S;
 }
 
@@ -648,7 +667,7 @@ extern "C" int thb_conv_f32_fwd(const thb_conv_desc *d, const void *w_split, con
     p.H = d->H; p.W = d->W; p.in_ld = d->in_ld; p.oW = d->oW; p.oHW = d->oH * d->oW;
     p.dH = d->dH; p.dW = d->dW; p.padH = d->padH; p.padW = d->padW; p.kW = d->kW;
     p.Cout = d->Cout; p.Cout_pad = d->Cout_pad; p.out_ld = d->out_ld;
-    p.n_kchunks = d->Ktot_pad / 4; p.nkb = k_blocks(d); p.n_tiles = d->Cout_pad / tile_n(d);
+    p.n_kchunks = d->Ktot_pad / 4; p.nkb = k_blocks(d);
     p.scale = d->scale; p.shift = d->shift; p.slope = d->act.kind == THB_ACT_PRELU ? d->act.slope : nullptr;
     p.res = (const float *)d->res; p.res_ld = d->res_ld; p.self_coef = d->self_coef; p.res_coef = d->res_coef;
     p.act_kind = d->act.kind; p.act_th = d->act.threshold; p.act_val = d->act.value; p.act_alpha = d->act.alpha;
@@ -661,11 +680,14 @@ extern "C" int thb_conv_f32_fwd(const thb_conv_desc *d, const void *w_split, con
     p.splits = d->splits > 0 ? d->splits : thb_conv_f32_splits(d);
     if (p.splits != 1 && p.splits != 2 && p.splits != 4 && p.splits != 8) return THB_ERR_ARG;
     while (p.splits > p.nkb) p.splits /= 2;
+    const int bn = launch_n(d, p.splits, kn.sms);
+    p.n_tiles = d->Cout_pad / bn;
+    p.halves = bn < tile_n(d);
     p.parts = (const uint8_t *)w_split;
     static const CUtensorMap none = {};
     const CUtensorMap *a = p.mode ? thb_activation_tmap(d, x, p.mode) : &none;
     if (!a) return thb_note_launch(cudaErrorUnknown, "conv_f32: tensor map");
     const cudaStream_t st = (cudaStream_t)s;
-    if (tile_n(d) == 128) return p.mode ? launch<2, false>(a, p, st) : launch<2, true>(a, p, st);
+    if (bn == 128) return p.mode ? launch<2, false>(a, p, st) : launch<2, true>(a, p, st);
     return p.mode ? launch<1, false>(a, p, st) : launch<1, true>(a, p, st);
 }
