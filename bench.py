@@ -379,7 +379,7 @@ def measure(arm, steps, warmup, world, barrier, max_over_ranks, peaks):
         peak = peaks["tflops_burst"] * (2 if u8 else 1)
         ach = conv_fl / (conv_ms * 1e-3) / 1e12 if conv_ms > 0 else 0.0
         roof = {"bound": "tensor",
-                "kernel": "conv_simt_kernel" if arm.dtype == "fp32" else "conv_tc_kernel" if u8 else "conv_tc_kernel + conv_patch_tc_kernel",
+                "kernel": "conv_f32_kernel" if arm.dtype == "fp32" else "conv_tc_kernel" if u8 else "conv_tc_kernel + conv_patch_tc_kernel",
                 "achieved": ach, "peak": peak, "unit": "TFLOP/s" if not u8 else "TOP/s", "frac": ach / peak,
                 "peak_source": "of " + peaks["src"] + (": bf16_tflops (burst)" if not u8 else ": 2 x bf16_tflops (burst)"),
                 "frac_of_sustained_peak": ach / (peaks["tflops"] * (2 if u8 else 1)),

@@ -13,10 +13,10 @@
 // all taps stay resident in shared memory for the whole launch.  Per patch: one copy, one barrier round, and
 // kH*kW*(pixel bytes / 32) back-to-back tcgen05.mma per accumulator.
 //
-// Epilogue (8 warps, one thread per patch row): TMEM -> scale/shift/activation -> a 128-byte row of a shared-memory
-// tile, then either a 4-D TMA store of the CR x CC outputs, or -- when a stride-2 max pooling follows
-// (modules/SpatialMaxPooling.c:168-247) -- the patch holds whole pooling windows (CR = 2(PR-1)+kp), the 256 epilogue
-// threads pool it on chip with windows clipped to the image as the reference clips them, and only the PR x PC pooled
+// Epilogue (16 warps on a patch; with pooling groups of eight, a patch each; one thread per patch row and half or all of its
+// channels): TMEM -> scale/shift/activation -> a 128-byte row of a shared-memory tile, then either a 4-D TMA store of the
+// CR x CC outputs, or -- when a stride-2 max pooling follows (modules/SpatialMaxPooling.c:168-247) -- the patch holds
+// whole pooling windows (CR = 2(PR-1)+kp), the group's threads pool it on chip with windows clipped to the image as the reference clips them, and only the PR x PC pooled
 // tile is stored: the convolution's own output never reaches global memory.
 // Every wait is bounded; a wait that runs out records a code in *status and the CTA drains and exits.
 #include "common.cuh"

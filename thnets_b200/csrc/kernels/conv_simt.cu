@@ -1,4 +1,5 @@
-// fp32 implicit-GEMM convolution with exact FFMA accumulation (the fp32 mode's 1e-4 parity path).
+// fp32 implicit-GEMM convolution by chains of FFMA: for layers that conv_f32_tc.cu does not take (few products a sum, channel counts
+// that neither its copies nor its gather fit), and for callers that hold no split copy of the weights.
 //
 // D[pixel][cout] = sum_k A[pixel][k] * Wk[k][cout], k = tap*Cin_pad + c over NHWC fp32 activations.
 //
