@@ -66,20 +66,26 @@ CASES = [  # n, cin, h, w, cout, k, stride, pad
 ]
 
 
+def error(y, ref):
+    return np.linalg.norm(y - ref) / np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("relu", [False, True], ids=["signed", "relu"])
 @pytest.mark.parametrize("case", CASES)
-def test_tiles_and_splits(lib, case):
+def test_tiles_and_splits(lib, case, relu):
     n, cin, h, w, cout, k, s, p = case
     rng = np.random.default_rng(cin + k)
     x = rng.standard_normal((n, cin, h, w)).astype(np.float32)
+    if relu:
+        x = np.maximum(x, 0)
     wt = (rng.standard_normal((cout, cin, k, k)) * (cin * k * k) ** -0.5).astype(np.float32)
     ref = double(x, wt, s, p)
     c = Split(lib, x, wt, s, p)
-    err = lambda y: np.linalg.norm(y - ref) / np.linalg.norm(ref)  # noqa: E731
-    before = err(c.ffma())
+    before = error(c.ffma(), ref)
     for splits in (0, 1, 2, 4, 8):
         y = c.run(splits, pad=4)
-        # half an ulp of a result (3e-8 of it on average), and what a truncated sum of 32 loses on the way (4e-8)
-        assert err(y) <= max(before, 1.2e-7), splits
+        # never further from the exact result than the FFMA kernel: measured 6.0e-8 to 2.3e-7 against 7.8e-8 to 4.3e-7
+        assert error(y, ref) <= before, splits
         assert G.rel_err(y, ref) < 1e-6, splits
         assert np.array_equal(y, c.run(splits)), splits
     # residual, scale, shift and the activations
@@ -99,7 +105,7 @@ def test_tiles_and_splits(lib, case):
 
 
 def test_values_the_parts_cannot_hold(lib):
-    """Infinities, NaN and values near the end of fp32's range come out as the FFMA kernel has them; small values keep their bits."""
+    """Infinities, NaN and values near the end of fp32's range come out as the FFMA kernel has them."""
     rng = np.random.default_rng(5)
     x = rng.standard_normal((1, 64, 12, 12)).astype(np.float32)
     wt = (rng.standard_normal((64, 64, 3, 3)) * 0.1).astype(np.float32)
@@ -118,8 +124,71 @@ def test_values_the_parts_cannot_hold(lib):
         assert np.array_equal(a[same], b[same])
         fin = np.isfinite(a)
         assert np.abs(a[fin] / b[fin] - 1).max() < 1e-3 and G.rel_err(b[fin], a[fin]) < 1e-6
-    tiny = Split(lib, (x := rng.standard_normal((1, 64, 12, 12)).astype(np.float32) * 1e-30), wt, 1, 1)
-    assert G.rel_err(tiny.run(1), double(x, wt, 1, 1)) < 1e-6
+
+
+SHAPES = [(1, 64, 12, 12, 64, 3, 1, 1), (1, 128, 9, 9, 128, 1, 1, 0), (1, 3, 20, 20, 128, 7, 2, 3)]  # im2col, matrix (wide tiles), gathered
+SCALES = [(1e-20, 1), (1e-30, 1), (1e-33, 1), (1e-35, 1), (1e-37, 1), (1e-40, 1), (1e-43, 1), (1, 1e-30), (1, 1e-35), (1, 1e-37), (1, 1e-41),
+          (1e-20, 1e-15), (1e-20, 1e-19), (1e10, 1e-40), (1e25, 1e-37), (1e-37, 1e20), (1e30, 1e-33), (1e-38, 1e37), (1e30, 1e-43)]
+
+
+def no_worse(c, ref, shape):
+    """Every split's result is as near to the exact one as the FFMA kernel's, but for the last bits of fp32's smallest numbers: a product
+    and its addition round by half of 2^-149, once for each of the K products and once more for each of their sums of 32."""
+    _, cin, _, _, _, k, _, _ = shape
+    before, quantum = error(c.ffma(), ref), 2.0 ** -150 * cin * k * k * 33 / 32
+    for splits in (0, 1, 2, 8):
+        y = c.run(splits)
+        small = np.abs(ref) < 2.0 ** -110
+        assert not small.any() or (np.abs(y - ref) <= 1e-6 * np.abs(ref).max() + quantum)[small].all(), splits
+        assert np.abs(ref).max() < 2.0 ** -110 or error(y, ref) <= before, splits
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("xs,ws", SCALES)
+def test_magnitudes(lib, shape, xs, ws):
+    """Values of any size keep their bits, down to where bf16 has none left."""
+    n, cin, h, w, cout, k, s, p = shape
+    rng = np.random.default_rng(cin)
+    x = (rng.standard_normal((n, cin, h, w)) * xs).astype(np.float32)
+    wt = (rng.standard_normal((cout, cin, k, k)) * 0.1 * ws).astype(np.float32)
+    c = Split(lib, x, wt, s, p)
+    no_worse(c, double(x, wt, s, p), shape)
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_mixed_magnitudes(lib, shape):
+    """Tiny values beside large ones: in a row of activations, in a channel of weights, between the channels; sums that are zero."""
+    n, cin, h, w, cout, k, s, p = shape
+    rng = np.random.default_rng(cin + 1)
+    x0 = rng.standard_normal((n, cin, h, w)).astype(np.float32)
+    w0 = (rng.standard_normal((cout, cin, k, k)) * 0.1).astype(np.float32)
+    zeros = np.zeros_like(x0)
+    zeros[:, cin // 2, h // 2, w // 2] = 1e-42    # alone: a row whose every product vanishes
+    zeros[:, cin // 2, 0, 0] = 1e-36
+    c = Split(lib, zeros, w0, s, p)
+    no_worse(c, double(zeros, w0, s, p), shape)
+    wide = w0 * np.float32(1e-37)
+    wide[:, 0] = 1                                # the channels' largest weights meet zeros
+    wide[1::2] *= np.float32(1e-3)
+    for xs in (1, 1e20, 1e37):
+        x = x0 * np.float32(xs)
+        x[:, 0] = 0
+        c = Split(lib, x, wide, s, p)
+        no_worse(c, double(x, wide, s, p), shape)
+    apart = w0 * (10.0 ** rng.uniform(-44, 10, (cout, 1, 1, 1)))  # channels of all sizes, one of them zero
+    apart[3] = 0
+    apart = apart.astype(np.float32)
+    c = Split(lib, x0, apart, s, p)
+    ref, rounding = double(x0, apart, s, p), 2.0 ** -150 * cin * k * k * 33 / 32
+    scale = (10.0 ** rng.uniform(-40, 3, cout)).astype(np.float32)
+    for sc in (np.ones(cout, np.float32), scale):
+        c.conv.set_affine(sc, None)
+        want, before = ref * sc[None, :, None, None], c.ffma()
+        for splits in (1, 2, 8):
+            y = c.run(splits)
+            for o in range(cout):
+                bound = 1e-6 * np.abs(want[:, o]).max() + rounding * sc[o] + 2.0 ** -150
+                assert np.abs(y[:, o] - want[:, o]).max() <= max(np.abs(before[:, o] - want[:, o]).max(), bound), (splits, o)
 
 
 def test_bounded_wait(lib, monkeypatch):
@@ -173,11 +242,9 @@ def test_half_tiles(lib, cin, h, w, cout, k, s, p):
     n = -(-(sms + 1) * 64 * 128 // (d.Cout_pad * d.oH * d.oW)) + 1
     many = Split(lib, np.repeat(x, n, 0), wt, s, p)
     ref = double(x, wt, s, p)
-    err = lambda y: np.linalg.norm(y - ref) / np.linalg.norm(ref)  # noqa: E731
-    # the bound of test_tiles_and_splits: 1.2e-7, and for long reductions (each K block is one more rounded addition) the FFMA chain's
-    bound = max(err(one.ffma()), 1.2e-7)
+    bound = error(one.ffma(), ref)
     for splits in (1, 2, 4, 8):
         y = one.run(splits, pad=4)
-        assert err(y) <= bound, splits
+        assert error(y, ref) <= bound, splits
         wide = many.run(splits)
         assert np.array_equal(wide[:1], y) and np.array_equal(wide[-1:], y), splits

@@ -1,7 +1,8 @@
 // fp32 convolution on the tensor cores: every operand as three bf16 parts, partial sums added in fp32.
 //
-// An fp32 value is b1 + b2 + b3 exactly, each part the bf16 nearest to what the parts before leave (8 + 8 + 8 bits).  A product is
-// then nine bf16 products, exact in fp32; the three of them below 2^-24 of it are left out:
+// An fp32 value of 2^-110 or more is b1 + b2 + b3 exactly, each part the bf16 nearest to what the parts before leave (8 + 8 + 8 bits);
+// a smaller one up to 2^-134, half of the smallest bf16.  A product is then nine bf16 products, exact in fp32; the three of them
+// below 2^-24 of it are left out:
 //     x w = x1 w1 + (x1 w2 + x2 w1) + (x2 w2 + x1 w3 + x3 w1) + O(2^-25).
 // The tensor core truncates its sums, so it never adds for long: the products of one K block of 32, smallest first, go to a fresh
 // accumulator, and the running sums are kept in registers, fp32 additions rounded to nearest.  The result is nearer to a double-
@@ -21,8 +22,15 @@
 // owner as in conv_few_tc.cu.  The result passes through shared memory, so that global memory is read (residual) and written in
 // rows of 16-byte chunks.
 //
-// A sum that is not finite may be one that the parts have spoilt (infinity times a zero part, a value that rounds to an infinite
-// part): those outputs are computed again, as the FFMA kernel would, from the fp32 weights.
+// The parts are those of weights times a power of two, one for each channel (weight_units_kernel): no fp32 weight loses a bit then, and
+// the sums stay far from the ends of the range.  Some sums the parts may spoil all the same; those outputs are computed again by FFMA
+// from the fp32 weights (exact4):
+//   - a sum that is not finite: infinity times a zero part, a value that rounds to an infinite part;
+//   - a sum so small that the 2^-134 an activation may have lost show in its bits;
+//   - a sum of zero, if its activations have subnormal numbers among them: below 2^-134 all of their parts are zero;
+//   - every sum of a channel with weights of 2^26 or more.
+// To look at every sum costs 0 to 2.5 % (3x3 64->64 @56x56, 64 images 100.3 -> 102.1 us; 1x1 64->256 @56x56, 16 images 36.2 -> 36.9; tiles
+// of 128 channels the same).  What is found is slow: a blank input takes 2.5 to 6 times the time of an ordinary one, one of 1e-35 a hundred.
 //
 // Every mbarrier wait is bounded; one that runs out records a code in *status and the CTA drains.
 #include <cuda.h>
@@ -72,6 +80,7 @@ struct F32Params {
     int splits, pdl, test_withhold;
     int halves;        // NT = 1 on weights laid out for 128 channels: a tile's parts are halves of theirs
     const uint8_t *parts;  // the weights' parts, one stage after another: [column tile][K block][part][64 rows of 64 bytes, swizzled]
+    const float *units;    // per channel what its sums are in units of (negative: it has no weights but zero); then per channel the smallest ordinary sum
     int *status;
     long long wait_limit;
 };
@@ -120,6 +129,24 @@ __device__ __forceinline__ void split_store(uint32_t taddr, const float4 &a, con
     tmem_st4(taddr + 32, p3);
 }
 
+// twice an fp32's bits less one, as an unsigned number: in the order of the magnitudes, but for zero, which is above them all
+__device__ __forceinline__ uint32_t magnitude(float v) { return 2 * __float_as_uint(v) - 1; }
+// the largest and the smallest magnitude of four values (the largest: NaN if one of them is)
+__device__ __forceinline__ float max4(float a, float b, float c, float d)
+{
+    float m;
+    asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(c));
+    asm("max.NaN.abs.f32 %0, %1, %2, %2;" : "=f"(m) : "f"(m), "f"(d));
+    return m;
+}
+__device__ __forceinline__ float min4(float a, float b, float c, float d)
+{
+    float m;
+    asm("min.abs.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(c));
+    asm("min.abs.f32 %0, %1, %2, %2;" : "=f"(m) : "f"(m), "f"(d));
+    return m;
+}
+
 // Four channels of one pixel: y = act(self * (sum * scale + shift) + res_coef * residual), channels >= Cout zero.
 struct Affine4 {
     float sc[4], sh[4];
@@ -154,28 +181,96 @@ struct Affine4 {
     }
 };
 
-// Four channels of one pixel by a chain of FFMA over K, zeros outside the image: the order of the FFMA kernel.
+// The activations of one pixel's sums, four at a time, zeros outside the image
+struct Patch {
+    const F32Params &p;
+    int n, ih0, iw0;
+    __device__ __forceinline__ Patch(const F32Params &p, int pm) : p(p), n(pm / p.oHW)
+    {
+        const int rem = pm - n * p.oHW, oh = rem / p.oW;
+        ih0 = oh * p.dH - p.padH;
+        iw0 = (rem - oh * p.oW) * p.dW - p.padW;
+    }
+    __device__ __forceinline__ float4 chunk(int g) const
+    {
+        const int ki = __ldg(p.kinfo + g), ih = ih0 + ((ki >> 24) & 0x7f), iw = iw0 + ((ki >> 16) & 0xff);
+        if (ki < 0 || (unsigned)ih >= (unsigned)p.H || (unsigned)iw >= (unsigned)p.W) return make_float4(0.f, 0.f, 0.f, 0.f);
+        return *reinterpret_cast<const float4 *>(p.x + ((size_t)(n * p.H + ih) * p.W + iw) * p.in_ld + (ki & 0xffff) * 4);
+    }
+};
+
+// Four channels of one pixel by FFMA from the fp32 weights: chains of 32 products, whose sums are added.
 __device__ __forceinline__ float4 exact4(const F32Params &p, int pm, int c0)
 {
-    const int n = pm / p.oHW, rem = pm - n * p.oHW, oh = rem / p.oW, ow = rem - oh * p.oW;
-    const int ih0 = oh * p.dH - p.padH, iw0 = ow * p.dW - p.padW;
-    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    const Patch patch(p, pm);
+    float s[4] = {0.f, 0.f, 0.f, 0.f}, t[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
     for (int g = 0; g < p.n_kchunks; g++) {
-        const int ki = __ldg(p.kinfo + g);
-        const int ih = ih0 + ((ki >> 24) & 0x7f), iw = iw0 + ((ki >> 16) & 0xff);
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (ki >= 0 && (unsigned)ih < (unsigned)p.H && (unsigned)iw < (unsigned)p.W)
-            v = *reinterpret_cast<const float4 *>(p.x + ((size_t)(n * p.H + ih) * p.W + iw) * p.in_ld + (ki & 0xffff) * 4);
+        float4 v = patch.chunk(g);
 #pragma unroll 1
         for (int e = 0; e < 4; e++) {
             const float4 wv = *reinterpret_cast<const float4 *>(p.w + (size_t)(g * 4 + e) * p.Cout_pad + c0);
-            s[0] = fmaf(v.x, wv.x, s[0]); s[1] = fmaf(v.x, wv.y, s[1]);
-            s[2] = fmaf(v.x, wv.z, s[2]); s[3] = fmaf(v.x, wv.w, s[3]);
+            t[0] = fmaf(v.x, wv.x, t[0]); t[1] = fmaf(v.x, wv.y, t[1]);
+            t[2] = fmaf(v.x, wv.z, t[2]); t[3] = fmaf(v.x, wv.w, t[3]);
             v.x = v.y; v.y = v.z; v.z = v.w;
+        }
+        if ((g & 7) == 7 || g == p.n_kchunks - 1) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) { s[j] += t[j]; t[j] = 0.f; }
         }
     }
     return make_float4(s[0], s[1], s[2], s[3]);
+}
+
+// A warp: are there subnormal numbers among the activations of one pixel's sums?
+__device__ __forceinline__ bool subnormals(const F32Params &p, int pm, int lane)
+{
+    const Patch patch(p, pm);
+    uint32_t least = ~0u;
+#pragma unroll 2
+    for (int g = lane; g < p.n_kchunks; g += 32) {
+        const float4 v = patch.chunk(g);
+        least = min(min(least, min(magnitude(v.x), magnitude(v.y))), min(magnitude(v.z), magnitude(v.w)));
+    }
+    return __any_sync(~0u, least < 2 * 0x00800000u - 1);
+}
+
+// A warp's rows that have a sum which is not ordinary (bits of `rare`: a thread's rows r0, r0 + step, ...): those sums computed again
+// or not, and stored.  G lanes share a row.
+__device__ __forceinline__ void store_rare(const F32Params &p, const uint8_t *part, unsigned rare, int r0, int step, int S, int G, int m0, int c0)
+{
+    const int lane = threadIdx.x & 31;
+    for (unsigned any = __reduce_or_sync(~0u, rare); any; any &= any - 1) {
+        const int k = __ffs(any) - 1, r = r0 + k * step;
+        const bool mine = rare >> k & 1;
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        bool spoilt = false, zero = false;
+        if (mine) {
+            const float4 u4 = *reinterpret_cast<const float4 *>(p.units + c0), l4 = *reinterpret_cast<const float4 *>(p.units + p.Cout_pad + c0);
+            const float u[4] = {u4.x, u4.y, u4.z, u4.w}, l[4] = {l4.x, l4.y, l4.z, l4.w};
+            for (int q = 0; q < S; q++) {
+                const float4 t = *reinterpret_cast<const float4 *>(part + (q * G * RECV_ROWS + r) * 16);
+                v[0] += t.x; v[1] += t.y; v[2] += t.z; v[3] += t.w;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float m = fabsf(v[i]);
+                zero |= m == 0.f && u[i] > 0.f;
+                spoilt |= m != 0.f && !(m >= l[i] && m < INFINITY);
+                v[i] *= fabsf(u[i]);
+            }
+        }
+        if (__any_sync(~0u, zero))
+            for (int first = 0; first < 32; first += G) {  // the warp's rows number k: G lanes each
+                const bool here = zero && lane / G == first / G;
+                if (__any_sync(~0u, here)) spoilt |= subnormals(p, m0 + __shfl_sync(~0u, r, first), lane) && here;
+            }
+        if (!mine) continue;
+        const float4 rv = p.res ? *reinterpret_cast<const float4 *>(p.res + (size_t)(m0 + r) * p.res_ld + c0) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 sums = make_float4(v[0], v[1], v[2], v[3]);
+        if (spoilt) sums = exact4(p, m0 + r, c0);
+        Affine4(p, c0).store(p, m0 + r, c0, sums, rv);
+    }
 }
 
 template <int NT, bool GATHER>
@@ -479,16 +574,22 @@ __global__ void __launch_bounds__(Cfg<NT, GATHER>::NTHREADS, 3 - NT) conv_f32_ke
         }
         if (GATHER) cp_async_wait<0>();
     }
+    // A thread stores four channels of every step-th row.  Their constants are read while the last multiplies run.
+    const int t2 = tid - C::CONV * 32, step = 256 >> (wshift - 2), g = t2 & (G - 1), c0 = n0 + rank * W + g * 4;
+    const int r0 = t2 >> (wshift - 2), rows = c0 < p.Cout ? min(BM, p.P - m0) : 0;
+    Affine4 f(p, c0);
+    const float4 unit = *reinterpret_cast<const float4 *>(p.units + c0), least = *reinterpret_cast<const float4 *>(p.units + p.Cout_pad + c0);
+    // the units go into the scales where that loses nothing (they are 2^-100 at least); elsewhere no sum is ordinary
+    const bool folded = min(min(magnitude(f.sc[0]), magnitude(f.sc[1])), min(magnitude(f.sc[2]), magnitude(f.sc[3]))) > magnitude(0x1p-26f);
+    const bool idle = unit.x < 0.f || unit.y < 0.f || unit.z < 0.f || unit.w < 0.f;  // a channel without weights: its zeros are ordinary
+    const float ordinary = !folded ? INFINITY : idle ? 0.f : max4(least.x, least.y, least.z, least.w);
+    f.sc[0] *= fabsf(unit.x); f.sc[1] *= fabsf(unit.y); f.sc[2] *= fabsf(unit.z); f.sc[3] *= fabsf(unit.w);
     leave();
     gathered();
     if (*abort_flag) return;
 
-    const int t2 = tid - C::CONV * 32, step = 256 >> (wshift - 2), g = t2 & (G - 1), c0 = n0 + rank * W + g * 4;
-    if (c0 >= p.Cout) return;
-    Affine4 f(p, c0);
-    const int r0 = t2 >> (wshift - 2), rows = min(BM, p.P - m0);
     const uint8_t *part = recv + (size_t)g * RECV_ROWS * 16;
-    unsigned spoilt = 0;
+    unsigned rare = 0;  // the thread's rows that have a sum which is not ordinary
 #pragma unroll 1
     for (int r = r0, k = 0; r < rows; r += 2 * step, k += 2) {
         float4 rv[2], v[2];
@@ -509,27 +610,56 @@ __global__ void __launch_bounds__(Cfg<NT, GATHER>::NTHREADS, 3 - NT) conv_f32_ke
 #pragma unroll
         for (int j = 0; j < 2; j++) {
             if (r + j * step >= rows) continue;
-            // (s - s is zero for a finite sum, NaN otherwise)
-            if (!((v[j].x - v[j].x) + (v[j].y - v[j].y) + (v[j].z - v[j].z) + (v[j].w - v[j].w) == 0.f)) spoilt |= 1u << (k + j);
-            f.store(p, m0 + r + j * step, c0, v[j], rv[j]);
+            if (min4(v[j].x, v[j].y, v[j].z, v[j].w) >= ordinary && max4(v[j].x, v[j].y, v[j].z, v[j].w) < INFINITY)
+                f.store(p, m0 + r + j * step, c0, v[j], rv[j]);
+            else
+                rare |= 1u << (k + j);
         }
     }
-    for (; spoilt; spoilt &= spoilt - 1) {
-        const int pm = m0 + r0 + (__ffs(spoilt) - 1) * step;
-        float4 rv = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (p.res) rv = *reinterpret_cast<const float4 *>(p.res + (size_t)pm * p.res_ld + c0);
-        f.store(p, pm, c0, exact4(p, pm, c0), rv);
+    if (idle) {
+        // (in a loop of its own: the instructions would slow the loop above down, 3 to 7 %)
+        const float4 u = *reinterpret_cast<const float4 *>(p.units + c0), l = *reinterpret_cast<const float4 *>(p.units + p.Cout_pad + c0);
+#pragma unroll 1
+        for (int r = r0, k = 0; r < rows; r += step, k++) {
+            float4 v = *reinterpret_cast<const float4 *>(part + r * 16);
+            for (int q = 1; q < S; q++) {
+                const float4 t = *reinterpret_cast<const float4 *>(part + (q * G * RECV_ROWS + r) * 16);
+                v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+            }
+            if ((u.x > 0.f && fabsf(v.x) < l.x) || (u.y > 0.f && fabsf(v.y) < l.y) || (u.z > 0.f && fabsf(v.z) < l.z) || (u.w > 0.f && fabsf(v.w) < l.w)) rare |= 1u << k;
+        }
     }
+    if (__any_sync(~0u, rare)) store_rare(p, part, rare, r0, step, S, G, m0, c0);
+}
+
+// fp32 weights [Ktot][Cout_pad] -> F32Params.units, 32 channels to a block of 32 x 32 threads.  A channel of largest weight 2^e (to
+// 2^(e + 1)) is multiplied by 2^39, or more to bring it to 1, up to 2^100: its smallest weights, 2^-149, then come to 2^-110 or more,
+// and a product that vanishes, below 2^-165, vanishes in fp32 as well.  Its sums are trusted while what 2^16 activations may have lost,
+// 2^(-134 + 16) of its scaled weights, is below a quarter of their last bit; and from 2^-90 on, lest parts of products vanish.
+__global__ void weight_units_kernel(const float *w, int Ktot, int Cout_pad, float *units)
+{
+    __shared__ float most[32][33];
+    const int c = blockIdx.x * 32 + threadIdx.x;
+    float m = 0.f;
+#pragma unroll 4
+    for (int k = threadIdx.y; k < Ktot; k += 32) m = fmaxf(m, fabsf(w[(size_t)k * Cout_pad + c]));
+    most[threadIdx.y][threadIdx.x] = m;
+    __syncthreads();
+    if (threadIdx.y) return;
+    for (int i = 1; i < 32; i++) m = fmaxf(m, most[i][threadIdx.x]);
+    const int e = m == 0.f ? -39 : m < 0x1p26f ? ilogbf(m) : 26, up = max(39, min(100, -e));
+    units[c] = m == 0.f ? -0x1p-39f : ldexpf(1.f, -up);
+    units[Cout_pad + c] = e == 26 ? INFINITY : ldexpf(1.f, max(e + up - 91, -90));
 }
 
 // fp32 weights [Ktot][Cout_pad] -> F32Params.parts, zeros behind Ktot: 64 channels of one K block
-__global__ void split_weights_kernel(const float *w, int Ktot, int nkb, int Cout_pad, int BN, uint8_t *out)
+__global__ void split_weights_kernel(const float *w, const float *units, int Ktot, int nkb, int Cout_pad, int BN, uint8_t *out)
 {
     __shared__ float t[32][65];
     const int kb = blockIdx.x, n0 = blockIdx.y * 64;
     for (int i = threadIdx.x; i < 32 * 64; i += 256) {
         const int k = i / 64, n = i % 64;
-        t[k][n] = kb * 32 + k < Ktot ? w[(size_t)(kb * 32 + k) * Cout_pad + n0 + n] : 0.f;
+        t[k][n] = kb * 32 + k < Ktot ? w[(size_t)(kb * 32 + k) * Cout_pad + n0 + n] * (1.f / fabsf(units[n0 + n])) : 0.f;
     }
     __syncthreads();
     const int part = BN * 64;  // bytes
@@ -616,14 +746,20 @@ extern "C" int thb_conv_f32_supported(const thb_conv_desc *d)
     return d->dtype == THB_F32 && d->kH * d->kW * d->Cin >= 64 && !d->x2 && !d->in_row_pitch && d->Cout_pad % 64 == 0 && operand_mode(d) >= 0 && d->kH <= 127 && d->kW <= 255;
 }
 
-extern "C" size_t thb_conv_f32_split_bytes(const thb_conv_desc *d) { return (size_t)d->Cout_pad * k_blocks(d) * 3 * BK * 2; }
+static size_t parts_bytes(const thb_conv_desc *d) { return (size_t)d->Cout_pad * k_blocks(d) * 3 * BK * 2; }
+
+extern "C" size_t thb_conv_f32_split_bytes(const thb_conv_desc *d) { return parts_bytes(d) + 2 * d->Cout_pad * sizeof(float); }
 
 extern "C" int thb_conv_f32_split_weights(const thb_conv_desc *d, void *w_split, thb_stream s)
 {
     if (!thb_conv_f32_supported(d)) return THB_ERR_UNSUPPORTED;
     if (!d->w || !w_split) return THB_ERR_ARG;
-    split_weights_kernel<<<dim3(k_blocks(d), d->Cout_pad / 64), 256, 0, (cudaStream_t)s>>>((const float *)d->w, d->Ktot_pad, k_blocks(d),
-                                                                                          d->Cout_pad, tile_n(d), (uint8_t *)w_split);
+    float *units = (float *)((uint8_t *)w_split + parts_bytes(d));
+    weight_units_kernel<<<d->Cout_pad / 32, dim3(32, 32), 0, (cudaStream_t)s>>>((const float *)d->w, d->Ktot_pad, d->Cout_pad, units);
+    const int rc = THB_LAUNCH_CHECK("weight_units_kernel");
+    if (rc != THB_OK) return rc;
+    split_weights_kernel<<<dim3(k_blocks(d), d->Cout_pad / 64), 256, 0, (cudaStream_t)s>>>((const float *)d->w, units, d->Ktot_pad, k_blocks(d),
+                                                                                                d->Cout_pad, tile_n(d), (uint8_t *)w_split);
     return THB_LAUNCH_CHECK("split_weights_kernel");
 }
 
@@ -684,6 +820,7 @@ extern "C" int thb_conv_f32_fwd(const thb_conv_desc *d, const void *w_split, con
     p.n_tiles = d->Cout_pad / bn;
     p.halves = bn < tile_n(d);
     p.parts = (const uint8_t *)w_split;
+    p.units = (const float *)(p.parts + parts_bytes(d));
     static const CUtensorMap none = {};
     const CUtensorMap *a = p.mode ? thb_activation_tmap(d, x, p.mode) : &none;
     if (!a) return thb_note_launch(cudaErrorUnknown, "conv_f32: tensor map");
