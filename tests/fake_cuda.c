@@ -4,6 +4,7 @@
 #include <cuda_runtime_api.h>
 #include <stdlib.h>
 #include <string.h>
+#include "thb200_kernels.h"
 
 /* ---- what a test sets and reads ---- */
 size_t fake_budget = (size_t)1 << 50, fake_live; /* device bytes */
@@ -11,6 +12,7 @@ int fake_devices = 1, fake_streams;              /* GPUs; streams alive */
 int fake_minmax, fake_boundaries, fake_empty;    /* launches: of the device's range pass, of boundary kernels in, of those on nothing */
 int fake_images;                                 /* that boundary kernels in were launched on */
 float fake_q_sub, fake_q_mult;                   /* the input quantisation of the last boundary kernel in */
+int fake_f32_tc, fake_splits, fake_tc_launches;  /* fp32 convolutions may go to the tensor cores; weights split for them; launches there */
 
 static void boundary(int n, float q_sub, float q_mult)
 {
@@ -117,6 +119,11 @@ int thb_minmax_normalized(const float *x, int N, int C, int H, int W, const floa
     return 0;
 }
 
+/* fp32 on the tensor cores (the host library's own rules where a test has switched them on) */
+int thb_conv_f32_supported(const thb_conv_desc *d) { return fake_f32_tc && d->dtype == THB_F32 && d->kH * d->kW * d->Cin >= 64 && !d->x2 && d->Cout_pad % 64 == 0; }
+int thb_conv_f32_split_weights(const thb_conv_desc *d, void *w, void *st) { fake_splits++; return 0; }
+int thb_conv_f32_fwd(const thb_conv_desc *d, const void *w, const void *x, void *y, void *st) { fake_tc_launches++; return 0; }
+
 /* ---- the rest ---- */
 unsigned short thb_float_to_half_bits(float v, int bf16) { (void)v; (void)bf16; return 0; }
 int thb_kernel_launch_count(void) { return 0; }
@@ -132,5 +139,5 @@ NOTHING(thb_conv_make_tmap) NOTHING(thb_conv_maxpool_fwd) NOTHING(thb_conv_nchw_
 NOTHING(thb_gemv_fwd) NOTHING(thb_l2_normalize) NOTHING(thb_logsoftmax) NOTHING(thb_max_unpool) NOTHING(thb_maxpool)
 NOTHING(thb_postprocess_status) NOTHING(thb_preprocess_images) NOTHING(thb_preprocess_images_lowp) NOTHING(thb_preprocess_yuyv)
 NOTHING(thb_reflect_pad) NOTHING(thb_slice_channels) NOTHING(thb_softmax) NOTHING(thb_to_nchw) NOTHING(thb_u8_channel_sum_rows)
-NOTHING(thb_conv_f32_fwd) NOTHING(thb_conv_f32_split_weights) NOTHING(thb_conv_f32_supported) NOTHING(thb_maxpool_sums) NOTHING(thb_maxpool_sums_supported)
+NOTHING(thb_maxpool_sums) NOTHING(thb_maxpool_sums_supported)
 NOTHING(thb_u8_combine) NOTHING(thb_u8_threshold) NOTHING(thb_upsample2x) NOTHING(thb_zero_pad)

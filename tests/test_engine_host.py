@@ -233,3 +233,48 @@ for fn in (lib.THB200_ProcessFloatConst, lib.THProcessFloat):
     parts.append(fake.boundaries)
 assert parts[0] == parts[1] > 1, parts
 """, tmp_path)
+
+
+def test_split_weights_make_room(engine, tmp_path):
+    """The second copies of fp32 weights never cost a call its memory: where a plan, or its sub-batches, fit without them only, they go
+    and the convolutions run on the FP32 units; a smaller shape gets them back.  THB200_NO_F32_TC=1 does without them from the start."""
+    engine("""
+fake.f32_tc = 1
+g = fx.resnet18(width=0.5, size=64, classes=10)
+x = pinned((64, 3, 64, 64))
+def held(chunks, env=None):
+    if env:
+        os.environ["THB200_NO_F32_TC"] = env
+    lib.THB200_SetPipelineChunks(chunks)
+    net = network(g, 0)
+    fake.splits = fake.tc_launches = 0
+    assert call(net, x) > 0
+    live = fake.live
+    assert (fake.splits > 0) == (fake.tc_launches > 0) == (env != "1")
+    th.free_network(net)
+    assert fake.live == 0
+    os.environ.pop("THB200_NO_F32_TC", None)
+    return live
+for chunks in (1, 2):
+    without, full = held(chunks, "1"), held(chunks, "0")
+    assert full > 1.1 * without
+    for part in (0.0, 0.02, 0.2, 0.5, 0.9, 0.999, 1.0):
+        net = network(g, 0)
+        fake.budget = without + int(part * (full - without))
+        fake.tc_launches = 0
+        for _ in range(2):
+            assert call(net, x) > 0, (chunks, part, lib.THB200_LastErrorString())
+        assert fake.live <= fake.budget and (part < 1 or fake.tc_launches > 0)
+        fake.budget = 1 << 50
+        fake.tc_launches = 0
+        assert call(net, x[:3]) > 0 and fake.tc_launches > 0, "a shape planned later has them again"
+        assert call(net, x) > 0
+        th.free_network(net)
+        assert fake.live == 0 and fake.streams == 0
+    net = network(g, 0)
+    fake.budget = without - (1 << 20)
+    assert call(net, x) <= 0
+    fake.budget = 1 << 50
+    assert call(net, x) > 0
+    th.free_network(net)
+""", tmp_path)

@@ -175,6 +175,7 @@ typedef struct shape_plan {
     int chunks, pipe_built, pipe_chunks;
     const unsigned char *cut; /* boundaries of the sub-batches in sixteenths (sub_batch_cuts), NULL: thb_slice_sub_batches */
     int peer_gather;
+    int no_split; /* planned without second copies of fp32 weights: with them it did not fit */
     unsigned long long used; /* forward counter of the last use */
 } shape_plan;
 
@@ -586,12 +587,13 @@ static float *weights_oihw(const thb_model *M, const thb_conv_desc *d, const wso
 }
 
 /* The second copy of an fp32 convolution's weights, which sends it to the tensor cores; none, and so the kernel on the FP32 units,
- * where that one does not take the layer, where the device has no room for the copy and with THB200_NO_F32_TC=1. */
+ * where that one does not take the layer, where the device has no room for the copy, or none for the plan beside the copies, and
+ * with THB200_NO_F32_TC=1. */
 static const void *conv_split_weights(planner *P, const thb_conv_desc *d, const int *conv_key)
 {
     thb_engine *E = P->E;
     const char *off = getenv("THB200_NO_F32_TC");
-    if ((off && atoi(off)) || !thb_conv_f32_supported(d)) return 0;
+    if ((off && atoi(off)) || E->cur->no_split || !thb_conv_f32_supported(d)) return 0;
     int key[BLOB_KEY];
     memcpy(key, conv_key, sizeof(key));
     key[1] = BL_SPLIT;
@@ -2285,6 +2287,23 @@ static int plans_make_way(thb_engine *E)
     return 1;
 }
 
+/* After a plan that did not fit although no other is left: are there second copies of fp32 weights that could make way? */
+static int splits_held(const thb_engine *E)
+{
+    int held = 0;
+    for (int i = 0; i < E->nblobs; i++) held += E->blobs[i].key[1] == BL_SPLIT;
+    return E->out_of_memory && held;
+}
+/* They go: no plan uses them any more. */
+static void splits_drop(thb_engine *E)
+{
+    for (int i = 0; i < E->nblobs; i++)
+        if (E->blobs[i].key[1] == BL_SPLIT) {
+            if (cudaSetDevice(E->blobs[i].device) == cudaSuccess) cudaFree(E->blobs[i].ptr);
+            E->blobs[i--] = E->blobs[--E->nblobs];
+        }
+}
+
 /* Plans beyond MAX_PLAN_BYTES are dropped, the least recently used first and the current one never. */
 static void plans_bound(thb_engine *E)
 {
@@ -2315,14 +2334,18 @@ static int select_plan(thb_engine *E, int N, int C, int H, int W, int rank, int 
     for (int i = 0; i < MAX_PLANS && slot < 0; i++)
         if (!E->plans[i]) slot = i;
     if (slot < 0) plan_drop(E, slot = plan_oldest(E, 0));
-    for (;;) {
+    for (int no_split = 0;;) {
         shape_plan *p = E->plans[slot] = E->cur = calloc(1, sizeof(*p));
         if (!p) { thb_set_error("out of memory"); return -1; }
         p->N = N; p->C = C; p->H = H; p->W = W; p->rank = rank; p->cp = cp;
+        p->no_split = no_split;
         p->used = E->clock;
         if (!plan_build(E)) break;
         plan_drop(E, slot);
-        if (!plans_make_way(E)) return -1;
+        if (plans_make_way(E)) continue;
+        if (!splits_held(E)) return -1;
+        splits_drop(E);
+        no_split = 1;
     }
     plans_bound(E);
     return 0;
@@ -2467,7 +2490,18 @@ static int pipe_build(thb_engine *E, int S)
     pipe_free(E->cur);
     while (pipe_instances(E, S)) {
         pipe_free(E->cur);
-        if (!plans_make_way(E)) return -1;
+        if (plans_make_way(E)) continue;
+        if (!splits_held(E)) return -1;
+        /* the shape's own plan uses them: it is made again without */
+        shape_plan *p = E->cur;
+        for (int g = 0; g < 8; g++) instance_free(&p->inst[g]);
+        splits_drop(E);
+        p->built = 0;
+        p->no_split = 1;
+        if (!plan_build(E)) continue;
+        for (int i = 0; i < MAX_PLANS; i++)
+            if (E->plans[i] == p) plan_drop(E, i);
+        return -1;
     }
     plans_bound(E);
     return 0;
