@@ -13,6 +13,7 @@ int fake_minmax, fake_boundaries, fake_empty;    /* launches: of the device's ra
 int fake_images;                                 /* that boundary kernels in were launched on */
 float fake_q_sub, fake_q_mult;                   /* the input quantisation of the last boundary kernel in */
 int fake_f32_tc, fake_splits, fake_tc_launches;  /* fp32 convolutions may go to the tensor cores; weights split for them; launches there */
+int fake_waits;                                  /* waits for the legacy stream */
 
 static void boundary(int n, float q_sub, float q_mult)
 {
@@ -76,6 +77,7 @@ cudaError_t cudaPointerGetAttributes(struct cudaPointerAttributes *a, const void
 static cudaError_t stream_create(cudaStream_t *s) { *s = (cudaStream_t)malloc(1); fake_streams++; return cudaSuccess; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned f) { (void)f; return stream_create(s); }
 cudaError_t cudaStreamCreateWithPriority(cudaStream_t *s, unsigned f, int p) { (void)f; (void)p; return stream_create(s); }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) { fake_waits += !s; return cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t s) { free(s); fake_streams--; return cudaSuccess; }
 cudaError_t cudaEventCreate(cudaEvent_t *e) { *e = (cudaEvent_t)malloc(1); return cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned f) { (void)f; return cudaEventCreate(e); }
@@ -133,7 +135,7 @@ void thb_count_launches(int n) { (void)n; }
 NOTHING(cudaDeviceEnablePeerAccess) NOTHING(cudaEventRecord) NOTHING(cudaGetLastError) NOTHING(cudaGraphDestroy)
 NOTHING(cudaGraphExecDestroy) NOTHING(cudaGraphInstantiate) NOTHING(cudaGraphLaunch) NOTHING(cudaMemcpy) NOTHING(cudaMemcpy2DAsync)
 NOTHING(cudaMemcpyAsync) NOTHING(cudaMemcpyPeerAsync) NOTHING(cudaMemset) NOTHING(cudaMemsetAsync) NOTHING(cudaSetDevice)
-NOTHING(cudaStreamEndCapture) NOTHING(cudaStreamSynchronize) NOTHING(cudaStreamWaitEvent)
+NOTHING(cudaStreamEndCapture) NOTHING(cudaStreamWaitEvent)
 NOTHING(thb_affine_act) NOTHING(thb_avgpool) NOTHING(thb_cmax) NOTHING(thb_col2im) NOTHING(thb_combine) NOTHING(thb_conv_fwd)
 NOTHING(thb_conv_make_tmap) NOTHING(thb_conv_maxpool_fwd) NOTHING(thb_conv_nchw_fwd) NOTHING(thb_copy_channels) NOTHING(thb_from_nchw)
 NOTHING(thb_gemv_fwd) NOTHING(thb_l2_normalize) NOTHING(thb_logsoftmax) NOTHING(thb_max_unpool) NOTHING(thb_maxpool)

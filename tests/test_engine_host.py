@@ -278,3 +278,20 @@ for chunks in (1, 2):
     assert call(net, x) > 0
     th.free_network(net)
 """, tmp_path)
+
+
+def test_one_wait_a_plan(engine, tmp_path):
+    """What a plan launches to lay its weights out is waited for once, however many layers it has."""
+    engine("""
+fake.f32_tc = 1
+net = network(fx.resnet18(width=0.5, size=64, classes=10), 0)
+x = pinned((8, 3, 64, 64))
+lib.THB200_SetPipelineChunks(1)
+for n in (1, 2, 8):
+    fake.waits = 0
+    assert call(net, x[:n]) > 0
+    assert fake.waits == 1
+    assert call(net, x[:n]) > 0
+    assert fake.waits == 1
+assert fake.splits > 10
+""", tmp_path)

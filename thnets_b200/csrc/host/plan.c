@@ -604,7 +604,7 @@ static const void *conv_split_weights(planner *P, const thb_conv_desc *d, const 
         E->out_of_memory = 0;
         return 0;
     }
-    if (thb_conv_f32_split_weights(d, w->ptr, 0) || cudaStreamSynchronize(0) != cudaSuccess) {
+    if (thb_conv_f32_split_weights(d, w->ptr, 0)) { /* (waited for at the end of the plan) */
         cudaFree(w->ptr);
         E->nblobs--;
         return 0;
@@ -1859,6 +1859,8 @@ static int instance_build(thb_engine *E, instance *I, int device, int slice_off,
         /* padded channels are never read as data, but stale NaN/Inf bit patterns would poison the
          * zero-weight products: start from a clean arena */
         if (!rc && cudaMemset(I->arena, 0, I->arena_bytes) != cudaSuccess) { thb_set_error("arena memset failed"); rc = -1; }
+        /* that, and the layers' split weights, are launches on the legacy stream, for which the instance's does not wait */
+        if (!rc && cudaStreamSynchronize(0) != cudaSuccess) { thb_set_error("laying the weights out failed"); rc = -1; }
     }
     free(P.val); free(P.uses); free(P.absorbed); free(P.leader);
     if (th_debug && !rc)
