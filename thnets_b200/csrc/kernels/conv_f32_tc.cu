@@ -702,7 +702,7 @@ int launch_n(const thb_conv_desc *d, int splits, long sms)
     return tile_n(d) == 128 && tiles * splits * 2 > sms ? 128 : 64;
 }
 
-template <int NT, bool GATHER> int launch(const CUtensorMap *a, const F32Params &p, cudaStream_t st)
+template <int NT, bool GATHER> int launch(const CUtensorMap &a, const F32Params &p, cudaStream_t st)
 {
     using C = Cfg<NT, GATHER>;
     const auto kern = conv_f32_kernel<NT, GATHER>;
@@ -734,7 +734,7 @@ template <int NT, bool GATHER> int launch(const CUtensorMap *a, const F32Params 
     }
     cfg.attrs = attr;
     cfg.numAttrs = n;
-    const cudaError_t le = cudaLaunchKernelEx(&cfg, kern, *a, p);
+    const cudaError_t le = cudaLaunchKernelEx(&cfg, kern, a, p);
     return thb_note_launch(le != cudaSuccess ? le : cudaGetLastError(), "conv_f32_kernel");
 }
 
@@ -821,9 +821,8 @@ extern "C" int thb_conv_f32_fwd(const thb_conv_desc *d, const void *w_split, con
     p.halves = bn < tile_n(d);
     p.parts = (const uint8_t *)w_split;
     p.units = (const float *)(p.parts + parts_bytes(d));
-    static const CUtensorMap none = {};
-    const CUtensorMap *a = p.mode ? thb_activation_tmap(d, x, p.mode) : &none;
-    if (!a) return thb_note_launch(cudaErrorUnknown, "conv_f32: tensor map");
+    CUtensorMap a = {};
+    if (p.mode && !thb_activation_tmap(d, x, p.mode, &a)) return thb_note_launch(cudaErrorUnknown, "conv_f32: tensor map");
     const cudaStream_t st = (cudaStream_t)s;
     if (bn == 128) return p.mode ? launch<2, false>(a, p, st) : launch<2, true>(a, p, st);
     return p.mode ? launch<1, false>(a, p, st) : launch<1, true>(a, p, st);

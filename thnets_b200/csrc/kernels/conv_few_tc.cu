@@ -658,7 +658,7 @@ bool eligible(const thb_conv_desc *d)
 }
 
 template <int KIND, int EW>
-int launch(const CUtensorMap *w, const CUtensorMap *a, const CUtensorMap *a2, const FewParams &p, int ctas, int smem, cudaStream_t st)
+int launch(const CUtensorMap &w, const CUtensorMap &a, const CUtensorMap &a2, const FewParams &p, int ctas, int smem, cudaStream_t st)
 {
     static bool set[64];
     int dev = 0;
@@ -689,7 +689,7 @@ int launch(const CUtensorMap *w, const CUtensorMap *a, const CUtensorMap *a2, co
     }
     cfg.attrs = attr;
     cfg.numAttrs = n;
-    const cudaError_t le = cudaLaunchKernelEx(&cfg, kern, *w, *a, *a2, p);
+    const cudaError_t le = cudaLaunchKernelEx(&cfg, kern, w, a, a2, p);
     return thb_note_launch(le != cudaSuccess ? le : cudaGetLastError(), "conv_few_kernel");
 }
 
@@ -792,7 +792,8 @@ static int few_fwd(const thb_conv_desc *d, const void *x, void *y, float *y_nchw
     if (p.splits > p.nkb) return THB_ERR_ARG;
     const ThbConvLaunch kn = thb_conv_launch_knobs();
     p.pdl = kn.pdl; p.wait_limit = kn.wait_limit; p.test_withhold = kn.test_withhold;
-    const CUtensorMap *w = thb_weights_tmap(d, BN, p.half ? 64 : 128), *a, *a2;
+    CUtensorMap w, a, a2;
+    bool ok = thb_weights_tmap(d, BN, p.half ? 64 : 128, &w);
     if (d->x2) {
         const int cin2 = d->Cin - d->cin1;
         if (d->res || p.mode != 1 || d->in_row_pitch || d->cin1 <= 0 || d->cin1 % 64 || cin2 <= 0 || cin2 % 64 || d->x2_d < 1 || d->x2_d > 8 ||
@@ -801,19 +802,21 @@ static int few_fwd(const thb_conv_desc *d, const void *x, void *y, float *y_nchw
         p.nkb1 = d->cin1 / 64;
         p.a2_d = d->x2_d;
         p.a2_mode = d->x2_d == 1 ? 1 : 2;
-        a = thb_matrix_tmap(x, p.P, d->cin1, d->in_ld, d->dtype, 64);
-        if (p.a2_mode == 1) a2 = thb_matrix_tmap(d->x2, p.P, cin2, d->x2_ld, d->dtype, 64);
+        ok = ok && thb_matrix_tmap(x, p.P, d->cin1, d->in_ld, d->dtype, 64, &a);
+        if (p.a2_mode == 1) ok = ok && thb_matrix_tmap(d->x2, p.P, cin2, d->x2_ld, d->dtype, 64, &a2);
         else {
             thb_conv_desc d2;
             memset(&d2, 0, sizeof(d2));
             d2.dtype = d->dtype;
             d2.N = d->N; d2.H = d->x2_H; d2.W = d->x2_W; d2.Cin = d2.Cin_pad = cin2; d2.in_ld = d->x2_ld;
             d2.kH = d2.kW = 1; d2.dH = d2.dW = d->x2_d; d2.oH = d->oH; d2.oW = d->oW;
-            a2 = thb_activation_tmap(&d2, d->x2, 2);
+            ok = ok && thb_activation_tmap(&d2, d->x2, 2, &a2);
         }
-    } else
-        a = a2 = thb_activation_tmap(d, x, tmap_mode);
-    if (!w || !a || !a2) return thb_note_launch(cudaErrorUnknown, "conv_few: tensor map");
+    } else {
+        ok = ok && thb_activation_tmap(d, x, tmap_mode, &a);
+        a2 = a;
+    }
+    if (!ok) return thb_note_launch(cudaErrorUnknown, "conv_few: tensor map");
     const int per = (p.nkb + p.splits - 1) / p.splits;
     const int ctas = ((p.P + BM - 1) / BM) * p.n_tiles * p.splits;
     // stages: as many as fit the CTAs an SM gets.  Clusters always leave room for two CTAs to an SM, or a GPC holds too few of

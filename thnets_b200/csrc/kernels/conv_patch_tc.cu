@@ -20,6 +20,7 @@
 // tile is stored: the convolution's own output never reaches global memory.
 // Every wait is bounded; a wait that runs out records a code in *status and the CTA drains and exits.
 #include "common.cuh"
+#include "conv_maps.cuh"
 #include <cuda.h>
 #include <string.h>
 #include <stdio.h>
@@ -712,11 +713,12 @@ bool patch_geometry_ok(const thb_conv_desc *d, int pk, int ps, int ppad)
     return true;
 }
 
-// (the cache holds tensor maps only, i.e. addresses and shapes: nothing in it can go stale when memory is reused)
-struct PtMapEntry {
-    const void *x, *y, *wptr, *res;
-    int key[20];
-    alignas(64) CUtensorMap w, a, y_map, r_map;
+struct PatchKey {
+    const void *x, *y, *w, *res;
+    int shape[20];
+};
+struct PatchMaps {
+    CUtensorMap w, a, y, r;
 };
 
 int patch_launch(const thb_conv_desc *d, int pk, int ppad, int pH, int pW, const void *x, void *y, int y_ld, thb_stream s)
@@ -742,16 +744,13 @@ int patch_launch(const thb_conv_desc *d, int pk, int ppad, int pH, int pW, const
     const size_t smem = g.smem;
 
     // tensor maps of the weights (one tap per box), the input (patch box) and the output (tile box), cached by buffer and shape
-    static PtMapEntry cache[128];
-    static int used = 0, next = 0;
-    const int key[20] = {d->dtype, d->N, d->H, d->W, d->Cin_pad, d->in_ld, d->in_row_pitch, d->oH, d->oW, pH, pW, y_ld, d->Cout,
-                         p.CR, p.CC, p.PR, p.PC, d->kH * 16 + d->kW, d->res ? d->res_ld : 0, d->Ktot_pad};
-    PtMapEntry *e = nullptr;
-    for (int i = 0; i < used; i++)
-        if (cache[i].x == x && cache[i].y == y && cache[i].wptr == d->w && cache[i].res == d->res && !memcmp(cache[i].key, key, sizeof(key))) { e = &cache[i]; break; }
-    if (!e) {
-        e = &cache[used < 128 ? used++ : (next++ % 128)];
-        e->x = nullptr;
+    static ThbMapCache<PatchKey, PatchMaps, 128> cache;
+    const PatchKey key = {x, y, d->w, d->res,
+                          {d->dtype, d->N, d->H, d->W, d->Cin_pad, d->in_ld, d->in_row_pitch, d->oH, d->oW, pH, pW, y_ld, d->Cout,
+                           p.CR, p.CC, p.PR, p.PC, d->kH * 16 + d->kW, d->res ? d->res_ld : 0, d->Ktot_pad}};
+    static_assert(sizeof(key) == 112, "no padding");
+    PatchMaps maps;
+    if (!cache.find(key, &maps)) {
         const CUtensorMapDataType t = d->dtype == THB_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
         const CUtensorMapSwizzle sw = p.px_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_32B;
         cuuint32_t estr[4] = {1, 1, 1, 1};
@@ -759,7 +758,7 @@ int patch_launch(const thb_conv_desc *d, int pk, int ppad, int pH, int pW, const
             cuuint64_t dims[2] = {(cuuint64_t)d->Ktot_pad, (cuuint64_t)d->Cout_pad};
             cuuint64_t strides[1] = {(cuuint64_t)d->Ktot_pad * 2};
             cuuint32_t box[2] = {(cuuint32_t)d->Cin_pad, 64};
-            if (enc(&e->w, t, 2, const_cast<void *>(d->w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
+            if (enc(&maps.w, t, 2, const_cast<void *>(d->w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
                 return thb_note_launch(cudaErrorInvalidValue, "conv_patch: weight tensor map");
         }
@@ -768,7 +767,7 @@ int patch_launch(const thb_conv_desc *d, int pk, int ppad, int pH, int pW, const
             cuuint64_t dims[4] = {(cuuint64_t)d->Cin_pad, (cuuint64_t)Wst, (cuuint64_t)d->H, (cuuint64_t)d->N};
             cuuint64_t strides[3] = {(cuuint64_t)d->in_ld * 2, (cuuint64_t)Wst * d->in_ld * 2, (cuuint64_t)d->H * Wst * d->in_ld * 2};
             cuuint32_t box[4] = {(cuuint32_t)d->Cin_pad, (cuuint32_t)p.P, (cuuint32_t)(p.CR + p.kH - 1), 1};
-            if (enc(&e->a, t, 4, const_cast<void *>(x), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
+            if (enc(&maps.a, t, 4, const_cast<void *>(x), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
                 return thb_note_launch(cudaErrorInvalidValue, "conv_patch: input tensor map");
         }
@@ -779,7 +778,7 @@ int patch_launch(const thb_conv_desc *d, int pk, int ppad, int pH, int pW, const
             cuuint64_t strides[3] = {(cuuint64_t)y_ld * 2, (cuuint64_t)yW * y_ld * 2, (cuuint64_t)yH * yW * y_ld * 2};
             cuuint32_t box[4] = {64, (cuuint32_t)(pk ? p.PC : p.CC), (cuuint32_t)(pk ? p.PR : p.CR), 1};
             // the pooled tile is written as plain rows; the convolution tile carries the 128-byte XOR pattern
-            if (enc(&e->y_map, t, 4, y, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            if (enc(&maps.y, t, 4, y, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     pk ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
                 return thb_note_launch(cudaErrorInvalidValue, "conv_patch: output tensor map");
@@ -790,12 +789,12 @@ int patch_launch(const thb_conv_desc *d, int pk, int ppad, int pH, int pW, const
             cuuint64_t dims[4] = {(cuuint64_t)c8, (cuuint64_t)d->oW, (cuuint64_t)d->oH, (cuuint64_t)d->N};
             cuuint64_t strides[3] = {(cuuint64_t)d->res_ld * 2, (cuuint64_t)d->oW * d->res_ld * 2, (cuuint64_t)d->oH * d->oW * d->res_ld * 2};
             cuuint32_t box[4] = {64, (cuuint32_t)p.CC, (cuuint32_t)p.CR, 1};
-            if (enc(&e->r_map, t, 4, const_cast<void *>(d->res), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            if (enc(&maps.r, t, 4, const_cast<void *>(d->res), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
                 return thb_note_launch(cudaErrorInvalidValue, "conv_patch: residual tensor map");
         }
-        e->x = x; e->y = y; e->wptr = d->w; e->res = d->res;
-        memcpy(e->key, key, sizeof(key));
+        if (!d->res) maps.r = maps.y;
+        cache.keep(key, maps);
     }
 
     // The per-channel constants travel as kernel parameters: from the descriptor's host copies when it has them, else
@@ -854,7 +853,7 @@ int patch_launch(const thb_conv_desc *d, int pk, int ppad, int pH, int pW, const
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = use_pdl ? 1 : 0;
-    const cudaError_t le = cudaLaunchKernelEx(&cfg, kern, e->w, e->a, e->y_map, p.has_res ? e->r_map : e->y_map, p);
+    const cudaError_t le = cudaLaunchKernelEx(&cfg, kern, maps.w, maps.a, maps.y, maps.r, p);
     return thb_note_launch(le != cudaSuccess ? le : cudaGetLastError(), "conv_patch_tc_kernel");
 }
 

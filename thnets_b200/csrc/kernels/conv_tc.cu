@@ -1535,7 +1535,8 @@ int num_sms()
 }
 
 struct ConvTmaps {
-    const CUtensorMap *w, *a, *y, *r;  // weights, activation operand, output, residual (unused ones alias w)
+    CUtensorMap w, a, y, r;  // weights, activation operand, output, residual or second operand (unused ones are copies of w)
+    bool has_y, has_r;
 };
 
 template <int KIND, int BN, int STAGES>
@@ -1606,7 +1607,7 @@ int launch_tc(const ConvTmaps &tm, ConvTcParams p, cudaStream_t st)
         if (kn.epi_groups >= 0) p.epi_groups = kn.epi_groups == 3 && KIND == 2 && p.a_tma && BN < 256 ? 3 : 2;
     }
     if (L::TMA_EPI) {
-        if (!tm.y || (p.res && !tm.r)) return thb_note_launch(cudaErrorUnknown, "conv_tc: output tensor map");
+        if (!tm.has_y || (p.res && !tm.has_r)) return thb_note_launch(cudaErrorUnknown, "conv_tc: output tensor map");
         // Shared memory is split between pipeline stages and the epilogue's 16 KB tiles (groups x tiles per group); which
         // split wins was measured per layer shape.  A single K block with 128 output channels per tile lives off its
         // epilogue: three groups (warps 0-3 join when they have nothing to gather) of two tiles.  One or two K blocks with
@@ -1640,8 +1641,7 @@ int launch_tc(const ConvTmaps &tm, ConvTcParams p, cudaStream_t st)
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = use_pdl ? 1 : 0;
-    const cudaError_t le = cudaLaunchKernelEx(&cfg, p.splits > 1 ? kern_split : kern_plain, *tm.w, *tm.a, tm.y ? *tm.y : *tm.w,
-                                              tm.r ? *tm.r : *tm.w, p);
+    const cudaError_t le = cudaLaunchKernelEx(&cfg, p.splits > 1 ? kern_split : kern_plain, tm.w, tm.a, tm.y, tm.r, p);
     const int rc = thb_note_launch(le != cudaSuccess ? le : cudaGetLastError(), "conv_tc_kernel");
     if (rc != THB_OK || p.splits <= 1) return rc;
     if constexpr (KIND != 2) {
@@ -1710,64 +1710,52 @@ CUtensorMapDataType tmap_type(int dtype)
 
 // TMA descriptors of plain row-major matrices [rows][cols] with a row pitch (activation operand of a 1x1
 // convolution, output and residual tensors), keyed by what they encode and built once per buffer and shape.
-struct MTmapEntry {
+struct MatrixKey {
     const void *x;
     long rows;
     int cols, ld, dtype, box_cols;
-    alignas(64) CUtensorMap map;
 };
-const CUtensorMap *matrix_tmap(const void *x, long rows, int cols, int ld, int dtype, int box_cols)
+bool matrix_tmap(const void *x, long rows, int cols, int ld, int dtype, int box_cols, CUtensorMap *out)
 {
-    static MTmapEntry cache[1024];
-    static int used = 0, next = 0;
-    for (int i = 0; i < used; i++) {
-        MTmapEntry &e = cache[i];
-        if (e.x == x && e.rows == rows && e.cols == cols && e.ld == ld && e.dtype == dtype && e.box_cols == box_cols) return &e.map;
-    }
+    static ThbMapCache<MatrixKey, CUtensorMap, 1024> cache;
+    const MatrixKey key = {x, rows, cols, ld, dtype, box_cols};
+    static_assert(sizeof(key) == 32, "no padding");
+    if (cache.find(key, out)) return true;
     encode_tiled_fn enc = get_encode_fn();
-    if (!enc) return nullptr;
-    MTmapEntry &e = cache[used < 1024 ? used++ : (next++ % 1024)];
-    e.x = nullptr;
+    if (!enc) return false;
     const size_t es = tmap_esize(dtype);
     const CUtensorMapDataType t = tmap_type(dtype);
     cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
     cuuint64_t strides[1] = {(cuuint64_t)ld * es};
     cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)BM};
     cuuint32_t estr[2] = {1, 1};
-    if (enc(&e.map, t, 2, const_cast<void *>(x), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    if (enc(out, t, 2, const_cast<void *>(x), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return nullptr;
-    e.x = x; e.rows = rows; e.cols = cols; e.ld = ld; e.dtype = dtype; e.box_cols = box_cols;
-    return &e.map;
+        return false;
+    cache.keep(key, *out);
+    return true;
 }
 
 // TMA descriptors of activation operands, keyed by what they encode (built once per buffer and shape).
 // mode 1: the plain [pixels][Cin] matrix of a 1x1 stride-1 convolution; mode 2: im2col over {C, W, H, N}.
-struct ATmapEntry {
+struct ActivationKey {
     const void *x;
-    int mode, N, H, W, cin_pad, in_ld, dtype, geom[8];
-    alignas(64) CUtensorMap map;
+    int mode, N, H, W, cin_pad, in_ld, dtype, geom[8], zero;
 };
-const CUtensorMap *activation_tmap(const thb_conv_desc *d, const void *x, int mode)
+bool activation_tmap(const thb_conv_desc *d, const void *x, int mode, CUtensorMap *out)
 {
     if (mode == 1)
-        return matrix_tmap(x, (long)d->N * d->H * d->W, d->Cin_pad, d->in_ld, d->dtype, (int)(128 / tmap_esize(d->dtype)));
-    static ATmapEntry cache[512];
-    static int used = 0, next = 0;
-    const int geom[8] = {d->kH, d->kW, d->dH, d->dW, d->padH, mode == 3 || mode == 5 ? d->in_row_pitch : d->padW, d->oH, d->oW};
-    for (int i = 0; i < used; i++) {
-        ATmapEntry &e = cache[i];
-        if (e.x == x && e.mode == mode && e.N == d->N && e.H == d->H && e.W == d->W && e.cin_pad == d->Cin_pad &&
-            e.in_ld == d->in_ld && e.dtype == d->dtype && (mode == 1 || !memcmp(e.geom, geom, sizeof(geom))))
-            return &e.map;
-    }
-    ATmapEntry &e = cache[used < 512 ? used++ : (next++ % 512)];
-    e.x = nullptr;
+        return matrix_tmap(x, (long)d->N * d->H * d->W, d->Cin_pad, d->in_ld, d->dtype, (int)(128 / tmap_esize(d->dtype)), out);
+    static ThbMapCache<ActivationKey, CUtensorMap, 512> cache;
+    const ActivationKey key = {x, mode, d->N, d->H, d->W, d->Cin_pad, d->in_ld, d->dtype,
+                               {d->kH, d->kW, d->dH, d->dW, d->padH, mode == 3 || mode == 5 ? d->in_row_pitch : d->padW, d->oH, d->oW}, 0};
+    static_assert(sizeof(key) == 72, "no padding");
+    if (cache.find(key, out)) return true;
     const size_t es = tmap_esize(d->dtype);
     const CUtensorMapDataType t = tmap_type(d->dtype);
     {
         encode_im2col_fn enc = get_encode_im2col_fn();
-        if (!enc) return nullptr;
+        if (!enc) return false;
         // The bounding box that base pixels (tap (0,0) positions) live in: from -pad up to the position of the last
         // output pixel (dim + pad - (k - 1) for a full convolution), so that stepping by the convolution stride visits
         // exactly oW x oH positions per image.
@@ -1790,43 +1778,36 @@ const CUtensorMap *activation_tmap(const thb_conv_desc *d, const void *x, int mo
         }
         cuuint32_t estr[4] = {1, (cuuint32_t)d->dW, (cuuint32_t)d->dH, 1};
         // modes 4 and 5: a tap (a row of taps) is 64 bytes of channels; the box is 64 bytes wide and lands as rows of 64 bytes with the 64-byte swizzle
-        if (enc(&e.map, t, 4, const_cast<void *>(x), dims, strides, lower, upper, (cuuint32_t)((mode >= 4 ? 64 : 128) / es),
+        if (enc(out, t, 4, const_cast<void *>(x), dims, strides, lower, upper, (cuuint32_t)((mode >= 4 ? 64 : 128) / es),
                 (cuuint32_t)BM, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                 mode >= 4 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return nullptr;
+            return false;
         // Drivers up to CUDA 13.1 encode im2col descriptors of tensors smaller than 128 KiB with a flag (bit 21 of
         // the second 64-bit word) that makes the load misbehave; CUTLASS clears it for those drivers, and so do we.
         int drv = 0;
         if (cudaDriverGetVersion(&drv) == cudaSuccess && drv <= 13010 &&
             (size_t)d->N * d->H * (mode == 3 || mode == 5 ? d->in_row_pitch : d->W) * d->in_ld * es < 131072)
-            reinterpret_cast<uint64_t *>(&e.map)[1] &= ~(1ull << 21);
+            reinterpret_cast<uint64_t *>(out)[1] &= ~(1ull << 21);
     }
-    e.x = x; e.mode = mode; e.N = d->N; e.H = d->H; e.W = d->W; e.cin_pad = d->Cin_pad; e.in_ld = d->in_ld; e.dtype = d->dtype;
-    memcpy(e.geom, geom, sizeof(geom));
-    return &e.map;
+    cache.keep(key, *out);
+    return true;
 }
 
 // Descriptor of the packed weights read in boxes of box_rows channels x 128 or 64 bytes (SWIZZLE_64B: convolutions whose taps
 // are 64 bytes).
-struct WBoxEntry {
+struct WeightsKey {
     const void *w;
-    int ktot, cout_pad, rows, bytes, dtype;
-    alignas(64) CUtensorMap map;
+    int ktot, cout_pad, rows, bytes, dtype, zero;
 };
-const CUtensorMap *weights_box_tmap(const thb_conv_desc *d, int box_rows, int box_bytes)
+bool weights_box_tmap(const thb_conv_desc *d, int box_rows, int box_bytes, CUtensorMap *out)
 {
-    static WBoxEntry cache[512];
-    static int used = 0, next = 0;
-    for (int i = 0; i < used; i++) {
-        WBoxEntry &e = cache[i];
-        if (e.w == d->w && e.ktot == d->Ktot_pad && e.cout_pad == d->Cout_pad && e.rows == box_rows && e.bytes == box_bytes && e.dtype == d->dtype)
-            return &e.map;
-    }
+    static ThbMapCache<WeightsKey, CUtensorMap, 512> cache;
+    const WeightsKey key = {d->w, d->Ktot_pad, d->Cout_pad, box_rows, box_bytes, d->dtype, 0};
+    static_assert(sizeof(key) == 32, "no padding");
+    if (cache.find(key, out)) return true;
     encode_tiled_fn enc = get_encode_fn();
-    if (!enc) return nullptr;
-    WBoxEntry &e = cache[used < 512 ? used++ : (next++ % 512)];
-    e.w = nullptr;
+    if (!enc) return false;
     const int es = d->dtype == THB_U8 ? 1 : 2;
     CUtensorMapDataType t = d->dtype == THB_U8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8
                             : d->dtype == THB_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -1834,12 +1815,12 @@ const CUtensorMap *weights_box_tmap(const thb_conv_desc *d, int box_rows, int bo
     cuuint64_t strides[1] = {(cuuint64_t)d->Ktot_pad * es};
     cuuint32_t box[2] = {(cuuint32_t)(box_bytes / es), (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
-    if (enc(&e.map, t, 2, const_cast<void *>(d->w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    if (enc(out, t, 2, const_cast<void *>(d->w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
             box_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return nullptr;
-    e.w = d->w; e.ktot = d->Ktot_pad; e.cout_pad = d->Cout_pad; e.rows = box_rows; e.bytes = box_bytes; e.dtype = d->dtype;
-    return &e.map;
+        return false;
+    cache.keep(key, *out);
+    return true;
 }
 
 }  // namespace
@@ -1853,12 +1834,12 @@ bool thb_im2col_ok(const thb_conv_desc *d)
            box_corner_ok((d->oH - 1) * d->dH + 1 - d->H - d->padH, d->H + d->padH) &&
            box_corner_ok((d->oW - 1) * d->dW + 1 - d->W - d->padW, d->W + d->padW);
 }
-const CUtensorMap *thb_matrix_tmap(const void *x, long rows, int cols, int ld, int dtype, int box_cols)
+bool thb_matrix_tmap(const void *x, long rows, int cols, int ld, int dtype, int box_cols, CUtensorMap *out)
 {
-    return matrix_tmap(x, rows, cols, ld, dtype, box_cols);
+    return matrix_tmap(x, rows, cols, ld, dtype, box_cols, out);
 }
-const CUtensorMap *thb_activation_tmap(const thb_conv_desc *d, const void *x, int mode) { return activation_tmap(d, x, mode); }
-const CUtensorMap *thb_weights_tmap(const thb_conv_desc *d, int box_rows, int box_bytes) { return weights_box_tmap(d, box_rows, box_bytes); }
+bool thb_activation_tmap(const thb_conv_desc *d, const void *x, int mode, CUtensorMap *out) { return activation_tmap(d, x, mode, out); }
+bool thb_weights_tmap(const thb_conv_desc *d, int box_rows, int box_bytes, CUtensorMap *out) { return weights_box_tmap(d, box_rows, box_bytes, out); }
 int thb_pdl_enabled() { return knobs().pdl; }
 ThbConvLaunch thb_conv_launch_knobs()
 {
@@ -1910,7 +1891,8 @@ extern "C" int thb_conv_padded_rows_supported(int dtype)
         d.N = 2; d.H = 8; d.W = 8; d.kH = d.kW = 4; d.dH = d.dW = 1; d.padH = d.padW = 2; d.oH = d.oW = 8;
         d.Cin_pad = d.in_ld = 32 / es;
         d.in_row_pitch = 12; d.in_pad_left = 2;
-        ok[dtype] = activation_tmap(&d, reinterpret_cast<const void *>(uintptr_t(1) << 20), 3) != nullptr;
+        CUtensorMap map;
+        ok[dtype] = activation_tmap(&d, reinterpret_cast<const void *>(uintptr_t(1) << 20), 3, &map);
     }
     return ok[dtype];
 }
@@ -1968,7 +1950,7 @@ extern "C" int thb_conv_fwd_tc(const thb_conv_desc *d, const void *x, void *y, t
     p.by_ohw = FastDiv::of((uint32_t)p.oHW);
     p.by_ow = FastDiv::of((uint32_t)p.oW);
     const CUtensorMap &tm = *reinterpret_cast<const CUtensorMap *>(d->tmap);
-    const CUtensorMap *ta = &tm;
+    ConvTmaps maps = {tm, tm, tm, tm, false, false};
     // a 1x1 stride-1 unpadded convolution (and every Linear) reads a plain [pixels][Cin] matrix: TMA loads it
     p.a_tma = d->kH == 1 && d->kW == 1 && d->dH == 1 && d->dW == 1 && d->padH == 0 && d->padW == 0 &&
               d->oH == d->H && d->oW == d->W;
@@ -2017,20 +1999,15 @@ extern "C" int thb_conv_fwd_tc(const thb_conv_desc *d, const void *x, void *y, t
         if (p.a_tma > allow) p.a_tma = 0, p.half = 0;
         if (allow == 22 && p.a_tma == 1) p.a_tma = 2;  // experiment: im2col mode for a plain matrix too
     }
-    if (p.a_tma) {
-        ta = activation_tmap(d, x, tmap_mode);
-        if (!ta) p.a_tma = 0, p.half = 0, ta = &tm;
-    }
-    ConvTmaps maps = {&tm, ta, nullptr, nullptr};
+    if (p.a_tma && !activation_tmap(d, x, tmap_mode, &maps.a)) p.a_tma = 0, p.half = 0, maps.a = tm;
     if (p.half) {
-        maps.w = weights_box_tmap(d, d->BN, 64);
-        if (!maps.w) return thb_note_launch(cudaErrorUnknown, "conv_tc: weight tensor map");
+        if (!weights_box_tmap(d, d->BN, 64, &maps.w)) return thb_note_launch(cudaErrorUnknown, "conv_tc: weight tensor map");
     }
     if (d->dtype != THB_U8 && d->BN >= 64) {
         // output and residual go through TMA: [pixels][channels rounded up to 8] matrices with their own pitch
         const int c8 = (d->Cout + 7) & ~7;
-        maps.y = matrix_tmap(y, p.P, c8, d->out_ld, d->dtype, 64);
-        if (d->res) maps.r = matrix_tmap(d->res, p.P, c8, d->res_ld, d->dtype, 64);
+        maps.has_y = matrix_tmap(y, p.P, c8, d->out_ld, d->dtype, 64, &maps.y);
+        if (d->res) maps.has_r = matrix_tmap(d->res, p.P, c8, d->res_ld, d->dtype, 64, &maps.r);
         if (d->x2) {
             // second activation operand: its descriptor travels in the residual's slot (there is no residual then)
             const int cin2 = d->Cin - d->cin1;
@@ -2039,10 +2016,10 @@ extern "C" int thb_conv_fwd_tc(const thb_conv_desc *d, const void *x, void *y, t
                 return THB_ERR_UNSUPPORTED;
             p.nkb1 = d->cin1 / 64;
             p.a2_d = d->x2_d;
-            maps.a = matrix_tmap(x, p.P, d->cin1, d->in_ld, d->dtype, 64);
+            const bool has_a = matrix_tmap(x, p.P, d->cin1, d->in_ld, d->dtype, 64, &maps.a);
             if (d->x2_d == 1) {
                 p.a2_mode = 1;
-                maps.r = matrix_tmap(d->x2, p.P, cin2, d->x2_ld, d->dtype, 64);
+                maps.has_r = matrix_tmap(d->x2, p.P, cin2, d->x2_ld, d->dtype, 64, &maps.r);
             } else {
                 thb_conv_desc d2;
                 memset(&d2, 0, sizeof(d2));
@@ -2050,9 +2027,9 @@ extern "C" int thb_conv_fwd_tc(const thb_conv_desc *d, const void *x, void *y, t
                 d2.N = d->N; d2.H = d->x2_H; d2.W = d->x2_W; d2.Cin = d2.Cin_pad = cin2; d2.in_ld = d->x2_ld;
                 d2.kH = d2.kW = 1; d2.dH = d2.dW = d->x2_d; d2.oH = d->oH; d2.oW = d->oW;
                 p.a2_mode = 2;
-                maps.r = activation_tmap(&d2, d->x2, 2);
+                maps.has_r = activation_tmap(&d2, d->x2, 2, &maps.r);
             }
-            if (!maps.a || !maps.r) return thb_note_launch(cudaErrorUnknown, "conv_tc: second operand tensor map");
+            if (!has_a || !maps.has_r) return thb_note_launch(cudaErrorUnknown, "conv_tc: second operand tensor map");
         }
     }
     if (d->x2 && !p.nkb1) return THB_ERR_UNSUPPORTED;  // (narrow tiles and uint8 have no second operand)
