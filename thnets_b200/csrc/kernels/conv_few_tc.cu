@@ -541,7 +541,7 @@ __global__ void __launch_bounds__(nthreads(EW), EW == 8 ? 2 : 3) conv_few_kernel
             }
             __syncwarp();
             if (S > 1) {
-                cluster_arrive_relaxed();  // (waited for at the end: no CTA leaves while a peer may still write to it)
+                cluster_arrive_relaxed();  // (waited for at the end: no CTA leaves before its peers have pushed what they will)
                 if (have && !mbar_wait_bounded(smem_u32(recv_full), 0, p.wait_limit)) {
                     report(p.status, 5);
                     *abort_flag = 1;
@@ -595,9 +595,12 @@ __global__ void __launch_bounds__(nthreads(EW), EW == 8 ? 2 : 3) conv_few_kernel
     tc_fence_before();
     __syncthreads();
     if (*abort_flag && warp == W_A && lane == 0) {
-        // a wait ran out: copies still on their way must land before the CTA may leave
+        // a wait ran out: copies still on their way must land before the CTA may leave, and so must what the peers have pushed, all of it
+        // on its way since cluster_wait (a CTA whose own accumulator never came has not waited for it; nor will all of it come where a
+        // peer has given up).
         const int n = kb1 - kb0 < nst ? kb1 - kb0 : nst;
-        for (int s = 0; s < n; s++) mbar_wait_bounded(smem_u32(&full[s]), ((kb1 - kb0 - 1 - s) / nst) & 1, p.wait_limit);
+        for (int s = S > 1 ? -1 : 0; s < n; s++)
+            mbar_wait_bounded(smem_u32(s < 0 ? recv_full : &full[s]), s < 0 ? 0 : ((kb1 - kb0 - 1 - s) / nst) & 1, p.wait_limit);
     }
     __syncthreads();
     tc_fence_after();
