@@ -380,6 +380,20 @@ def test_static_scratch_entry_validates_before_any_launch():
     assert lib.thb_conv_u8_fwd_static(None, fake, fake, None) == ARG
 
 
+def test_pooling_refuses_sums_it_cannot_leave():
+    """thb_maxpool_sums answers before any launch where only the kernel that knows no sums would do."""
+    from thnets_b200 import kernels_abi as K
+    lib = K.load()
+    lib.thb_maxpool_sums.argtypes = [C.c_int, C.c_void_p] + [C.c_int] * 13 + [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]
+
+    def call(x=1 << 20, y=1 << 21, n=1, h=8, w=8, c=64, ld=64, k=2, ow=4):
+        return lib.thb_maxpool_sums(K.THB_U8, x, n, h, w, c, ld, k, k, 2, 2, 0, 0, 4, ow, y, ld, 1 << 22, None)
+
+    assert call(x=(1 << 20) + 8) == call(y=(1 << 21) + 4) == -1
+    assert call(c=512, ld=512, w=2 * (65535 * 8 + 8), ow=65535 * 8 + 8) == -1
+    assert call(k=4) == call(c=48, ld=48) == call(ld=72) == -1
+
+
 def test_split_plan_is_for_launches_that_leave_the_machine_idle():
     """thb_conv_splitk_plan (host arithmetic only; without a device it assumes 148 SMs): a handful of tiles with a long
     reduction is split so that the units fill the machine, with at least four K blocks per part and a bounded scratch;

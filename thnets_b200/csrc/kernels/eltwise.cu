@@ -1242,7 +1242,9 @@ int thb_maxpool_sums(int dtype, const void *x, int N, int H, int W, int C, int x
     const bool vectors = x_ld % al == 0 && y_ld % al == 0 && (((uintptr_t)x | (uintptr_t)y) & 15) == 0;
     // (uint8: the maximum starts from byte 0 as lowp_SpatialMaxPooling.c does; fp32: from the smallest finite value)
     const uint32_t lowest = dtype == THB_F16 ? 0xFC00FC00u : dtype == THB_BF16 ? 0xFF80FF80u : dtype == THB_U8 ? 0u : 0xFF7FFFFFu;
-    if (kH == kW && (kH == 2 || kH == 3) && vectors && (long)N * oH <= 0x7fffffffL && ((long)oW * cvecs + 255) / 256 <= 65535) {
+    const bool by_vectors = kH == kW && (kH == 2 || kH == 3) && vectors && (long)N * oH <= 0x7fffffffL && ((long)oW * cvecs + 255) / 256 <= 65535;
+    if (csum && !by_vectors) return THB_ERR_UNSUPPORTED;  // (the other kernel knows no sums)
+    if (by_vectors) {
         const dim3 grid((unsigned)(N * oH), (unsigned)((oW * cvecs + 255) / 256));
 #define MAXPOOL_KERNEL(K) \
     (dtype == THB_F16 ? maxpool_kernel<__half2, K> : dtype == THB_BF16 ? maxpool_kernel<__nv_bfloat162, K> : dtype == THB_U8 ? maxpool_kernel<U8x4, K> : maxpool_kernel<float, K>)
