@@ -41,6 +41,9 @@ CASES = [  # n, c, h, w, k, stride, pad, output rows and columns
     (1, 512, 6, 5, 2, 2, 0, 3, 3),       # 32 groups; the last column's window is half outside
     (2, 256, 13, 11, 3, 2, 0, 6, 5),
     (2, 33, 10, 10, 3, 3, 1, 4, 4),      # three groups: no sums
+    (2, 64, 11, 9, 3, 2, 1, 6, 5),       # 3x3 stride 2: two rows of outputs a thread (16-bit types), the last
+    (1, 32, 14, 6, 3, 2, 0, 7, 3),       # thread's second one inside, or beyond the output
+    (300, 16, 23, 7, 3, 2, 0, 11, 3),    # in uint8 from this many blocks on
     (1, 3, 1, 1, 2, 2, 0, 1, 1),
 ]
 

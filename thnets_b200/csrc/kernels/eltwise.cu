@@ -3,6 +3,7 @@
 // All of them walk channels-innermost tensors in 16-byte channel vectors so that every global access
 // of a warp is a run of full sectors.
 #include "common.cuh"
+#include <type_traits>
 #include <float.h>
 #include <math.h>
 
@@ -676,32 +677,54 @@ __device__ __forceinline__ void pixel_sum(const uint4 &v, int cvecs, bool write,
     if (write && (lane & (cvecs - 1)) == 0) *csum = sum;
 }
 
-// K x K max pooling, any stride and padding: a thread owns one 16-byte vector of an output pixel, a block a piece of an output
-// row, so that a pixel costs one division; all of its loads are on their way before the first maximum.  HBM-bound.  3x3 stride 2,
-// fp16, 112x112x64: 1 image 6.9 -> 6.4 us, 32 images 16.3 -> 12.4, 256 images 127 -> 104 against threads that walked down strips of
-// rows and carried the row two windows share (uint8: 8.8 -> 6.2, 16.5 -> 11.5, 75 -> 79).  VGG-16's five 2x2 poolings in uint8, 32 images, with the sums of the pooled
-// pixels for the next layers: 77 us (28.6 for the first, 129 MB: 4.5 TB/s) against 119 for the general kernel and 41 for passes of
-// their own over its results.
-template <typename T2, int K>
-__global__ void __launch_bounds__(256) maxpool_kernel(const uint4 *__restrict__ x, int H, int W, int cvecs, int x_ld, int dH, int dW, int padH, int padW,
+// K x K max pooling, any stride and padding: a thread owns one 16-byte vector of an output pixel (ROWS = 2, stride 2: of two, one above
+// the other, which share a row of inputs), a block a piece of an output row, so that a pixel costs one division; all of its loads are
+// on their way before the first maximum.  HBM-bound.  3x3 stride 2, 112x112x64, us for threads that walked down strips of rows / for
+// one row a thread / for two (* chosen):
+//   fp16    1 image 6.9 / 6.8 / 6.8*    32 images 13.6 / 12.3 / 11.2*    256 images 107 / 96 / 85* (514 MB: 6.0 TB/s)
+//   uint8   1 image 8.6 / 6.6* / 6.6    32 images 16.1 / 11.4* / 11.6    256 images 74 / 77 / 72*
+//   fp32    1 image 5.2 / 5.1*          32 images 41 / 26*               256 images 297 / 191*   (strips: the general kernel)
+// (48 registers for one row, five blocks to an SM: with 50, and four, fp32 takes 217.)
+// VGG-16's five 2x2 poolings in uint8, 32 images, with the sums of the pooled pixels for the next layers: 77 us (28.6 for the first, 129
+// MB: 4.5 TB/s) against 119 for the general kernel and 41 for passes of their own over its results.
+template <typename T2, int K, int ROWS>
+__global__ void __launch_bounds__(256, K == 3 && ROWS == 1 ? 5 : 1) maxpool_kernel(const uint4 *__restrict__ x, int H, int W, int cvecs, int x_ld, int dH, int dW, int padH, int padW,
                                                       int oH, int oW, uint32_t lowest, uint4 *__restrict__ y, int y_ld, int *csum)
 {
     pdl_enter();
-    const int n = blockIdx.x / oH, ih0 = (blockIdx.x - n * oH) * dH - padH;
+    constexpr int IN = 2 * (ROWS - 1) + K;  // (ROWS > 1: stride 2)
+    const int rows = (oH + ROWS - 1) / ROWS, n = blockIdx.x / rows, oh0 = (blockIdx.x - n * rows) * ROWS, ih0 = oh0 * dH - padH;
     const int it = blockIdx.y * 256 + threadIdx.x, ow = it / cvecs, cv = it - ow * cvecs, iw0 = ow * dW - padW;
-    const bool real = ow < oW;
     const uint4 *img = x + (size_t)n * H * W * x_ld + cv;
-    uint4 v[K * K], m = make_uint4(lowest, lowest, lowest, lowest);
+    const uint4 none = make_uint4(lowest, lowest, lowest, lowest);
+    uint4 v[IN * K];
 #pragma unroll
-    for (int k = 0; k < K * K; k++) {
+    for (int k = 0; k < IN * K; k++) {
         const int ih = ih0 + k / K, iw = iw0 + k % K;
-        v[k] = real && (unsigned)ih < (unsigned)H && (unsigned)iw < (unsigned)W ? __ldg(img + ((size_t)ih * W + iw) * x_ld) : m;
+        v[k] = ow < oW && (unsigned)ih < (unsigned)H && (unsigned)iw < (unsigned)W ? __ldg(img + ((size_t)ih * W + iw) * x_ld) : none;
     }
+    if constexpr (std::is_same<T2, float>::value) {  // in order, so that NaN is passed over wherever it stands; one row, no sums
+        uint4 m = none;
 #pragma unroll
-    for (int k = 0; k < K * K; k++) m = max8<T2>(m, v[k]);
-    const size_t pix = (size_t)blockIdx.x * oW + ow;
-    if (real) y[pix * y_ld + cv] = m;
-    if (csum) pixel_sum(m, cvecs, real, csum + pix);
+        for (int k = 0; k < K * K; k++) m = max8<T2>(m, v[k]);
+        if (ow < oW) y[((size_t)blockIdx.x * oW + ow) * y_ld + cv] = m;
+    } else {
+        // the maxima of each row's K once, also for the row that two windows share
+#pragma unroll
+        for (int r = 0; r < IN; r++)
+#pragma unroll
+            for (int k = 1; k < K; k++) v[r * K] = max8<T2>(v[r * K], v[r * K + k]);
+#pragma unroll
+        for (int r = 0; r < ROWS; r++) {
+            uint4 m = none;
+#pragma unroll
+            for (int k = 0; k < K; k++) m = max8<T2>(m, v[(2 * r + k) * K]);
+            const bool real = ow < oW && (ROWS == 1 || oh0 + r < oH);
+            const size_t pix = (ROWS == 1 ? (size_t)blockIdx.x : (size_t)n * oH + oh0 + r) * oW + ow;
+            if (real) y[pix * y_ld + cv] = m;
+            if (csum) pixel_sum(m, cvecs, real, csum + pix);
+        }
+    }
 }
 
 // ---- y = act(x*scale[c] + shift[c]) ----------------------------------------------------------------------
@@ -1245,10 +1268,13 @@ int thb_maxpool_sums(int dtype, const void *x, int N, int H, int W, int C, int x
     const bool by_vectors = kH == kW && (kH == 2 || kH == 3) && vectors && (long)N * oH <= 0x7fffffffL && ((long)oW * cvecs + 255) / 256 <= 65535;
     if (csum && !by_vectors) return THB_ERR_UNSUPPORTED;  // (the other kernel knows no sums)
     if (by_vectors) {
-        const dim3 grid((unsigned)(N * oH), (unsigned)((oW * cvecs + 255) / 256));
-#define MAXPOOL_KERNEL(K) \
-    (dtype == THB_F16 ? maxpool_kernel<__half2, K> : dtype == THB_BF16 ? maxpool_kernel<__nv_bfloat162, K> : dtype == THB_U8 ? maxpool_kernel<U8x4, K> : maxpool_kernel<float, K>)
-        const auto kern = kH == 2 ? MAXPOOL_KERNEL(2) : MAXPOOL_KERNEL(3);
+        // two rows of outputs a thread (see maxpool_kernel); uint8 from four waves of blocks on (three of them fit an SM)
+        const int pieces = (oW * cvecs + 255) / 256;
+        const bool two = kH == 3 && dH == 2 && (dtype == THB_F16 || dtype == THB_BF16 || (dtype == THB_U8 && (long)N * ((oH + 1) / 2) * pieces >= 4 * 3 * 148));
+        const dim3 grid((unsigned)(N * (two ? (oH + 1) / 2 : oH)), (unsigned)pieces);
+#define MAXPOOL_KERNEL(K, ROWS) \
+    (dtype == THB_F16 ? maxpool_kernel<__half2, K, ROWS> : dtype == THB_BF16 ? maxpool_kernel<__nv_bfloat162, K, ROWS> : dtype == THB_U8 ? maxpool_kernel<U8x4, K, ROWS> : maxpool_kernel<float, K, 1>)
+        const auto kern = kH == 2 ? MAXPOOL_KERNEL(2, 1) : two ? MAXPOOL_KERNEL(3, 2) : MAXPOOL_KERNEL(3, 1);
 #undef MAXPOOL_KERNEL
         thb_launch(kern, grid, 256, s, (const uint4 *)x, H, W, cvecs, x_ld / al, dH, dW, padH, padW, oH, oW, lowest, (uint4 *)y, y_ld / al, csum);
         return THB_LAUNCH_CHECK("maxpool_kernel");
