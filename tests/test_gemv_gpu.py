@@ -1,4 +1,4 @@
-"""Linear on up to eight rows: every count of rows of x, weight rows that do not divide among the CTAs or their groups of four, and
+"""Linear on up to eight rows: every count of rows of x, weight rows that do not divide among the CTAs or their groups of four or two, and
 reductions of less than, exactly and just over whole batches of 256 vectors."""
 import ctypes as C
 
@@ -21,7 +21,7 @@ def lib():
 
 
 @pytest.mark.parametrize("dtype", [K.THB_F32, K.THB_F16, K.THB_BF16])
-@pytest.mark.parametrize("m,vectors", [(1, 1), (5, 255), (296, 256), (593, 257), (1000, 512), (1187, 3), (4096, 769)])
+@pytest.mark.parametrize("m,vectors", [(1, 1), (5, 255), (296, 256), (593, 257), (1000, 512), (1187, 3), (4096, 769), (592, 1025), (1184, 513)])
 def test_gemv_edges(lib, dtype, m, vectors):
     per = 4 if dtype == K.THB_F32 else 8
     k, td = vectors * per, TORCH[dtype]

@@ -2,11 +2,19 @@
 // HBM-bound on the weight matrix: W is streamed once with 16-byte loads (four to eight in flight per thread, marked to leave the
 // L2 first: as ordinary lines they push the convolutions' weights out, AlexNet fp32 on one image 120 -> 125 us of kernels), the x
 // rows stay in L1/L2, sums are fp32.
-// us per chain of launches, weights from HBM, one row of W at a time (a batch four vectors of it) / four rows (a batch a vector of
-// each): 9216->4096->4096->1000 fp32, 1 row of x 37.1 / 38.3, 2 rows 45.2 / 41.5, 8 rows 101 / 78; fp16, 1 row 32.5 / 24.0, 4 rows
-// 72 / 43, 8 rows 132 / 63; 25088->4096->4096->1000 fp16 54 / 43; 2048->1000 fp16, 8 rows 7.8 / 4.2; 1024->30000 fp32 44 / 21.
-// (Four rows: x is read a quarter as often, and a reduction of 4096 halves fills its batches.)  A ring of cp.async in shared memory
-// in place of the registers: 23.6 and 3.7 for the fp16 ones, but such copies cannot be marked: 130 us for AlexNet's forward.
+// A CTA takes 4, 2 or 1 rows of W at a time: a batch is one vector a thread of each of four rows, two of each of two, four of one.  Four
+// rows read x a quarter as often, and short reductions fill their batches; where a CTA has one or two rows in all, groups of four would
+// leave most of its loads empty (the sums are the same bits).  us a launch in a chain, weights from HBM, one row at a time by an earlier
+// kernel / four rows always / by the CTA's rows:
+//                 fp32, 1 row of x     fp16, 1             fp32, 8             fp16, 8
+//   9216->4096    22.9 / 22.7 / 22.7   18.9 / 13.2 / 13.0  61.5 / 47.5 / 41.1  80.8 / 37.3 / 33.9
+//   4096->1000    3.43 / 4.27 / 3.42   3.43 / 3.25 / 2.77  9.06 / 7.07 / 6.70  12.3 / 5.81 / 5.84
+//   2048->1000    2.78 / 2.78 / 2.35   2.80 / 2.58 / 2.23  6.19 / 4.45 / 4.49  7.93 / 4.21 / 4.19
+//   512->1000     2.53 / 2.13 / 2.11   2.55 / 2.06 / 2.14  4.16 / 3.04 / 3.07  4.92 / 3.10 / 3.17
+//   8192->300     3.09 / 5.52 / 3.84   2.82 / 4.75 / 2.74  8.21 / 9.70 / 5.98  10.7 / 8.07 / 6.56
+//   1024->30000   43.7 / 20.5 / 20.4   53.3 / 19.5 / 17.5  95.4 / 65.0 / 64.1  122 / 61.8 / 62.6
+// A ring of cp.async in shared memory in place of the registers: as fast, but such copies cannot be marked: 130 us for AlexNet's
+// forward instead of 120.
 #include "common.cuh"
 
 namespace {
@@ -44,33 +52,32 @@ template <> struct V16<__nv_bfloat16> {
     }
 };
 
-// A CTA owns a contiguous range of rows and takes them ROWS at a time: a thread owns the vectors tid, tid + 256, ... of each, so a
-// batch is a vector of every row and is multiplied by one vector of x per image.  The batch after the one being multiplied is
+// A CTA owns a contiguous range of rows and takes them ROWS at a time: a thread owns the vectors tid, tid + 256, ... of each, and a
+// batch is VECS of them of every row, each multiplied by one vector of x per image.  The batch after the one being multiplied is
 // already in flight (two register buffers, running on into the CTA's next rows), so the stream of loads never drains.
-constexpr int ROWS = 4;
 constexpr int ctas_per_sm(int nb) { return nb <= 2 ? 4 : 2; }
 
-template <typename T, int NB>
+template <typename T, int NB, int ROWS>
 __global__ void __launch_bounds__(256, ctas_per_sm(NB)) gemv_kernel(const T *x, int K, int x_ld, const T *w, int M, const float *scale,
                                                                     const float *shift, thb_act act, T *y, int y_ld)
 {
-    constexpr int VN = V16<T>::N;
+    constexpr int VN = V16<T>::N, VECS = 4 / ROWS;
     __shared__ float part[2][8][ROWS * NB];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int nvec = K / VN, nkb = (nvec + 255) / 256;
+    const int nvec = K / VN, nkb = (nvec + 256 * VECS - 1) / (256 * VECS);
     const int r0 = (int)((long long)M * blockIdx.x / gridDim.x), r1 = (int)((long long)M * (blockIdx.x + 1) / gridDim.x);
     const uint4 *wv = reinterpret_cast<const uint4 *>(w) + tid;
 
     int lrow = r0, lkb = 0;  // next batch to load
-    auto load = [&](uint4 (&buf)[ROWS]) {
-        if (lkb * 256 + tid < nvec) {
+    auto load = [&](uint4 (&buf)[4]) {
 #pragma unroll
-            for (int r = 0; r < ROWS; r++)
-                if (lrow + r < r1) buf[r] = __ldcs(wv + (size_t)(lrow + r) * nvec + lkb * 256);
+        for (int i = 0; i < 4; i++) {
+            const int r = i / VECS, v = (lkb * VECS + i % VECS) * 256;
+            if (v + tid < nvec && lrow + r < r1) buf[i] = __ldcs(wv + (size_t)(lrow + r) * nvec + v);
         }
         if (++lkb == nkb) { lkb = 0; lrow += ROWS; }
     };
-    uint4 buf0[ROWS] = {}, buf1[ROWS] = {};
+    uint4 buf0[4] = {}, buf1[4] = {};
     // Programmatic dependent launch: the weights do not depend on the kernel before this one, so the first two
     // batches of every CTA are on their way while that kernel drains (and the next kernel of the stream may start its own
     // in the same way); x is read and y written only after the wait.
@@ -91,12 +98,14 @@ __global__ void __launch_bounds__(256, ctas_per_sm(NB)) gemv_kernel(const T *x, 
         for (int n = 0; n < NB; n++) acc[r][n] = 0.f;
     int row = r0, kb = 0, parity = 0;
 
-    auto consume = [&](const uint4 (&buf)[ROWS]) {
-        const int v = kb * 256 + tid;
-        if (v < nvec) {
+    auto consume = [&](const uint4 (&buf)[4]) {
+#pragma unroll
+        for (int j = 0; j < VECS; j++) {
+            const int v = (kb * VECS + j) * 256 + tid;
+            if (v >= nvec) break;
             float wf[ROWS][VN];
 #pragma unroll
-            for (int r = 0; r < ROWS; r++) V16<T>::unpack(buf[r], wf[r]);
+            for (int r = 0; r < ROWS; r++) V16<T>::unpack(buf[r * VECS + j], wf[r]);
 #pragma unroll
             for (int n = 0; n < NB; n++) {
                 float xf[VN];
@@ -169,10 +178,12 @@ int launch_gemv(const void *x, int N, int K, int x_ld, const void *w, int M, con
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     cudaError_t le = cudaSuccess;
-#define GEMV_CASE(NB)                                                                                                   \
-    case NB:                                                                                                            \
-        le = cudaLaunchKernelEx(&cfg, gemv_kernel<T, NB>, (const T *)x, K, x_ld, (const T *)w, M, scale, shift, a, (T *)y, y_ld); \
-        break;
+#define GEMV_CASE(NB)                                                                                                              \
+    case NB: {                                                                                                                     \
+        const auto kern = M <= grid ? gemv_kernel<T, NB, 1> : M <= 2 * grid ? gemv_kernel<T, NB, 2> : gemv_kernel<T, NB, 4>;       \
+        le = cudaLaunchKernelEx(&cfg, kern, (const T *)x, K, x_ld, (const T *)w, M, scale, shift, a, (T *)y, y_ld);                \
+        break;                                                                                                                     \
+    }
     switch (N) {
         GEMV_CASE(1) GEMV_CASE(2) GEMV_CASE(3) GEMV_CASE(4) GEMV_CASE(5) GEMV_CASE(6) GEMV_CASE(7) GEMV_CASE(8)
     default: return THB_ERR_UNSUPPORTED;
