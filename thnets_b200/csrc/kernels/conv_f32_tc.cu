@@ -780,7 +780,7 @@ extern "C" int thb_conv_f32_split_weights(const thb_conv_desc *d, void *w_split,
 //   5x5 64->192 @27x27, 1 image               29 / 18 / 13 / 13*       before  27    9.4e-8 / 2.0e-7
 //   3x3 384->256 @13x13, 1 image              53 / 31 / 20 / 15*       before  17    1.1e-7 / 2.7e-7
 //   3x3 512->512 @7x7, 1 image                67 / 38 / 23 / 16*       before  20    1.1e-7 / 2.3e-7
-//   6x6 256->4096 @18x25, 1 image            146* / 151 / 146 / 196    before 681    3.1e-7 / not measured
+//   6x6 256->4096 @18x25, 1 image            146* / 151 / 146 / 196    before 681    3.1e-7 / 6.1e-7 (of 512 channels)
 //   512->1000 of 9 rows                       11 / 9.8 / 8.7 / 8.8*    before 7.5    8.5e-8 / 1.6e-7
 extern "C" int thb_conv_f32_splits(const thb_conv_desc *d)
 {
