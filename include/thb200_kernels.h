@@ -147,7 +147,7 @@ int thb_conv_simt_splits(const thb_conv_desc *d);
 int thb_conv_few_supported(const thb_conv_desc *d);
 /* F32 on the tensor cores: the convolution of thb_conv_fwd from a second copy of the weights, each value as three bf16 parts
  * (w_split: split_bytes of device memory, filled from d->w by split_weights on the stream).  d->w and d->kinfo stay in use (sums
- * that are not finite are computed from them), d->status has to be set, and d->splits is the number of CTAs that share a tile's
+ * that the parts may have spoilt, not finite or very small ones, are computed from them), d->status has to be set, and d->splits is the number of CTAs that share a tile's
  * reduction (1, 2, 4 or 8; 0: thb_conv_f32_splits).  supported: up to 16 padded input channels, or a
  * multiple of 32 of them, and at least 64 products to a sum. */
 int thb_conv_f32_supported(const thb_conv_desc *d);
